@@ -1,8 +1,8 @@
 """Autotuner of the FISTA step kernel's SpMV structure.
 
 For each precision and each class of instances (average nonzeros per row x number of rows) it
-times every kernel variant -- block-staged tile (0), warp-staged rows (64) and 1/2/4/8/16/32
-lanes per row -- on a representative planted instance, with the engine's own step-kernel timer
+times every kernel variant -- the engine's own rule (-1: sliced rows where it applies), block-
+staged tile (0), warp-staged rows (64) and 1/2/4/8/16/32 lanes per row -- on a representative planted instance, with the engine's own step-kernel timer
 (bqp_profile_step: CUDA events around back-to-back launches on the engine stream), and writes
 the fastest per class to boxqp/tuning.json.  Run on the target GPU:
 
@@ -19,7 +19,7 @@ from pathlib import Path
 
 HERE = Path(__file__).resolve().parent
 TABLE = HERE / 'tuning.json'
-VARIANTS = [0, 64, 1, 2, 4, 8, 16, 32]
+VARIANTS = [-1, 0, 64, 1, 2, 4, 8, 16, 32]
 # (row-length bucket lower bound, upper bound, generator: family preset and edges/vertex)
 ROW_CLASSES = [(0, 4, ('graph10k', 1)), (4, 6, ('grid', None)), (6, 9, ('graph10k', 3)),
                (9, 13, ('graph10k', 5)), (13, 20, ('graph10k', 7)), (20, 48, ('graph10k', 14)),
@@ -60,6 +60,8 @@ def _instance(boxqp, family, epv, n):
 def tune(quick=False, launches=30):
     sys.path.insert(0, str(HERE.parent))
     import boxqp
+    import boxqp.autotune as live
+    live._table = {'entries': []}  # variant -1 must reach the engine's rule, not the table being replaced
     eng = boxqp.Engine(0)
     entries = []
     sizes = SIZE_CLASSES[1:] if quick else SIZE_CLASSES

@@ -67,10 +67,13 @@ struct Layout {
     size_t col_ff = kNone, hi_ff = kNone, lo_ff = kNone, cnt_ff = kNone, start_ff = kNone;
     size_t sstep = kNone, lprec = kNone, s = kNone, gate = kNone;
     size_t pc_inv = kNone, pc_e = kNone, pc_tile = kNone;
+    size_t slice_len = kNone, slice_row = kNone, slice_base = kNone;
     size_t total = 0;
 };
 
-Layout make_layout(int64_t n, int64_t nnz, int64_t tiles, int precision) {
+// Sliced FP64 solves hold their rows' order in place of the row pointers, which they need (with the
+// CSR as uploaded) only during admission, in a buffer of its own.
+Layout make_layout(int64_t n, int64_t nnz, int64_t tiles, int precision, bool sliced) {
     Layout L;
     size_t o = 0;
     // 64 bytes of slack behind every array keep 16-byte vector loads of a tail in bounds.
@@ -80,7 +83,13 @@ Layout make_layout(int64_t n, int64_t nnz, int64_t tiles, int precision) {
         return at;
     };
     const size_t N = static_cast<size_t>(n), Z = static_cast<size_t>(nnz);
-    L.rowptr = take((N + 1) * 4);
+    if (sliced) {
+        L.slice_len = take(N);
+        L.slice_row = take(N);
+        L.slice_base = take((N + 31) / 32 * 4);
+    } else {
+        L.rowptr = take((N + 1) * 4);
+    }
     L.col = take(Z * 4);
     if (precision == PREC_MIXED) {
         L.vhi = take(Z * 4);
@@ -224,7 +233,11 @@ struct Job {
     };
     std::vector<Piece> pieces;
     size_t piece = 0, piece_off = 0;
-    void* tmp = nullptr;
+    void* tmp = nullptr;      // ... or a sliced solve's CSR as uploaded and the positions of its rows
+    int32_t* csr_rowptr = nullptr;
+    int32_t* csr_col = nullptr;
+    double* csr_val = nullptr;
+    uint8_t* position_of = nullptr;
     void* power = nullptr;
     double t_upload = 0;
     std::vector<double> x;    // primal of a solve that holds no device memory (finished at submission)
@@ -234,6 +247,10 @@ struct Job {
     double t_submit = 0, t_done = 0;
     ~Job() { HostBufferCache::get().release(own, own_bytes); }
 };
+
+Layout layout_of(const Job& j) {
+    return make_layout(j.n, j.nnz, static_cast<int64_t>(j.tiles.size()), j.opt.precision, is_sliced(j.variant));
+}
 
 void free_inputs(Job& j) {
     HostBufferCache::get().release(j.own, j.own_bytes);
@@ -281,11 +298,15 @@ void set_unsupported(bqp_stats& st) {
     st.dual_bound = -HUGE_VAL;
 }
 
-// Default SpMV structure of the step kernel when the caller's options do not name one
-// (kernel_variant < 0): rows longer than a warp use sub-warps, the rest the block-staged tile.
-int default_variant(int64_t n, int64_t nnz, int precision) {
-    if (precision == PREC_FP64_EXACT) return 1;
+// SpMV structure when the caller's options do not name one (kernel_variant < 0).  The FP64 engines
+// take sliced rows unless a row is too long for a lane (kSliceMaxRow) or the rows are long on average
+// (kSliceMaxAverage), where several lanes per row give a small instance more loads in flight;
+// long rows elsewhere take sub-warps, the rest the block-staged tile.
+int default_variant(int64_t n, int64_t nnz, int64_t longest_row, int precision) {
     const double avg = n > 0 ? static_cast<double>(nnz) / static_cast<double>(n) : 1.0;
+    if (precision != PREC_MIXED && longest_row <= kSliceMaxRow && avg < kSliceMaxAverage)
+        return n <= kSliceSmall ? VAR_SLICE_SMALL : VAR_SLICE;
+    if (precision == PREC_FP64_EXACT) return 1;
     if (avg >= 48) return 32;
     return VAR_TILE;
 }
@@ -294,7 +315,9 @@ int default_variant(int64_t n, int64_t nnz, int precision) {
 // index, units}: as many units as the product kernel has resident blocks (`slots`), so that one
 // round runs them on the whole GPU, but units of about kCgUnitMin tiles at least; the tiles are
 // spread evenly (sizes differ by one at most), and no unit goes above kCgRowsum rows (the row
-// sums' shared buffer; units of kCgUnitMin tiles always fit).  Depends on the instance alone, so
+// sums' shared buffer; units of kCgUnitMin tiles always fit).  At least 4 / 2 / 1 tiles: a 10k-row mixed
+// solve 457 / 430 / 420 us, the FP64 one 2.10 / 1.95 / 1.95 ms, 256 uneven solves 2.00 / 2.03 / 2.12 ms
+// on the device.  Depends on the instance alone, so
 // the product's partial sums, and the CG iterates, are the same in a batch as solo.
 void cg_units(const Tile* t, int count, int first, int slots, std::vector<int4>& out) {
     const int fewest = (count + kCgUnitMax - 1) / kCgUnitMax;
@@ -434,6 +457,7 @@ public:
 private:
     void loop();
     bool upload(Job& j, std::string& why);
+    bool alloc_upload(Job& j, size_t bytes, std::string& why);
     bool upload_begin(Job& j, std::string& why);
     bool upload_copy(Job& j, size_t budget);
     bool upload_finish(Job& j, std::string& why);
@@ -453,7 +477,7 @@ private:
         if (uploading_) return true;
         if (queue_.empty() || queue_.front()->resolve) return false;
         const Job* j = queue_.front();
-        return resident_bytes_ + make_layout(j->n, j->nnz, static_cast<int64_t>(j->tiles.size()), j->opt.precision).total <= cap_;
+        return resident_bytes_ + layout_of(*j).total <= cap_;
     }
     bool install(std::vector<Job*>& jobs, std::string& why);
     void upload_waiting();
@@ -469,13 +493,36 @@ private:
     // step groups of precision `prec` that a body launches (bits of graph_groups_)
     std::vector<int> body_groups(int prec) const {
         std::vector<int> g;
-        for (int k = 0; k < kStepGroups; ++k)
+        for (int k = 0; k < 2 * kVariants; ++k)
             if (((graph_groups_ >> k) & 1u) && (k >= kVariants) == (prec == PREC_MIXED)) g.push_back(k);
         return g;
     }
+    // the FP64_EXACT engine: its sliced instances' group, and the kernel over the table for the others
+    int exact_slices() const { return static_cast<int>((graph_groups_ >> kExactSlices) & 3u); }
+    bool exact_csr() const { return (graph_groups_ & kExactCsrBit) || !exact_slices(); }
+    int check_families() const {
+        int f = 0;
+        for (int k = 0; k <= kStepGroups; ++k) {
+            if (!((graph_groups_ >> k) & 1u)) continue;
+            if (k == step_group(PREC_FP64, VAR_SLICE) || k == step_group(PREC_FP64, VAR_SLICE_SMALL) ||
+                (k >= kExactSlices && k < kStepGroups)) f |= kCheckSlices;
+            else if (k >= kVariants && k < 2 * kVariants) f |= kCheckMixed;
+            else f |= kCheckFp64;
+        }
+        return f;
+    }
+    // precisions with instances in the graph (bit k)
+    unsigned present_precisions() const {
+        return (body_groups(PREC_FP64).empty() ? 0u : 1u << PREC_FP64) | (body_groups(PREC_MIXED).empty() ? 0u : 1u << PREC_MIXED) |
+               (exact_slices() != 0 || (graph_groups_ & kExactCsrBit) ? 1u << PREC_FP64_EXACT : 0u);
+    }
     void launch_body_steps(const View& v, int prec, int K, int grid, cudaStream_t s) const {
         if (prec == PREC_FP64_EXACT) {
-            for (int j = 0; j < K; ++j) launch_step_exact(v, j, grid, s);
+            for (int j = 0; j < K; ++j) {
+                for (int k = 0; k < 2; ++k)
+                    if ((exact_slices() >> k) & 1) launch_step_group(v, kExactSlices + k, j, grid, s);
+                if (exact_csr()) launch_step_exact(v, j, grid, s);
+            }
             return;
         }
         std::vector<int> groups = body_groups(prec);
@@ -487,7 +534,9 @@ private:
         StepLaunches L;
         L.n[PREC_FP64] = K * std::max<int>(1, static_cast<int>(body_groups(PREC_FP64).size()));
         L.n[PREC_MIXED] = K * std::max<int>(1, static_cast<int>(body_groups(PREC_MIXED).size()));
-        L.n[PREC_FP64_EXACT] = K;
+        L.n[PREC_FP64_EXACT] = K * ((exact_slices() & 1) + (exact_slices() >> 1) + (exact_csr() ? 1 : 0));
+        L.checks = check_launches(check_families());
+        L.present = present_precisions();
         return L;
     }
     bool ensure_tables(int need_inst, int need_tiles, std::string& why);
@@ -503,6 +552,7 @@ private:
         v.ranges = d_ranges_;
         v.group_tiles = d_group_tiles_;
         v.units = d_units_;
+        v.momentum = d_momentum_;
         return v;
     }
     bool cuda_ok(cudaError_t e, std::string& why, const char* what) {
@@ -547,6 +597,7 @@ private:
     Tile* d_tiles_ = nullptr;
     Partial* d_partial_ = nullptr;
     Ctrl* d_ctrl_ = nullptr;
+    double2* d_momentum_ = nullptr;
     Ctrl* h_ctrl_ = nullptr;       // pinned
     int32_t* h_status_ = nullptr;  // pinned
     int inst_cap_ = 0, tile_cap_ = 0;
@@ -564,16 +615,17 @@ private:
     std::vector<int2> h_ranges_;
     std::vector<Job*> slot_job_;
     std::vector<int32_t> slot_prec_;      // precision of the solve in each slot
-    std::vector<int32_t> h_group_tiles_;  // tile indices ordered by step group
+    std::vector<Tile> h_group_tiles_;     // the tiles ordered by step group
     // page-locked staging of the tables above: their copies to the device run as DMA behind the
     // engine stream instead of a pageable copy each (rewritten only after that stream drained)
     unsigned char* h_table_stage_ = nullptr;
     size_t table_stage_bytes_ = 0;
     std::vector<int4> h_units_;           // CG work units: first tile, tiles, index, units of the instance
     int32_t group_begin_[kStepGroups + 1] = {};
-    uint32_t groups_present_ = 0;         // step groups with tiles
+    static constexpr uint32_t kExactCsrBit = 1u << kStepGroups;  // FP64_EXACT instances over the CSR
+    uint32_t groups_present_ = 0;         // step groups with tiles (and kExactCsrBit)
     uint32_t graph_groups_ = 0;           // step groups the graph launches
-    int32_t* d_group_tiles_ = nullptr;
+    Tile* d_group_tiles_ = nullptr;
     int4* d_units_ = nullptr;
     std::vector<int> free_slots_;
     int n_inst_ = 0;
@@ -676,6 +728,20 @@ bool Engine::init(std::string& why) {
     if (!cuda_ok(cudaMemset(d_ctrl_, 0, sizeof(Ctrl)), why, "control block")) return false;
     if (!cuda_ok(cudaMallocHost(&h_ctrl_, sizeof(Ctrl)), why, "pinned control")) return false;
     std::memset(h_ctrl_, 0, sizeof(Ctrl));
+    {
+        // the reference's momentum recurrence, each operation rounded as its CPU loop rounds it
+        std::vector<double2> m(kMomentumTable);
+        double t = 1.0;
+        for (double2& e : m) {
+            const double nt = (1.0 + std::sqrt(1.0 + 4.0 * t * t)) / 2.0;
+            e.x = (t - 1.0) / nt;
+            e.y = nt;
+            t = nt;
+        }
+        if (!cuda_ok(cudaMalloc(&d_momentum_, sizeof(double2) * m.size()), why, "momentum table")) return false;
+        if (!cuda_ok(cudaMemcpy(d_momentum_, m.data(), sizeof(double2) * m.size(), cudaMemcpyHostToDevice), why, "momentum table"))
+            return false;
+    }
     if (!ensure_tables(256, 1024, why)) return false;
     cudaSetDevice(prev);
     thread_ = std::thread([this] { loop(); });
@@ -704,9 +770,9 @@ void Engine::shutdown() {
     exec_ = nullptr;
     graph_ = nullptr;
     cudaFree(d_inst_); cudaFree(d_ranges_); cudaFree(d_tile_done_); cudaFree(d_status_);
-    cudaFree(d_tiles_); cudaFree(d_partial_); cudaFree(d_ctrl_); cudaFree(d_group_tiles_); cudaFree(d_units_);
+    cudaFree(d_tiles_); cudaFree(d_partial_); cudaFree(d_ctrl_); cudaFree(d_momentum_); cudaFree(d_group_tiles_); cudaFree(d_units_);
     d_inst_ = nullptr; d_ranges_ = nullptr; d_tile_done_ = nullptr; d_status_ = nullptr;
-    d_tiles_ = nullptr; d_partial_ = nullptr; d_ctrl_ = nullptr; d_group_tiles_ = nullptr; d_units_ = nullptr;
+    d_tiles_ = nullptr; d_partial_ = nullptr; d_ctrl_ = nullptr; d_momentum_ = nullptr; d_group_tiles_ = nullptr; d_units_ = nullptr;
     if (h_ctrl_) cudaFreeHost(h_ctrl_);
     if (h_stage_) cudaFreeHost(h_stage_);
     if (h_stage_slots_) cudaFreeHost(h_stage_slots_);
@@ -787,11 +853,11 @@ bool Engine::ensure_tables(int need_inst, int need_tiles, std::string& why) {
         int cap = std::max(need_tiles, std::max(1024, tile_cap_ * 2));
         Tile* tiles = nullptr;
         Partial* partial = nullptr;
-        int32_t* group_tiles = nullptr;
+        Tile* group_tiles = nullptr;
         int4* units = nullptr;
         if (!cuda_ok(cudaMalloc(&tiles, sizeof(Tile) * cap), why, "tile table")) return false;
         if (!cuda_ok(cudaMalloc(&partial, sizeof(Partial) * cap), why, "partials")) return false;
-        if (!cuda_ok(cudaMalloc(&group_tiles, sizeof(int32_t) * cap), why, "step groups")) return false;
+        if (!cuda_ok(cudaMalloc(&group_tiles, sizeof(Tile) * cap * (kTileRows / kSlicePiece)), why, "step groups")) return false;
         if (!cuda_ok(cudaMalloc(&units, sizeof(int4) * cap), why, "CG work units")) return false;
         cudaFree(d_tiles_);
         cudaFree(d_partial_);
@@ -828,9 +894,9 @@ bool Engine::run_stream(int cap, std::string& why) {
     int bodies = 0;
     for (; bodies < cap; ++bodies) {
         if (profile_phases_) cudaEventRecord(pev_[0], stream_);
-        launch_check(v, grid, stream_);
+        launch_check(v, check_families(), grid, stream_);
         launch_gate_plain(v, K, stream_);
-        kernels += 4;
+        kernels += check_launches(check_families()) + 1;
         cudaMemcpyAsync(h_ctrl_, d_ctrl_, sizeof(Ctrl), cudaMemcpyDeviceToHost, stream_);
         if (!cuda_ok(cudaStreamSynchronize(stream_), why, "engine check")) return false;
         if (profile_phases_) cudaEventRecord(pev_[1], stream_);
@@ -892,12 +958,15 @@ bool Engine::build_graph(std::string& why) {
     const View v = view();
 
     if (!cuda_ok(cudaGraphCreate(&graph_, 0), why, "graph create")) return false;
-    cudaGraphConditionalHandle h_loop, h_f[3], h_pol, h_cg;
+    cudaGraphConditionalHandle h_loop, h_f[3] = {}, h_pol = 0, h_cg = 0;
     if (!cuda_ok(cudaGraphConditionalHandleCreate(&h_loop, graph_, 1, cudaGraphCondAssignDefault), why, "conditional handle")) return false;
+    const unsigned present = present_precisions();
+    const bool mixed = (present >> PREC_MIXED) & 1u;
     for (int k = 0; k < 3; ++k)
-        if (!cuda_ok(cudaGraphConditionalHandleCreate(&h_f[k], graph_, 0, cudaGraphCondAssignDefault), why, "conditional handle")) return false;
-    if (!cuda_ok(cudaGraphConditionalHandleCreate(&h_pol, graph_, 0, cudaGraphCondAssignDefault), why, "conditional handle")) return false;
-    if (!cuda_ok(cudaGraphConditionalHandleCreate(&h_cg, graph_, 0, cudaGraphCondAssignDefault), why, "conditional handle")) return false;
+        if (((present >> k) & 1u) &&
+            !cuda_ok(cudaGraphConditionalHandleCreate(&h_f[k], graph_, 0, cudaGraphCondAssignDefault), why, "conditional handle")) return false;
+    if (mixed && !cuda_ok(cudaGraphConditionalHandleCreate(&h_pol, graph_, 0, cudaGraphCondAssignDefault), why, "conditional handle")) return false;
+    if (mixed && !cuda_ok(cudaGraphConditionalHandleCreate(&h_cg, graph_, 0, cudaGraphCondAssignDefault), why, "conditional handle")) return false;
 
     cudaGraphNodeParams wp = {cudaGraphNodeTypeConditional};
     wp.conditional.handle = h_loop;
@@ -938,11 +1007,14 @@ bool Engine::build_graph(std::string& why) {
 
     cudaGraphNode_t last = nullptr;
     if (!capture(body, nullptr, 0, [&] {
-            launch_check(v, grid, capture_);
+            launch_check(v, check_families(), grid, capture_);
             launch_gate(v, h_f, h_pol, h_cg, body_launches(K), K, capture_);
         }, &last)) return false;
     const int precisions[3] = {PREC_FP64, PREC_MIXED, PREC_FP64_EXACT};
+    // branches only for the precisions that have instances: an idle conditional node costs a body
+    // about as much as an idle launch
     for (int k = 0; k < 3; ++k) {
+        if (!((present >> k) & 1u)) continue;
         cudaGraphNode_t node;
         cudaGraph_t inner;
         if (!add_if(last, h_f[k], &node, &inner)) return false;
@@ -950,7 +1022,7 @@ bool Engine::build_graph(std::string& why) {
             return false;
         last = node;
     }
-    {
+    if (mixed) {
         cudaGraphNode_t node;
         cudaGraph_t inner;
         if (!add_if(last, h_pol, &node, &inner)) return false;
@@ -1281,10 +1353,22 @@ bool Engine::upload(Job& j, std::string& why) {
     return upload_finish(j, why);
 }
 
+// The solve's upload buffer (j.tmp) on ustream_, freed behind the admission kernels; an exhausted
+// pool is reported like one that cannot hold the slab.
+bool Engine::alloc_upload(Job& j, size_t bytes, std::string& why) {
+    const cudaError_t e = cudaMallocFromPoolAsync(&j.tmp, bytes, pool_, ustream_);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        j.out_of_memory = true;
+        j.tmp = nullptr;
+    }
+    return cuda_ok(e, why, "allocate upload buffer");
+}
+
 bool Engine::upload_begin(Job& j, std::string& why) {
     j.t_upload = host_seconds();
     const int prec = j.opt.precision;
-    j.layout = make_layout(j.n, j.nnz, static_cast<int64_t>(j.tiles.size()), prec);
+    j.layout = layout_of(j);
     void* slab = nullptr;
     // host-side fault injection (bqp_inject_admission_oom): fail as an exhausted pool would,
     // without any device call
@@ -1309,14 +1393,31 @@ bool Engine::upload_begin(Job& j, std::string& why) {
     const size_t N = static_cast<size_t>(j.n), Z = static_cast<size_t>(j.nnz);
     j.pieces.clear();
     j.piece = j.piece_off = 0;
-    j.pieces.push_back({at<int32_t>(slab, L.rowptr), j.rowptr, (N + 1) * 4});
-    if (Z) j.pieces.push_back({at<int32_t>(slab, L.col), j.col, Z * 4});
+    const bool sliced = is_sliced(j.variant);
+    j.tmp = nullptr;
+    if (sliced) {
+        const size_t b_val = align_up(Z * 8 + 64), b_col = align_up(Z * 4 + 64);
+        const size_t b_rowptr = align_up((N + 1) * 4);
+        if (!alloc_upload(j, b_val + b_col + b_rowptr + N, why)) return false;
+        j.csr_val = static_cast<double*>(j.tmp);
+        j.csr_col = reinterpret_cast<int32_t*>(static_cast<char*>(j.tmp) + b_val);
+        j.csr_rowptr = reinterpret_cast<int32_t*>(static_cast<char*>(j.tmp) + b_val + b_col);
+        j.position_of = reinterpret_cast<uint8_t*>(static_cast<char*>(j.tmp) + b_val + b_col + b_rowptr);
+        j.pieces.push_back({j.csr_rowptr, j.rowptr, (N + 1) * 4});
+        if (Z) j.pieces.push_back({j.csr_col, j.col, Z * 4});
+    } else {
+        j.pieces.push_back({at<int32_t>(slab, L.rowptr), j.rowptr, (N + 1) * 4});
+        if (Z) j.pieces.push_back({at<int32_t>(slab, L.col), j.col, Z * 4});
+    }
     j.pieces.push_back({at<double>(slab, L.c), j.c, N * 8});
     j.pieces.push_back({at<double>(slab, L.l), j.l, N * 8});
     j.pieces.push_back({at<double>(slab, L.u), j.u, N * 8});
     InstDev& R = j.rec;
     std::memset(&R, 0, sizeof(R));
     R.rowptr = at<int32_t>(slab, L.rowptr);
+    R.slice_len = at<uint8_t>(slab, L.slice_len);
+    R.slice_row = at<uint8_t>(slab, L.slice_row);
+    R.slice_base = at<int32_t>(slab, L.slice_base);
     R.col = at<int32_t>(slab, L.col);
     R.val64 = at<double>(slab, L.val64);
     R.vhi = at<float>(slab, L.vhi);
@@ -1395,16 +1496,15 @@ bool Engine::upload_begin(Job& j, std::string& why) {
     R.step_switch = 3.0 * j.opt.polish_switch;
     R.lip_device = j.opt.lipschitz == BQP_LIPSCHITZ_POWER ? 1 : 0;
     j.power = nullptr;
-    j.tmp = nullptr;
     if (R.lip_device &&
         !cuda_ok(cudaMallocFromPoolAsync(&j.power, power_scratch_bytes(j.n), pool_, ustream_), why, "allocate power scratch"))
         return false;
     if (prec == PREC_MIXED) {
         // FP64 values only for the admission kernels (hi/lo split, diagonal, preconditioner)
-        if (!cuda_ok(cudaMallocFromPoolAsync(&j.tmp, Z * 8 + 64, pool_, ustream_), why, "allocate upload buffer")) return false;
+        if (!alloc_upload(j, Z * 8 + 64, why)) return false;
         if (Z) j.pieces.push_back({j.tmp, j.val, Z * 8});
     } else if (Z) {
-        j.pieces.push_back({at<double>(slab, L.val64), j.val, Z * 8});
+        j.pieces.push_back({sliced ? j.csr_val : at<double>(slab, L.val64), j.val, Z * 8});
     }
     return true;
 }
@@ -1427,8 +1527,14 @@ bool Engine::upload_copy(Job& j, size_t budget) {
 }
 
 bool Engine::upload_finish(Job& j, std::string& why) {
-    InstDev& R = j.rec;
+    InstDev R = j.rec;  // as the admission kernels read it: a sliced solve's CSR still in its upload buffer
     const int prec = j.opt.precision;
+    const bool sliced = is_sliced(j.variant);
+    if (sliced) {
+        R.rowptr = j.csr_rowptr;
+        R.col = j.csr_col;
+        R.val64 = j.csr_val;
+    }
     // the convexity gate and the Gershgorin bound first: the other admission kernels read L from
     // its result, and the engine thread reads the result back before it installs the solve
     j.gate_host = acquire_gate_slot();
@@ -1448,6 +1554,12 @@ bool Engine::upload_finish(Job& j, std::string& why) {
         if (R.lip_device) {
             cudaMemcpyAsync(R.lprec, &R.gate->lip_bits, sizeof(double), cudaMemcpyDeviceToDevice, ustream_);
             launch_power_lipschitz(R, j.n, val, false, j.power, ustream_);
+        }
+        if (sliced) {
+            const Layout& L = j.layout;
+            launch_slice_rows(R, j.n, j.nnz, R.rowptr, R.col, val, j.position_of, at<int32_t>(j.slab, L.col),
+                              at<double>(j.slab, L.val64), ustream_);
+            cudaFreeAsync(j.tmp, ustream_);
         }
     }
     if (j.power) cudaFreeAsync(j.power, ustream_);
@@ -1504,7 +1616,7 @@ void Engine::upload_waiting() {
             if (queue_.empty()) break;
             j = queue_.front();
             if (j->resolve) break;
-            const size_t need = make_layout(j->n, j->nnz, static_cast<int64_t>(j->tiles.size()), j->opt.precision).total;
+            const size_t need = layout_of(*j).total;
             if (resident_bytes_ + need > cap_) break;
             queue_.pop_front();
             j->state = JOB_ADMITTING;
@@ -1615,6 +1727,9 @@ void Engine::finish_refused(Job* j) {
 // CUDA error.  Caller holds mu_.
 void Engine::fail_admission(Job* j, size_t reserved, const std::string& why) {
     release_gate_slot(*j);
+    if (j->tmp) cudaFreeAsync(j->tmp, ustream_);
+    if (j->power) cudaFreeAsync(j->power, ustream_);
+    j->tmp = j->power = nullptr;
     resident_bytes_ -= reserved;
     if (j->resident) {
         pending_free_.emplace_back(-1, j->slab);
@@ -1660,12 +1775,18 @@ void Engine::process_frees() {
 // invalidates it.
 void Engine::upload_tables() {
     if (!tables_dirty_) return;
+    // a sliced instance's tiles go to its group in pieces of kSlicePiece rows
+    auto pieces = [](const Tile& t) {
+        return is_sliced(t.variant) ? (t.row_end - t.row_begin + kSlicePiece - 1) / kSlicePiece : 1;
+    };
     int32_t count[kStepGroups + 1] = {};
+    uint32_t exact_csr = 0;
     for (const Tile& t : h_tiles_) {
         const int g = step_group(slot_prec_[t.inst], t.variant);
-        if (g >= 0) count[g + 1]++;
+        if (g >= 0) count[g + 1] += pieces(t);
+        else exact_csr = kExactCsrBit;
     }
-    groups_present_ = 0;
+    groups_present_ = exact_csr;
     for (int g = 0; g < kStepGroups; ++g) {
         if (count[g + 1]) groups_present_ |= 1u << g;
         count[g + 1] += count[g];
@@ -1673,8 +1794,12 @@ void Engine::upload_tables() {
     std::memcpy(group_begin_, count, sizeof(group_begin_));
     h_group_tiles_.resize(static_cast<size_t>(count[kStepGroups]));
     for (int k = 0; k < static_cast<int>(h_tiles_.size()); ++k) {
-        const int g = step_group(slot_prec_[h_tiles_[k].inst], h_tiles_[k].variant);
-        if (g >= 0) h_group_tiles_[static_cast<size_t>(count[g]++)] = k;
+        const Tile& t = h_tiles_[k];
+        const int g = step_group(slot_prec_[t.inst], t.variant);
+        if (g < 0) continue;
+        const int rows = is_sliced(t.variant) ? kSlicePiece : t.row_end - t.row_begin;
+        for (int r = t.row_begin; r < t.row_end; r += rows)
+            h_group_tiles_[static_cast<size_t>(count[g]++)] = Tile{t.inst, r, std::min(r + rows, t.row_end), t.variant};
     }
     // CG work units: runs of consecutive tiles of one instance (cg_units; a unit depends on the
     // instance alone, not on the batch)
@@ -1685,7 +1810,7 @@ void Engine::upload_tables() {
     }
     // the four tables through one page-locked staging buffer (16-byte aligned parts)
     const size_t b_tiles = sizeof(Tile) * h_tiles_.size();
-    const size_t b_group = sizeof(int32_t) * h_group_tiles_.size();
+    const size_t b_group = sizeof(Tile) * h_group_tiles_.size();
     const size_t b_units = sizeof(int4) * h_units_.size();
     const size_t b_ranges = sizeof(int2) * static_cast<size_t>(std::max(n_inst_, 1));
     auto up16 = [](size_t b) { return (b + 15) & ~size_t(15); };
@@ -1813,13 +1938,18 @@ void Engine::collect(std::unique_lock<std::mutex>& lk) {
     // larger one stays in the slab (final, untouched until release or re-run) and bqp_fetch
     // copies it straight to the caller's array, off the engine thread.
     std::vector<std::vector<float>> x32(finished.size());
-    bool small = false;
+    bool small = false, unsliced = false;
     for (size_t k = 0; k < finished.size(); ++k) {
         Job& j = *finished[k];
         const InstDev& R = recs[k];
         j.x_f32 = R.result_src == 1;
         j.x_dev = R.result_src == 1 ? static_cast<const void*>(R.x32)
                                     : static_cast<const void*>(R.result_src == 2 ? R.xp : R.x64);
+        if (is_sliced(j.variant)) {  // back into row order, in the momentum buffer the next run starts from anew
+            launch_unslice(j.n, R.slice_row, R.x64, R.w64[0], stream_);
+            j.x_dev = R.w64[0];
+            unsliced = true;
+        }
         j.x.clear();
         if (j.n > kHostPrimal) continue;
         small = true;
@@ -1831,7 +1961,8 @@ void Engine::collect(std::unique_lock<std::mutex>& lk) {
         }
         cudaMemcpyAsync(dst, j.x_dev, (j.x_f32 ? 4 : 8) * static_cast<size_t>(j.n), cudaMemcpyDeviceToHost, stream_);
     }
-    if (small) cudaStreamSynchronize(stream_);
+    // (bqp_fetch copies the larger ones on another stream)
+    if (small || unsliced) cudaStreamSynchronize(stream_);
     const double now = host_seconds();
     for (size_t k = 0; k < finished.size(); ++k) {
         Job& j = *finished[k];
@@ -2054,7 +2185,7 @@ void Engine::loop() {
                 continue;
             }
             if (uploading_) break;  // FIFO: the paused upload goes first
-            const size_t need = make_layout(j->n, j->nnz, static_cast<int64_t>(j->tiles.size()), j->opt.precision).total;
+            const size_t need = layout_of(*j).total;
             if (resident_bytes_ + need > cap_) {
                 if (n_running_ == 0 && uploaded_.empty()) {
                     queue_.pop_front();
@@ -2205,6 +2336,7 @@ struct Scan {
     int error = 0;  // 1 row pointers, 2 coefficient/bound, 3 Hessian entry
     bool nonzero = false;
     bool infeasible = false;
+    int64_t longest = 0;  // entries of the longest row
 };
 
 // Destination of the host copy taken during the scan (asynchronous submit), or all null.
@@ -2241,6 +2373,7 @@ Scan scan_rows(int64_t r0, int64_t r1, int64_t n, int64_t nnz, const int32_t* ro
             return s;
         }
         if (l[i] > u[i]) s.infeasible = true;
+        if (b - a > s.longest) s.longest = b - a;
         // rows [copied, i] validated: their nonzeros lie in [rowptr[copied], rowptr[i + 1]] within [0, nnz]
         if (dst.rowptr && (b - rowptr[copied] >= 16384 || i + 1 - copied >= 4096 || i + 1 == r1)) copy_rows(i + 1);
     }
@@ -2264,6 +2397,7 @@ Scan scan_problem(int64_t n, int64_t nnz, const int32_t* rowptr, const int32_t* 
     for (const Scan& p : part) {
         if (p.error && !s.error) s.error = p.error;
         s.infeasible = s.infeasible || p.infeasible;
+        s.longest = std::max(s.longest, p.longest);
     }
     return s;
 }
@@ -2386,9 +2520,8 @@ int make_job(int64_t n, int64_t nnz, const int32_t* rowptr, const int32_t* col, 
         *out = j.release();
         return BQP_OK;
     }
-    if (o.precision == BQP_PRECISION_FP64_EXACT) j->variant = 1;
-    else if (o.kernel_variant >= 0) j->variant = o.kernel_variant;
-    else j->variant = bqp::default_variant(n, nnz, o.precision);
+    if (o.precision != BQP_PRECISION_FP64_EXACT && o.kernel_variant >= 0) j->variant = o.kernel_variant;
+    else j->variant = bqp::default_variant(n, nnz, scan.longest, o.precision);
     j->tiles = bqp::make_tiles(n, rowptr, j->variant);
     const double t_tiles = host_seconds();
     if (copy) {

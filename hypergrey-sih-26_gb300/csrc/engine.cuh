@@ -15,11 +15,12 @@ constexpr int kBlock = 256;          // threads per CTA of every tile kernel
 constexpr int kMaxInterval = 32;     // maximum check interval (iterations per chunk)
 constexpr int kTileNnz = 4096;       // target nonzeros per tile
 constexpr int kTileRows = 512;       // maximum rows per tile
-constexpr int kCgUnitMin = 4;        // tiles per work unit of the polish CG product kernel: about
+constexpr int kCgUnitMin = 2;        // tiles per work unit of the polish CG product and the sliced check: about
 constexpr int kCgUnitMax = 8;        //   this many at least, and up to this many for large instances (cg_units)
-constexpr int kCgRowsum = kCgUnitMin * kTileRows;  // rows per CG work unit at most (its row sums, 16 KB)
+constexpr int kCgRowsum = 4 * kTileRows;  // rows per CG work unit at most (its row sums, 16 KB)
 constexpr int kCgGroups = 2;         // row groups per warp whose loads the CG product keeps in flight
 constexpr int kCgUnroll = 2;         // entries per row group and lane (and epilogue rows per thread) per pass of the CG product
+constexpr int kMomentumTable = 8192; // FISTA momenta kept in a table (View::momentum)
 constexpr int kRearmRows = 1024;     // rows per block when re-arming resident solves (8192: 32 us on 1M rows, latency-bound)
 constexpr int64_t kHostPrimal = 131072;  // primals up to this size come back at completion, larger at fetch
 
@@ -45,21 +46,41 @@ enum Precision : int32_t { PREC_FP64 = 0, PREC_MIXED = 1, PREC_FP64_EXACT = 2 };
 enum Variant : int32_t {
     VAR_TILE = 0,    // block-staged: products of the whole tile, then one thread per row
     VAR_WARP = 64,   // warp-staged: 32 rows per warp, products then one lane per row
+    VAR_SLICE = 65,  // sliced rows (below): one lane per row over interleaved entries
+    VAR_SLICE_SMALL = 66,  // the same for small instances: whole rows loaded ahead of the previous step's end
     // 1, 2, 4, 8, 16, 32: sub-warp rows, that many lanes per row
 };
 
 // Step-kernel groups: one kernel per (precision, variant) for the FP64 and mixed engines, each
 // over its own list of tiles, so a kernel carries one SpMV structure and the registers of that
 // structure alone (the FP64_EXACT engine has one structure and no groups).
-constexpr int kVariants = 8;
-constexpr int kStepGroups = 2 * kVariants;
+constexpr int kVariants = 10;
+constexpr int kExactSlices = 2 * kVariants;  // the FP64_EXACT engine's sliced instances, then the small ones
+constexpr int kStepGroups = 2 * kVariants + 2;
+__host__ __device__ constexpr bool is_sliced(int variant) { return variant == VAR_SLICE || variant == VAR_SLICE_SMALL; }
 __host__ __device__ constexpr int variant_index(int variant) {
-    return variant == VAR_WARP ? 7 : variant == 32 ? 6 : variant == 16 ? 5 : variant == 8 ? 4 : variant == 4 ? 3
+    return variant == VAR_SLICE_SMALL ? 9 : variant == VAR_SLICE ? 8 : variant == VAR_WARP ? 7 : variant == 32 ? 6 : variant == 16 ? 5 : variant == 8 ? 4 : variant == 4 ? 3
          : variant == 2 ? 2 : variant == 1 ? 1 : 0;
 }
 __host__ __device__ constexpr int step_group(int precision, int variant) {
-    return precision == PREC_FP64_EXACT ? -1 : (precision == PREC_MIXED ? kVariants : 0) + variant_index(variant);
+    return precision == PREC_FP64_EXACT ? (is_sliced(variant) ? kExactSlices + (variant == VAR_SLICE_SMALL) : -1) : (precision == PREC_MIXED ? kVariants : 0) + variant_index(variant);
 }
+
+// Sliced rows (VAR_SLICE).  The rows of each window of kSliceWindow rows are ordered by descending
+// length (ties in row order), and the whole instance is kept in that order: position p of a window
+// holds one of its rows, every vector is stored by position and the columns are positions.  A
+// slice is 32 consecutive positions, one per lane of a warp.  A slice's entries are stored column by
+// column without padding: first the first entry of each of its rows, then the second entry of
+// each row that has one, and so on.  Because the rows of a slice are in descending length, the rows
+// still active at any column are its first lanes, so every load of values, columns and vectors is
+// one dense run, each row's sum runs in its own lane in column order (no shuffles, the per-row
+// epilogue on full warps), and the lanes of a warp finish nearly together.  The entries of a window
+// keep their CSR extent; the order is undone when the primal is handed out.
+constexpr int kSliceWindow = 256;
+constexpr int kSlicePiece = 128;     // rows of a step work item (a block's four warps take a slice each)
+constexpr int64_t kSliceSmall = 65536;  // rows up to which an instance is VAR_SLICE_SMALL
+constexpr int kSliceMaxRow = 127;    // longest row of a sliced instance (a tile holds 32 such rows, so tiles begin on slices)
+constexpr int kSliceMaxAverage = 48; // longer average rows keep the sub-warp structures (default_variant)
 
 struct Tile {
     int32_t inst;
@@ -108,6 +129,9 @@ struct __align__(16) InstDev {
     const double* val64;   // FP64 values (PREC_FP64, PREC_FP64_EXACT)
     const float* vhi;      // FP32 high part (PREC_MIXED)
     const float* vlo;      // FP32 low part, val ~= hi + lo (PREC_MIXED)
+    const uint8_t* slice_len;    // VAR_SLICE: per position, the row's length
+    const uint8_t* slice_row;    // VAR_SLICE: per position, the row within its window
+    const int32_t* slice_base;   // VAR_SLICE: per slice, its first entry in col / val64
     const double* c;
     const double* l;
     const double* u;
@@ -244,7 +268,8 @@ struct View {
     Ctrl* ctrl;
     int32_t* status_mirror;  // per-instance status, rewritten by the control kernel every body
     const int2* ranges;      // per-instance tile range [x, y) in the tile table
-    const int32_t* group_tiles;  // tile indices ordered by step group (Ctrl::group_begin)
+    const Tile* group_tiles;     // the tiles (sliced instances: pieces of kSlicePiece rows) ordered by step group (Ctrl::group_begin)
+    const double2* momentum;     // FISTA: beta_k and t_{k+1} for k < kMomentumTable (they depend on k alone)
     const int4* units;           // CG work units: x the first tile of a run of y consecutive tiles of one
                                  // instance, z the unit's index within the instance, w its unit count
 };

@@ -71,6 +71,14 @@ __device__ __forceinline__ unsigned long long dbits(double v) {
 __device__ __forceinline__ double bdouble(unsigned long long b) { return __longlong_as_double(static_cast<long long>(b)); }
 __device__ __forceinline__ unsigned long long umax64(unsigned long long a, unsigned long long b) { return a < b ? b : a; }
 
+// smax(l, smin(u, v)) on the bit patterns: the same value as the FP64 comparisons give (NaNs and
+// zeros of either sign included) without their issue slots on the FP64 pipe.
+__device__ __forceinline__ double clip_bits(double v, double l, double u) {
+    const uint64_t vb = dbits(v), lb = dbits(l), ub = dbits(u);
+    const uint64_t t = less_bits(vb, ub) ? vb : ub;
+    return bdouble(less_bits(lb, t) ? t : lb);
+}
+
 struct Acc {
     double obj, bnd, sep, a;
     unsigned long long stat, prim, b;
@@ -491,6 +499,62 @@ __device__ __forceinline__ void tile_rows(int variant, const int32_t* __restrict
     }
 }
 
+// ---- sliced rows (engine.cuh: VAR_SLICE) -------------------------------------------------------
+// One slice, one row per lane: the sum of the row's products in column order.  `len` is the lane's
+// row length (descending over the lanes), `base` the slice's first entry.  At column j the rows
+// still active are the first lanes, so the column's entries are base + the entries of the columns
+// before it + lane: the lane's address advances by the count of active lanes.  AHEAD columns
+// are loaded together (entries, then gathers) before the first product.
+// EXACT: products and sums rounded separately from 0.0, the reference loop's arithmetic.
+template <int AHEAD>
+struct SliceColumns {  // AHEAD columns of a slice: this lane's columns (-1: the row has ended) and values
+    int c[AHEAD];
+    double a[AHEAD];
+    __device__ __forceinline__ void load(const int32_t* __restrict__ col, const double* __restrict__ val, int left, int& k) {
+#pragma unroll
+        for (int q = 0; q < AHEAD; ++q) {
+            const bool in = q < left;
+            c[q] = in ? __ldg(col + k) : -1;
+            a[q] = in ? __ldg(val + k) : 0.0;
+            k += __popc(__ballot_sync(0xffffffffu, in));
+        }
+    }
+    // adds the first `columns` (warp-uniform) of them; a column past the slice's longest row costs
+    // no FP64 issue slot
+    template <bool EXACT>
+    __device__ __forceinline__ double add(const double* x, int columns, double acc) const {
+        double xv[AHEAD];
+#pragma unroll
+        for (int q = 0; q < AHEAD; ++q) xv[q] = c[q] >= 0 ? x[c[q]] : 0.0;
+        return sum<EXACT, 0>(xv, columns, acc);
+    }
+
+private:
+    template <bool EXACT, int Q>
+    __device__ __forceinline__ double sum(const double* xv, int columns, double acc) const {
+        if constexpr (Q < AHEAD) {
+            if (Q >= columns) return acc;
+            if (c[Q] >= 0) acc = EXACT ? __dadd_rn(acc, __dmul_rn(a[Q], xv[Q])) : fma(a[Q], xv[Q], acc);
+            return sum<EXACT, Q + 1>(xv, columns, acc);
+        } else {
+            return acc;
+        }
+    }
+};
+template <bool EXACT, int AHEAD>
+__device__ __forceinline__ double slice_dot(const int32_t* __restrict__ col, const double* __restrict__ val,
+                                            const double* x, int base, int len) {
+    const int longest = __shfl_sync(0xffffffffu, len, 0);
+    int k = base + (threadIdx.x & 31);
+    double acc = 0.0;
+    SliceColumns<AHEAD> e;
+    for (int j = 0; j < longest; j += AHEAD) {  // warp-uniform
+        e.load(col, val, len - j, k);
+        acc = e.template add<EXACT>(x, longest - j, acc);
+    }
+    return acc;
+}
+
 // FP32 "double-float" arithmetic: an unevaluated pair (hi, lo) carries ~46 significant bits.
 // The products of the mixed engine's checks and polish run on the FP32 pipes with it, since
 // GB300's FP64 rate is 1/64 of its FP32 rate; FP64 is used once per row.
@@ -680,7 +744,24 @@ __device__ __forceinline__ CheckSrc source_of(const InstDev& I) {
 }
 
 // ---- the state machine after a check (thread 0 of the finalizing block) -------------------
-__device__ void fista_betas(InstDev& I, int64_t count) {
+// Momenta of iterations [I.it0, I.it0 + count).  The sequence depends on the iteration alone, so it
+// comes from a table the host filled with the same IEEE operations: one thread's recurrence (a
+// square root and two divisions per iteration, each waiting for the one before) took 20 us per
+// chunk of 25 on this GPU's FP64 pipe.  Past the table the recurrence goes on from I.t.
+__device__ void fista_betas(const View& v, InstDev& I, int64_t count) {
+    const int64_t first = I.it0;
+    if (first + count <= kMomentumTable) {
+        double t = I.t;
+#pragma unroll 8
+        for (int64_t j = 0; j < count; ++j) {
+            const double2 m = __ldg(v.momentum + first + j);
+            I.beta[j] = m.x;
+            I.beta32[j] = static_cast<float>(m.x);
+            t = m.y;
+        }
+        I.t = t;
+        return;
+    }
     // t_{k+1} = (1 + sqrt(1 + 4 t_k^2)) / 2, beta_k = (t_k - 1) / t_{k+1}
     // (src/accelerated_qp.cpp:47), each operation rounded as the reference's CPU loop rounds it.
     double t = I.t;
@@ -700,7 +781,7 @@ __device__ void finish(InstDev& I, int status, int src) {
     I.end_ns = now_ns();
 }
 
-__device__ void after_check(InstDev& I, const Acc& tot) {
+__device__ void after_check(const View& v, InstDev& I, const Acc& tot) {
     const int64_t it_check = I.it_next;
     const int ph = I.phase;
     I.checks++;
@@ -761,7 +842,7 @@ __device__ void after_check(InstDev& I, const Acc& tot) {
     I.moved[1] = 0;
     I.it_next = it_check + I.interval < I.max_iter ? it_check + I.interval : I.max_iter;
     const int64_t count = I.it_next - I.it0;
-    fista_betas(I, count);
+    fista_betas(v, I, count);
     I.fista_iters += count;
 }
 
@@ -1003,14 +1084,139 @@ template <int PREC, int VAR>
 __global__ void __launch_bounds__(kBlock, step_min_blocks<VAR>()) step_kernel(View v, int group, int j0) {
     if (j0 >= v.ctrl->step_due[PREC]) return;  // every chunk of this precision ends before step j0
     const int b = v.ctrl->group_begin[group], e = v.ctrl->group_begin[group + 1];
-    for (int t = b + static_cast<int>(blockIdx.x); t < e; t += gridDim.x) step_tile<PREC, VAR>(v, v.tiles[v.group_tiles[t]], j0);
+    for (int t = b + static_cast<int>(blockIdx.x); t < e; t += gridDim.x) step_tile<PREC, VAR>(v, v.group_tiles[t], j0);
 }
 
-// FP64_EXACT engine: one structure, every tile of the table (other precisions skip).
+// FP64_EXACT engine over the CSR: every tile of the table (other precisions and sliced instances skip).
 __global__ void __launch_bounds__(kBlock) step_exact_kernel(View v, int j0) {
     if (j0 >= v.ctrl->step_due[PREC_FP64_EXACT]) return;
     const int nt = v.ctrl->n_tiles;
-    for (int t = blockIdx.x; t < nt; t += gridDim.x) step_tile<PREC_FP64_EXACT, 1>(v, v.tiles[t], j0);
+    for (int t = blockIdx.x; t < nt; t += gridDim.x)
+        if (!is_sliced(v.tiles[t].variant)) step_tile<PREC_FP64_EXACT, 1>(v, v.tiles[t], j0);
+}
+
+// Sliced FP64 steps.  A work item is a piece of kSlicePiece positions, a slice per warp; where the
+// items leave blocks idle each block takes a half or a quarter of one (a small solve is bound by
+// the latency of its loads: one slice per block on many SMs beats four per block on few).
+//
+// The step launches of a body are chained by programmatic dependent launch: everything a step reads
+// but the iterates (the control fields, which only the kernels between bodies write, the matrix and
+// the bounds) is loaded before it waits for the step before it.  Every block waits, the idle
+// ones too, so that a launch that has ended implies that all launches before it have.
+//
+// Bounds: the FP64 pipe (16 cycles an SM per warp instruction: 3 + 3 a row on the tridiagonal family,
+// about 10 us for 1M rows, beside 80 MB from DRAM, 12 us) and the rate of random gathers (15M on the
+// random graph, 60 us).  Per step, against the CSR structures (one or two lanes per row): tridiagonal
+// 1M rows 26.4 -> 14.6 us, random graph 15M entries 95 -> 72 us, 10k rows 12 -> 3.5 us (of which
+// the overlap of launches 0.6 ms over 400 steps).
+constexpr int kSliceThreads = kSlicePiece;
+__device__ __forceinline__ void wait_for_previous_launch() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_launch_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// What a step reads of an instance's record, kept in registers from one item to the next while the
+// instance stays the same.
+struct SliceStep {
+    const uint8_t* len;
+    const int32_t* base;
+    const int32_t* col;
+    const double* val;
+    const double* win;
+    double* wout;
+    double* x;
+    const double* c;
+    const double* l;
+    const double* u;
+    double beta, scale;
+    int n;
+    bool due;
+};
+
+template <int PREC>
+__device__ __forceinline__ SliceStep slice_step(const InstDev& I, int j0) {
+    SliceStep S;
+    const int64_t it = I.it_cur + j0;
+    S.due = I.status == ST_RUNNING && I.phase == PH_FISTA && it < I.it_next;
+    const int in = static_cast<int>(it & 1);
+    S.len = I.slice_len;
+    S.base = I.slice_base;
+    S.col = I.col;
+    S.val = I.val64;
+    S.win = I.w64[in];
+    S.wout = I.w64[in ^ 1];
+    S.x = I.x64;
+    S.c = I.c;
+    S.l = I.l;
+    S.u = I.u;
+    S.beta = S.due ? I.beta[it - I.it0] : 0.0;
+    S.scale = PREC == PREC_FP64_EXACT ? I.L : I.invL;
+    S.n = I.n;
+    return S;
+}
+
+__device__ __forceinline__ int item_split(int items, int grid) {
+    int shift = 0;
+    while (shift < 2 && (items << (shift + 1)) <= grid) ++shift;
+    return shift;
+}
+
+// AHEAD columns of a row are in flight together (in the first round, loaded before the wait);
+// BLOCKS per SM.
+template <int PREC, int AHEAD, int BLOCKS>
+__global__ void __launch_bounds__(kSliceThreads, BLOCKS) step_slice_kernel(View v, int group, int j0) {
+    constexpr bool kExact = PREC == PREC_FP64_EXACT;
+    let_next_launch_begin();
+    const int b = v.ctrl->group_begin[group], items = v.ctrl->group_begin[group + 1] - b;
+    const int shift = item_split(items, gridDim.x), parts = items << shift;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int g = blockIdx.x;
+    if (j0 >= v.ctrl->step_due[PREC] || g >= parts) {
+        wait_for_previous_launch();
+        return;
+    }
+    Tile T = v.group_tiles[b + (g >> shift)];
+    SliceStep S = slice_step<PREC>(v.inst[T.inst], j0);
+    bool waited = false;
+    for (int turn = warp;; ++turn) {
+        // the slice of this warp: a window's slices come in descending length, so the warps take
+        // turns at the long ones
+        const int part = g & ((1 << shift) - 1), per = (kSlicePiece / 32) >> shift;
+        const int s = (T.row_begin >> 5) + part * per + (turn & (kSlicePiece / 32 - 1));
+        const bool mine = S.due && (turn & (kSlicePiece / 32 - 1)) < per && s * 32 < T.row_end;
+        const int inst = T.inst, p = s * 32 + lane;
+        const bool valid = mine && p < S.n;
+        const int len = valid ? __ldg(S.len + p) : 0;
+        int k = (mine ? __ldg(S.base + s) : 0) + lane;
+        const double ci = valid ? __ldg(S.c + p) : 0.0, lo = valid ? __ldg(S.l + p) : 0.0, up = valid ? __ldg(S.u + p) : 0.0;
+        const int longest = __shfl_sync(0xffffffffu, len, 0);
+        SliceColumns<AHEAD> e;
+        e.load(S.col, S.val, len, k);
+        g += gridDim.x;
+        if (g < parts) T = v.group_tiles[b + (g >> shift)];  // the next item, ahead of its use
+        if (!waited) wait_for_previous_launch();
+        waited = true;
+        const double wi = valid ? S.win[p] : 0.0, xo = valid ? S.x[p] : 0.0;
+        // the exact engine adds the cost to the finished sum, as the reference does
+        double acc = e.template add<kExact>(S.win, longest, kExact ? 0.0 : ci);
+        for (int j = AHEAD; j < longest; j += AHEAD) {  // warp-uniform
+            e.load(S.col, S.val, len - j, k);
+            acc = e.template add<kExact>(S.win, longest - j, acc);
+        }
+        if (valid) {
+            // FP64 work per row beside its products: the step, x+ - x and w+ (the cost starts the sum,
+            // clamping runs on the bit patterns)
+            double nx;
+            if constexpr (kExact) {
+                nx = clip_bits(__dsub_rn(wi, __ddiv_rn(__dadd_rn(acc, ci), S.scale)), lo, up);
+                S.wout[p] = __dadd_rn(nx, __dmul_rn(S.beta, __dsub_rn(nx, xo)));
+            } else {
+                nx = clip_bits(wi - acc * S.scale, lo, up);
+                S.wout[p] = nx + S.beta * (nx - xo);
+            }
+            S.x[p] = nx;
+        }
+        if (g >= parts) return;
+        if (T.inst != inst) S = slice_step<PREC>(v.inst[T.inst], j0);
+    }
 }
 
 // ---- check kernel -----------------------------------------------------------------------------
@@ -1026,6 +1232,7 @@ __global__ void __launch_bounds__(kBlock, 3) check_kernel(View v) {
     const int nt = v.ctrl->n_tiles;
     for (int t = blockIdx.x; t < nt; t += gridDim.x) {
         const Tile T = v.tiles[t];
+        if (FAMILY == FAMILY_FP64 && is_sliced(T.variant)) continue;  // check_slice_kernel's
         InstDev& I = v.inst[T.inst];
         if (I.status != ST_RUNNING) continue;
         if (I.phase == PH_FISTA && I.it_cur < I.it_next) continue;  // chunk still running
@@ -1051,8 +1258,48 @@ __global__ void __launch_bounds__(kBlock, 3) check_kernel(View v) {
         if (publish_and_test_last(v, t, T.inst, R.y - R.x, total)) {
             Acc inst_total = reduce_instance(v, R.x, R.y, s.gate != 0);
             if (threadIdx.x == 0) {
-                after_check(I, inst_total);
+                after_check(v, I, inst_total);
                 I.stat_floor = 0;  // the next check starts from nothing
+            }
+            __syncthreads();
+        }
+    }
+}
+
+// Check of the sliced FP64 instances over the work units (runs of consecutive tiles of one instance,
+// as many as resident blocks): a unit's rows accumulate in registers, one reduction and one
+// publication per unit (its partial in its instance's slot R.x + index).
+__global__ void __launch_bounds__(kBlock, 4) check_slice_kernel(View v) {
+    if (v.ctrl->check_due[FAMILY_FP64] == 0) return;
+    const int nu = v.ctrl->n_units;
+    for (int un = blockIdx.x; un < nu; un += gridDim.x) {
+        const int4 U = v.units[un];  // first tile, tiles, index and units of its instance
+        const Tile T = v.tiles[U.x];
+        if (!is_sliced(T.variant)) continue;
+        InstDev& I = v.inst[T.inst];
+        if (I.status != ST_RUNNING || I.phase != PH_FISTA || I.it_cur < I.it_next) continue;
+        const int last = (v.tiles[U.x + U.y - 1].row_end + 31) >> 5;
+        const unsigned long long floor = __ldcg(&I.stat_floor);
+        const int gate = I.diag_gate, n = I.n;
+        Acc a = acc_identity();
+        for (int s = (T.row_begin >> 5) + static_cast<int>(threadIdx.x >> 5); s < last; s += kBlock / 32) {
+            const int p = s * 32 + static_cast<int>(threadIdx.x & 31);
+            const bool valid = p < n;
+            const int len = valid ? __ldg(I.slice_len + p) : 0;
+            const double gq = slice_dot<false, 4>(I.col, I.val64, I.x64, __ldg(I.slice_base + s), len);
+            if (!valid) continue;
+            const double xi = I.x64[p], li = I.l[p], ui = I.u[p];
+            check_row(a, xi, gq, I.c[p], li, ui, gate ? I.diag[p] : 1.0, gate, p, less_equal_bits(dbits(xi), dbits(li)),
+                      less_equal_bits(dbits(ui), dbits(xi)), floor);
+        }
+        Acc total = block_reduce_check(a, gate != 0, true);
+        if (threadIdx.x == 0 && total.stat > floor) atomicMax(&I.stat_floor, total.stat);
+        const int2 R = v.ranges[T.inst];
+        if (publish_and_test_last(v, R.x + U.z, T.inst, U.w, total)) {
+            Acc inst_total = reduce_instance(v, R.x, R.x + U.w, gate != 0);
+            if (threadIdx.x == 0) {
+                after_check(v, I, inst_total);
+                I.stat_floor = 0;
             }
             __syncthreads();
         }
@@ -2002,15 +2249,15 @@ __global__ void gate_kernel(View v, cudaGraphConditionalHandle h_fp64, cudaGraph
         v.ctrl->n_polish = c.polish;
         v.ctrl->n_cg = c.polish;
         v.ctrl->cg_iters = 0;
-        long long launched = 4;  // three check kernels + gate
+        long long launched = steps.checks + 1;  // check kernels and gate
         for (int k = 0; k < 3; ++k) launched += c.fista[k] > 0 ? steps.n[k] : 0;
         launched += c.polish > 0 ? 2 : 0;
         v.ctrl->kernels += launched;
-        cudaGraphSetConditional(h_fp64, c.fista[0] > 0 ? 1u : 0u);
-        cudaGraphSetConditional(h_mixed, c.fista[1] > 0 ? 1u : 0u);
-        cudaGraphSetConditional(h_exact, c.fista[2] > 0 ? 1u : 0u);
-        cudaGraphSetConditional(h_polish, c.polish > 0 ? 1u : 0u);
-        cudaGraphSetConditional(h_cg, c.polish > 0 ? 1u : 0u);
+        if (steps.present & 1u) cudaGraphSetConditional(h_fp64, c.fista[0] > 0 ? 1u : 0u);
+        if (steps.present & 2u) cudaGraphSetConditional(h_mixed, c.fista[1] > 0 ? 1u : 0u);
+        if (steps.present & 4u) cudaGraphSetConditional(h_exact, c.fista[2] > 0 ? 1u : 0u);
+        if (steps.present & 2u) cudaGraphSetConditional(h_polish, c.polish > 0 ? 1u : 0u);
+        if (steps.present & 2u) cudaGraphSetConditional(h_cg, c.polish > 0 ? 1u : 0u);
     }
 }
 
@@ -2064,7 +2311,7 @@ __device__ __forceinline__ void init_row(const InstDev& I, int r) {
 }
 
 // Start of a solve: clock, deadline and (mixed) the first chunk.  One thread.
-__device__ void start_instance(InstDev& I) {
+__device__ void start_instance(const View& v, InstDev& I) {
         const int64_t start = now_ns();
         I.start_ns = start;
         I.deadline_ns = start + I.deadline_ns;  // host stores the budget in nanoseconds
@@ -2080,7 +2327,7 @@ __device__ void start_instance(InstDev& I) {
             I.moved[1] = 0;
             const int64_t first = I.interval <= 16 ? I.interval + I.interval / 2 : I.interval;
             I.it_next = first < I.max_iter ? first : I.max_iter;
-            fista_betas(I, I.it_next);
+            fista_betas(v, I, I.it_next);
             I.fista_iters += I.it_next;
         }
 }
@@ -2088,7 +2335,7 @@ __device__ void start_instance(InstDev& I) {
 __global__ void init_instance_kernel(View v, int slot, int n) {
     InstDev& I = v.inst[slot];
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) init_row(I, r);
-    if (blockIdx.x == 0 && threadIdx.x == 0) start_instance(I);
+    if (blockIdx.x == 0 && threadIdx.x == 0) start_instance(v, I);
 }
 
 // Re-arms a list of resident solves in one launch.  Block b takes rows [span.y, span.y + kRearmRows)
@@ -2114,7 +2361,7 @@ __global__ void __launch_bounds__(kBlock) rearm_kernel(View v, const InstDev* __
                 I.invL = 1.0 / I.L;
                 I.invLf = static_cast<float>(I.invL);
             }
-            start_instance(I);
+            start_instance(v, I);
         }
     }
 }
@@ -2282,6 +2529,131 @@ __global__ void __launch_bounds__(kGateWarps * 32) convexity_gate_kernel(const i
         if (nondominant) atomicOr(&out->nondominant, 1);
         if (flags) atomicOr(&out->flags, flags);
     }
+}
+
+// Admission of a sliced instance, first kernel: one block per window of kSliceWindow rows.  The rows
+// are ordered by descending length with a stable counting sort (ballots within a warp, one count
+// per warp and length, so the order does not depend on the run); the window's vectors move into that
+// order in place.
+__global__ void __launch_bounds__(kSliceWindow) slice_order_kernel(InstDev I, int n, const int32_t* __restrict__ rowptr,
+                                                                  uint8_t* __restrict__ position_of) {
+    constexpr int kBins = kSliceMaxRow + 1, kWarps = kSliceWindow / 32;
+    __shared__ int32_t hist[kWarps][kBins];
+    __shared__ int32_t bin_start[kBins];
+    __shared__ int32_t warp_total[kWarps];
+    __shared__ uint8_t row_at[kSliceWindow];  // per position: its row
+    __shared__ uint8_t len_at[kSliceWindow];  // per position: its row's length
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int w0 = blockIdx.x * kSliceWindow, rows = min(kSliceWindow, n - w0);
+    for (int b = t; b < kWarps * kBins; b += kSliceWindow) hist[b / kBins][b % kBins] = 0;
+    const bool valid = t < rows;
+    const int len = valid ? __ldg(rowptr + w0 + t + 1) - __ldg(rowptr + w0 + t) : 0;
+    const int bin = valid ? kSliceMaxRow - len : kBins;  // descending length; the rows past n apart
+    const unsigned peers = __match_any_sync(0xffffffffu, bin);
+    const int rank = __popc(peers & ((1u << lane) - 1u));
+    __syncthreads();
+    if (valid && rank == 0) hist[warp][bin] = __popc(peers);
+    __syncthreads();
+    int mine = 0;
+    if (t < kBins) {  // per bin: the warps' counts become offsets; mine: the bin's rows
+        for (int w = 0; w < kWarps; ++w) {
+            const int c = hist[w][t];
+            hist[w][t] = mine;
+            mine += c;
+        }
+    }
+    int incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31) warp_total[warp] = incl;
+    __syncthreads();
+    if (t < kBins) {
+        int before = 0;
+        for (int w = 0; w < warp; ++w) before += warp_total[w];
+        bin_start[t] = before + incl - mine;
+    }
+    __syncthreads();
+    if (valid) {
+        const int p = bin_start[bin] + hist[warp][bin] + rank;
+        row_at[p] = static_cast<uint8_t>(t);
+        len_at[p] = static_cast<uint8_t>(len);
+        position_of[w0 + t] = static_cast<uint8_t>(p);
+    }
+    __syncthreads();
+    const int my_len = valid ? len_at[t] : 0;
+    const int total = static_cast<int>(__reduce_add_sync(0xffffffffu, static_cast<unsigned>(my_len)));
+    if (lane == 0) warp_total[warp] = total;
+    double vec[4];
+    double* const arrays[4] = {const_cast<double*>(I.c), const_cast<double*>(I.l), const_cast<double*>(I.u),
+                               const_cast<double*>(I.diag)};
+    if (valid) {
+        const int r = w0 + row_at[t];
+        const_cast<uint8_t*>(I.slice_len)[w0 + t] = len_at[t];
+        const_cast<uint8_t*>(I.slice_row)[w0 + t] = row_at[t];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) vec[k] = arrays[k][r];
+    }
+    __syncthreads();  // every value of the window is read before its place is written
+    if (valid) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) arrays[k][w0 + t] = vec[k];
+    }
+    int base = __ldg(rowptr + w0);
+    for (int w = 0; w < warp; ++w) base += warp_total[w];
+    if (lane == 0 && valid) const_cast<int32_t*>(I.slice_base)[(w0 >> 5) + warp] = base;
+}
+
+// Second kernel: the window's entries, staged in shared memory by coalesced loads where they fit
+// (`cap` entries; a fuller window reads its rows from global memory), leave slice by slice, column by
+// column, their columns as positions.  Each entry is read and written once (24 bytes) and its column's
+// position gathered (one byte): 154 us for 15M entries, once per solve.  A column out of range passes through unchanged: the gate refuses
+// that solve.
+__global__ void __launch_bounds__(kSliceWindow) slice_entries_kernel(InstDev I, int n, const int32_t* __restrict__ rowptr,
+                                                                    const int32_t* __restrict__ col,
+                                                                    const double* __restrict__ val, int cap,
+                                                                    const uint8_t* __restrict__ position_of,
+                                                                    int32_t* __restrict__ col_out,
+                                                                    double* __restrict__ val_out) {
+    extern __shared__ __align__(16) unsigned char dyn_smem[];
+    double* sval = reinterpret_cast<double*>(dyn_smem);
+    int32_t* scol = reinterpret_cast<int32_t*>(sval + cap);
+    const int t = threadIdx.x, lane = t & 31;
+    const int w0 = blockIdx.x * kSliceWindow, rows = min(kSliceWindow, n - w0);
+    const int kb = __ldg(rowptr + w0), ke = __ldg(rowptr + w0 + rows);
+    const bool staged = ke - kb <= cap;
+    auto place = [&](int32_t c) {
+        return static_cast<uint32_t>(c) < static_cast<uint32_t>(n) ? (c & ~(kSliceWindow - 1)) | __ldg(position_of + c) : c;
+    };
+    if (staged) {
+#pragma unroll 4
+        for (int k = t; k < ke - kb; k += kSliceWindow) {
+            sval[k] = __ldg(val + kb + k);
+            scol[k] = place(__ldg(col + kb + k));
+        }
+    }
+    const bool valid = t < rows;
+    const int len = valid ? __ldg(I.slice_len + w0 + t) : 0;
+    const int src = valid ? __ldg(rowptr + w0 + __ldg(I.slice_row + w0 + t)) - kb : 0;
+    int k = valid ? __ldg(I.slice_base + ((w0 + t) >> 5)) + lane : 0;
+    __syncthreads();
+    const int longest = __shfl_sync(0xffffffffu, len, 0);
+    for (int j = 0; j < longest; ++j) {  // warp-uniform
+        const bool in = j < len;
+        if (in) {
+            val_out[k] = staged ? sval[src + j] : __ldg(val + kb + src + j);
+            col_out[k] = staged ? scol[src + j] : place(__ldg(col + kb + src + j));
+        }
+        k += __popc(__ballot_sync(0xffffffffu, in));
+    }
+}
+
+__global__ void __launch_bounds__(kBlock) unslice_kernel(int n, const uint8_t* __restrict__ slice_row,
+                                                         const double* __restrict__ x, double* __restrict__ out) {
+    for (int p = blockIdx.x * kBlock + threadIdx.x; p < n; p += gridDim.x * kBlock)
+        out[(p & ~(kSliceWindow - 1)) + __ldg(slice_row + p)] = x[p];
 }
 
 // Mixed engine, per row after the gate: 1/Q_ii (the polish's Jacobi preconditioner), the
@@ -2640,6 +3012,8 @@ namespace {
 // One full wave (SMs x resident blocks per SM) per tile kernel, computed once per process.
 struct Waves {
     int group[kStepGroups] = {};
+    int slices[4] = {};  // FP64, FP64 small, exact, exact small
+    int check_slices = 0;
     int exact = 0;
     int check = 0, check_mixed = 0, check_verify = 0, polish = 0, matvec = 0, residual = 0;
 };
@@ -2680,6 +3054,21 @@ void group_waves(int sms) {
     group_wave<PREC, VAR_WARP>(sms);
 }
 
+// Columns in flight and blocks per SM: 4 / 5 / 6 columns at 8 blocks (64 registers) measured 6.56 /
+// 6.13 / 6.83 ms per FP64 grid solve and 37.1 / 36.8 / 37.9 ms on the random graph; small instances
+// hide latency with whole rows in flight (12 columns, 128 registers: 10k rows 2.95 -> 2.47 ms per solve
+// against 8 columns at 6 blocks).  The two cross at about kSliceSmall rows: 40k rows 6.7 against 7.2 us a
+// step, 100k rows 10.4 against 10.2.
+using SliceKernel = void (*)(View, int, int);
+constexpr int kWideAhead = 5, kWideBlocks = 8, kSmallAhead = 12, kSmallBlocks = 4;
+SliceKernel slice_kernel(bool exact, bool small) {
+    if (exact) return small ? step_slice_kernel<PREC_FP64_EXACT, kSmallAhead, kSmallBlocks> : step_slice_kernel<PREC_FP64_EXACT, kWideAhead, kWideBlocks>;
+    return small ? step_slice_kernel<PREC_FP64, kSmallAhead, kSmallBlocks> : step_slice_kernel<PREC_FP64, kWideAhead, kWideBlocks>;
+}
+
+// Entries that slice_entries_kernel stages in shared memory at most (12 bytes each).
+constexpr int kSliceStageMax = 16384;
+
 template <int PREC, int VAR>
 void launch_group(const View& v, int group, int j, int grid, cudaStream_t s) {
     step_kernel<PREC, VAR><<<pick(grid, g_waves.group[group]), kBlock, step_smem<PREC, VAR>(), s>>>(v, group, j);
@@ -2704,6 +3093,13 @@ int tile_grid(int sms) {
     group_waves<PREC_FP64>(sms);
     group_waves<PREC_MIXED>(sms);
     g_waves.exact = wave_of(step_exact_kernel, sms, 0);
+    for (int k = 0; k < 4; ++k) {
+        int blocks = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, slice_kernel(k >= 2, k & 1), kSliceThreads, 0);
+        g_waves.slices[k] = sms * (blocks < 1 ? 1 : blocks);
+    }
+    g_waves.check_slices = wave_of(check_slice_kernel, sms, 0);
+    cudaFuncSetAttribute(slice_entries_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 12 * kSliceStageMax);
     g_waves.check = wave_of(check_kernel<FAMILY_FP64>, sms, kSmem8);
     g_waves.check_mixed = wave_of(check_kernel<FAMILY_MIXED>, sms, kSmem8);
     g_waves.check_verify = wave_of(check_kernel<FAMILY_VERIFY>, sms, kSmem8);
@@ -2713,22 +3109,41 @@ int tile_grid(int sms) {
     g_waves.polish = wave_of(cg_vector_kernel, sms, 0);
     int m = g_waves.exact;
     for (int w : g_waves.group) m = w > m ? w : m;
-    for (int w : {g_waves.check, g_waves.matvec, g_waves.polish})
+    for (int w : {g_waves.check, g_waves.matvec, g_waves.polish, g_waves.slices[0], g_waves.slices[1], g_waves.slices[2], g_waves.slices[3]})
         m = w > m ? w : m;
     return m;
 }
 
 int cg_matvec_slots() { return g_waves.matvec; }
 
-void launch_check(const View& v, int grid, cudaStream_t s) {
-    check_kernel<FAMILY_MIXED><<<pick(grid, g_waves.check_mixed), kBlock, kSmem8, s>>>(v);
-    check_kernel<FAMILY_VERIFY><<<pick(grid, g_waves.check_verify), kBlock, kSmem8, s>>>(v);
-    check_kernel<FAMILY_FP64><<<pick(grid, g_waves.check), kBlock, kSmem8, s>>>(v);
+void launch_check(const View& v, int families, int grid, cudaStream_t s) {
+    if (families & kCheckMixed) {
+        check_kernel<FAMILY_MIXED><<<pick(grid, g_waves.check_mixed), kBlock, kSmem8, s>>>(v);
+        check_kernel<FAMILY_VERIFY><<<pick(grid, g_waves.check_verify), kBlock, kSmem8, s>>>(v);
+    }
+    if (families & kCheckFp64) check_kernel<FAMILY_FP64><<<pick(grid, g_waves.check), kBlock, kSmem8, s>>>(v);
+    if (families & kCheckSlices) check_slice_kernel<<<pick(grid, g_waves.check_slices), kBlock, 0, s>>>(v);
 }
 
 void launch_step_group(const View& v, int group, int j, int grid, cudaStream_t s) {
-    if (group >= kVariants) launch_group_of<PREC_MIXED>(v, group, j, grid, s);
-    else launch_group_of<PREC_FP64>(v, group, j, grid, s);
+    const int wide = step_group(PREC_FP64, VAR_SLICE), small = step_group(PREC_FP64, VAR_SLICE_SMALL);
+    if (group >= kExactSlices || group == wide || group == small) {
+        const bool exact = group >= kExactSlices, is_small = group == small || group == kExactSlices + 1;
+        cudaLaunchAttribute overlap;
+        overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        overlap.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t config = {};
+        config.gridDim = dim3(static_cast<unsigned>(pick(8 * grid, g_waves.slices[2 * exact + is_small])));
+        config.blockDim = dim3(kSliceThreads);
+        config.stream = s;
+        config.attrs = &overlap;
+        config.numAttrs = j > 0 ? 1 : 0;  // the first step of a body reads what the kernels before it wrote
+        cudaLaunchKernelEx(&config, slice_kernel(exact, is_small), v, group, j);
+    } else if (group >= kVariants) {
+        launch_group_of<PREC_MIXED>(v, group, j, grid, s);
+    } else {
+        launch_group_of<PREC_FP64>(v, group, j, grid, s);
+    }
 }
 
 void launch_step_exact(const View& v, int j, int grid, cudaStream_t s) {
@@ -2838,6 +3253,22 @@ void launch_gate_raw(int64_t n, const int32_t* rowptr, const int32_t* col, const
     if (grid < 1) grid = 1;
     convexity_gate_kernel<<<static_cast<int>(grid), kGateWarps * 32, 0, s>>>(rowptr, col, val, static_cast<int>(n), out,
                                                                              diag, vhi, vlo);
+}
+
+void launch_slice_rows(const InstDev& rec, int64_t n, int64_t nnz, const int32_t* rowptr, const int32_t* col,
+                       const double* val, uint8_t* position_of, int32_t* col_out, double* val_out, cudaStream_t s) {
+    // shared memory for a window of average rows and a fifth more
+    const int64_t want = kSliceWindow * nnz / n * 6 / 5 + kSliceWindow;
+    const int cap = static_cast<int>(want < 1024 ? 1024 : want > kSliceStageMax ? kSliceStageMax : (want + 1) & ~int64_t(1));
+    const int windows = static_cast<int>((n + kSliceWindow - 1) / kSliceWindow), ni = static_cast<int>(n);
+    slice_order_kernel<<<windows, kSliceWindow, 0, s>>>(rec, ni, rowptr, position_of);
+    slice_entries_kernel<<<windows, kSliceWindow, 12 * cap, s>>>(rec, ni, rowptr, col, val, cap, position_of, col_out, val_out);
+}
+
+void launch_unslice(int64_t n, const uint8_t* slice_row, const double* x, double* out, cudaStream_t s) {
+    int64_t grid = (n + kBlock - 1) / kBlock;
+    if (grid > 152 * 8) grid = 152 * 8;
+    unslice_kernel<<<static_cast<int>(grid), kBlock, 0, s>>>(static_cast<int>(n), slice_row, x, out);
 }
 
 void launch_gate(const InstDev& rec, int64_t n, const double* val, cudaStream_t s) {

@@ -11,11 +11,18 @@ int tile_grid(int sms);
 // resident blocks of the CG product kernel (after tile_grid)
 int cg_matvec_slots();
 // Tile kernels: grid-stride over the tile table (the grid size is fixed at capture).
-void launch_check(const View& v, int grid, cudaStream_t s);
+void launch_check(const View& v, int families, int grid, cudaStream_t s);
 // Step j of a body: the step kernel of one group (step_group(precision, variant)) over the group's
 // tiles, or the FP64_EXACT step over the whole table.
 void launch_step_group(const View& v, int group, int j, int grid, cudaStream_t s);
 void launch_step_exact(const View& v, int j, int grid, cudaStream_t s);
+// Check kernels of a body: one per family that has instances (bits of kCheck*).
+constexpr int kCheckFp64 = 1;    // FP64 engines over the CSR
+constexpr int kCheckSlices = 2;  // FP64 engines over sliced rows
+constexpr int kCheckMixed = 4;   // mixed engine: the FP32 iterate and the polished point (two kernels)
+constexpr int check_launches(int families) {
+    return ((families & kCheckFp64) ? 1 : 0) + ((families & kCheckSlices) ? 1 : 0) + ((families & kCheckMixed) ? 2 : 0);
+}
 void launch_polish_init(const View& v, int grid, cudaStream_t s);
 void launch_polish_residual(const View& v, int grid, cudaStream_t s);
 void launch_cg_matvec(const View& v, int grid, cudaStream_t s);
@@ -28,6 +35,8 @@ void launch_cg_vector(const View& v, int grid, cudaStream_t s, cudaGraphConditio
 // precision-k FISTA body (steps per body x step groups launched).
 struct StepLaunches {
     int n[3];
+    int checks;        // check kernels of a body
+    unsigned present;  // bit k: the graph has a branch for precision k (bit 1: and the polish)
 };
 void launch_gate(const View& v, const cudaGraphConditionalHandle* fista, cudaGraphConditionalHandle polish,
                  cudaGraphConditionalHandle cg_loop, StepLaunches steps, int body_steps, cudaStream_t s);
@@ -40,6 +49,14 @@ void launch_control_plain(const View& v, int steps, cudaStream_t s);
 // (FP64 values `val`) into *rec.gate (cleared first), the FP64 diagonal into rec.diag and, for the
 // mixed engine, the hi/lo FP32 values into rec.vhi/rec.vlo.  The later admission kernels read L there.
 void launch_gate(const InstDev& rec, int64_t n, const double* val, cudaStream_t s);
+// Admission of a sliced instance, after the gate: the order of its rows (slice_len, slice_row,
+// slice_base of `rec`), its vectors (c, l, u, diag) brought into that order in place, and its entries
+// (columns as positions) into col_out, val_out.  rowptr, col, val: the uploaded CSR; position_of: n
+// bytes of scratch.
+void launch_slice_rows(const InstDev& rec, int64_t n, int64_t nnz, const int32_t* rowptr, const int32_t* col,
+                       const double* val, uint8_t* position_of, int32_t* col_out, double* val_out, cudaStream_t s);
+// x of a sliced instance in row order: out[row] = x[position].
+void launch_unslice(int64_t n, const uint8_t* slice_row, const double* x, double* out, cudaStream_t s);
 // The same pass on raw device pointers (diag, vhi, vlo may be null: not stored).
 void launch_gate_raw(int64_t n, const int32_t* rowptr, const int32_t* col, const double* val, GateResult* out,
                      double* diag, float* vhi, float* vlo, cudaStream_t s);
