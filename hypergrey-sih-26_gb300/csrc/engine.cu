@@ -211,6 +211,8 @@ struct Job {
     int diag_gate = 0;  // -1: decided by the admission gate (a diagonal Hessian with a positive diagonal)
     int variant = 0;
     std::vector<Tile> tiles;  // local tiles (inst field filled at admission)
+    std::vector<Tile> items;  // step work items of a sliced solve: its tiles in pieces of kSlicePiece rows
+    std::vector<int4> units;  // CG and check work units, tiles counted from the solve's first (cg_units)
     int state = JOB_QUEUED;
     bool resolve = false;     // re-run of a resident solve
     bool notify = false;      // report completion through the completion queue (bqp_wait_any)
@@ -311,15 +313,15 @@ int default_variant(int64_t n, int64_t nnz, int64_t longest_row, int precision) 
     return VAR_TILE;
 }
 
-// CG work units of one instance (its `count` tiles at t), appended to `out` as {first tile, tiles,
-// index, units}: as many units as the product kernel has resident blocks (`slots`), so that one
+// CG and check work units of one instance (its `count` tiles at t), appended to `out` as {first tile, tiles,
+// index, units}, the tiles counted from the instance's first: as many units as the product kernel has resident blocks (`slots`), so that one
 // round runs them on the whole GPU, but units of about kCgUnitMin tiles at least; the tiles are
 // spread evenly (sizes differ by one at most), and no unit goes above kCgRowsum rows (the row
 // sums' shared buffer; units of kCgUnitMin tiles always fit).  At least 4 / 2 / 1 tiles: a 10k-row mixed
 // solve 457 / 430 / 420 us, the FP64 one 2.10 / 1.95 / 1.95 ms, 256 uneven solves 2.00 / 2.03 / 2.12 ms
 // on the device.  Depends on the instance alone, so
 // the product's partial sums, and the CG iterates, are the same in a batch as solo.
-void cg_units(const Tile* t, int count, int first, int slots, std::vector<int4>& out) {
+void cg_units(const Tile* t, int count, int slots, std::vector<int4>& out) {
     const int fewest = (count + kCgUnitMax - 1) / kCgUnitMax;
     const int most = std::max(1, (count + kCgUnitMin - 1) / kCgUnitMin);
     int u = std::max(fewest, std::min(std::max(slots, 1), most));
@@ -334,7 +336,7 @@ void cg_units(const Tile* t, int count, int first, int slots, std::vector<int4>&
     }
     for (int k = 0, b = 0; k < u; ++k) {
         const int len = count / u + (k < count % u ? 1 : 0);
-        out.push_back(make_int4(first + b, len, k, u));
+        out.push_back(make_int4(b, len, k, u));
         b += len;
     }
 }
@@ -455,6 +457,15 @@ public:
     }
 
 private:
+    // graphs built so far, by the step groups, the steps per body and the grid they launch: a stream
+    // of different solves goes back and forth between a few (kept up to kGraphs, dropped together)
+    struct Graph {
+        cudaGraph_t graph;
+        cudaGraphExec_t exec;
+        uint32_t groups;
+        int interval, grid;
+        int stand_in;  // launches for tables that need fewer groups
+    };
     void loop();
     bool upload(Job& j, std::string& why);
     bool alloc_upload(Job& j, size_t bytes, std::string& why);
@@ -487,9 +498,11 @@ private:
     bool run_once(std::string& why);
     bool run_stream(int cap, std::string& why);
     void update_grid();
+    bool select_graph(std::string& why);
     void collect(std::unique_lock<std::mutex>& lk);
     void process_frees();
-    void upload_tables();
+    std::vector<Job*> running_jobs() const;
+    bool upload_tables(const std::vector<Job*>& jobs, std::string& why);
     // step groups of precision `prec` that a body launches (bits of graph_groups_)
     std::vector<int> body_groups(int prec) const {
         std::vector<int> g;
@@ -540,7 +553,7 @@ private:
         return L;
     }
     bool ensure_tables(int need_inst, int need_tiles, std::string& why);
-    bool build_graph(std::string& why);
+    bool build_graph(Graph& out, std::string& why);
     View view() const {
         View v;
         v.inst = d_inst_;
@@ -611,16 +624,16 @@ private:
     int stage_cap_ = 0, span_cap_ = 0;
 
     // host mirrors
-    std::vector<Tile> h_tiles_;
     std::vector<int2> h_ranges_;
     std::vector<Job*> slot_job_;
-    std::vector<int32_t> slot_prec_;      // precision of the solve in each slot
-    std::vector<Tile> h_group_tiles_;     // the tiles ordered by step group
     // page-locked staging of the tables above: their copies to the device run as DMA behind the
     // engine stream instead of a pageable copy each (rewritten only after that stream drained)
     unsigned char* h_table_stage_ = nullptr;
     size_t table_stage_bytes_ = 0;
-    std::vector<int4> h_units_;           // CG work units: first tile, tiles, index, units of the instance
+    // the device tables (tiles, step groups, work units) hold the solves that run, and no others: a
+    // launch's kernels do not walk over the tiles of resident solves that have finished
+    std::vector<std::pair<int, uint64_t>> table_jobs_;  // slot and id of each solve in the tables
+    int n_tiles_ = 0, n_units_ = 0;
     int32_t group_begin_[kStepGroups + 1] = {};
     static constexpr uint32_t kExactCsrBit = 1u << kStepGroups;  // FP64_EXACT instances over the CSR
     uint32_t groups_present_ = 0;         // step groups with tiles (and kExactCsrBit)
@@ -632,11 +645,19 @@ private:
     bool tables_dirty_ = false;
 
     // graph
-    cudaGraph_t graph_ = nullptr;
-    cudaGraphExec_t exec_ = nullptr;
+    static constexpr size_t kGraphs = 16;
+    std::vector<Graph> graphs_;
+    Graph* graph_now_ = nullptr;
     int graph_grid_ = 0;
     int graph_interval_ = 25;
-    bool graph_valid_ = false;
+    void drop_graphs() {
+        for (Graph& g : graphs_) {
+            if (g.exec) cudaGraphExecDestroy(g.exec);
+            if (g.graph) cudaGraphDestroy(g.graph);
+        }
+        graphs_.clear();
+        graph_now_ = nullptr;
+    }
 
     // jobs
     mutable std::mutex mu_;
@@ -765,10 +786,7 @@ void Engine::shutdown() {
         cudaStreamSynchronize(stream_);
     }
     jobs_.clear();
-    if (exec_) cudaGraphExecDestroy(exec_);
-    if (graph_) cudaGraphDestroy(graph_);
-    exec_ = nullptr;
-    graph_ = nullptr;
+    drop_graphs();
     cudaFree(d_inst_); cudaFree(d_ranges_); cudaFree(d_tile_done_); cudaFree(d_status_);
     cudaFree(d_tiles_); cudaFree(d_partial_); cudaFree(d_ctrl_); cudaFree(d_momentum_); cudaFree(d_group_tiles_); cudaFree(d_units_);
     d_inst_ = nullptr; d_ranges_ = nullptr; d_tile_done_ = nullptr; d_status_ = nullptr;
@@ -845,9 +863,8 @@ bool Engine::ensure_tables(int need_inst, int need_tiles, std::string& why) {
         inst_cap_ = cap;
         h_ranges_.resize(cap, int2{0, 0});
         slot_job_.resize(cap, nullptr);
-        slot_prec_.resize(cap, 0);
         tables_dirty_ = true;
-        graph_valid_ = false;
+        drop_graphs();
     }
     if (need_tiles > tile_cap_) {
         int cap = std::max(need_tiles, std::max(1024, tile_cap_ * 2));
@@ -869,16 +886,45 @@ bool Engine::ensure_tables(int need_inst, int need_tiles, std::string& why) {
         d_units_ = units;
         tile_cap_ = cap;
         tables_dirty_ = true;
-        graph_valid_ = false;
+        drop_graphs();
     }
     return true;
 }
 
+// Grid cap of the tile kernels for the tables at hand: the tiles rounded up to a power of two (64 at
+// least), so that tables of about the same size share a graph.
 void Engine::update_grid() {
-    const int grid_max = grid_max_;
-    int want = static_cast<int>(std::min<size_t>(static_cast<size_t>(grid_max), align_up(std::max<size_t>(h_tiles_.size(), 1), 32)));
-    graph_grid_ = std::max(want, graph_grid_);
-    if (graph_grid_ > grid_max) graph_grid_ = grid_max;
+    int want = 64;
+    while (want < grid_max_ && want < n_tiles_) want *= 2;
+    graph_grid_ = std::min(want, grid_max_);
+}
+
+// The graph for the tables at hand: one built for these groups, or one that launches more (its idle
+// launches cost less than building another, unless that goes on), or a new one.
+bool Engine::select_graph(std::string& why) {
+    constexpr int kStandIns = 8;
+    update_grid();
+    graph_now_ = nullptr;
+    for (Graph& g : graphs_) {
+        if (g.interval != graph_interval_ || g.grid < graph_grid_ || (groups_present_ & ~g.groups)) continue;
+        const bool exact = g.groups == groups_present_ && g.grid == graph_grid_;
+        if (exact) {
+            graph_now_ = &g;
+            return true;
+        }
+        if (!graph_now_ || g.grid < graph_now_->grid) graph_now_ = &g;
+    }
+    if (graph_now_ && ++graph_now_->stand_in <= kStandIns) return true;
+    if (graph_now_) graph_now_->stand_in = 0;
+    if (graphs_.size() >= kGraphs) drop_graphs();
+    graphs_.push_back(Graph{nullptr, nullptr, groups_present_, graph_interval_, graph_grid_, 0});
+    graph_groups_ = groups_present_;
+    if (!build_graph(graphs_.back(), why)) {
+        drop_graphs();
+        return false;
+    }
+    graph_now_ = &graphs_.back();
+    return true;
 }
 
 // Host-driven launches of the same loop body: the host reads the gate's phase counts after
@@ -946,34 +992,28 @@ bool Engine::run_stream(int cap, std::string& why) {
     return cuda_ok(cudaGetLastError(), why, "stream launches");
 }
 
-bool Engine::build_graph(std::string& why) {
-    if (exec_) cudaGraphExecDestroy(exec_);
-    if (graph_) cudaGraphDestroy(graph_);
-    exec_ = nullptr;
-    graph_ = nullptr;
-    update_grid();
-    graph_groups_ = groups_present_;
+bool Engine::build_graph(Graph& out, std::string& why) {
     const int grid = graph_grid_;
     const int K = graph_interval_;
     const View v = view();
 
-    if (!cuda_ok(cudaGraphCreate(&graph_, 0), why, "graph create")) return false;
+    if (!cuda_ok(cudaGraphCreate(&out.graph, 0), why, "graph create")) return false;
     cudaGraphConditionalHandle h_loop, h_f[3] = {}, h_pol = 0, h_cg = 0;
-    if (!cuda_ok(cudaGraphConditionalHandleCreate(&h_loop, graph_, 1, cudaGraphCondAssignDefault), why, "conditional handle")) return false;
+    if (!cuda_ok(cudaGraphConditionalHandleCreate(&h_loop, out.graph, 1, cudaGraphCondAssignDefault), why, "conditional handle")) return false;
     const unsigned present = present_precisions();
     const bool mixed = (present >> PREC_MIXED) & 1u;
     for (int k = 0; k < 3; ++k)
         if (((present >> k) & 1u) &&
-            !cuda_ok(cudaGraphConditionalHandleCreate(&h_f[k], graph_, 0, cudaGraphCondAssignDefault), why, "conditional handle")) return false;
-    if (mixed && !cuda_ok(cudaGraphConditionalHandleCreate(&h_pol, graph_, 0, cudaGraphCondAssignDefault), why, "conditional handle")) return false;
-    if (mixed && !cuda_ok(cudaGraphConditionalHandleCreate(&h_cg, graph_, 0, cudaGraphCondAssignDefault), why, "conditional handle")) return false;
+            !cuda_ok(cudaGraphConditionalHandleCreate(&h_f[k], out.graph, 0, cudaGraphCondAssignDefault), why, "conditional handle")) return false;
+    if (mixed && !cuda_ok(cudaGraphConditionalHandleCreate(&h_pol, out.graph, 0, cudaGraphCondAssignDefault), why, "conditional handle")) return false;
+    if (mixed && !cuda_ok(cudaGraphConditionalHandleCreate(&h_cg, out.graph, 0, cudaGraphCondAssignDefault), why, "conditional handle")) return false;
 
     cudaGraphNodeParams wp = {cudaGraphNodeTypeConditional};
     wp.conditional.handle = h_loop;
     wp.conditional.type = cudaGraphCondTypeWhile;
     wp.conditional.size = 1;
     cudaGraphNode_t wnode;
-    if (!cuda_ok(cudaGraphAddNode(&wnode, graph_, nullptr, nullptr, 0, &wp), why, "while node")) return false;
+    if (!cuda_ok(cudaGraphAddNode(&wnode, out.graph, nullptr, nullptr, 0, &wp), why, "while node")) return false;
     cudaGraph_t body = wp.conditional.phGraph_out[0];
 
     auto capture = [&](cudaGraph_t g, const cudaGraphNode_t* deps, size_t ndeps, auto&& launches,
@@ -1042,8 +1082,7 @@ bool Engine::build_graph(std::string& why) {
         last = node;
     }
     if (!capture(body, &last, 1, [&] { launch_control(v, h_loop, K, capture_); }, nullptr)) return false;
-    if (!cuda_ok(cudaGraphInstantiate(&exec_, graph_, 0), why, "graph instantiate")) return false;
-    graph_valid_ = true;
+    if (!cuda_ok(cudaGraphInstantiate(&out.exec, out.graph, 0), why, "graph instantiate")) return false;
     return true;
 }
 
@@ -1335,10 +1374,7 @@ void Engine::update_steps() {
         }
     if (!any) return;
     steps = std::max(1, steps);
-    if (steps != graph_interval_) {
-        graph_interval_ = steps;
-        graph_valid_ = false;
-    }
+    graph_interval_ = steps;
 }
 
 // Uploads one new solve on the upload stream (inputs, slab, device-side forms), without touching
@@ -1591,17 +1627,13 @@ bool Engine::install(std::vector<Job*>& jobs, std::string& why) {
             slot = n_inst_++;
         }
         j.slot = slot;
-        slot_prec_[slot] = j.opt.precision;
         for (Tile& t : j.tiles) t.inst = slot;
-        const int begin = static_cast<int>(h_tiles_.size());
-        if (!ensure_tables(0, begin + static_cast<int>(j.tiles.size()), why)) return false;
-        h_tiles_.insert(h_tiles_.end(), j.tiles.begin(), j.tiles.end());
-        h_ranges_[slot] = int2{begin, static_cast<int>(h_tiles_.size())};
-        tables_dirty_ = true;
+        for (Tile& t : j.items) t.inst = slot;
+        j.units.clear();
+        cg_units(j.tiles.data(), static_cast<int>(j.tiles.size()), cg_slots_, j.units);
     }
     if (!cuda_ok(cudaStreamWaitEvent(stream_, uev_, 0), why, "upload order")) return false;
     if (!rearm(jobs, why)) return false;
-    if (graph_grid_ < grid_max_ && static_cast<int>(h_tiles_.size()) > graph_grid_) graph_valid_ = false;
     return true;
 }
 
@@ -1746,117 +1778,113 @@ void Engine::fail_admission(Job* j, size_t reserved, const std::string& why) {
 
 void Engine::process_frees() {
     if (pending_free_.empty()) return;
-    std::vector<char> dead(static_cast<size_t>(std::max(n_inst_, 1)), 0);
     for (auto& pf : pending_free_) {
         if (pf.second) cudaFreeAsync(pf.second, stream_);
         if (pf.first >= 0) {
-            dead[pf.first] = 1;
             slot_job_[pf.first] = nullptr;
             free_slots_.push_back(pf.first);
-            h_ranges_[pf.first] = int2{0, 0};
         }
     }
     pending_free_.clear();
-    std::vector<Tile> kept;
-    kept.reserve(h_tiles_.size());
-    for (const Tile& t : h_tiles_) if (!dead[t.inst]) kept.push_back(t);
-    h_tiles_.swap(kept);
-    for (int s = 0; s < n_inst_; ++s) h_ranges_[s] = int2{0, 0};
-    for (int k = 0; k < static_cast<int>(h_tiles_.size()); ++k) {
-        int2& r = h_ranges_[h_tiles_[k].inst];
-        if (r.y == 0) r.x = k;
-        r.y = k + 1;
-    }
-    tables_dirty_ = true;
 }
 
-// Uploads the tile and range tables and the step groups (tiles ordered by (precision, variant),
-// a counting sort in table order) when they changed.  A group the graph does not launch yet
-// invalidates it.
-void Engine::upload_tables() {
-    if (!tables_dirty_) return;
-    // a sliced instance's tiles go to its group in pieces of kSlicePiece rows
-    auto pieces = [](const Tile& t) {
-        return is_sliced(t.variant) ? (t.row_end - t.row_begin + kSlicePiece - 1) / kSlicePiece : 1;
-    };
+// The solves in the running state, in slot order (caller holds mu_).
+std::vector<Job*> Engine::running_jobs() const {
+    std::vector<Job*> jobs;
+    for (int s = 0; s < n_inst_; ++s)
+        if (slot_job_[s] && slot_job_[s]->state == JOB_RUNNING) jobs.push_back(slot_job_[s]);
+    return jobs;
+}
+
+// Uploads the tables of the solves `jobs` (tiles, step groups: items by (precision, variant), work
+// units, ranges) unless the device already has them.  Each solve keeps its own lists, so this is
+// one copy of each into the page-locked staging buffer.
+bool Engine::upload_tables(const std::vector<Job*>& jobs, std::string& why) {
+    std::vector<std::pair<int, uint64_t>> ids;
+    ids.reserve(jobs.size());
+    for (const Job* j : jobs) ids.emplace_back(j->slot, j->id);
+    if (!tables_dirty_ && ids == table_jobs_) return true;
+    size_t tiles = 0, units = 0, items = 0;
     int32_t count[kStepGroups + 1] = {};
-    uint32_t exact_csr = 0;
-    for (const Tile& t : h_tiles_) {
-        const int g = step_group(slot_prec_[t.inst], t.variant);
-        if (g >= 0) count[g + 1] += pieces(t);
-        else exact_csr = kExactCsrBit;
+    groups_present_ = 0;
+    auto items_of = [](const Job& j) -> const std::vector<Tile>& { return is_sliced(j.variant) ? j.items : j.tiles; };
+    for (const Job* j : jobs) {
+        tiles += j->tiles.size();
+        units += j->units.size();
+        const int g = step_group(j->opt.precision, j->variant);
+        if (g < 0) {
+            groups_present_ |= kExactCsrBit;
+            continue;
+        }
+        groups_present_ |= 1u << g;
+        count[g + 1] += static_cast<int32_t>(items_of(*j).size());
+        items += items_of(*j).size();
     }
-    groups_present_ = exact_csr;
-    for (int g = 0; g < kStepGroups; ++g) {
-        if (count[g + 1]) groups_present_ |= 1u << g;
-        count[g + 1] += count[g];
-    }
+    for (int g = 0; g < kStepGroups; ++g) count[g + 1] += count[g];
     std::memcpy(group_begin_, count, sizeof(group_begin_));
-    h_group_tiles_.resize(static_cast<size_t>(count[kStepGroups]));
-    for (int k = 0; k < static_cast<int>(h_tiles_.size()); ++k) {
-        const Tile& t = h_tiles_[k];
-        const int g = step_group(slot_prec_[t.inst], t.variant);
-        if (g < 0) continue;
-        const int rows = is_sliced(t.variant) ? kSlicePiece : t.row_end - t.row_begin;
-        for (int r = t.row_begin; r < t.row_end; r += rows)
-            h_group_tiles_[static_cast<size_t>(count[g]++)] = Tile{t.inst, r, std::min(r + rows, t.row_end), t.variant};
-    }
-    // CG work units: runs of consecutive tiles of one instance (cg_units; a unit depends on the
-    // instance alone, not on the batch)
-    h_units_.clear();
-    for (int i = 0; i < n_inst_; ++i) {
-        const int2 R = h_ranges_[i];
-        if (R.y > R.x) cg_units(h_tiles_.data() + R.x, R.y - R.x, R.x, cg_slots_, h_units_);
-    }
-    // the four tables through one page-locked staging buffer (16-byte aligned parts)
-    const size_t b_tiles = sizeof(Tile) * h_tiles_.size();
-    const size_t b_group = sizeof(Tile) * h_group_tiles_.size();
-    const size_t b_units = sizeof(int4) * h_units_.size();
+    if (!ensure_tables(0, static_cast<int>(tiles), why)) return false;
+    tables_dirty_ = true;  // until the copies below are queued
+    const size_t b_tiles = sizeof(Tile) * tiles, b_group = sizeof(Tile) * items, b_units = sizeof(int4) * units;
     const size_t b_ranges = sizeof(int2) * static_cast<size_t>(std::max(n_inst_, 1));
-    auto up16 = [](size_t b) { return (b + 15) & ~size_t(15); };
-    const size_t need = up16(b_tiles) + up16(b_group) + up16(b_units) + up16(b_ranges);
+    const size_t need = b_tiles + b_group + b_units + b_ranges;
     if (need > table_stage_bytes_) {
         const size_t cap = std::max(need, 2 * table_stage_bytes_);
         if (h_table_stage_) cudaFreeHost(h_table_stage_);
         h_table_stage_ = nullptr;
         table_stage_bytes_ = 0;
-        if (cudaMallocHost(&h_table_stage_, cap) == cudaSuccess) table_stage_bytes_ = cap;
+        if (!cuda_ok(cudaMallocHost(&h_table_stage_, cap), why, "table staging")) return false;
+        table_stage_bytes_ = cap;
     }
-    auto stage = [&](void* dst, const void* src, size_t bytes, size_t& at) {
-        if (bytes == 0) return;
-        if (h_table_stage_) {
-            std::memcpy(h_table_stage_ + at, src, bytes);
-            cudaMemcpyAsync(dst, h_table_stage_ + at, bytes, cudaMemcpyHostToDevice, stream_);
-            at += up16(bytes);
-        } else {
-            cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream_);  // pageable fallback
+    // the staging buffer is rewritten only here, after the engine stream drained
+    Tile* t = reinterpret_cast<Tile*>(h_table_stage_);
+    Tile* it = t + tiles;
+    int4* un = reinterpret_cast<int4*>(it + items);
+    n_tiles_ = 0;
+    for (const Job* j : jobs) {
+        std::memcpy(t + n_tiles_, j->tiles.data(), sizeof(Tile) * j->tiles.size());
+        const int g = step_group(j->opt.precision, j->variant);
+        if (g >= 0) {
+            const std::vector<Tile>& list = items_of(*j);
+            std::memcpy(it + count[g], list.data(), sizeof(Tile) * list.size());
+            count[g] += static_cast<int32_t>(list.size());
         }
+        for (const int4& u : j->units) *un++ = make_int4(u.x + n_tiles_, u.y, u.z, u.w);
+        h_ranges_[j->slot] = int2{n_tiles_, n_tiles_ + static_cast<int>(j->tiles.size())};
+        n_tiles_ += static_cast<int>(j->tiles.size());
+    }
+    n_units_ = static_cast<int>(units);
+    std::memcpy(un, h_ranges_.data(), b_ranges);
+    const unsigned char* at = h_table_stage_;
+    auto copy = [&](void* dst, size_t bytes) {
+        if (bytes) cudaMemcpyAsync(dst, at, bytes, cudaMemcpyHostToDevice, stream_);
+        at += bytes;
     };
-    size_t at = 0;
-    stage(d_tiles_, h_tiles_.data(), b_tiles, at);
-    stage(d_group_tiles_, h_group_tiles_.data(), b_group, at);
-    stage(d_units_, h_units_.data(), b_units, at);
-    stage(d_ranges_, h_ranges_.data(), b_ranges, at);
-    // the staging buffer is rewritten only by the next call, after the engine stream drained
-    if (groups_present_ & ~graph_groups_) graph_valid_ = false;
+    copy(d_tiles_, b_tiles);
+    copy(d_group_tiles_, b_group);
+    copy(d_units_, b_units);
+    copy(d_ranges_, b_ranges);
+    table_jobs_.swap(ids);
     tables_dirty_ = false;
+    return true;
 }
 
 bool Engine::run_once(std::string& why) {
     const double t_enter = host_profile() ? host_seconds() : 0.0;
-    upload_tables();
-    const double t_tables = host_profile() ? host_seconds() : 0.0;
-    if (!stream_mode_ && !graph_valid_ && !build_graph(why)) return false;
     int cap = std::numeric_limits<int>::max() / 2;
     double latency;
+    std::vector<Job*> jobs;
     {
         std::lock_guard<std::mutex> g(mu_);
         latency = latency_ms_;
+        jobs = running_jobs();
     }
+    if (!upload_tables(jobs, why)) return false;
+    const double t_tables = host_profile() ? host_seconds() : 0.0;
+    if (!stream_mode_ && !select_graph(why)) return false;
     if (latency > 0) cap = std::max(1, static_cast<int>(latency / std::max(body_ms_, 1e-3)));
     h_ctrl_->n_inst = n_inst_;
-    h_ctrl_->n_tiles = static_cast<int32_t>(h_tiles_.size());
-    h_ctrl_->n_units = static_cast<int32_t>(h_units_.size());
+    h_ctrl_->n_tiles = n_tiles_;
+    h_ctrl_->n_units = n_units_;
     std::memcpy(h_ctrl_->group_begin, group_begin_, sizeof(group_begin_));
     for (int k = 0; k < 3; ++k) {
         h_ctrl_->check_due[k] = 1;  // the first body checks whatever is due; later ones as counted
@@ -1872,7 +1900,7 @@ bool Engine::run_once(std::string& why) {
     if (stream_mode_) {
         if (!run_stream(cap, why)) return false;
         cudaMemcpyAsync(d_ctrl_, h_ctrl_, sizeof(Ctrl), cudaMemcpyHostToDevice, stream_);
-    } else if (!cuda_ok(cudaGraphLaunch(exec_, stream_), why, "graph launch")) {
+    } else if (!cuda_ok(cudaGraphLaunch(graph_now_->exec, stream_), why, "graph launch")) {
         return false;
     }
     if (host_profile()) {
@@ -2014,6 +2042,10 @@ int Engine::profile_step(uint64_t id, int launches, double* ms_out, double* byte
     if (j.state != JOB_DONE || !j.resident || n_running_ != 0 || !queue_.empty() || launches < 1) return BQP_ERR_NOT_READY;
     cudaSetDevice(device_);
     std::string why;
+    if (!upload_tables({&j}, why)) {
+        set_error(why);
+        return BQP_ERR_CUDA;
+    }
     update_grid();
     InstDev saved;
     cudaMemcpy(&saved, &d_inst_[j.slot], sizeof(InstDev), cudaMemcpyDeviceToHost);
@@ -2028,10 +2060,9 @@ int Engine::profile_step(uint64_t id, int launches, double* ms_out, double* byte
         R.beta32[k] = 0.5f;
     }
     cudaMemcpyAsync(&d_inst_[j.slot], &R, sizeof(InstDev), cudaMemcpyHostToDevice, stream_);
-    upload_tables();
     h_ctrl_->n_inst = n_inst_;
-    h_ctrl_->n_tiles = static_cast<int32_t>(h_tiles_.size());
-    h_ctrl_->n_units = static_cast<int32_t>(h_units_.size());
+    h_ctrl_->n_tiles = n_tiles_;
+    h_ctrl_->n_units = n_units_;
     std::memcpy(h_ctrl_->group_begin, group_begin_, sizeof(group_begin_));
     for (int k = 0; k < 3; ++k) h_ctrl_->step_due[k] = kMaxInterval;
     cudaMemcpyAsync(d_ctrl_, h_ctrl_, sizeof(Ctrl), cudaMemcpyHostToDevice, stream_);
@@ -2075,6 +2106,11 @@ int Engine::profile_cg(uint64_t id, int iterations, double* ms_matvec, double* m
         j.opt.precision != PREC_MIXED)
         return BQP_ERR_NOT_READY;
     cudaSetDevice(device_);
+    std::string why;
+    if (!upload_tables({&j}, why)) {
+        set_error(why);
+        return BQP_ERR_CUDA;
+    }
     update_grid();
     InstDev saved;
     cudaMemcpy(&saved, &d_inst_[j.slot], sizeof(InstDev), cudaMemcpyDeviceToHost);
@@ -2088,10 +2124,9 @@ int Engine::profile_cg(uint64_t id, int iterations, double* ms_matvec, double* m
     R.ff_nnz = 0;
     R.ff_rows = 0;
     cudaMemcpyAsync(&d_inst_[j.slot], &R, sizeof(InstDev), cudaMemcpyHostToDevice, stream_);
-    upload_tables();
     h_ctrl_->n_inst = n_inst_;
-    h_ctrl_->n_tiles = static_cast<int32_t>(h_tiles_.size());
-    h_ctrl_->n_units = static_cast<int32_t>(h_units_.size());
+    h_ctrl_->n_tiles = n_tiles_;
+    h_ctrl_->n_units = n_units_;
     h_ctrl_->n_cg = 1;
     cudaMemcpyAsync(d_ctrl_, h_ctrl_, sizeof(Ctrl), cudaMemcpyHostToDevice, stream_);
     const View v = view();
@@ -2523,6 +2558,10 @@ int make_job(int64_t n, int64_t nnz, const int32_t* rowptr, const int32_t* col, 
     if (o.precision != BQP_PRECISION_FP64_EXACT && o.kernel_variant >= 0) j->variant = o.kernel_variant;
     else j->variant = bqp::default_variant(n, nnz, scan.longest, o.precision);
     j->tiles = bqp::make_tiles(n, rowptr, j->variant);
+    if (bqp::is_sliced(j->variant))
+        for (const bqp::Tile& t : j->tiles)
+            for (int32_t r = t.row_begin; r < t.row_end; r += bqp::kSlicePiece)
+                j->items.push_back(bqp::Tile{0, r, std::min(r + bqp::kSlicePiece, t.row_end), t.variant});
     const double t_tiles = host_seconds();
     if (copy) {
         j->rowptr = dst.rowptr; j->col = dst.col; j->val = dst.val; j->c = dst.c; j->l = dst.l; j->u = dst.u;
