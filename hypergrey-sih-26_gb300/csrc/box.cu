@@ -22,7 +22,7 @@
 struct bqp_box {
     int device = 0;
     int64_t n = 0, nnz = 0;
-    double L = 0;
+    bqp::KnownDivisor L{};
     int32_t* rowptr = nullptr;
     int32_t* col = nullptr;
     double* val = nullptr;
@@ -31,6 +31,10 @@ struct bqp_box {
     double* u = nullptr;
     double* x = nullptr;
     double* w[2] = {nullptr, nullptr};
+    // sliced rows (engine.cuh): the arrays above in slice order, no row pointers
+    uint8_t* slice_len = nullptr;
+    uint8_t* slice_row = nullptr;
+    int32_t* slice_base = nullptr;
     int cur = 0;
     cudaStream_t stream = nullptr;
     std::string error;
@@ -43,6 +47,7 @@ void box_free(bqp_box* b) {
     if (!b) return;
     cudaFree(b->rowptr); cudaFree(b->col); cudaFree(b->val); cudaFree(b->c); cudaFree(b->l); cudaFree(b->u);
     cudaFree(b->x); cudaFree(b->w[0]); cudaFree(b->w[1]);
+    cudaFree(b->slice_len); cudaFree(b->slice_row); cudaFree(b->slice_base);
     if (b->stream) cudaStreamDestroy(b->stream);
     delete b;
 }
@@ -52,6 +57,57 @@ bool ok(cudaError_t e, std::string& why) {
     why = std::string("CUDA: ") + cudaGetErrorString(e);
     return false;
 }
+
+// Brings an uploaded problem into slice order where its rows allow it (sliceable: the row pointers
+// are consistent and no row is too long for a lane).  Without memory for the second copy of the
+// entries, or for other rows, it stays in CSR.
+bool slice_box(bqp_box* b, const int32_t* rowptr, std::string& why) {
+    int64_t longest = 0;
+    bool consistent = rowptr[0] == 0 && rowptr[b->n] == b->nnz;
+    for (int64_t i = 0; i < b->n && consistent; ++i) {
+        const int64_t len = static_cast<int64_t>(rowptr[i + 1]) - rowptr[i];
+        consistent = len >= 0;
+        if (len > longest) longest = len;
+    }
+    if (!consistent || !bqp::sliceable(b->n, b->nnz, longest)) return true;
+    const size_t N = static_cast<size_t>(b->n), Z = static_cast<size_t>(b->nnz);
+    int32_t* col = nullptr;
+    double* val = nullptr;
+    uint8_t* position_of = nullptr;
+    if (cudaMalloc(&col, Z * 4 + 16) != cudaSuccess || cudaMalloc(&val, Z * 8 + 16) != cudaSuccess ||
+        cudaMalloc(&position_of, N) != cudaSuccess || cudaMalloc(&b->slice_len, N) != cudaSuccess ||
+        cudaMalloc(&b->slice_row, N) != cudaSuccess || cudaMalloc(&b->slice_base, (N + 31) / 32 * 4) != cudaSuccess) {
+        cudaGetLastError();  // not sticky
+        cudaFree(col); cudaFree(val); cudaFree(position_of);
+        cudaFree(b->slice_len); cudaFree(b->slice_row); cudaFree(b->slice_base);
+        b->slice_len = b->slice_row = nullptr;
+        b->slice_base = nullptr;
+        return true;
+    }
+    bqp::InstDev rec{};
+    rec.slice_len = b->slice_len;
+    rec.slice_row = b->slice_row;
+    rec.slice_base = b->slice_base;
+    rec.c = b->c;
+    rec.l = b->l;
+    rec.u = b->u;
+    bqp::launch_slice_rows(rec, b->n, b->nnz, b->rowptr, b->col, b->val, position_of, col, val, b->stream);
+    const bool good = ok(cudaGetLastError(), why) && ok(cudaStreamSynchronize(b->stream), why);
+    cudaFree(position_of); cudaFree(b->rowptr); cudaFree(b->col); cudaFree(b->val);
+    b->rowptr = nullptr;
+    b->col = col;
+    b->val = val;
+    return good;
+}
+
+// x0 = w0 = clip(0, l, u) (CudaBox::initial, src/cuda_box.cu:25), in the order of l and u
+__global__ void box_start_kernel(int64_t n, const double* l, const double* u, double* x, double* w) {
+    for (int64_t j = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; j < n; j += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        const double v = 0.0 < u[j] ? 0.0 : u[j];
+        x[j] = w[j] = l[j] < v ? v : l[j];
+    }
+}
+
 // ---- scratch of bqp_check_device_noalloc ------------------------------------------------------
 // The verification reduction needs global scratch for its per-block partials, its completion
 // counter and its 8 result values.  bqp_check_device_noalloc takes that scratch from this
@@ -150,15 +206,9 @@ bqp_box* bqp_box_create(int device, int64_t n, int64_t nnz, const int32_t* rowpt
     b->device = device;
     b->n = n;
     b->nnz = nnz;
-    b->L = lipschitz;
+    b->L = bqp::known_divisor(lipschitz);
     std::string why;
     const size_t N = static_cast<size_t>(n), Z = static_cast<size_t>(nnz);
-    // x0 = w0 = clip(0, l, u) (CudaBox::initial, src/cuda_box.cu:25)
-    std::vector<double> x0(N);
-    for (size_t j = 0; j < N; ++j) {
-        double v = (0.0 < upper[j]) ? 0.0 : upper[j];
-        x0[j] = (lower[j] < v) ? v : lower[j];
-    }
     bool good = ok(cudaSetDevice(device), why) && ok(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking), why) &&
                 ok(cudaMalloc(&b->rowptr, (N + 1) * 4), why) && ok(cudaMalloc(&b->col, Z * 4 + 16), why) &&
                 ok(cudaMalloc(&b->val, Z * 8 + 16), why) && ok(cudaMalloc(&b->c, N * 8), why) &&
@@ -170,9 +220,12 @@ bqp_box* bqp_box_create(int device, int64_t n, int64_t nnz, const int32_t* rowpt
                 (Z == 0 || ok(cudaMemcpy(b->val, val, Z * 8, cudaMemcpyHostToDevice), why)) &&
                 ok(cudaMemcpy(b->c, c, N * 8, cudaMemcpyHostToDevice), why) &&
                 ok(cudaMemcpy(b->l, lower, N * 8, cudaMemcpyHostToDevice), why) &&
-                ok(cudaMemcpy(b->u, upper, N * 8, cudaMemcpyHostToDevice), why) &&
-                ok(cudaMemcpy(b->x, x0.data(), N * 8, cudaMemcpyHostToDevice), why) &&
-                ok(cudaMemcpy(b->w[0], x0.data(), N * 8, cudaMemcpyHostToDevice), why);
+                ok(cudaMemcpy(b->u, upper, N * 8, cudaMemcpyHostToDevice), why) && slice_box(b, rowptr, why);
+    if (good) {
+        box_start_kernel<<<static_cast<int>((N + 255) / 256 < 4096 ? (N + 255) / 256 : 4096), 256, 0, b->stream>>>(n, b->l, b->u, b->x,
+                                                                                                          b->w[0]);
+        good = ok(cudaGetLastError(), why) && ok(cudaStreamSynchronize(b->stream), why);
+    }
     if (!good) {
         g_box_error = why;
         box_free(b);
@@ -184,8 +237,8 @@ bqp_box* bqp_box_create(int device, int64_t n, int64_t nnz, const int32_t* rowpt
 int bqp_box_step(bqp_box* b, double momentum) {
     if (!b) return BQP_ERR_INVALID;
     cudaSetDevice(b->device);
-    bqp::launch_box_step(b->n, b->rowptr, b->col, b->val, b->c, b->l, b->u, b->L, momentum, b->x, b->w[b->cur],
-                         b->w[b->cur ^ 1], b->stream);
+    const bqp::BoxStep step{b->n, b->rowptr, b->slice_len, b->slice_base, b->col, b->val, b->c, b->l, b->u, b->L};
+    bqp::launch_box_step(step, momentum, b->x, b->w[b->cur], b->w[b->cur ^ 1], b->stream);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         b->error = std::string("CUDA: ") + cudaGetErrorString(e);
@@ -198,7 +251,12 @@ int bqp_box_step(bqp_box* b, double momentum) {
 int bqp_box_primal(bqp_box* b, double* x) {
     if (!b || !x) return BQP_ERR_INVALID;
     cudaSetDevice(b->device);
-    cudaError_t e = cudaMemcpyAsync(x, b->x, static_cast<size_t>(b->n) * 8, cudaMemcpyDeviceToHost, b->stream);
+    const double* from = b->x;
+    if (b->slice_row) {  // row order, in the buffer the next step writes
+        bqp::launch_unslice(b->n, b->slice_row, b->x, b->w[b->cur ^ 1], b->stream);
+        from = b->w[b->cur ^ 1];
+    }
+    cudaError_t e = cudaMemcpyAsync(x, from, static_cast<size_t>(b->n) * 8, cudaMemcpyDeviceToHost, b->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
     if (e != cudaSuccess) {
         b->error = std::string("CUDA: ") + cudaGetErrorString(e);

@@ -306,7 +306,7 @@ void set_unsupported(bqp_stats& st) {
 // long rows elsewhere take sub-warps, the rest the block-staged tile.
 int default_variant(int64_t n, int64_t nnz, int64_t longest_row, int precision) {
     const double avg = n > 0 ? static_cast<double>(nnz) / static_cast<double>(n) : 1.0;
-    if (precision != PREC_MIXED && longest_row <= kSliceMaxRow && avg < kSliceMaxAverage)
+    if (precision != PREC_MIXED && sliceable(n, nnz, longest_row))
         return n <= kSliceSmall ? VAR_SLICE_SMALL : VAR_SLICE;
     if (precision == PREC_FP64_EXACT) return 1;
     if (avg >= 48) return 32;
@@ -1512,6 +1512,8 @@ bool Engine::upload_begin(Job& j, std::string& why) {
     R.L = j.lipschitz;
     R.invL = 1.0 / j.lipschitz;
     R.invLf = static_cast<float>(1.0 / j.lipschitz);
+    R.invL_lo = 0.0;  // set with L once the gate has found it
+    R.div_span = 0;
     R.tol = j.opt.tolerance;
     R.offset = j.opt.offset;
     R.interval = j.opt.check_interval;
@@ -1730,7 +1732,10 @@ bool Engine::gate_uploaded(std::vector<Job*>& batch, std::vector<Job*>& refused,
         std::memcpy(&L, &g.lip_bits, sizeof(double));
         j->lipschitz = L;
         j->rec.L = L;
-        j->rec.invL = 1.0 / L;
+        const KnownDivisor d = known_divisor(L);
+        j->rec.invL = d.hi;
+        j->rec.invL_lo = d.lo;
+        j->rec.div_span = d.span;
         j->rec.invLf = static_cast<float>(1.0 / L);
         keep.push_back(j);
     }

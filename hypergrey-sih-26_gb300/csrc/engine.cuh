@@ -6,6 +6,7 @@
 // instances that are not in the phase the kernel serves, so one captured graph serves
 // any mix of instances that are admitted, iterating, polishing or retired.
 #pragma once
+#include <cmath>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -81,6 +82,10 @@ constexpr int kSlicePiece = 128;     // rows of a step work item (a block's four
 constexpr int64_t kSliceSmall = 65536;  // rows up to which an instance is VAR_SLICE_SMALL
 constexpr int kSliceMaxRow = 127;    // longest row of a sliced instance (a tile holds 32 such rows, so tiles begin on slices)
 constexpr int kSliceMaxAverage = 48; // longer average rows keep the sub-warp structures (default_variant)
+
+inline bool sliceable(int64_t n, int64_t nnz, int64_t longest_row) {
+    return n > 0 && nnz > 0 && longest_row <= kSliceMaxRow && nnz < kSliceMaxAverage * n;
+}
 
 struct Tile {
     int32_t inst;
@@ -202,7 +207,9 @@ struct __align__(16) InstDev {
     int64_t end_ns;
     double L;
     double invL;
+    double invL_lo;        // exact engine: 1/L - invL, and the dividends' exponent range (KnownDivisor)
     float invLf;
+    int32_t div_span;
     int32_t result_src;    // where the answer lives: 0 x64, 1 x32, 2 xp
     double tol;
     double offset;
@@ -240,6 +247,28 @@ struct __align__(16) InstDev {
     double polish_bytes;   // polish: algorithmic bytes of the residual passes and CG iterations
 };
 static_assert(sizeof(InstDev) % 16 == 0, "rearm_kernel copies records as 16-byte words");
+
+// Division by a divisor known in advance, correctly rounded: hi = RN(1/b), lo = RN(1/b - hi), then
+// q = RN(a hi + RN(a lo)) is within an ulp of a/b, r = a - q b is exact (one fused operation), and
+// RN(q + r hi) is RN(a/b) (P. Markstein, IBM J. Res. Dev. 34, 1990; the two-part reciprocal of
+// N. Brisebarre, J.-M. Muller and S. K. Raina, IEEE Trans. Computers 53, 2004).  Four FP64
+// operations, where the general division takes several times as many.  The theorem wants every
+// step clear of underflow and overflow: divisors of 2^-100..2^100 and dividends of biased exponent
+// kDivLow.. kDivLow + kDivSpan; span 0 (divisor outside) and other dividends (zeros, whose signs
+// the remainder would lose, among them) take the general division.
+constexpr int kDivLow = 200, kDivSpan = 1647;
+struct KnownDivisor {
+    double b, hi, lo;
+    int32_t span;
+};
+inline KnownDivisor known_divisor(double b) {
+    KnownDivisor d{b, 1.0 / b, 0.0, 0};
+    if (b >= 0x1p-100 && b <= 0x1p100) {
+        d.lo = std::fma(-d.hi, b, 1.0) / b;  // the remainder is exact
+        d.span = kDivSpan;
+    }
+    return d;
+}
 
 struct Ctrl {
     int32_t n_inst;        // instance records in use

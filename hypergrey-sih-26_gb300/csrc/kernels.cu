@@ -79,6 +79,14 @@ __device__ __forceinline__ double clip_bits(double v, double l, double u) {
     return bdouble(less_bits(lb, t) ? t : lb);
 }
 
+// a / d.b, correctly rounded (engine.cuh: KnownDivisor)
+__device__ __forceinline__ double divide_known(double a, const KnownDivisor& d) {
+    const int e = static_cast<int>(dbits(a) >> 52) & 0x7ff;
+    if (static_cast<unsigned>(e - kDivLow) >= static_cast<unsigned>(d.span)) return __ddiv_rn(a, d.b);
+    const double q = __fma_rn(a, d.hi, __dmul_rn(a, d.lo));
+    return __fma_rn(__fma_rn(-q, d.b, a), d.hi, q);
+}
+
 struct Acc {
     double obj, bnd, sep, a;
     unsigned long long stat, prim, b;
@@ -1126,7 +1134,8 @@ struct SliceStep {
     const double* c;
     const double* l;
     const double* u;
-    double beta, scale;
+    double beta;
+    KnownDivisor L;  // the exact engine divides by L, the plain one multiplies by L.hi
     int n;
     bool due;
 };
@@ -1148,7 +1157,12 @@ __device__ __forceinline__ SliceStep slice_step(const InstDev& I, int j0) {
     S.l = I.l;
     S.u = I.u;
     S.beta = S.due ? I.beta[it - I.it0] : 0.0;
-    S.scale = PREC == PREC_FP64_EXACT ? I.L : I.invL;
+    S.L.hi = I.invL;
+    if (PREC == PREC_FP64_EXACT) {
+        S.L.b = I.L;
+        S.L.lo = I.invL_lo;
+        S.L.span = I.div_span;
+    }
     S.n = I.n;
     return S;
 }
@@ -1206,10 +1220,10 @@ __global__ void __launch_bounds__(kSliceThreads, BLOCKS) step_slice_kernel(View 
             // clamping runs on the bit patterns)
             double nx;
             if constexpr (kExact) {
-                nx = clip_bits(__dsub_rn(wi, __ddiv_rn(__dadd_rn(acc, ci), S.scale)), lo, up);
+                nx = clip_bits(__dsub_rn(wi, divide_known(__dadd_rn(acc, ci), S.L)), lo, up);
                 S.wout[p] = __dadd_rn(nx, __dmul_rn(S.beta, __dsub_rn(nx, xo)));
             } else {
-                nx = clip_bits(wi - acc * S.scale, lo, up);
+                nx = clip_bits(wi - acc * S.L.hi, lo, up);
                 S.wout[p] = nx + S.beta * (nx - xo);
             }
             S.x[p] = nx;
@@ -2359,6 +2373,8 @@ __global__ void __launch_bounds__(kBlock) rearm_kernel(View v, const InstDev* __
             if (I.lip_device) {
                 I.L = *I.lprec;
                 I.invL = 1.0 / I.L;
+                I.invL_lo = __ddiv_rn(__fma_rn(-I.invL, I.L, 1.0), I.L);
+                I.div_span = I.L >= 0x1p-100 && I.L <= 0x1p100 ? kDivSpan : 0;
                 I.invLf = static_cast<float>(I.invL);
             }
             start_instance(v, I);
@@ -2594,12 +2610,13 @@ __global__ void __launch_bounds__(kSliceWindow) slice_order_kernel(InstDev I, in
         const_cast<uint8_t*>(I.slice_len)[w0 + t] = len_at[t];
         const_cast<uint8_t*>(I.slice_row)[w0 + t] = row_at[t];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) vec[k] = arrays[k][r];
+        for (int k = 0; k < 4; ++k) vec[k] = arrays[k] ? arrays[k][r] : 0.0;
     }
     __syncthreads();  // every value of the window is read before its place is written
     if (valid) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) arrays[k][w0 + t] = vec[k];
+        for (int k = 0; k < 4; ++k)
+            if (arrays[k]) arrays[k][w0 + t] = vec[k];
     }
     int base = __ldg(rowptr + w0);
     for (int w = 0; w < warp; ++w) base += warp_total[w];
@@ -2986,23 +3003,47 @@ __global__ void __launch_bounds__(kBlock) check_standalone_kernel(CheckSrc s, in
 }
 
 // ---- plugin-level FISTA step --------------------------------------------------------------------
-__global__ void __launch_bounds__(kBlock) box_step_kernel(int n, const int32_t* __restrict__ rowptr,
-                                                          const int32_t* __restrict__ col,
-                                                          const double* __restrict__ val,
-                                                          const double* __restrict__ c,
-                                                          const double* __restrict__ l,
-                                                          const double* __restrict__ u, double L, double beta,
-                                                          double* __restrict__ x, const double* __restrict__ w_in,
-                                                          double* __restrict__ w_out) {
+__global__ void __launch_bounds__(kBlock) box_step_kernel(BoxStep b, double beta, double* __restrict__ x,
+                                                          const double* __restrict__ w_in, double* __restrict__ w_out) {
+    const int n = static_cast<int>(b.n);
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
         double acc = 0.0;
-        const int ks = __ldg(rowptr + r), ke = __ldg(rowptr + r + 1);
-        for (int k = ks; k < ke; ++k) acc = __dadd_rn(acc, __dmul_rn(__ldg(val + k), __ldg(w_in + __ldg(col + k))));
-        const double v = __dsub_rn(__ldg(w_in + r), __ddiv_rn(__dadd_rn(acc, __ldg(c + r)), L));
-        const double nx = smax(__ldg(l + r), smin(__ldg(u + r), v));
+        const int ks = __ldg(b.rowptr + r), ke = __ldg(b.rowptr + r + 1);
+        for (int k = ks; k < ke; ++k) acc = __dadd_rn(acc, __dmul_rn(__ldg(b.val + k), __ldg(w_in + __ldg(b.col + k))));
+        const double v = __dsub_rn(__ldg(w_in + r), divide_known(__dadd_rn(acc, __ldg(b.c + r)), b.L));
+        const double nx = smax(__ldg(b.l + r), smin(__ldg(b.u + r), v));
         w_out[r] = __dadd_rn(nx, __dmul_rn(beta, __dsub_rn(nx, x[r])));
         x[r] = nx;
     }
+}
+
+// Over sliced rows, a slice per warp; the matrix, cost and bounds of the first columns are loaded
+// before the wait for the step before (programmatic dependent launch).  300k rows of 11 entries:
+// one thread per CSR row with the general division 45 us a step (uncoalesced rows, FP64 pipe).
+constexpr int kBoxAhead = 8;
+__global__ void __launch_bounds__(kSliceThreads, 6) box_step_slice_kernel(BoxStep b, double beta, double* x, const double* w_in,
+                                                                       double* w_out) {
+    let_next_launch_begin();
+    const int lane = threadIdx.x & 31, s = blockIdx.x * (kSliceThreads / 32) + static_cast<int>(threadIdx.x >> 5);
+    const int n = static_cast<int>(b.n), p = s * 32 + lane;
+    const bool valid = p < n;
+    const int len = valid ? __ldg(b.slice_len + p) : 0;
+    int k = (s * 32 < n ? __ldg(b.slice_base + s) : 0) + lane;
+    const double ci = valid ? __ldg(b.c + p) : 0.0, lo = valid ? __ldg(b.l + p) : 0.0, up = valid ? __ldg(b.u + p) : 0.0;
+    const int longest = __shfl_sync(0xffffffffu, len, 0);
+    SliceColumns<kBoxAhead> e;
+    e.load(b.col, b.val, len, k);
+    wait_for_previous_launch();
+    const double wi = valid ? w_in[p] : 0.0, xo = valid ? x[p] : 0.0;
+    double acc = e.add<true>(w_in, longest, 0.0);
+    for (int j = kBoxAhead; j < longest; j += kBoxAhead) {
+        e.load(b.col, b.val, len - j, k);
+        acc = e.add<true>(w_in, longest - j, acc);
+    }
+    if (!valid) return;
+    const double nx = clip_bits(__dsub_rn(wi, divide_known(__dadd_rn(acc, ci), b.L)), lo, up);
+    w_out[p] = __dadd_rn(nx, __dmul_rn(beta, __dsub_rn(nx, xo)));
+    x[p] = nx;
 }
 
 }  // namespace
@@ -3261,6 +3302,7 @@ void launch_slice_rows(const InstDev& rec, int64_t n, int64_t nnz, const int32_t
     const int64_t want = kSliceWindow * nnz / n * 6 / 5 + kSliceWindow;
     const int cap = static_cast<int>(want < 1024 ? 1024 : want > kSliceStageMax ? kSliceStageMax : (want + 1) & ~int64_t(1));
     const int windows = static_cast<int>((n + kSliceWindow - 1) / kSliceWindow), ni = static_cast<int>(n);
+    cudaFuncSetAttribute(slice_entries_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 12 * kSliceStageMax);
     slice_order_kernel<<<windows, kSliceWindow, 0, s>>>(rec, ni, rowptr, position_of);
     slice_entries_kernel<<<windows, kSliceWindow, 12 * cap, s>>>(rec, ni, rowptr, col, val, cap, position_of, col_out, val_out);
 }
@@ -3321,13 +3363,24 @@ cudaError_t load_check_standalone() {
     return cudaFuncGetAttributes(&attr, check_standalone_kernel);
 }
 
-void launch_box_step(int64_t n, const int32_t* rowptr, const int32_t* col, const double* val,
-                     const double* c, const double* l, const double* u, double L, double beta,
-                     double* x, const double* w_in, double* w_out, cudaStream_t s) {
-    int grid = static_cast<int>((n + kBlock - 1) / kBlock);
+void launch_box_step(const BoxStep& b, double beta, double* x, const double* w_in, double* w_out, cudaStream_t s) {
+    if (b.slice_len) {
+        cudaLaunchAttribute overlap;
+        overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        overlap.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t config = {};
+        config.gridDim = dim3(static_cast<unsigned>((b.n + kSliceThreads - 1) / kSliceThreads));
+        config.blockDim = dim3(kSliceThreads);
+        config.stream = s;
+        config.attrs = &overlap;
+        config.numAttrs = 1;
+        cudaLaunchKernelEx(&config, box_step_slice_kernel, b, beta, x, w_in, w_out);
+        return;
+    }
+    int grid = static_cast<int>((b.n + kBlock - 1) / kBlock);
     if (grid > 152 * 16) grid = 152 * 16;
     if (grid < 1) grid = 1;
-    box_step_kernel<<<grid, kBlock, 0, s>>>(static_cast<int>(n), rowptr, col, val, c, l, u, L, beta, x, w_in, w_out);
+    box_step_kernel<<<grid, kBlock, 0, s>>>(b, beta, x, w_in, w_out);
 }
 
 }  // namespace bqp

@@ -93,9 +93,21 @@ void launch_check_standalone(int64_t n, const int32_t* rowptr, const int32_t* co
 // its first launch would load it) and opts it into its shared-memory size.
 cudaError_t load_check_standalone();
 
-// Plugin-level FISTA step (reference numerics: FP64, division by L, no FMA), ping-pong w.
-void launch_box_step(int64_t n, const int32_t* rowptr, const int32_t* col, const double* val,
-                     const double* c, const double* l, const double* u, double L, double beta,
-                     double* x, const double* w_in, double* w_out, cudaStream_t s);
+// Plugin-level FISTA step (reference numerics: FP64, division by L, no FMA), ping-pong w.  The
+// problem over the uploaded CSR, or over sliced rows (slice_len set: every array in slice order,
+// the launches of one stream chained by programmatic dependent launch).
+struct BoxStep {
+    int64_t n;
+    const int32_t* rowptr;
+    const uint8_t* slice_len;
+    const int32_t* slice_base;
+    const int32_t* col;
+    const double* val;
+    const double* c;
+    const double* l;
+    const double* u;
+    KnownDivisor L;
+};
+void launch_box_step(const BoxStep& b, double beta, double* x, const double* w_in, double* w_out, cudaStream_t s);
 
 }  // namespace bqp
