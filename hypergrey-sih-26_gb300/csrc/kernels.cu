@@ -20,6 +20,7 @@
 // whatever its active lanes).
 #include "kernels.cuh"
 #include "fpbits.h"
+#include "slices.cuh"
 
 #include <atomic>
 #include <cmath>
@@ -505,62 +506,6 @@ __device__ __forceinline__ void tile_rows(int variant, const int32_t* __restrict
     case 32: subwarp_rows<32, T>(rowptr, rb, re, prod, add, zero, epi); break;
     default: warp_groups<T>(rowptr, rb, re, warp_buffer<T>(), prod, add, zero, epi); break;
     }
-}
-
-// ---- sliced rows (engine.cuh: VAR_SLICE) -------------------------------------------------------
-// One slice, one row per lane: the sum of the row's products in column order.  `len` is the lane's
-// row length (descending over the lanes), `base` the slice's first entry.  At column j the rows
-// still active are the first lanes, so the column's entries are base + the entries of the columns
-// before it + lane: the lane's address advances by the count of active lanes.  AHEAD columns
-// are loaded together (entries, then gathers) before the first product.
-// EXACT: products and sums rounded separately from 0.0, the reference loop's arithmetic.
-template <int AHEAD>
-struct SliceColumns {  // AHEAD columns of a slice: this lane's columns (-1: the row has ended) and values
-    int c[AHEAD];
-    double a[AHEAD];
-    __device__ __forceinline__ void load(const int32_t* __restrict__ col, const double* __restrict__ val, int left, int& k) {
-#pragma unroll
-        for (int q = 0; q < AHEAD; ++q) {
-            const bool in = q < left;
-            c[q] = in ? __ldg(col + k) : -1;
-            a[q] = in ? __ldg(val + k) : 0.0;
-            k += __popc(__ballot_sync(0xffffffffu, in));
-        }
-    }
-    // adds the first `columns` (warp-uniform) of them; a column past the slice's longest row costs
-    // no FP64 issue slot
-    template <bool EXACT>
-    __device__ __forceinline__ double add(const double* x, int columns, double acc) const {
-        double xv[AHEAD];
-#pragma unroll
-        for (int q = 0; q < AHEAD; ++q) xv[q] = c[q] >= 0 ? x[c[q]] : 0.0;
-        return sum<EXACT, 0>(xv, columns, acc);
-    }
-
-private:
-    template <bool EXACT, int Q>
-    __device__ __forceinline__ double sum(const double* xv, int columns, double acc) const {
-        if constexpr (Q < AHEAD) {
-            if (Q >= columns) return acc;
-            if (c[Q] >= 0) acc = EXACT ? __dadd_rn(acc, __dmul_rn(a[Q], xv[Q])) : fma(a[Q], xv[Q], acc);
-            return sum<EXACT, Q + 1>(xv, columns, acc);
-        } else {
-            return acc;
-        }
-    }
-};
-template <bool EXACT, int AHEAD>
-__device__ __forceinline__ double slice_dot(const int32_t* __restrict__ col, const double* __restrict__ val,
-                                            const double* x, int base, int len) {
-    const int longest = __shfl_sync(0xffffffffu, len, 0);
-    int k = base + (threadIdx.x & 31);
-    double acc = 0.0;
-    SliceColumns<AHEAD> e;
-    for (int j = 0; j < longest; j += AHEAD) {  // warp-uniform
-        e.load(col, val, len - j, k);
-        acc = e.template add<EXACT>(x, longest - j, acc);
-    }
-    return acc;
 }
 
 // FP32 "double-float" arithmetic: an unevaluated pair (hi, lo) carries ~46 significant bits.
@@ -1109,8 +1054,7 @@ __global__ void __launch_bounds__(kBlock) step_exact_kernel(View v, int j0) {
 //
 // The step launches of a body are chained by programmatic dependent launch: everything a step reads
 // but the iterates (the control fields, which only the kernels between bodies write, the matrix and
-// the bounds) is loaded before it waits for the step before it.  Every block waits, the idle
-// ones too, so that a launch that has ended implies that all launches before it have.
+// the bounds) is loaded before it waits for the step before it.
 //
 // Bounds: the FP64 pipe (16 cycles an SM per warp instruction: 3 + 3 a row on the tridiagonal family,
 // about 10 us for 1M rows, beside 80 MB from DRAM, 12 us) and the rate of random gathers (15M on the
@@ -1118,8 +1062,6 @@ __global__ void __launch_bounds__(kBlock) step_exact_kernel(View v, int j0) {
 // 1M rows 26.4 -> 14.6 us, random graph 15M entries 95 -> 72 us, 10k rows 12 -> 3.5 us (of which
 // the overlap of launches 0.6 ms over 400 steps).
 constexpr int kSliceThreads = kSlicePiece;
-__device__ __forceinline__ void wait_for_previous_launch() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void let_next_launch_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // What a step reads of an instance's record, kept in registers from one item to the next while the
 // instance stays the same.
@@ -2628,7 +2570,8 @@ __global__ void __launch_bounds__(kSliceWindow) slice_order_kernel(InstDev I, in
 // column, their columns as positions.  Each entry is read and written once (24 bytes) and its column's
 // position gathered (one byte): 154 us for 15M entries, once per solve.  A column out of range passes through unchanged: the gate refuses
 // that solve.
-__global__ void __launch_bounds__(kSliceWindow) slice_entries_kernel(InstDev I, int n, const int32_t* __restrict__ rowptr,
+__global__ void __launch_bounds__(kSliceWindow) slice_entries_kernel(InstDev I, int n, int columns,
+                                                                    const int32_t* __restrict__ rowptr,
                                                                     const int32_t* __restrict__ col,
                                                                     const double* __restrict__ val, int cap,
                                                                     const uint8_t* __restrict__ position_of,
@@ -2642,7 +2585,7 @@ __global__ void __launch_bounds__(kSliceWindow) slice_entries_kernel(InstDev I, 
     const int kb = __ldg(rowptr + w0), ke = __ldg(rowptr + w0 + rows);
     const bool staged = ke - kb <= cap;
     auto place = [&](int32_t c) {
-        return static_cast<uint32_t>(c) < static_cast<uint32_t>(n) ? (c & ~(kSliceWindow - 1)) | __ldg(position_of + c) : c;
+        return static_cast<uint32_t>(c) < static_cast<uint32_t>(columns) ? (c & ~(kSliceWindow - 1)) | __ldg(position_of + c) : c;
     };
     if (staged) {
 #pragma unroll 4
@@ -2665,6 +2608,12 @@ __global__ void __launch_bounds__(kSliceWindow) slice_entries_kernel(InstDev I, 
         }
         k += __popc(__ballot_sync(0xffffffffu, in));
     }
+}
+
+__global__ void __launch_bounds__(kBlock) slice_vector_kernel(int n, const uint8_t* __restrict__ slice_row,
+                                                              const double* __restrict__ x, double* __restrict__ out) {
+    for (int p = blockIdx.x * kBlock + threadIdx.x; p < n; p += gridDim.x * kBlock)
+        out[p] = x[(p & ~(kSliceWindow - 1)) + __ldg(slice_row + p)];
 }
 
 __global__ void __launch_bounds__(kBlock) unslice_kernel(int n, const uint8_t* __restrict__ slice_row,
@@ -3296,21 +3245,41 @@ void launch_gate_raw(int64_t n, const int32_t* rowptr, const int32_t* col, const
                                                                              diag, vhi, vlo);
 }
 
-void launch_slice_rows(const InstDev& rec, int64_t n, int64_t nnz, const int32_t* rowptr, const int32_t* col,
-                       const double* val, uint8_t* position_of, int32_t* col_out, double* val_out, cudaStream_t s) {
+void launch_slice_order(const InstDev& rec, int64_t n, const int32_t* rowptr, uint8_t* position_of, cudaStream_t s) {
+    const int windows = static_cast<int>((n + kSliceWindow - 1) / kSliceWindow);
+    slice_order_kernel<<<windows, kSliceWindow, 0, s>>>(rec, static_cast<int>(n), rowptr, position_of);
+}
+
+void launch_slice_entries(const InstDev& rec, int64_t n, int64_t columns, int64_t nnz, const int32_t* rowptr,
+                          const int32_t* col, const double* val, const uint8_t* position_of, int32_t* col_out,
+                          double* val_out, cudaStream_t s) {
     // shared memory for a window of average rows and a fifth more
     const int64_t want = kSliceWindow * nnz / n * 6 / 5 + kSliceWindow;
     const int cap = static_cast<int>(want < 1024 ? 1024 : want > kSliceStageMax ? kSliceStageMax : (want + 1) & ~int64_t(1));
-    const int windows = static_cast<int>((n + kSliceWindow - 1) / kSliceWindow), ni = static_cast<int>(n);
+    const int windows = static_cast<int>((n + kSliceWindow - 1) / kSliceWindow);
     cudaFuncSetAttribute(slice_entries_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 12 * kSliceStageMax);
-    slice_order_kernel<<<windows, kSliceWindow, 0, s>>>(rec, ni, rowptr, position_of);
-    slice_entries_kernel<<<windows, kSliceWindow, 12 * cap, s>>>(rec, ni, rowptr, col, val, cap, position_of, col_out, val_out);
+    slice_entries_kernel<<<windows, kSliceWindow, 12 * cap, s>>>(rec, static_cast<int>(n), static_cast<int>(columns), rowptr, col,
+                                                               val, cap, position_of, col_out, val_out);
+}
+
+void launch_slice_rows(const InstDev& rec, int64_t n, int64_t nnz, const int32_t* rowptr, const int32_t* col,
+                       const double* val, uint8_t* position_of, int32_t* col_out, double* val_out, cudaStream_t s) {
+    launch_slice_order(rec, n, rowptr, position_of, s);
+    launch_slice_entries(rec, n, n, nnz, rowptr, col, val, position_of, col_out, val_out, s);
 }
 
 void launch_unslice(int64_t n, const uint8_t* slice_row, const double* x, double* out, cudaStream_t s) {
+    if (n <= 0) return;
     int64_t grid = (n + kBlock - 1) / kBlock;
     if (grid > 152 * 8) grid = 152 * 8;
     unslice_kernel<<<static_cast<int>(grid), kBlock, 0, s>>>(static_cast<int>(n), slice_row, x, out);
+}
+
+void launch_slice_vector(int64_t n, const uint8_t* slice_row, const double* x, double* out, cudaStream_t s) {
+    if (n <= 0) return;
+    int64_t grid = (n + kBlock - 1) / kBlock;
+    if (grid > 152 * 8) grid = 152 * 8;
+    slice_vector_kernel<<<static_cast<int>(grid), kBlock, 0, s>>>(static_cast<int>(n), slice_row, x, out);
 }
 
 void launch_gate(const InstDev& rec, int64_t n, const double* val, cudaStream_t s) {

@@ -55,6 +55,14 @@ void launch_gate(const InstDev& rec, int64_t n, const double* val, cudaStream_t 
 // bytes of scratch.
 void launch_slice_rows(const InstDev& rec, int64_t n, int64_t nnz, const int32_t* rowptr, const int32_t* col,
                        const double* val, uint8_t* position_of, int32_t* col_out, double* val_out, cudaStream_t s);
+// The two steps by themselves: the order of `n` rows (rec's vectors may be null), and their entries, whose
+// columns (below `columns`) are mapped by position_of.
+void launch_slice_order(const InstDev& rec, int64_t n, const int32_t* rowptr, uint8_t* position_of, cudaStream_t s);
+void launch_slice_entries(const InstDev& rec, int64_t n, int64_t columns, int64_t nnz, const int32_t* rowptr,
+                          const int32_t* col, const double* val, const uint8_t* position_of, int32_t* col_out,
+                          double* val_out, cudaStream_t s);
+// A vector brought into slice order: out[position] = x[row].
+void launch_slice_vector(int64_t n, const uint8_t* slice_row, const double* x, double* out, cudaStream_t s);
 // x of a sliced instance in row order: out[row] = x[position].
 void launch_unslice(int64_t n, const uint8_t* slice_row, const double* x, double* out, cudaStream_t s);
 // The same pass on raw device pointers (diag, vhi, vlo may be null: not stored).
