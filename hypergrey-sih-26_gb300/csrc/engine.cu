@@ -474,14 +474,17 @@ private:
     bool upload_finish(Job& j, std::string& why);
     void fail_admission(Job* j, size_t reserved, const std::string& why);  // caller holds mu_
     void finish_paused_upload(std::unique_lock<std::mutex>& lk);
+    // host callback behind a launch that the engine thread no longer polls (kPollSeconds)
     static void CUDART_CB on_launch_done(void* self) {
         Engine* e = static_cast<Engine*>(self);
-        {
-            std::lock_guard<std::mutex> g(e->mu_);
-            e->launch_done_ = true;
-            e->t_launch_done_ = host_seconds();
-        }
+        std::lock_guard<std::mutex> g(e->mu_);
+        e->launch_done_.store(true);
         e->cv_work_.notify_all();
+    }
+    // whether the current launch has ended (engine thread)
+    bool launch_ended() {
+        if (!launch_done_.load() && cudaEventQuery(done_ev_) == cudaSuccess) launch_done_.store(true);
+        return launch_done_.load();
     }
     // a new solve at the head of the queue that fits under the cap (caller holds mu_)
     bool uploadable_head() const {
@@ -499,6 +502,7 @@ private:
     bool run_stream(int cap, std::string& why);
     void update_grid();
     bool select_graph(std::string& why);
+    bool queue_collection(const std::vector<Job*>& jobs, std::string& why);
     void collect(std::unique_lock<std::mutex>& lk);
     void process_frees();
     std::vector<Job*> running_jobs() const;
@@ -561,7 +565,6 @@ private:
         v.partial = d_partial_;
         v.tile_done = d_tile_done_;
         v.ctrl = d_ctrl_;
-        v.status_mirror = d_status_;
         v.ranges = d_ranges_;
         v.group_tiles = d_group_tiles_;
         v.units = d_units_;
@@ -596,8 +599,21 @@ private:
     // during the next launch, so a stream of large solves overlaps each upload with the
     // previous solve instead of idling the device for the whole queue's copies.
     static constexpr size_t kSyncUploadBudget = size_t(64) << 20;
-    bool launch_done_ = true;          // the host callback behind the current launch has run (mu_)
-    double t_launch_done_ = 0;         // host time of that callback (BOXQP_PROFILE: gap to the next launch)
+    // The engine thread polls a launch for its first kPollSeconds (waking through a host callback costs
+    // tens of microseconds, a tenth of a small solve), then waits for the callback; uploads that
+    // arrive meanwhile are seen either way (arrivals_).
+    static constexpr double kPollSeconds = 4e-3;
+    std::atomic<bool> launch_done_{true};
+    std::atomic<uint64_t> arrivals_{0};  // submissions so far
+    cudaEvent_t done_ev_ = nullptr;      // end of the current launch and its collection
+    double t_launch_done_ = 0;           // host time at which that was seen (BOXQP_PROFILE: gap to the next launch)
+    // collection of finished solves (page-locked): jobs, spans, records, primals; rewritten per launch
+    unsigned char* h_collect_ = nullptr;
+    size_t collect_bytes_ = 0;
+    static constexpr size_t kCollectMax = size_t(64) << 20;  // primals beyond this are copied one by one
+    std::vector<CollectJob> collect_jobs_;                   // the current launch's, as the kernel reads them
+    bool pageable_access_ = false;       // the device reads pageable host memory
+    static constexpr size_t kUploadKernelBytes = size_t(2) << 20;
     // BOXQP_PROFILE: host times of the steps between two launches (engine thread)
     double t_synced_ = 0, t_collected_ = 0, t_freed_ = 0, t_gated_ = 0, t_installed_ = 0;
     cudaMemPool_t pool_ = nullptr;
@@ -606,7 +622,6 @@ private:
     InstDev* d_inst_ = nullptr;
     int2* d_ranges_ = nullptr;
     int32_t* d_tile_done_ = nullptr;
-    int32_t* d_status_ = nullptr;
     Tile* d_tiles_ = nullptr;
     Partial* d_partial_ = nullptr;
     Ctrl* d_ctrl_ = nullptr;
@@ -614,13 +629,10 @@ private:
     Ctrl* h_ctrl_ = nullptr;       // pinned
     int32_t* h_status_ = nullptr;  // pinned
     int inst_cap_ = 0, tile_cap_ = 0;
-    // re-arm staging (pinned host / device): records, slots, row spans
+    // re-arm staging (page-locked, read by the kernel from there): records, slots, row spans
     InstDev* h_stage_ = nullptr;
-    InstDev* d_stage_ = nullptr;
     int32_t* h_stage_slots_ = nullptr;
-    int32_t* d_stage_slots_ = nullptr;
     int2* h_spans_ = nullptr;
-    int2* d_spans_ = nullptr;
     int stage_cap_ = 0, span_cap_ = 0;
 
     // host mirrors
@@ -724,6 +736,10 @@ bool Engine::init(std::string& why) {
     if (!cuda_ok(cudaStreamCreateWithPriority(&ustream_, cudaStreamNonBlocking, prio_least), why, "stream")) return false;
     if (!cuda_ok(cudaStreamCreateWithFlags(&fstream_, cudaStreamNonBlocking), why, "stream")) return false;
     if (!cuda_ok(cudaEventCreateWithFlags(&uev_, cudaEventDisableTiming), why, "event")) return false;
+    if (!cuda_ok(cudaEventCreateWithFlags(&done_ev_, cudaEventDisableTiming), why, "event")) return false;
+    int pageable = 0;
+    cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, device_);
+    pageable_access_ = pageable != 0;
     cudaMemPoolProps props;
     std::memset(&props, 0, sizeof(props));
     props.allocType = cudaMemAllocationTypePinned;
@@ -787,9 +803,9 @@ void Engine::shutdown() {
     }
     jobs_.clear();
     drop_graphs();
-    cudaFree(d_inst_); cudaFree(d_ranges_); cudaFree(d_tile_done_); cudaFree(d_status_);
+    cudaFree(d_inst_); cudaFree(d_ranges_); cudaFree(d_tile_done_);
     cudaFree(d_tiles_); cudaFree(d_partial_); cudaFree(d_ctrl_); cudaFree(d_momentum_); cudaFree(d_group_tiles_); cudaFree(d_units_);
-    d_inst_ = nullptr; d_ranges_ = nullptr; d_tile_done_ = nullptr; d_status_ = nullptr;
+    d_inst_ = nullptr; d_ranges_ = nullptr; d_tile_done_ = nullptr;
     d_tiles_ = nullptr; d_partial_ = nullptr; d_ctrl_ = nullptr; d_momentum_ = nullptr; d_group_tiles_ = nullptr; d_units_ = nullptr;
     if (h_ctrl_) cudaFreeHost(h_ctrl_);
     if (h_stage_) cudaFreeHost(h_stage_);
@@ -801,11 +817,10 @@ void Engine::shutdown() {
     for (GateResult* c : gate_chunks_) cudaFreeHost(c);
     gate_chunks_.clear();
     gate_free_.clear();
-    cudaFree(d_stage_);
-    cudaFree(d_stage_slots_);
-    cudaFree(d_spans_);
     h_stage_ = nullptr; h_stage_slots_ = nullptr; h_spans_ = nullptr;
-    d_stage_ = nullptr; d_stage_slots_ = nullptr; d_spans_ = nullptr;
+    if (h_collect_) cudaFreeHost(h_collect_);
+    h_collect_ = nullptr;
+    collect_bytes_ = 0;
     if (h_status_) cudaFreeHost(h_status_);
     h_ctrl_ = nullptr;
     h_status_ = nullptr;
@@ -829,6 +844,8 @@ void Engine::shutdown() {
     if (ustream_) cudaStreamDestroy(ustream_);
     if (fstream_) cudaStreamDestroy(fstream_);
     if (uev_) cudaEventDestroy(uev_);
+    if (done_ev_) cudaEventDestroy(done_ev_);
+    done_ev_ = nullptr;
     stream_ = nullptr;
     capture_ = nullptr;
     ustream_ = nullptr;
@@ -842,24 +859,22 @@ bool Engine::ensure_tables(int need_inst, int need_tiles, std::string& why) {
         int cap = std::max(need_inst, std::max(256, inst_cap_ * 2));
         InstDev* inst = nullptr;
         int2* ranges = nullptr;
-        int32_t *done = nullptr, *status = nullptr, *h_status = nullptr;
+        int32_t *done = nullptr, *h_status = nullptr;
         if (!cuda_ok(cudaMalloc(&inst, sizeof(InstDev) * cap), why, "instance table")) return false;
         if (!cuda_ok(cudaMalloc(&ranges, sizeof(int2) * cap), why, "range table")) return false;
         if (!cuda_ok(cudaMalloc(&done, sizeof(int32_t) * cap), why, "tile counters")) return false;
-        if (!cuda_ok(cudaMalloc(&status, sizeof(int32_t) * cap), why, "status mirror")) return false;
         if (!cuda_ok(cudaMallocHost(&h_status, sizeof(int32_t) * cap), why, "pinned status")) return false;
         cudaMemsetAsync(inst, 0, sizeof(InstDev) * cap, stream_);
         cudaMemsetAsync(ranges, 0, sizeof(int2) * cap, stream_);
         cudaMemsetAsync(done, 0, sizeof(int32_t) * cap, stream_);
-        cudaMemsetAsync(status, 0xff, sizeof(int32_t) * cap, stream_);
         if (d_inst_) {
             cudaMemcpyAsync(inst, d_inst_, sizeof(InstDev) * inst_cap_, cudaMemcpyDeviceToDevice, stream_);
             cudaMemcpyAsync(done, d_tile_done_, sizeof(int32_t) * inst_cap_, cudaMemcpyDeviceToDevice, stream_);
         }
         cudaStreamSynchronize(stream_);
-        cudaFree(d_inst_); cudaFree(d_ranges_); cudaFree(d_tile_done_); cudaFree(d_status_);
+        cudaFree(d_inst_); cudaFree(d_ranges_); cudaFree(d_tile_done_);
         if (h_status_) cudaFreeHost(h_status_);
-        d_inst_ = inst; d_ranges_ = ranges; d_tile_done_ = done; d_status_ = status; h_status_ = h_status;
+        d_inst_ = inst; d_ranges_ = ranges; d_tile_done_ = done; h_status_ = h_status;
         inst_cap_ = cap;
         h_ranges_.resize(cap, int2{0, 0});
         slot_job_.resize(cap, nullptr);
@@ -1102,6 +1117,7 @@ int Engine::submit(Job* raw, uint64_t* id) {
     }
     if (!done) {
         queue_.push_back(j);
+        arrivals_.fetch_add(1);
         cv_work_.notify_all();
     }
     return BQP_OK;
@@ -1296,8 +1312,8 @@ void Engine::reset_record(Job& j) {
     R.moved[1] = 0;
 }
 
-// Re-arms resident solves (bqp_resolve): one upload of the staged records and one kernel for the
-// whole batch.  Engine thread only.
+// Re-arms resident solves (bqp_resolve): one kernel for the whole batch, which reads the staged
+// records from page-locked memory.  Engine thread only.
 bool Engine::rearm(const std::vector<Job*>& batch, std::string& why) {
     // the staging buffers are reused (or reallocated): the previous re-arm must have completed
     // (in steady state it has, long before)
@@ -1309,24 +1325,18 @@ bool Engine::rearm(const std::vector<Job*>& batch, std::string& why) {
         const int cap = std::max(count, std::max(256, 2 * stage_cap_));
         if (h_stage_) cudaFreeHost(h_stage_);
         if (h_stage_slots_) cudaFreeHost(h_stage_slots_);
-        cudaFree(d_stage_);
-        cudaFree(d_stage_slots_);
-        h_stage_ = nullptr; h_stage_slots_ = nullptr; d_stage_ = nullptr; d_stage_slots_ = nullptr;
+        h_stage_ = nullptr; h_stage_slots_ = nullptr;
         stage_cap_ = 0;
         if (!cuda_ok(cudaMallocHost(&h_stage_, sizeof(InstDev) * cap), why, "re-arm staging")) return false;
         if (!cuda_ok(cudaMallocHost(&h_stage_slots_, sizeof(int32_t) * cap), why, "re-arm staging")) return false;
-        if (!cuda_ok(cudaMalloc(&d_stage_, sizeof(InstDev) * cap), why, "re-arm staging")) return false;
-        if (!cuda_ok(cudaMalloc(&d_stage_slots_, sizeof(int32_t) * cap), why, "re-arm staging")) return false;
         stage_cap_ = cap;
     }
     if (spans > span_cap_) {
         const int cap = std::max(spans, std::max(256, 2 * span_cap_));
         if (h_spans_) cudaFreeHost(h_spans_);
-        cudaFree(d_spans_);
-        h_spans_ = nullptr; d_spans_ = nullptr;
+        h_spans_ = nullptr;
         span_cap_ = 0;
         if (!cuda_ok(cudaMallocHost(&h_spans_, sizeof(int2) * cap), why, "re-arm staging")) return false;
-        if (!cuda_ok(cudaMalloc(&d_spans_, sizeof(int2) * cap), why, "re-arm staging")) return false;
         span_cap_ = cap;
     }
     int s = 0;
@@ -1338,10 +1348,7 @@ bool Engine::rearm(const std::vector<Job*>& batch, std::string& why) {
         for (int64_t r = 0; r < j.n; r += kRearmRows) h_spans_[s++] = int2{k, static_cast<int>(r)};
     }
     cudaEventRecord(rev0_, stream_);
-    cudaMemcpyAsync(d_stage_, h_stage_, sizeof(InstDev) * count, cudaMemcpyHostToDevice, stream_);
-    cudaMemcpyAsync(d_stage_slots_, h_stage_slots_, sizeof(int32_t) * count, cudaMemcpyHostToDevice, stream_);
-    cudaMemcpyAsync(d_spans_, h_spans_, sizeof(int2) * spans, cudaMemcpyHostToDevice, stream_);
-    launch_rearm(view(), d_stage_, d_stage_slots_, d_spans_, spans, stream_);
+    launch_rearm(view(), h_stage_, h_stage_slots_, h_spans_, spans, stream_);
     cudaEventRecord(rev1_, stream_);
     if (!cuda_ok(cudaGetLastError(), why, "re-arm kernel")) return false;
     rearm_pending_ = true;  // the next launch on stream_ runs after it
@@ -1547,8 +1554,25 @@ bool Engine::upload_begin(Job& j, std::string& why) {
     return true;
 }
 
-// Issues copies of up to `budget` bytes; true once every copy of the solve is issued.
+// Issues copies of up to `budget` bytes; true once every copy of the solve is issued.  A small solve's
+// arrays go in one launch that reads them where they are (six copies of pageable memory take the
+// engine thread longer than the data does).
 bool Engine::upload_copy(Job& j, size_t budget) {
+    if (j.piece == 0 && j.piece_off == 0 && pageable_access_ && j.pieces.size() <= UploadPieces::kMost) {
+        size_t bytes = 0;
+        UploadPieces p;
+        for (const Job::Piece& q : j.pieces) {
+            bytes += q.bytes;
+            p.src[p.count] = static_cast<const uint32_t*>(q.src);
+            p.dst[p.count] = static_cast<uint32_t*>(q.dst);
+            p.words[p.count++] = static_cast<uint32_t>(q.bytes / 4);
+        }
+        if (bytes <= kUploadKernelBytes) {
+            launch_upload(p, ustream_);
+            j.piece = j.pieces.size();
+            return true;
+        }
+    }
     while (j.piece < j.pieces.size() && budget > 0) {
         const Job::Piece& p = j.pieces[j.piece];
         const size_t take = std::min(budget, p.bytes - j.piece_off);
@@ -1644,7 +1668,7 @@ bool Engine::install(std::vector<Job*>& jobs, std::string& why) {
 // so that the next launch is not held up by the host staging of a large solve.
 void Engine::upload_waiting() {
     std::unique_lock<std::mutex> lk(mu_);
-    while (!stop_ && !launch_done_) {
+    while (!stop_ && !launch_ended()) {
         Job* j = uploading_;
         if (!j) {
             if (queue_.empty()) break;
@@ -1923,21 +1947,27 @@ bool Engine::run_once(std::string& why) {
                      since(t_gated_), since(t_installed_));
     }
     cudaEventRecord(ev1_, stream_);
-    cudaMemcpyAsync(h_status_, d_status_, sizeof(int32_t) * std::max(n_inst_, 1), cudaMemcpyDeviceToHost, stream_);
-    cudaMemcpyAsync(h_ctrl_, d_ctrl_, sizeof(Ctrl), cudaMemcpyDeviceToHost, stream_);
+    if (!queue_collection(jobs, why)) return false;
     // while the device runs the launch, upload the new solves that arrive (they are installed
-    // before the next launch); a host callback behind the launch ends the wait
-    {
-        std::lock_guard<std::mutex> g(mu_);
-        launch_done_ = false;
-    }
-    if (!cuda_ok(cudaLaunchHostFunc(stream_, &Engine::on_launch_done, this), why, "launch callback")) return false;
-    for (;;) {
+    // before the next launch)
+    launch_done_.store(false);
+    if (!cuda_ok(cudaEventRecord(done_ev_, stream_), why, "launch end")) return false;
+    const double poll_until = host_seconds() + kPollSeconds;
+    for (bool called_back = false;;) {
+        const uint64_t seen = arrivals_.load();
         upload_waiting();
+        if (!called_back) {
+            while (!launch_ended() && arrivals_.load() == seen && host_seconds() < poll_until) std::this_thread::yield();
+            if (launch_ended()) break;
+            if (arrivals_.load() != seen || host_seconds() < poll_until) continue;
+            called_back = true;
+            if (!cuda_ok(cudaLaunchHostFunc(stream_, &Engine::on_launch_done, this), why, "launch callback")) return false;
+        }
         std::unique_lock<std::mutex> lk(mu_);
-        cv_work_.wait(lk, [&] { return launch_done_ || stop_ || uploadable_head(); });
-        if (launch_done_ || stop_) break;
+        cv_work_.wait(lk, [&] { return launch_done_.load() || stop_ || uploadable_head(); });
+        if (launch_done_.load() || stop_) break;
     }
+    if (host_profile()) t_launch_done_ = host_seconds();
     if (!cuda_ok(cudaStreamSynchronize(stream_), why, "engine launch")) return false;
     if (host_profile()) t_synced_ = host_seconds();
     if (!settle_rearm(why)) return false;  // completed before the launch: no wait
@@ -1954,57 +1984,100 @@ bool Engine::run_once(std::string& why) {
     return true;
 }
 
-// Moves finished solves to the done state: copies their records and primals back.
+// Queues the collection behind a launch of `jobs`: one kernel writes each finished solve's status,
+// record and primal (in row order) to page-locked memory, so that collect() needs no copies of its
+// own.  A primal of more than kHostPrimal variables stays on the device until bqp_fetch copies it
+// straight to the caller's array, off the engine thread (a sliced one is brought into row order in
+// the momentum buffer, which the next run starts from anew).
+bool Engine::queue_collection(const std::vector<Job*>& jobs, std::string& why) {
+    collect_jobs_.clear();
+    size_t spans = 0, primals = 0;
+    for (const Job* j : jobs) {
+        CollectJob c{};
+        c.slot = j->slot;
+        const size_t bytes = sizeof(double) * static_cast<size_t>(j->n);
+        if (j->n > kHostPrimal) {
+            if (is_sliced(j->variant)) {
+                c.n = static_cast<int32_t>(j->n);
+                c.x = j->rec.w64[0];
+            }
+        } else if (primals + bytes <= kCollectMax) {
+            c.n = static_cast<int32_t>(j->n);
+            primals += bytes;
+        }
+        spans += static_cast<size_t>(std::max(1, (c.n + kCollectRows - 1) / kCollectRows));
+        collect_jobs_.push_back(c);
+    }
+    const size_t count = jobs.size();
+    const size_t o_spans = align_up(sizeof(CollectJob) * count), o_records = o_spans + align_up(sizeof(int2) * spans);
+    const size_t o_x = o_records + align_up(sizeof(InstDev) * count), need = o_x + primals;
+    if (need > collect_bytes_) {
+        const size_t cap = std::max(need, 2 * collect_bytes_);
+        if (h_collect_) cudaFreeHost(h_collect_);
+        h_collect_ = nullptr;
+        collect_bytes_ = 0;
+        if (!cuda_ok(cudaMallocHost(&h_collect_, cap), why, "collection staging")) return false;
+        collect_bytes_ = cap;
+    }
+    int2* sp = reinterpret_cast<int2*>(h_collect_ + o_spans);
+    double* x = reinterpret_cast<double*>(h_collect_ + o_x);
+    for (size_t k = 0; k < count; ++k) {
+        CollectJob& c = collect_jobs_[k];
+        c.record = reinterpret_cast<InstDev*>(h_collect_ + o_records) + k;
+        if (c.n > 0 && !c.x) {
+            c.x = x;
+            x += c.n;
+        }
+        for (int r = 0; r == 0 || r < c.n; r += kCollectRows) *sp++ = int2{static_cast<int>(k), r};
+    }
+    if (count) std::memcpy(h_collect_, collect_jobs_.data(), sizeof(CollectJob) * count);
+    launch_collect(view(), reinterpret_cast<const CollectJob*>(h_collect_), reinterpret_cast<const int2*>(h_collect_ + o_spans),
+                   static_cast<int>(spans), h_status_, h_ctrl_, stream_);
+    return cuda_ok(cudaGetLastError(), why, "collect kernel");
+}
+
+// Moves finished solves to the done state, their records and primals as the collection wrote them.
 void Engine::collect(std::unique_lock<std::mutex>& lk) {
     std::vector<Job*> finished;
-    for (int s = 0; s < n_inst_; ++s) {
-        Job* j = slot_job_[s];
-        if (j && j->state == JOB_RUNNING && h_status_[s] != ST_RUNNING) finished.push_back(j);
+    std::vector<const CollectJob*> from;
+    for (const CollectJob& c : collect_jobs_) {
+        Job* j = slot_job_[c.slot];
+        if (j && j->state == JOB_RUNNING && h_status_[c.slot] != ST_RUNNING) {
+            finished.push_back(j);
+            from.push_back(&c);
+        }
     }
     if (finished.empty()) return;
     lk.unlock();
-    std::vector<InstDev> recs(finished.size());
-    for (size_t k = 0; k < finished.size(); ++k)
-        cudaMemcpyAsync(&recs[k], &d_inst_[finished[k]->slot], sizeof(InstDev), cudaMemcpyDeviceToHost, stream_);
-    cudaStreamSynchronize(stream_);
-    // Primals of up to kHostPrimal variables come back now, all behind one synchronisation; a
-    // larger one stays in the slab (final, untouched until release or re-run) and bqp_fetch
-    // copies it straight to the caller's array, off the engine thread.
-    std::vector<std::vector<float>> x32(finished.size());
-    bool small = false, unsliced = false;
     for (size_t k = 0; k < finished.size(); ++k) {
         Job& j = *finished[k];
-        const InstDev& R = recs[k];
-        j.x_f32 = R.result_src == 1;
-        j.x_dev = R.result_src == 1 ? static_cast<const void*>(R.x32)
-                                    : static_cast<const void*>(R.result_src == 2 ? R.xp : R.x64);
-        if (is_sliced(j.variant)) {  // back into row order, in the momentum buffer the next run starts from anew
-            launch_unslice(j.n, R.slice_row, R.x64, R.w64[0], stream_);
-            j.x_dev = R.w64[0];
-            unsliced = true;
+        const CollectJob& c = *from[k];
+        const InstDev& R = *c.record;
+        j.x_f32 = false;
+        j.x_dev = nullptr;
+        if (j.n <= kHostPrimal && c.n > 0) {
+            j.x.resize(static_cast<size_t>(j.n));
+            std::memcpy(j.x.data(), c.x, sizeof(double) * static_cast<size_t>(j.n));
+            continue;
         }
         j.x.clear();
-        if (j.n > kHostPrimal) continue;
-        small = true;
-        j.x.resize(static_cast<size_t>(j.n));
-        void* dst = j.x.data();
-        if (j.x_f32) {
-            x32[k].resize(static_cast<size_t>(j.n));
-            dst = x32[k].data();
+        if (c.n > 0) {
+            j.x_dev = c.x;  // row order
+        } else {
+            j.x_f32 = R.result_src == 1;
+            j.x_dev = R.result_src == 1 ? static_cast<const void*>(R.x32)
+                                        : static_cast<const void*>(R.result_src == 2 ? R.xp : R.x64);
+            if (is_sliced(j.variant)) {
+                launch_unslice(j.n, R.slice_row, R.x64, R.w64[0], stream_);
+                j.x_dev = R.w64[0];
+                cudaStreamSynchronize(stream_);
+            }
         }
-        cudaMemcpyAsync(dst, j.x_dev, (j.x_f32 ? 4 : 8) * static_cast<size_t>(j.n), cudaMemcpyDeviceToHost, stream_);
     }
-    // (bqp_fetch copies the larger ones on another stream)
-    if (small || unsliced) cudaStreamSynchronize(stream_);
     const double now = host_seconds();
     for (size_t k = 0; k < finished.size(); ++k) {
         Job& j = *finished[k];
-        const InstDev& R = recs[k];
-        if (!j.x.empty()) {
-            if (j.x_f32)
-                for (int64_t i = 0; i < j.n; ++i) j.x[i] = static_cast<double>(x32[k][i]);
-            j.x_dev = nullptr;
-        }
+        const InstDev& R = *from[k]->record;
         bqp_stats& s = j.stats;
         s.status = status_code(R.status);
         s.verified = R.verified;

@@ -288,6 +288,15 @@ struct Ctrl {
     int32_t step_due[3];   // per precision: step launches of this body with work (later ones return at once)
 };
 
+// What the collect kernel hands out of one solve when a launch has ended (CollectSpan: its blocks).
+struct CollectJob {
+    int32_t slot;
+    int32_t n;          // rows of the primal to write (0: the record alone)
+    InstDev* record;    // page-locked
+    double* x;          // page-locked, or device memory for a primal that bqp_fetch will copy
+};
+constexpr int kCollectRows = 1024;  // rows per block, whole slice windows
+
 // Everything a tile kernel needs, passed by value.
 struct View {
     InstDev* inst;
@@ -295,7 +304,6 @@ struct View {
     Partial* partial;
     int32_t* tile_done;    // per-instance count of finished tiles (check / CG reductions)
     Ctrl* ctrl;
-    int32_t* status_mirror;  // per-instance status, rewritten by the control kernel every body
     const int2* ranges;      // per-instance tile range [x, y) in the tile table
     const Tile* group_tiles;     // the tiles (sliced instances: pieces of kSlicePiece rows) ordered by step group (Ctrl::group_begin)
     const double2* momentum;     // FISTA: beta_k and t_{k+1} for k < kMomentumTable (they depend on k alone)

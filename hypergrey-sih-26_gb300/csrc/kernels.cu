@@ -2120,7 +2120,7 @@ struct Counts {
 };
 
 // steps > 0: also the step launches with work per precision (a chunk needs it_next - it_cur more)
-__device__ Counts count_phases(const View& v, bool mirror, int steps = 0) {
+__device__ Counts count_phases(const View& v, int steps = 0) {
     __shared__ int s[11];
     if (threadIdx.x < 11) s[threadIdx.x] = 0;
     __syncthreads();
@@ -2129,7 +2129,6 @@ __device__ Counts count_phases(const View& v, bool mirror, int steps = 0) {
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         const InstDev& I = v.inst[i];
         const int st = I.status;
-        if (mirror) v.status_mirror[i] = st;
         if (st != ST_RUNNING) continue;
         nr++;
         const int pk = I.precision == PREC_MIXED ? 1 : I.precision == PREC_FP64_EXACT ? 2 : 0;
@@ -2196,7 +2195,7 @@ __device__ void advance_chunks(const View& v, int steps) {
 __global__ void gate_kernel(View v, cudaGraphConditionalHandle h_fp64, cudaGraphConditionalHandle h_mixed,
                             cudaGraphConditionalHandle h_exact, cudaGraphConditionalHandle h_polish,
                             cudaGraphConditionalHandle h_cg, StepLaunches steps, int body_steps) {
-    const Counts c = count_phases(v, false, body_steps);
+    const Counts c = count_phases(v, body_steps);
     if (threadIdx.x == 0) {
         for (int k = 0; k < 3; ++k) {
             v.ctrl->n_fista[k] = c.fista[k];
@@ -2219,7 +2218,7 @@ __global__ void gate_kernel(View v, cudaGraphConditionalHandle h_fp64, cudaGraph
 
 __global__ void control_kernel(View v, cudaGraphConditionalHandle loop_h, int steps) {
     advance_chunks(v, steps);
-    const Counts c = count_phases(v, true);
+    const Counts c = count_phases(v);
     if (threadIdx.x == 0) {
         for (int k = 0; k < 3; ++k) v.ctrl->check_due[k] = c.check_due[k];
         Ctrl* ctrl = v.ctrl;
@@ -2231,7 +2230,7 @@ __global__ void control_kernel(View v, cudaGraphConditionalHandle loop_h, int st
 }
 
 __global__ void gate_plain_kernel(View v, int steps) {
-    const Counts c = count_phases(v, false, steps);
+    const Counts c = count_phases(v, steps);
     if (threadIdx.x == 0) {
         for (int k = 0; k < 3; ++k) {
             v.ctrl->n_fista[k] = c.fista[k];
@@ -2245,7 +2244,7 @@ __global__ void gate_plain_kernel(View v, int steps) {
 
 __global__ void control_plain_kernel(View v, int steps) {
     advance_chunks(v, steps);
-    const Counts c = count_phases(v, true);
+    const Counts c = count_phases(v);
     if (threadIdx.x == 0) {
         for (int k = 0; k < 3; ++k) v.ctrl->check_due[k] = c.check_due[k];
         v.ctrl->bodies++;
@@ -2288,12 +2287,6 @@ __device__ void start_instance(const View& v, InstDev& I) {
         }
 }
 
-__global__ void init_instance_kernel(View v, int slot, int n) {
-    InstDev& I = v.inst[slot];
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) init_row(I, r);
-    if (blockIdx.x == 0 && threadIdx.x == 0) start_instance(v, I);
-}
-
 // Re-arms a list of resident solves in one launch.  Block b takes rows [span.y, span.y + kRearmRows)
 // of staged record span.x; the block holding row 0 also installs the record in its slot and
 // starts the solve.
@@ -2321,6 +2314,55 @@ __global__ void __launch_bounds__(kBlock) rearm_kernel(View v, const InstDev* __
             }
             start_instance(v, I);
         }
+    }
+}
+
+// End of a launch: one block per span of kCollectRows rows.  A solve still running only reports its
+// status.  The primal goes out in row order as FP64 (a sliced one through shared memory, so that the
+// writes, over the link to the host, are dense).
+__global__ void __launch_bounds__(kBlock) collect_kernel(View v, const CollectJob* __restrict__ jobs,
+                                                         const int2* __restrict__ spans, int32_t* statuses, Ctrl* ctrl) {
+    __shared__ double rows[kCollectRows];
+    const int t = threadIdx.x;
+    if (blockIdx.x == 0)
+        for (int w = t; w < static_cast<int>(sizeof(Ctrl) / 4); w += kBlock)
+            reinterpret_cast<uint32_t*>(ctrl)[w] = reinterpret_cast<const uint32_t*>(v.ctrl)[w];
+    const int2 sp = spans[blockIdx.x];
+    const CollectJob J = jobs[sp.x];
+    const InstDev& I = v.inst[J.slot];
+    const int status = I.status;
+    if (sp.y == 0 && t == 0) statuses[J.slot] = status;
+    if (status == ST_RUNNING) return;
+    if (sp.y == 0)
+        for (int w = t; w < static_cast<int>(sizeof(InstDev) / 16); w += kBlock)
+            reinterpret_cast<uint4*>(J.record)[w] = reinterpret_cast<const uint4*>(&I)[w];
+    const int count = min(kCollectRows, J.n - sp.y);
+    if (count <= 0) return;
+    const uint8_t* order = I.slice_row;
+    for (int k = t; k < count; k += kBlock) {
+        const int p = sp.y + k;
+        const double x = I.result_src == 1 ? widen_float(I.x32[p]) : I.result_src == 2 ? I.xp[p] : I.x64[p];
+        if (order) rows[(k & ~(kSliceWindow - 1)) + order[p]] = x;
+        else J.x[p] = x;
+    }
+    if (!order) return;
+    __syncthreads();
+    for (int k = t; k < count; k += kBlock) J.x[sp.y + k] = rows[k];
+}
+
+__global__ void __launch_bounds__(kBlock) upload_kernel(UploadPieces p) {
+    const int i0 = blockIdx.x * kBlock + threadIdx.x, stride = gridDim.x * kBlock;
+    for (int k = 0; k < p.count; ++k) {
+        const uint32_t* __restrict__ src = p.src[k];
+        uint32_t* __restrict__ dst = p.dst[k];
+        const int n = static_cast<int>(p.words[k]);
+        int done = 0;
+        if (((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0) {
+            const int quads = n / 4;
+            for (int i = i0; i < quads; i += stride) reinterpret_cast<uint4*>(dst)[i] = reinterpret_cast<const uint4*>(src)[i];
+            done = 4 * quads;
+        }
+        for (int i = done + i0; i < n; i += stride) dst[i] = src[i];
     }
 }
 
@@ -3163,17 +3205,21 @@ void launch_control(const View& v, cudaGraphConditionalHandle loop, int steps, c
 void launch_gate_plain(const View& v, int steps, cudaStream_t s) { gate_plain_kernel<<<1, 1024, 0, s>>>(v, steps); }
 void launch_control_plain(const View& v, int steps, cudaStream_t s) { control_plain_kernel<<<1, 1024, 0, s>>>(v, steps); }
 
-void launch_init_instance(const View& v, int slot, int n, int precision, cudaStream_t s) {
-    int grid = (n + kBlock - 1) / kBlock;
-    if (grid > 4096) grid = 4096;
-    if (grid < 1) grid = 1;
-    (void)precision;
-    init_instance_kernel<<<grid, kBlock, 0, s>>>(v, slot, n);
-}
-
 void launch_rearm(const View& v, const InstDev* stage, const int32_t* slots, const int2* spans, int n_spans,
                   cudaStream_t s) {
     if (n_spans > 0) rearm_kernel<<<n_spans, kBlock, 0, s>>>(v, stage, slots, spans);
+}
+
+void launch_collect(const View& v, const CollectJob* jobs, const int2* spans, int n_spans, int32_t* statuses, Ctrl* ctrl,
+                    cudaStream_t s) {
+    if (n_spans > 0) collect_kernel<<<n_spans, kBlock, 0, s>>>(v, jobs, spans, statuses, ctrl);
+}
+
+void launch_upload(const UploadPieces& p, cudaStream_t s) {
+    int64_t quads = 0;
+    for (int k = 0; k < p.count; ++k) quads += p.words[k] / 4;
+    const int64_t grid = (quads + 2 * kBlock - 1) / (2 * kBlock);
+    upload_kernel<<<static_cast<int>(grid < 1 ? 1 : grid > 152 * 2 ? 152 * 2 : grid), kBlock, 0, s>>>(p);
 }
 
 // Lanes per row of the admission kernels: the residual pass's choice (about a sixth of the

@@ -82,12 +82,25 @@ void launch_precondition(const InstDev& rec, int64_t n, const double* val, bool 
 // and the estimate after.  scratch: power_scratch_bytes(n) bytes of device memory, 256-aligned.
 size_t power_scratch_bytes(int64_t n);
 void launch_power_lipschitz(const InstDev& rec, int64_t n, const double* val, bool scaled, void* scratch, cudaStream_t s);
-// Admission: x0 = clip(0, l, u), w = x0, start clock; one instance.
-// Re-arm of resident solves: records staged on the device, spans (staged index, first row) of
-// kRearmRows rows each, one block per span.
+// Re-arm of resident solves: records staged in page-locked host memory (read from there by the kernel),
+// spans (staged index, first row) of kRearmRows rows each, one block per span.
 void launch_rearm(const View& v, const InstDev* stage, const int32_t* slots, const int2* spans, int n_spans,
                   cudaStream_t s);
-void launch_init_instance(const View& v, int slot, int n, int precision, cudaStream_t s);
+
+// After a launch: statuses, the control block and, of the solves that have finished, the records and
+// primals in row order, written to where `jobs` says (spans: job index, first row; all page-locked).
+void launch_collect(const View& v, const CollectJob* jobs, const int2* spans, int n_spans, int32_t* statuses, Ctrl* ctrl,
+                    cudaStream_t s);
+// One launch in place of a copy per array: pieces of host memory that the device can read directly
+// (page-locked, or any on a device with access to pageable memory), 4-byte multiples.
+struct UploadPieces {
+    static constexpr int kMost = 8;
+    int count = 0;
+    const uint32_t* src[kMost];
+    uint32_t* dst[kMost];
+    uint32_t words[kMost];
+};
+void launch_upload(const UploadPieces& p, cudaStream_t s);
 
 // Standalone FP64 check on caller device arrays (one instance, block partials in scratch).
 // scratch must hold check_scratch_bytes(n) bytes.
