@@ -832,8 +832,14 @@ cudaError_t bqp_admm::slice(int64_t hz, int64_t az) {
         a.slice_len = a_len; a.slice_row = a_row; a.slice_base = a_base;
         bqp::launch_slice_order(k, n, rp, position_of, stream);
         if (m) bqp::launch_slice_order(a, m, arp, position_of + t0, stream);
-        bqp::launch_slice_entries(k, n, t0 + m, hz + az, rp, ci, va, position_of, k_col, k_val, stream);
-        if (m) bqp::launch_slice_entries(a, m, n, az, arp, aci, ava, position_of, a_col, a_val, stream);
+        bqp::launch_slice_columns(hz + az, t0 + m, ci, position_of, stream);
+        bqp::launch_slice_entries(k, n, hz + az, rp, ci, va, k_col, k_val, stream);
+        if (m) {
+            // into a copy: without success the CSR stays in use
+            cudaMemcpyAsync(ci, aci, Z * 4, cudaMemcpyDeviceToDevice, stream);
+            bqp::launch_slice_columns(az, n, ci, position_of, stream);
+            bqp::launch_slice_entries(a, m, az, arp, ci, ava, a_col, a_val, stream);
+        }
         e = cudaGetLastError();
         const cudaError_t done = cudaStreamSynchronize(stream);
         if (!e) e = done;

@@ -91,7 +91,9 @@ bool slice_box(bqp_box* b, const int32_t* rowptr, std::string& why) {
     rec.c = b->c;
     rec.l = b->l;
     rec.u = b->u;
-    bqp::launch_slice_rows(rec, b->n, b->nnz, b->rowptr, b->col, b->val, position_of, col, val, b->stream);
+    bqp::launch_slice_order(rec, b->n, b->rowptr, position_of, b->stream);
+    bqp::launch_slice_columns(b->nnz, b->n, b->col, position_of, b->stream);
+    bqp::launch_slice_entries(rec, b->n, b->nnz, b->rowptr, b->col, b->val, col, val, b->stream);
     const bool good = ok(cudaGetLastError(), why) && ok(cudaStreamSynchronize(b->stream), why);
     cudaFree(position_of); cudaFree(b->rowptr); cudaFree(b->col); cudaFree(b->val);
     b->rowptr = nullptr;
@@ -330,7 +332,7 @@ int bqp_gate_device(int64_t n, const int32_t* d_rowptr, const int32_t* d_col, co
         return BQP_ERR_NO_MEMORY;
     }
     bqp::GateResult host{};
-    bqp::launch_gate_raw(n, d_rowptr, d_col, d_val, out, d_diag, nullptr, nullptr, s);
+    bqp::launch_gate_raw(n, d_rowptr, d_col, d_val, out, d_diag, nullptr, nullptr, nullptr, s);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(&host, out, sizeof(host), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);

@@ -4,7 +4,7 @@
 // The graph is one WHILE loop whose body is
 //     check -> gate -> IF(fp64) K x (step per fp64 group) -> IF(mixed) K x (step per mixed group)
 //           -> IF(exact) K x step -> IF(polish) [polish_init, polish_residual,
-//              WHILE(an instance iterates, <= 25 per body) (cg_matvec, cg_vector)] -> control
+//              WHILE(an instance iterates, <= 24 per body) (cg_matvec, cg_vector)] -> control
 // (K: the shortest check interval among the running solves; a group: one SpMV structure).
 // The check kernel's per-instance finalizers decide each instance's next phase, the gate kernel
 // arms the IF nodes for the phases present, and the control kernel ends the loop when no
@@ -54,7 +54,7 @@ bool host_profile() {
 
 
 size_t align_up(size_t x, size_t a = 256) { return (x + a - 1) / a * a; }
-constexpr int kCgPerBody = 25;  // CG iterations per polish body
+constexpr int kCgPerBody = 24;  // CG iterations per polish branch, a multiple of kCgTurns
 constexpr size_t kNone = std::numeric_limits<size_t>::max();
 
 struct Layout {
@@ -210,6 +210,7 @@ struct Job {
     double lipschitz = 0;
     int diag_gate = 0;  // -1: decided by the admission gate (a diagonal Hessian with a positive diagonal)
     int variant = 0;
+    int sum_lanes = 0;        // sliced mixed solves: InstDev::sum_lanes
     std::vector<Tile> tiles;  // local tiles (inst field filled at admission)
     std::vector<Tile> items;  // step work items of a sliced solve: its tiles in pieces of kSlicePiece rows
     std::vector<int4> units;  // CG and check work units, tiles counted from the solve's first (cg_units)
@@ -240,6 +241,7 @@ struct Job {
     int32_t* csr_col = nullptr;
     double* csr_val = nullptr;
     uint8_t* position_of = nullptr;
+    bool columns_sliced = false;  // slice_columns has run
     void* power = nullptr;
     double t_upload = 0;
     std::vector<double> x;    // primal of a solve that holds no device memory (finished at submission)
@@ -300,17 +302,26 @@ void set_unsupported(bqp_stats& st) {
     st.dual_bound = -HUGE_VAL;
 }
 
-// SpMV structure when the caller's options do not name one (kernel_variant < 0).  The FP64 engines
-// take sliced rows unless a row is too long for a lane (kSliceMaxRow) or the rows are long on average
-// (kSliceMaxAverage), where several lanes per row give a small instance more loads in flight;
-// long rows elsewhere take sub-warps, the rest the block-staged tile.
-int default_variant(int64_t n, int64_t nnz, int64_t longest_row, int precision) {
+// Structure of a solve's kernels.  Sliced rows unless a row is too long for a lane (kSliceMaxRow), the rows
+// are long on average, where several lanes per row give a small instance more loads in flight
+// (kSliceMaxAverage; the mixed engine's FP32 rows gain from it only below kSliceMaxAverageMixed), or the
+// power estimate wants the CSR.  For the FP64 engine a structure that the options name is taken as named;
+// for the mixed engine it names the order of a row's FP32 sum, which the sliced step keeps
+// (slice_sums; not named: the block-staged tile's).  Over the CSR, FP64 rows that the options leave open
+// take the structures that the autotuner's timings (boxqp/tuning.json) rank first or within a few
+// percent of it per class.
+int choose_variant(int64_t n, int64_t nnz, int64_t longest_row, const bqp_options& o, int* sums) {
     const double avg = n > 0 ? static_cast<double>(nnz) / static_cast<double>(n) : 1.0;
-    if (precision != PREC_MIXED && sliceable(n, nnz, longest_row))
-        return n <= kSliceSmall ? VAR_SLICE_SMALL : VAR_SLICE;
-    if (precision == PREC_FP64_EXACT) return 1;
-    if (avg >= 48) return 32;
-    return VAR_TILE;
+    const int sliced = n <= kSliceSmall ? VAR_SLICE_SMALL : VAR_SLICE;
+    const bool rows_fit = sliceable(n, nnz, longest_row) && o.lipschitz != BQP_LIPSCHITZ_POWER;
+    if (o.precision == PREC_FP64_EXACT) return rows_fit ? sliced : 1;
+    if (o.precision == PREC_FP64) {
+        if (o.kernel_variant >= 0) return o.kernel_variant;
+        return rows_fit ? sliced : avg >= 48 ? 32 : avg < 9 ? 1 : 2;
+    }
+    const int named = o.kernel_variant >= 0 ? o.kernel_variant : avg >= 48 ? 32 : VAR_TILE;
+    *sums = slice_sums(named);
+    return rows_fit && avg < kSliceMaxAverageMixed && *sums >= 0 ? sliced : named;
 }
 
 // CG and check work units of one instance (its `count` tiles at t), appended to `out` as {first tile, tiles,
@@ -357,7 +368,9 @@ std::vector<Tile> make_tiles(int64_t n, const int32_t* rowptr, int variant) {
         const int32_t* p = std::upper_bound(rowptr + r + 2, rowptr + hi + 1, limit,
                                             [](int64_t v, int32_t x) { return v < static_cast<int64_t>(x); });
         int64_t e = (p - rowptr) - 1;
-        if (e < n) {
+        if (is_sliced(variant)) {  // whole windows, one at least
+            e = std::min<int64_t>(n, r + std::max<int64_t>(1, (e - r) / kSliceWindow) * kSliceWindow);
+        } else if (e < n) {
             const int64_t rows = e - r;
             if (rows >= kBlock) e = r + rows / kBlock * kBlock;
             else if (rows >= 32) e = r + rows / 32 * 32;
@@ -469,6 +482,8 @@ private:
     void loop();
     bool upload(Job& j, std::string& why);
     bool alloc_upload(Job& j, size_t bytes, std::string& why);
+    static bool slice_early(const Job& j);
+    void slice_columns(Job& j);
     bool upload_begin(Job& j, std::string& why);
     bool upload_copy(Job& j, size_t budget);
     bool upload_finish(Job& j, std::string& why);
@@ -523,6 +538,7 @@ private:
             if (!((graph_groups_ >> k) & 1u)) continue;
             if (k == step_group(PREC_FP64, VAR_SLICE) || k == step_group(PREC_FP64, VAR_SLICE_SMALL) ||
                 (k >= kExactSlices && k < kStepGroups)) f |= kCheckSlices;
+            else if (k == step_group(PREC_MIXED, VAR_SLICE) || k == step_group(PREC_MIXED, VAR_SLICE_SMALL)) f |= kCheckMixedSlices;
             else if (k >= kVariants && k < 2 * kVariants) f |= kCheckMixed;
             else f |= kCheckFp64;
         }
@@ -553,6 +569,7 @@ private:
         L.n[PREC_MIXED] = K * std::max<int>(1, static_cast<int>(body_groups(PREC_MIXED).size()));
         L.n[PREC_FP64_EXACT] = K * ((exact_slices() & 1) + (exact_slices() >> 1) + (exact_csr() ? 1 : 0));
         L.checks = check_launches(check_families());
+        L.polish = 1 + polish_launches(check_families());
         L.present = present_precisions();
         return L;
     }
@@ -585,6 +602,8 @@ private:
     cudaStream_t stream_ = nullptr;
     cudaStream_t capture_ = nullptr;
     cudaStream_t ustream_ = nullptr;   // uploads of new solves, overlapping the running graph
+    cudaStream_t pstream_ = nullptr;   // a sliced solve's order and columns, beside the copy of its values
+    cudaEvent_t pev_slice_ = nullptr;
     cudaStream_t fstream_ = nullptr;   // bqp_fetch copies of finished primals (caller threads, fmu_)
     std::mutex fmu_;
     cudaEvent_t uev_ = nullptr;        // end of the latest upload on ustream_
@@ -612,7 +631,8 @@ private:
     size_t collect_bytes_ = 0;
     static constexpr size_t kCollectMax = size_t(64) << 20;  // primals beyond this are copied one by one
     std::vector<CollectJob> collect_jobs_;                   // the current launch's, as the kernel reads them
-    bool pageable_access_ = false;       // the device reads pageable host memory
+    unsigned char* h_upload_ = nullptr;  // page-locked staging of small uploads (upload_copy)
+    cudaEvent_t stage_ev_ = nullptr;     // the last kernel that reads it
     static constexpr size_t kUploadKernelBytes = size_t(2) << 20;
     // BOXQP_PROFILE: host times of the steps between two launches (engine thread)
     double t_synced_ = 0, t_collected_ = 0, t_freed_ = 0, t_gated_ = 0, t_installed_ = 0;
@@ -734,12 +754,13 @@ bool Engine::init(std::string& why) {
     if (!cuda_ok(cudaStreamCreateWithPriority(&stream_, cudaStreamNonBlocking, prio_greatest), why, "stream")) return false;
     if (!cuda_ok(cudaStreamCreateWithFlags(&capture_, cudaStreamNonBlocking), why, "stream")) return false;
     if (!cuda_ok(cudaStreamCreateWithPriority(&ustream_, cudaStreamNonBlocking, prio_least), why, "stream")) return false;
+    if (!cuda_ok(cudaStreamCreateWithPriority(&pstream_, cudaStreamNonBlocking, prio_least), why, "stream")) return false;
+    if (!cuda_ok(cudaEventCreateWithFlags(&pev_slice_, cudaEventDisableTiming), why, "event")) return false;
+    if (!cuda_ok(cudaEventCreateWithFlags(&stage_ev_, cudaEventDisableTiming), why, "event")) return false;
+    if (!cuda_ok(cudaMallocHost(&h_upload_, kUploadKernelBytes), why, "upload staging")) return false;
     if (!cuda_ok(cudaStreamCreateWithFlags(&fstream_, cudaStreamNonBlocking), why, "stream")) return false;
     if (!cuda_ok(cudaEventCreateWithFlags(&uev_, cudaEventDisableTiming), why, "event")) return false;
     if (!cuda_ok(cudaEventCreateWithFlags(&done_ev_, cudaEventDisableTiming), why, "event")) return false;
-    int pageable = 0;
-    cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, device_);
-    pageable_access_ = pageable != 0;
     cudaMemPoolProps props;
     std::memset(&props, 0, sizeof(props));
     props.allocType = cudaMemAllocationTypePinned;
@@ -796,6 +817,7 @@ void Engine::shutdown() {
     if (stream_) {
         cudaSetDevice(device_);
         if (ustream_) cudaStreamSynchronize(ustream_);
+        if (pstream_) cudaStreamSynchronize(pstream_);
         cudaStreamSynchronize(stream_);
         for (auto& kv : jobs_) if (kv.second->slab) cudaFreeAsync(kv.second->slab, stream_);
         for (auto& pf : pending_free_) if (pf.second) cudaFreeAsync(pf.second, stream_);
@@ -843,6 +865,13 @@ void Engine::shutdown() {
     if (capture_) cudaStreamDestroy(capture_);
     if (ustream_) cudaStreamDestroy(ustream_);
     if (fstream_) cudaStreamDestroy(fstream_);
+    if (pstream_) cudaStreamDestroy(pstream_);
+    if (pev_slice_) cudaEventDestroy(pev_slice_);
+    if (stage_ev_) cudaEventDestroy(stage_ev_);
+    if (h_upload_) cudaFreeHost(h_upload_);
+    pstream_ = nullptr;
+    pev_slice_ = stage_ev_ = nullptr;
+    h_upload_ = nullptr;
     if (uev_) cudaEventDestroy(uev_);
     if (done_ev_) cudaEventDestroy(done_ev_);
     done_ev_ = nullptr;
@@ -969,15 +998,16 @@ bool Engine::run_stream(int cap, std::string& why) {
         }
         if (profile_phases_) cudaEventRecord(pev_[2], stream_);
         if (h_ctrl_->n_polish > 0) {
+            const int families = check_families(), products = polish_launches(families);
             launch_polish_init(v, grid, stream_);
-            launch_polish_residual(v, grid, stream_);
-            kernels += 2;
+            launch_polish_residual(v, families, grid, stream_);
+            kernels += 1 + products;
             // the CG loop as the graph runs it: stop once no instance iterates (read back after
             // every iteration; this mode serves per-kernel profiling, not speed)
             for (int j = 0; j < kCgPerBody; ++j) {
-                launch_cg_matvec(v, grid, stream_);
-                launch_cg_vector(v, grid, stream_);
-                kernels += 2;
+                launch_cg_matvec(v, families, grid, stream_);
+                launch_cg_vector(v, products, grid, stream_);
+                kernels += products + 1;
                 cudaMemcpyAsync(h_ctrl_, d_ctrl_, sizeof(Ctrl), cudaMemcpyDeviceToHost, stream_);
                 if (!cuda_ok(cudaStreamSynchronize(stream_), why, "engine polish")) return false;
                 if (h_ctrl_->n_cg <= 0) break;
@@ -1087,12 +1117,14 @@ bool Engine::build_graph(Graph& out, std::string& why) {
         cudaGraph_t loop_body;
         if (!capture(inner, nullptr, 0, [&] {
                 launch_polish_init(v, grid, capture_);
-                launch_polish_residual(v, grid, capture_);
+                launch_polish_residual(v, check_families(), grid, capture_);
             }, &head)) return false;
         if (!add_cond(inner, head, h_cg, cudaGraphCondTypeWhile, &loop_node, &loop_body)) return false;
         if (!capture(loop_body, nullptr, 0, [&] {
-                launch_cg_matvec(v, grid, capture_);
-                launch_cg_vector(v, grid, capture_, h_cg, kCgPerBody);
+                for (int turn = 0; turn < kCgTurns; ++turn) {
+                    launch_cg_matvec(v, check_families(), grid, capture_);
+                    launch_cg_vector(v, polish_launches(check_families()), grid, capture_, h_cg, kCgPerBody, turn);
+                }
             }, nullptr)) return false;
         last = node;
     }
@@ -1436,6 +1468,7 @@ bool Engine::upload_begin(Job& j, std::string& why) {
     const size_t N = static_cast<size_t>(j.n), Z = static_cast<size_t>(j.nnz);
     j.pieces.clear();
     j.piece = j.piece_off = 0;
+    j.columns_sliced = false;
     const bool sliced = is_sliced(j.variant);
     j.tmp = nullptr;
     if (sliced) {
@@ -1514,6 +1547,8 @@ bool Engine::upload_begin(Job& j, std::string& why) {
     R.lanes_res = lanes_for(avg_row);
     R.lanes_cg = lanes_for(0.5 * avg_row);
     R.n = static_cast<int32_t>(j.n);
+    R.nnz = j.nnz;
+    R.sum_lanes = j.sum_lanes;
     R.diag_gate = j.diag_gate > 0 ? 1 : 0;
     R.precision = prec;
     R.L = j.lipschitz;
@@ -1544,31 +1579,56 @@ bool Engine::upload_begin(Job& j, std::string& why) {
     if (R.lip_device &&
         !cuda_ok(cudaMallocFromPoolAsync(&j.power, power_scratch_bytes(j.n), pool_, ustream_), why, "allocate power scratch"))
         return false;
-    if (prec == PREC_MIXED) {
+    if (sliced) {
+        if (Z) j.pieces.push_back({j.csr_val, j.val, Z * 8});
+    } else if (prec == PREC_MIXED) {
         // FP64 values only for the admission kernels (hi/lo split, diagonal, preconditioner)
         if (!alloc_upload(j, Z * 8 + 64, why)) return false;
         if (Z) j.pieces.push_back({j.tmp, j.val, Z * 8});
     } else if (Z) {
-        j.pieces.push_back({sliced ? j.csr_val : at<double>(slab, L.val64), j.val, Z * 8});
+        j.pieces.push_back({at<double>(slab, L.val64), j.val, Z * 8});
     }
     return true;
 }
 
+// Whether a solve's columns become positions before its gate runs (the power estimate multiplies by the
+// CSR as uploaded, after the gate).
+bool Engine::slice_early(const Job& j) { return is_sliced(j.variant) && j.rec.lip_device == 0; }
+
+// The row order and the columns as positions, on a stream of their own behind what ustream_ has copied so
+// far: row pointers, vectors and columns; the values are still on their way.
+void Engine::slice_columns(Job& j) {
+    InstDev R = j.rec;
+    R.diag = nullptr;  // the gate writes it in slice order
+    cudaEventRecord(pev_slice_, ustream_);
+    cudaStreamWaitEvent(pstream_, pev_slice_, 0);
+    launch_slice_order(R, j.n, j.csr_rowptr, j.position_of, pstream_);
+    launch_slice_columns(j.nnz, j.n, j.csr_col, j.position_of, pstream_);
+    cudaEventRecord(pev_slice_, pstream_);
+    j.columns_sliced = true;
+}
+
 // Issues copies of up to `budget` bytes; true once every copy of the solve is issued.  A small solve's
-// arrays go in one launch that reads them where they are (six copies of pageable memory take the
-// engine thread longer than the data does).
+// arrays go through page-locked staging in one launch (six copies of pageable memory take the engine
+// thread longer; the device could read pageable memory itself, but pages it has not seen cost about
+// 2 us each: 870 us for the 1.8 MB of a 10k-row solve).
 bool Engine::upload_copy(Job& j, size_t budget) {
-    if (j.piece == 0 && j.piece_off == 0 && pageable_access_ && j.pieces.size() <= UploadPieces::kMost) {
+    if (j.piece == 0 && j.piece_off == 0 && j.pieces.size() <= UploadPieces::kMost) {
         size_t bytes = 0;
-        UploadPieces p;
-        for (const Job::Piece& q : j.pieces) {
-            bytes += q.bytes;
-            p.src[p.count] = static_cast<const uint32_t*>(q.src);
-            p.dst[p.count] = static_cast<uint32_t*>(q.dst);
-            p.words[p.count++] = static_cast<uint32_t>(q.bytes / 4);
-        }
+        for (const Job::Piece& q : j.pieces) bytes += align_up(q.bytes, 16);
         if (bytes <= kUploadKernelBytes) {
+            cudaEventSynchronize(stage_ev_);
+            UploadPieces p;
+            unsigned char* to = h_upload_;
+            for (const Job::Piece& q : j.pieces) {
+                std::memcpy(to, q.src, q.bytes);
+                p.src[p.count] = reinterpret_cast<const uint32_t*>(to);
+                p.dst[p.count] = static_cast<uint32_t*>(q.dst);
+                p.words[p.count++] = static_cast<uint32_t>(q.bytes / 4);
+                to += align_up(q.bytes, 16);
+            }
             launch_upload(p, ustream_);
+            cudaEventRecord(stage_ev_, ustream_);
             j.piece = j.pieces.size();
             return true;
         }
@@ -1583,6 +1643,7 @@ bool Engine::upload_copy(Job& j, size_t budget) {
         if (j.piece_off == p.bytes) {
             ++j.piece;
             j.piece_off = 0;
+            if (j.piece + 1 == j.pieces.size() && slice_early(j)) slice_columns(j);  // all but the values
         }
     }
     return j.piece == j.pieces.size();
@@ -1597,33 +1658,42 @@ bool Engine::upload_finish(Job& j, std::string& why) {
         R.col = j.csr_col;
         R.val64 = j.csr_val;
     }
-    // the convexity gate and the Gershgorin bound first: the other admission kernels read L from
-    // its result, and the engine thread reads the result back before it installs the solve
     j.gate_host = acquire_gate_slot();
     if (!j.gate_host) {
         why = "host memory for the convexity gate result";
         return false;
     }
-    launch_gate(R, j.n, prec == PREC_MIXED ? static_cast<const double*>(j.tmp) : R.val64, ustream_);
+    const Layout& L = j.layout;
+    const double* uploaded = sliced ? j.csr_val : prec == PREC_MIXED ? static_cast<const double*>(j.tmp) : R.val64;
+    const bool placed = slice_early(j);  // the columns are positions already (slice_columns)
+    if (placed && !j.columns_sliced) slice_columns(j);
+    if (placed) cudaStreamWaitEvent(ustream_, pev_slice_, 0);
+    // the convexity gate and the Gershgorin bound: the other admission kernels read L from
+    // its result, and the engine thread reads the result back before it installs the solve
+    launch_gate(R, j.n, uploaded, prec == PREC_MIXED && !sliced, placed ? j.position_of : nullptr, ustream_);
     cudaMemcpyAsync(j.gate_host, R.gate, sizeof(GateResult), cudaMemcpyDeviceToHost, ustream_);
-    if (prec == PREC_MIXED) {
-        launch_prepare_instance(R, j.n, ustream_);
-        launch_precondition(R, j.n, static_cast<const double*>(j.tmp), j.opt.scaling != 2, j.power, ustream_);
-        cudaFreeAsync(j.tmp, ustream_);
-    } else {
-        const double* val = R.val64;
-        launch_prepare_instance(R, j.n, ustream_);
-        if (R.lip_device) {
-            cudaMemcpyAsync(R.lprec, &R.gate->lip_bits, sizeof(double), cudaMemcpyDeviceToDevice, ustream_);
-            launch_power_lipschitz(R, j.n, val, false, j.power, ustream_);
-        }
-        if (sliced) {
-            const Layout& L = j.layout;
-            launch_slice_rows(R, j.n, j.nnz, R.rowptr, R.col, val, j.position_of, at<int32_t>(j.slab, L.col),
-                              at<double>(j.slab, L.val64), ustream_);
-            cudaFreeAsync(j.tmp, ustream_);
-        }
+    if (R.lip_device && prec != PREC_MIXED) {
+        cudaMemcpyAsync(R.lprec, &R.gate->lip_bits, sizeof(double), cudaMemcpyDeviceToDevice, ustream_);
+        launch_power_lipschitz(R, j.n, uploaded, false, j.power, ustream_);
     }
+    if (sliced && !placed) {
+        launch_slice_order(R, j.n, R.rowptr, j.position_of, ustream_);
+        launch_slice_columns(j.nnz, j.n, j.csr_col, j.position_of, ustream_);
+    }
+    if (sliced && prec == PREC_MIXED)
+        launch_slice_entries_split(R, j.n, j.nnz, R.rowptr, R.col, uploaded, at<int32_t>(j.slab, L.col), const_cast<float*>(R.vhi),
+                                   const_cast<float*>(R.vlo), ustream_);
+    else if (sliced)
+        launch_slice_entries(R, j.n, j.nnz, R.rowptr, R.col, uploaded, at<int32_t>(j.slab, L.col), at<double>(j.slab, L.val64), ustream_);
+    if (sliced) {
+        R.rowptr = nullptr;
+        R.col = j.rec.col;
+    }
+    if (prec == PREC_MIXED) {  // in slice order where sliced
+        launch_prepare_instance(R, j.n, ustream_);
+        launch_precondition(R, j.n, uploaded, j.opt.scaling != 2, j.power, ustream_);
+    }
+    if (j.tmp) cudaFreeAsync(j.tmp, ustream_);
     if (j.power) cudaFreeAsync(j.power, ustream_);
     j.tmp = nullptr;
     j.power = nullptr;
@@ -1988,7 +2058,7 @@ bool Engine::run_once(std::string& why) {
 // record and primal (in row order) to page-locked memory, so that collect() needs no copies of its
 // own.  A primal of more than kHostPrimal variables stays on the device until bqp_fetch copies it
 // straight to the caller's array, off the engine thread (a sliced one is brought into row order in
-// the momentum buffer, which the next run starts from anew).
+// a buffer that the next run writes before it reads it: the first momentum buffer, or CG's r).
 bool Engine::queue_collection(const std::vector<Job*>& jobs, std::string& why) {
     collect_jobs_.clear();
     size_t spans = 0, primals = 0;
@@ -1996,14 +2066,12 @@ bool Engine::queue_collection(const std::vector<Job*>& jobs, std::string& why) {
         CollectJob c{};
         c.slot = j->slot;
         const size_t bytes = sizeof(double) * static_cast<size_t>(j->n);
-        if (j->n > kHostPrimal) {
-            if (is_sliced(j->variant)) {
-                c.n = static_cast<int32_t>(j->n);
-                c.x = j->rec.w64[0];
-            }
-        } else if (primals + bytes <= kCollectMax) {
+        if (j->n <= kHostPrimal && primals + bytes <= kCollectMax) {
             c.n = static_cast<int32_t>(j->n);
             primals += bytes;
+        } else if (is_sliced(j->variant)) {
+            c.n = static_cast<int32_t>(j->n);
+            c.x = j->opt.precision == PREC_MIXED ? j->rec.r : j->rec.w64[0];
         }
         spans += static_cast<size_t>(std::max(1, (c.n + kCollectRows - 1) / kCollectRows));
         collect_jobs_.push_back(c);
@@ -2055,7 +2123,8 @@ void Engine::collect(std::unique_lock<std::mutex>& lk) {
         const InstDev& R = *c.record;
         j.x_f32 = false;
         j.x_dev = nullptr;
-        if (j.n <= kHostPrimal && c.n > 0) {
+        const bool on_host = c.n > 0 && c.x != j.rec.r && c.x != j.rec.w64[0];
+        if (on_host) {
             j.x.resize(static_cast<size_t>(j.n));
             std::memcpy(j.x.data(), c.x, sizeof(double) * static_cast<size_t>(j.n));
             continue;
@@ -2067,11 +2136,6 @@ void Engine::collect(std::unique_lock<std::mutex>& lk) {
             j.x_f32 = R.result_src == 1;
             j.x_dev = R.result_src == 1 ? static_cast<const void*>(R.x32)
                                         : static_cast<const void*>(R.result_src == 2 ? R.xp : R.x64);
-            if (is_sliced(j.variant)) {
-                launch_unslice(j.n, R.slice_row, R.x64, R.w64[0], stream_);
-                j.x_dev = R.w64[0];
-                cudaStreamSynchronize(stream_);
-            }
         }
     }
     const double now = host_seconds();
@@ -2210,14 +2274,15 @@ int Engine::profile_cg(uint64_t id, int iterations, double* ms_matvec, double* m
     const View v = view();
     const int grid = graph_grid_;
     launch_polish_init(v, grid, stream_);
-    launch_polish_residual(v, grid, stream_);
+    const int families = is_sliced(j.variant) ? kCheckMixedSlices : kCheckMixed;
+    launch_polish_residual(v, families, grid, stream_);
     std::vector<cudaEvent_t> ev(static_cast<size_t>(2 * iterations + 1), nullptr);
     for (auto& e : ev) cudaEventCreate(&e);
     cudaEventRecord(ev[0], stream_);
     for (int k = 0; k < iterations; ++k) {
-        launch_cg_matvec(v, grid, stream_);
+        launch_cg_matvec(v, families, grid, stream_);
         cudaEventRecord(ev[2 * k + 1], stream_);
-        launch_cg_vector(v, grid, stream_);
+        launch_cg_vector(v, 1, grid, stream_);
         cudaEventRecord(ev[2 * k + 2], stream_);
     }
     InstDev after;
@@ -2633,8 +2698,7 @@ int make_job(int64_t n, int64_t nnz, const int32_t* rowptr, const int32_t* col, 
         *out = j.release();
         return BQP_OK;
     }
-    if (o.precision != BQP_PRECISION_FP64_EXACT && o.kernel_variant >= 0) j->variant = o.kernel_variant;
-    else j->variant = bqp::default_variant(n, nnz, scan.longest, o.precision);
+    j->variant = bqp::choose_variant(n, nnz, scan.longest, o, &j->sum_lanes);
     j->tiles = bqp::make_tiles(n, rowptr, j->variant);
     if (bqp::is_sliced(j->variant))
         for (const bqp::Tile& t : j->tiles)

@@ -19,6 +19,7 @@ constexpr int kTileRows = 512;       // maximum rows per tile
 constexpr int kCgUnitMin = 2;        // tiles per work unit of the polish CG product and the sliced check: about
 constexpr int kCgUnitMax = 8;        //   this many at least, and up to this many for large instances (cg_units)
 constexpr int kCgRowsum = 4 * kTileRows;  // rows per CG work unit at most (its row sums, 16 KB)
+constexpr int kCgTurns = 2;          // CG iterations per body of the graph's CG loop (a body's start costs several us)
 constexpr int kCgGroups = 2;         // row groups per warp whose loads the CG product keeps in flight
 constexpr int kCgUnroll = 2;         // entries per row group and lane (and epilogue rows per thread) per pass of the CG product
 constexpr int kMomentumTable = 8192; // FISTA momenta kept in a table (View::momentum)
@@ -83,6 +84,16 @@ constexpr int64_t kSliceSmall = 65536;  // rows up to which an instance is VAR_S
 constexpr int kSliceMaxRow = 127;    // longest row of a sliced instance (a tile holds 32 such rows, so tiles begin on slices)
 constexpr int kSliceMaxAverage = 48; // longer average rows keep the sub-warp structures (default_variant)
 
+// Mixed instances longer than this on average keep the sub-warp structures: their FP32 steps are bound by the
+// gathers on either layout, while admission and the residual pass cost more on slices.
+constexpr int kSliceMaxAverageMixed = 20;
+// Order of a row's FP32 sum in the sliced mixed step for a named structure (kernel_variant), the one that
+// structure's own kernel has, so that the layout does not change the iterates: 0 rounded products summed
+// in column order (block- and warp-staged), 1 fused in column order, 2 two interleaved fused sums (one or
+// two lanes per row); -1: none (more lanes keep their CSR kernels).
+inline int slice_sums(int variant) {
+    return variant == VAR_TILE || variant == VAR_WARP ? 0 : variant == 1 || variant == 2 ? variant : -1;
+}
 inline bool sliceable(int64_t n, int64_t nnz, int64_t longest_row) {
     return n > 0 && nnz > 0 && longest_row <= kSliceMaxRow && nnz < kSliceMaxAverage * n;
 }
@@ -136,7 +147,7 @@ struct __align__(16) InstDev {
     const float* vlo;      // FP32 low part, val ~= hi + lo (PREC_MIXED)
     const uint8_t* slice_len;    // VAR_SLICE: per position, the row's length
     const uint8_t* slice_row;    // VAR_SLICE: per position, the row within its window
-    const int32_t* slice_base;   // VAR_SLICE: per slice, its first entry in col / val64
+    const int32_t* slice_base;   // VAR_SLICE: per slice, its first entry in col / val64 (vhi, vlo)
     const double* c;
     const double* l;
     const double* u;
@@ -168,19 +179,23 @@ struct __align__(16) InstDev {
                            // free-list position (z; -1 held at a bound): one 16-byte gather per entry
                            // of the residual pass's products
     int32_t* pos_of;       // polish: the free-list positions alone (-1 held at a bound), for its count
-    int32_t* free_rows;    // polish: free rows of each tile, listed from the tile's first row
+    int32_t* free_rows;    // polish: free rows of each tile, listed from the tile's first row (sliced: their
+                           // positions, in row order)
     int32_t* free_cnt;     // polish: free rows per tile (index within the instance's tiles)
     int32_t* col_ff;       // polish: the free-column entries of a tile's free rows, packed row
     float* hi_ff;          //   after row (list order) from the start of the tile's own extent
     float* lo_ff;          //   [rowptr[row_begin], ...): row r at [start_ff[r], + cnt_ff[r])
     int32_t* cnt_ff;
-    int32_t* start_ff;
+    int32_t* start_ff;     //   (sliced: 32 list positions a slice, entries interleaved column by column as in
+                           //   the matrix, the slice's first entry at start_ff[its first position])
     double* pc_inv;        // polish preconditioner, per free-list position: 1 / pivot of the chain factorization (1 / Q_rr on a Jacobi row)
     double* pc_e;          //   and the kept coupling to the next position (0 ends a chain)
     int32_t* pc_tile;      //   per tile (index within the instance): 1 when the tile has a chain
     unsigned long long stat_floor;  // within a running check: the largest stationarity ratio (FP64
                                     // bits) published so far; rows that cannot exceed it skip the division
     // geometry (the instance's tile range lives in View::ranges)
+    int64_t nnz;
+    int32_t sum_lanes;     // sliced mixed steps: the order of a row's FP32 sum (slice_sums)
     int32_t n;
     int32_t diag_gate;
     // control
@@ -254,8 +269,8 @@ static_assert(sizeof(InstDev) % 16 == 0, "rearm_kernel copies records as 16-byte
 // N. Brisebarre, J.-M. Muller and S. K. Raina, IEEE Trans. Computers 53, 2004).  Four FP64
 // operations, where the general division takes several times as many.  The theorem wants every
 // step clear of underflow and overflow: divisors of 2^-100..2^100 and dividends of biased exponent
-// kDivLow.. kDivLow + kDivSpan; span 0 (divisor outside) and other dividends (zeros, whose signs
-// the remainder would lose, among them) take the general division.
+// kDivLow.. kDivLow + kDivSpan; span 0 (divisor outside) and other dividends take the general division
+// (a zero, whose sign the remainder would lose, stays as it is).
 constexpr int kDivLow = 200, kDivSpan = 1647;
 struct KnownDivisor {
     double b, hi, lo;
@@ -281,6 +296,7 @@ struct Ctrl {
     int32_t n_polish;
     int32_t error;         // non-zero: a kernel detected an inconsistency
     int32_t n_cg;          // instances that may still run CG iterations in this body
+    int32_t n_cg_before;   // n_cg as the last CG vector step found it
     int32_t cg_iters;      // CG iterations run in this body
     long long kernels;     // engine kernels executed by this launch (counted by gate/control)
     int32_t group_begin[kStepGroups + 1];  // step groups: [begin, end) in View::group_tiles

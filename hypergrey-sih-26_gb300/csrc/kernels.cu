@@ -1180,6 +1180,136 @@ __global__ void __launch_bounds__(kSliceThreads, BLOCKS) step_slice_kernel(View 
     }
 }
 
+// The FP32 step of the sliced mixed instances: the same structure on FP32 values and iterates, with the
+// per-row step and the active-set motion of the chunk's last two steps.
+struct SliceStepF {
+    const uint8_t* len;
+    const int32_t* base;
+    const int32_t* col;
+    const float* val;
+    const float* win;
+    float* wout;
+    float* x;
+    const float* c;
+    const float* l;
+    const float* u;
+    const float* step;
+    int32_t* moved;  // this step's flag, or null
+    float beta;
+    int sums;        // order of a row's sum (slice_sums)
+    int n;
+    bool due;
+};
+
+__device__ __forceinline__ SliceStepF slice_step_f32(InstDev& I, int j0) {
+    SliceStepF S;
+    const int64_t it = I.it_cur + j0;
+    S.due = I.status == ST_RUNNING && I.phase == PH_FISTA && it < I.it_next;
+    const int in = static_cast<int>(it & 1), j = static_cast<int>(it - I.it0), count = static_cast<int>(I.it_next - I.it0);
+    S.len = I.slice_len;
+    S.base = I.slice_base;
+    S.col = I.col;
+    S.val = I.vhi;
+    S.win = I.w32[in];
+    S.wout = I.w32[in ^ 1];
+    S.x = I.x32;
+    S.c = I.c32;
+    S.l = I.l32;
+    S.u = I.u32;
+    S.step = I.sstep;
+    S.moved = S.due && count >= 2 && j >= count - 2 ? &I.moved[j - (count - 2)] : nullptr;
+    S.beta = S.due ? I.beta32[j] : 0.0f;
+    S.sums = I.sum_lanes;
+    S.n = I.n;
+    return S;
+}
+
+// Adds a round of columns to a row's sum in the order `sums` (AHEAD is even: a round begins with an
+// even column).
+template <int AHEAD>
+__device__ __forceinline__ void add_columns(const SliceColumns<AHEAD, float>& e, const float* x, int sums, float& even,
+                                            float& odd) {
+    static_assert(AHEAD % 2 == 0, "a round begins with an even column");
+    float xv[AHEAD];
+#pragma unroll
+    for (int q = 0; q < AHEAD; ++q) xv[q] = e.c[q] >= 0 ? x[e.c[q]] : 0.f;
+    if (sums == 0) {
+#pragma unroll
+        for (int q = 0; q < AHEAD; ++q)
+            if (e.c[q] >= 0) even = __fadd_rn(even, __fmul_rn(e.a[q], xv[q]));
+    } else if (sums == 1) {
+#pragma unroll
+        for (int q = 0; q < AHEAD; ++q)
+            if (e.c[q] >= 0) even = __fmaf_rn(e.a[q], xv[q], even);
+    } else {
+#pragma unroll
+        for (int q = 0; q < AHEAD; q += 2) {
+            if (e.c[q] >= 0) even = __fmaf_rn(e.a[q], xv[q], even);
+            if (e.c[q + 1] >= 0) odd = __fmaf_rn(e.a[q + 1], xv[q + 1], odd);
+        }
+    }
+}
+
+// FP32 step of the sliced mixed engine, in the form of step_slice_kernel.  The random graph is bound by
+// its 15 million gathers (60 us), the grid by its 75 MB and the chain load, gather, store of each warp.
+// Against the CSR kernels the tuning table names: grid 1M 26 -> 19.6 us a step, random graph 1M
+// 76 -> 74 us, 10k rows 13.2 -> 7.9 us.  6 columns at 8 blocks per SM: 1.75 ms of device time per
+// random-graph solve, 4 columns 1.83, 8 columns 1.83, 10 blocks 1.81, 12 blocks 1.83.
+template <int AHEAD, int BLOCKS>
+__global__ void __launch_bounds__(kSliceThreads, BLOCKS) step_slice_f32_kernel(View v, int group, int j0) {
+    let_next_launch_begin();
+    const int b = v.ctrl->group_begin[group], items = v.ctrl->group_begin[group + 1] - b;
+    const int shift = item_split(items, gridDim.x), parts = items << shift;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int g = blockIdx.x;
+    if (j0 >= v.ctrl->step_due[PREC_MIXED] || g >= parts) {
+        wait_for_previous_launch();
+        return;
+    }
+    Tile T = v.group_tiles[b + (g >> shift)];
+    SliceStepF S = slice_step_f32(v.inst[T.inst], j0);
+    bool waited = false;
+    for (int turn = warp;; ++turn) {
+        const int part = g & ((1 << shift) - 1), per = (kSlicePiece / 32) >> shift;
+        const int s = (T.row_begin >> 5) + part * per + (turn & (kSlicePiece / 32 - 1));
+        const bool mine = S.due && (turn & (kSlicePiece / 32 - 1)) < per && s * 32 < T.row_end;
+        const int inst = T.inst, p = s * 32 + lane;
+        const bool valid = mine && p < S.n;
+        const int len = valid ? __ldg(S.len + p) : 0;
+        int k = (mine ? __ldg(S.base + s) : 0) + lane;
+        const float ci = valid ? __ldg(S.c + p) : 0.f, lo = valid ? __ldg(S.l + p) : 0.f, up = valid ? __ldg(S.u + p) : 0.f;
+        const float st = valid ? __ldg(S.step + p) : 0.f;
+        const int longest = __shfl_sync(0xffffffffu, len, 0);
+        SliceColumns<AHEAD, float> e;
+        e.load(S.col, S.val, len, k);
+        g += gridDim.x;
+        if (g < parts) T = v.group_tiles[b + (g >> shift)];  // the next item, ahead of its use
+        if (!waited) wait_for_previous_launch();
+        waited = true;
+        const float wi = valid ? S.win[p] : 0.f, xo = valid ? S.x[p] : 0.f;
+        float acc = 0.f, odd = 0.f;
+        add_columns(e, S.win, S.sums, acc, odd);
+        for (int j = AHEAD; j < longest; j += AHEAD) {  // warp-uniform
+            e.load(S.col, S.val, len - j, k);
+            add_columns(e, S.win, S.sums, acc, odd);
+        }
+        if (S.sums == 2) acc += odd;
+        bool moved = false;
+        if (valid) {
+            const float nx = smaxf(lo, sminf(up, wi - (acc + ci) * st));
+            S.wout[p] = nx + S.beta * (nx - xo);
+            S.x[p] = nx;
+            moved = bound_state(xo, lo, up) != bound_state(nx, lo, up);
+        }
+        if (S.moved && __any_sync(0xffffffffu, moved) && lane == 0) {
+            volatile int32_t* f = S.moved;
+            if (*f == 0) *f = 1;
+        }
+        if (g >= parts) return;
+        if (T.inst != inst) S = slice_step_f32(v.inst[T.inst], j0);
+    }
+}
+
 // ---- check kernel -----------------------------------------------------------------------------
 // One kernel per precision family (FAMILY_MIXED: FP32 iterate or polished point; FAMILY_FP64:
 // fp64 and fp64_exact), so each carries only its own check path and its own register budget.
@@ -1193,7 +1323,7 @@ __global__ void __launch_bounds__(kBlock, 3) check_kernel(View v) {
     const int nt = v.ctrl->n_tiles;
     for (int t = blockIdx.x; t < nt; t += gridDim.x) {
         const Tile T = v.tiles[t];
-        if (FAMILY == FAMILY_FP64 && is_sliced(T.variant)) continue;  // check_slice_kernel's
+        if (is_sliced(T.variant)) continue;  // the sliced checks'
         InstDev& I = v.inst[T.inst];
         if (I.status != ST_RUNNING) continue;
         if (I.phase == PH_FISTA && I.it_cur < I.it_next) continue;  // chunk still running
@@ -1238,7 +1368,7 @@ __global__ void __launch_bounds__(kBlock, 4) check_slice_kernel(View v) {
         const Tile T = v.tiles[U.x];
         if (!is_sliced(T.variant)) continue;
         InstDev& I = v.inst[T.inst];
-        if (I.status != ST_RUNNING || I.phase != PH_FISTA || I.it_cur < I.it_next) continue;
+        if (I.precision == PREC_MIXED || I.status != ST_RUNNING || I.phase != PH_FISTA || I.it_cur < I.it_next) continue;
         const int last = (v.tiles[U.x + U.y - 1].row_end + 31) >> 5;
         const unsigned long long floor = __ldcg(&I.stat_floor);
         const int gate = I.diag_gate, n = I.n;
@@ -1252,6 +1382,102 @@ __global__ void __launch_bounds__(kBlock, 4) check_slice_kernel(View v) {
             const double xi = I.x64[p], li = I.l[p], ui = I.u[p];
             check_row(a, xi, gq, I.c[p], li, ui, gate ? I.diag[p] : 1.0, gate, p, less_equal_bits(dbits(xi), dbits(li)),
                       less_equal_bits(dbits(ui), dbits(xi)), floor);
+        }
+        Acc total = block_reduce_check(a, gate != 0, true);
+        if (threadIdx.x == 0 && total.stat > floor) atomicMax(&I.stat_floor, total.stat);
+        const int2 R = v.ranges[T.inst];
+        if (publish_and_test_last(v, R.x + U.z, T.inst, U.w, total)) {
+            Acc inst_total = reduce_instance(v, R.x, R.x + U.w, gate != 0);
+            if (threadIdx.x == 0) {
+                after_check(v, I, inst_total);
+                I.stat_floor = 0;
+            }
+            __syncthreads();
+        }
+    }
+}
+
+// Columns of a slice of the mixed engine: hi/lo values and gathered FP32 numbers or pairs.
+template <int AHEAD>
+struct SlicePairs {
+    int c[AHEAD];
+    float h[AHEAD], l[AHEAD];
+    __device__ __forceinline__ void load(const int32_t* __restrict__ col, const float* __restrict__ vhi,
+                                         const float* __restrict__ vlo, int left, int& k) {
+#pragma unroll
+        for (int q = 0; q < AHEAD; ++q) {
+            const bool in = q < left;
+            c[q] = in ? __ldg(col + k) : -1;
+            h[q] = in ? __ldg(vhi + k) : 0.f;
+            l[q] = in ? __ldg(vlo + k) : 0.f;
+            k += __popc(__ballot_sync(0xffffffffu, in));
+        }
+    }
+    __device__ __forceinline__ float2 add(const float* x, float2 acc) const {
+        float xv[AHEAD];
+#pragma unroll
+        for (int q = 0; q < AHEAD; ++q) xv[q] = c[q] >= 0 ? x[c[q]] : 0.f;
+#pragma unroll
+        for (int q = 0; q < AHEAD; ++q)
+            if (c[q] >= 0) acc = df_add(acc, df_prod(h[q], l[q], xv[q]));
+        return acc;
+    }
+    __device__ __forceinline__ float2 add(const float2* x, float2 acc) const {
+        float2 xv[AHEAD];
+#pragma unroll
+        for (int q = 0; q < AHEAD; ++q) xv[q] = c[q] >= 0 ? x[c[q]] : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int q = 0; q < AHEAD; ++q)
+            if (c[q] >= 0) acc = df_add(acc, df_prod2(h[q], l[q], xv[q]));
+        return acc;
+    }
+};
+
+// Checks of the sliced mixed instances over the work units: the FP32 iterate (FAMILY_MIXED) or the
+// polished point (FAMILY_VERIFY), the arithmetic of check_rows<1> and <2>.  Bound by the gathers: the
+// pair arithmetic is FP32 and a row's FP64 epilogue runs on a full warp.  Verification of the random
+// graph 1M 170 -> 94 us (cold caches), grid 77 -> 59 us.
+template <int FAMILY>
+__global__ void __launch_bounds__(kBlock, 4) check_slice_mixed_kernel(View v) {
+    constexpr int kAheadPairs = 4;
+    if (v.ctrl->check_due[FAMILY] == 0) return;
+    const int nu = v.ctrl->n_units;
+    for (int un = blockIdx.x; un < nu; un += gridDim.x) {
+        const int4 U = v.units[un];  // first tile, tiles, index and units of its instance
+        const Tile T = v.tiles[U.x];
+        if (!is_sliced(T.variant)) continue;
+        InstDev& I = v.inst[T.inst];
+        if (I.precision != PREC_MIXED || I.status != ST_RUNNING) continue;
+        if (FAMILY == FAMILY_VERIFY ? I.phase != PH_POLISH_FINISH : I.phase != PH_FISTA || I.it_cur < I.it_next) continue;
+        const int last = (v.tiles[U.x + U.y - 1].row_end + 31) >> 5;
+        const unsigned long long floor = __ldcg(&I.stat_floor);
+        const int gate = I.diag_gate, n = I.n;
+        Acc a = acc_identity();
+        for (int s = (T.row_begin >> 5) + static_cast<int>(threadIdx.x >> 5); s < last; s += kBlock / 32) {
+            const int p = s * 32 + static_cast<int>(threadIdx.x & 31);
+            const bool valid = p < n;
+            const int len = valid ? __ldg(I.slice_len + p) : 0;
+            int k = __ldg(I.slice_base + s) + static_cast<int>(threadIdx.x & 31);
+            const int longest = __shfl_sync(0xffffffffu, len, 0);
+            float2 acc = make_float2(0.f, 0.f);
+            SlicePairs<kAheadPairs> e;
+            for (int j = 0; j < longest; j += kAheadPairs) {  // warp-uniform
+                e.load(I.col, I.vhi, I.vlo, len - j, k);
+                if constexpr (FAMILY == FAMILY_VERIFY) acc = e.add(I.xp2, acc);
+                else acc = e.add(I.x32, acc);
+            }
+            if (!valid) continue;
+            const double gq = df_value(acc), li = I.l[p], ui = I.u[p], ci = I.c[p];
+            if constexpr (FAMILY == FAMILY_VERIFY) {
+                const double xi = I.xp[p];
+                check_row(a, xi, gq, ci, li, ui, gate ? I.diag[p] : 1.0, gate, p, less_equal_bits(dbits(xi), dbits(li)),
+                          less_equal_bits(dbits(ui), dbits(xi)), floor);
+            } else {
+                const float xf = I.x32[p];
+                const bool at_lower = xf <= I.l32[p], at_upper = xf >= I.u32[p];
+                if (gate) check_row(a, static_cast<double>(xf), gq, ci, li, ui, I.diag[p], 1, p, at_lower, at_upper);
+                else check_row_f32(a, xf, gq, ci, li, ui, p, at_lower, at_upper);
+            }
         }
         Acc total = block_reduce_check(a, gate != 0, true);
         if (threadIdx.x == 0 && total.stat > floor) atomicMax(&I.stat_floor, total.stat);
@@ -1291,13 +1517,16 @@ __device__ __forceinline__ bool polish_phase(const InstDev& I, int phase) {
 }
 
 __global__ void __launch_bounds__(kBlock) polish_init_kernel(View v) {
+    static_assert(kBlock == kSliceWindow, "a turn of the loop over a tile's rows is a slice window");
     __shared__ int warp_free[kBlock / 32];
+    __shared__ uint8_t position[kSliceWindow];  // sliced: the position of each of the window's rows
     const int nt = v.ctrl->n_tiles;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int t = blockIdx.x; t < nt; t += gridDim.x) {
         const Tile T = v.tiles[t];
         const InstDev& I = v.inst[T.inst];
         if (!polish_phase(I, PH_POLISH_INIT)) continue;
+        const uint8_t* __restrict__ order = is_sliced(T.variant) ? I.slice_row : nullptr;
         const float* __restrict__ x32 = I.x32;
         const float* __restrict__ l32 = I.l32;
         const float* __restrict__ u32 = I.u32;
@@ -1310,10 +1539,16 @@ __global__ void __launch_bounds__(kBlock) polish_init_kernel(View v) {
         int32_t* __restrict__ list = I.free_rows + T.row_begin;
         int count = 0;
         for (int r0 = T.row_begin; r0 < T.row_end; r0 += kBlock) {
-            const int r = r0 + static_cast<int>(threadIdx.x);
+            int r = r0 + static_cast<int>(threadIdx.x);
+            const bool valid = r < T.row_end;
+            if (order) {  // the rows in their own order, each at its position
+                if (valid) position[order[r]] = static_cast<uint8_t>(threadIdx.x);
+                __syncthreads();
+                if (valid) r = r0 + position[threadIdx.x];
+            }
             bool is_free = false;
             float2 x2 = make_float2(0.f, 0.f);
-            if (r < T.row_end) {
+            if (valid) {
                 const float xf = x32[r];
                 double xv;
                 if (xf <= l32[r]) xv = l[r];
@@ -1332,7 +1567,7 @@ __global__ void __launch_bounds__(kBlock) polish_init_kernel(View v) {
                 before += w < warp ? warp_free[w] : 0;
                 total += warp_free[w];
             }
-            if (r < T.row_end) {
+            if (valid) {
                 const int j = before + __popc(m & ((1u << lane) - 1u));
                 if (is_free) list[j] = r;
                 const int pos = is_free ? T.row_begin + j : -1;
@@ -1522,13 +1757,16 @@ __device__ int block_sum_int(int v) {
     return total;
 }
 
-__device__ void residual_epilogue(const InstDev& I, const int32_t* __restrict__ list, int n, int tile,
-                                  const float2* rowsum, const float2* coupling, Acc& a) {
-    __shared__ double res[kTileRows];  // r per list position
-    __shared__ double dg[kTileRows];   // Q_rr per list position
-    __shared__ double ec[kTileRows];   // coupling to the next position; then the forward values
-    __shared__ double ek[kTileRows];   // kept coupling
-    __shared__ double zs[kTileRows];   // z of the chain rows
+// `list` indexes the vectors; `row_of` gives each list position's row (the list itself over the CSR);
+// scratch: kResidualScratch doubles of shared memory.
+constexpr int kResidualScratch = 5 * kTileRows;
+__device__ void residual_epilogue(const InstDev& I, const int32_t* __restrict__ list, const int32_t* row_of, int n, int tile,
+                                  const float2* rowsum, const float2* coupling, double* scratch, Acc& a) {
+    double* res = scratch;        // r per list position
+    double* dg = res + kTileRows;  // Q_rr per list position
+    double* ec = dg + kTileRows;   // coupling to the next position; then the forward values
+    double* ek = ec + kTileRows;   // kept coupling
+    double* zs = ek + kTileRows;   // z of the chain rows
     const double* __restrict__ c = I.c;
     const double* __restrict__ dinv = I.dinv;
     const double* __restrict__ diag = I.diag;
@@ -1559,14 +1797,14 @@ __device__ void residual_epilogue(const InstDev& I, const int32_t* __restrict__ 
         const int r = list[t];
         res[t] = -(df_value(rowsum[t]) + c[r]);
         double e = 0.0;
-        if (t + 1 < n && list[t + 1] == r + 1 && (t + 1) % kChain != 0)
+        if (t + 1 < n && row_of[t + 1] == row_of[t] + 1 && (t + 1) % kChain != 0)
             e = static_cast<double>(coupling[t].x) + coupling[t].y;
         ec[t] = e;
         if (e != 0.0) {
             any = true;
             dg[t] = diag[r];
         }
-        if (t > 0 && list[t - 1] == r - 1) dg[t] = diag[r];  // a possible chain row's pivot source
+        if (t > 0 && row_of[t - 1] == row_of[t] - 1) dg[t] = diag[r];  // a possible chain row's pivot source
     }
     bool chains = __syncthreads_or(any) != 0;
     if (chains) {
@@ -1854,6 +2092,7 @@ __device__ int polish_rows(const InstDev& I, int rb, int tile, int n_free, Acc& 
     __shared__ int32_t start_of[kTileRows];  // free-list positions of the packed rows
     __shared__ float2 rowsum[kTileRows];     // row sums handed to the FP64 epilogue
     __shared__ float2 coupling[kTileRows];   // Q(r, r + 1) of each free row (hi, lo)
+    __shared__ double scratch[kResidualScratch];
     const int32_t* list = I.free_rows + rb;
     const int base = __ldg(I.rowptr + rb);
     int kept;
@@ -1867,8 +2106,37 @@ __device__ int polish_rows(const InstDev& I, int rb, int tile, int n_free, Acc& 
     }
     // the FP64 epilogue, one free row (or one chain of rows) per thread on full warps
     __syncthreads();
-    residual_epilogue(I, list, n_free, tile, rowsum, coupling, a);
+    residual_epilogue(I, list, list, n_free, tile, rowsum, coupling, scratch, a);
     return kept;
+}
+
+// End of a work unit of the residual pass: the unit's Q_FF size and partial sums; the instance's last unit
+// starts its CG.
+__device__ void finish_residual(const View& v, InstDev& I, int inst, int2 R, int4 U, int kept, int n_free_unit, const Acc& a) {
+    if (threadIdx.x == 0) {  // Q_FF size of this polish round, for the byte accounting
+        atomicAdd(reinterpret_cast<unsigned long long*>(&I.ff_nnz), static_cast<unsigned long long>(kept));
+        atomicAdd(reinterpret_cast<unsigned long long*>(&I.ff_rows), static_cast<unsigned long long>(n_free_unit));
+    }
+    Acc total = block_reduce_ab(a, 1, true, true);
+        if (publish_and_test_last(v, R.x + U.z, inst, U.w, total)) {
+            Acc inst_total = reduce_instance_ab(v, R.x, R.x + U.w);
+            if (threadIdx.x == 0) {
+                // residual pass: the full CSR (hi/lo values + columns) and row pointers, xq (the
+                // snapped point's pairs and the positions, gathered) and c; the packed Q_FF
+                // written (hi/lo + column) with its row starts and counts; r, z, p, s, p2, x and
+                // the preconditioner's 1/pivot written and 1/diag read on the free rows
+                const double nnz = static_cast<double>(I.nnz);
+                const double N = static_cast<double>(I.n);
+                const double fz = static_cast<double>(I.ff_nnz), fr = static_cast<double>(I.ff_rows);
+                I.polish_bytes += 12.0 * nnz + 4.0 * (N + 1) + 24.0 * N + 12.0 * fz + 8.0 * fr + 64.0 * fr;
+                I.rz = inst_total.a;
+                I.cg_res = static_cast<double>(__uint_as_float(static_cast<unsigned>(inst_total.b)));
+                I.cg_it = 0;
+                I.phase = (I.cg_res <= I.cg_tol || !(I.rz > 0)) ? PH_POLISH_FINISH : PH_POLISH_CG;
+                if (I.phase == PH_POLISH_FINISH) atomicSub(&v.ctrl->n_cg, 1);
+            }
+            __syncthreads();
+        }
 }
 
 // Four blocks per SM (64 registers, a few spills): 2.307 ms per 1M random-graph solve against
@@ -1881,6 +2149,7 @@ __global__ void __launch_bounds__(kBlock, 4) polish_residual_kernel(View v) {
     for (int un = blockIdx.x; un < nu; un += gridDim.x) {
         const int4 U = v.units[un];  // first tile, tiles, index and units of its instance
         const Tile T0 = v.tiles[U.x];
+        if (is_sliced(T0.variant)) continue;  // polish_residual_slice_kernel's
         InstDev& I = v.inst[T0.inst];
         if (!polish_phase(I, PH_POLISH_INIT)) continue;
         const int2 R = v.ranges[T0.inst];
@@ -1893,60 +2162,15 @@ __global__ void __launch_bounds__(kBlock, 4) polish_residual_kernel(View v) {
             kept += polish_rows(I, v.tiles[t].row_begin, t - R.x, n_free, a);
             n_free_unit += n_free;
         }
-        if (threadIdx.x == 0) {  // Q_FF size of this polish round, for the byte accounting
-            atomicAdd(reinterpret_cast<unsigned long long*>(&I.ff_nnz), static_cast<unsigned long long>(kept));
-            atomicAdd(reinterpret_cast<unsigned long long*>(&I.ff_rows), static_cast<unsigned long long>(n_free_unit));
-        }
-        Acc total = block_reduce_ab(a, I.lanes_res, true, true);
-        if (publish_and_test_last(v, R.x + U.z, T0.inst, U.w, total)) {
-            Acc inst_total = reduce_instance_ab(v, R.x, R.x + U.w);
-            if (threadIdx.x == 0) {
-                // residual pass: the full CSR (hi/lo values + columns) and row pointers, xq (the
-                // snapped point's pairs and the positions, gathered) and c; the packed Q_FF
-                // written (hi/lo + column) with its row starts and counts; r, z, p, s, p2, x and
-                // the preconditioner's 1/pivot written and 1/diag read on the free rows
-                const double nnz = static_cast<double>(__ldg(I.rowptr + I.n));
-                const double N = static_cast<double>(I.n);
-                const double fz = static_cast<double>(I.ff_nnz), fr = static_cast<double>(I.ff_rows);
-                I.polish_bytes += 12.0 * nnz + 4.0 * (N + 1) + 24.0 * N + 12.0 * fz + 8.0 * fr + 64.0 * fr;
-                I.rz = inst_total.a;
-                I.cg_res = static_cast<double>(__uint_as_float(static_cast<unsigned>(inst_total.b)));
-                I.cg_it = 0;
-                I.phase = (I.cg_res <= I.cg_tol || !(I.rz > 0)) ? PH_POLISH_FINISH : PH_POLISH_CG;
-                if (I.phase == PH_POLISH_FINISH) atomicSub(&v.ctrl->n_cg, 1);
-            }
-            __syncthreads();
-        }
+        finish_residual(v, I, T0.inst, R, U, kept, n_free_unit, a);
     }
 }
 
-__global__ void __launch_bounds__(kBlock, 4) cg_matvec_kernel(View v) {
-    __shared__ int pre[kCgUnitMax + 1];
-    __shared__ int rbeg[kCgUnitMax];
-    __shared__ float2 rowsum[kCgRowsum];
-    const int nu = v.ctrl->n_units;
-    for (int un = blockIdx.x; un < nu; un += gridDim.x) {
-        const int4 U = v.units[un];  // first tile, tiles, index and units of its instance
-        const int t0 = U.x;
-        const Tile T = v.tiles[t0];
-        InstDev& I = v.inst[T.inst];
-        if (!polish_phase(I, PH_POLISH_CG)) continue;
-        const int2 R = v.ranges[T.inst];
-        const int nk = U.y;
-        unit_table(v, I, t0, R.x, nk, pre, rbeg);
-        const int total = pre[kCgUnitMax];
-        Acc a = acc_identity();
-        switch (I.lanes_cg) {
-        case 1: matvec_unit<1>(I, pre, rbeg, nk, total, rowsum, a); break;
-        case 2: matvec_unit<2>(I, pre, rbeg, nk, total, rowsum, a); break;
-        case 4: matvec_unit<4>(I, pre, rbeg, nk, total, rowsum, a); break;
-        case 8: matvec_unit<8>(I, pre, rbeg, nk, total, rowsum, a); break;
-        case 16: matvec_unit<16>(I, pre, rbeg, nk, total, rowsum, a); break;
-        default: matvec_unit<32>(I, pre, rbeg, nk, total, rowsum, a); break;
-        }
-        Acc tot = block_reduce_ab(a, I.lanes_cg, true, true);
+// End of a work unit of the CG product: its partial sums; the instance's last unit takes the CG step.
+__device__ void finish_product(const View& v, InstDev& I, int inst, int2 R, int4 U, const Acc& a) {
+    Acc tot = block_reduce_ab(a, 1, true, true);
         // the unit's partial in slot R.x + index: the instance's partials are contiguous
-        if (publish_and_test_last(v, R.x + U.z, T.inst, U.w, tot)) {
+        if (publish_and_test_last(v, R.x + U.z, inst, U.w, tot)) {
             Acc inst_total = reduce_instance_ab(v, R.x, R.x + U.w);
             if (threadIdx.x == 0) {
                 // Chronopoulos-Gear: gamma_i = r_i.u_i, delta_i = (Q u_i).u_i, beta_i =
@@ -1979,22 +2203,301 @@ __global__ void __launch_bounds__(kBlock, 4) cg_matvec_kernel(View v) {
             }
             __syncthreads();
         }
+}
+
+__global__ void __launch_bounds__(kBlock, 4) cg_matvec_kernel(View v) {
+    __shared__ int pre[kCgUnitMax + 1];
+    __shared__ int rbeg[kCgUnitMax];
+    __shared__ float2 rowsum[kCgRowsum];
+    let_next_launch_begin();
+    wait_for_previous_launch();
+    const int nu = v.ctrl->n_units;
+    for (int un = blockIdx.x; un < nu; un += gridDim.x) {
+        const int4 U = v.units[un];  // first tile, tiles, index and units of its instance
+        const int t0 = U.x;
+        const Tile T = v.tiles[t0];
+        if (is_sliced(T.variant)) continue;  // cg_matvec_slice_kernel's
+        InstDev& I = v.inst[T.inst];
+        if (!polish_phase(I, PH_POLISH_CG)) continue;
+        const int2 R = v.ranges[T.inst];
+        const int nk = U.y;
+        unit_table(v, I, t0, R.x, nk, pre, rbeg);
+        const int total = pre[kCgUnitMax];
+        Acc a = acc_identity();
+        switch (I.lanes_cg) {
+        case 1: matvec_unit<1>(I, pre, rbeg, nk, total, rowsum, a); break;
+        case 2: matvec_unit<2>(I, pre, rbeg, nk, total, rowsum, a); break;
+        case 4: matvec_unit<4>(I, pre, rbeg, nk, total, rowsum, a); break;
+        case 8: matvec_unit<8>(I, pre, rbeg, nk, total, rowsum, a); break;
+        case 16: matvec_unit<16>(I, pre, rbeg, nk, total, rowsum, a); break;
+        default: matvec_unit<32>(I, pre, rbeg, nk, total, rowsum, a); break;
+        }
+        finish_product(v, I, T.inst, R, U, a);
     }
+}
+
+// ---- the polish of sliced instances --------------------------------------------------------------
+// Residual pass over the sliced rows, a tile at a time.  Lane per position: the row's product, the
+// coupling to the next row, and each entry's list position, kept in shared memory; then the packing of
+// Q_FF over the free list, lane per list position, from those.  One gather per entry of the free rows, no
+// shuffles.  The free list, and with it the preconditioner's chains, keeps the row order.  What bounds
+// it is latency (three barriers a tile, rows of a window in descending length): four blocks per SM and
+// four columns in flight measured 1754 us per random-graph solve, three blocks with the kept values
+// staged too and six columns 1822, four blocks with eight columns (spills) 1831.
+constexpr int kResidualAhead = 4, kResidualBlocks = 4;
+constexpr int kResidualStage = 5120;  // entries of a tile whose list positions are kept in shared memory
+struct ResidualShared {
+    union {
+        int32_t place[kResidualStage];                       // per entry of the tile: the column's list position, or -1
+        double scratch[kResidualScratch];                    // the epilogue's, once Q_FF is packed
+    };
+    float2 rowsum[kTileRows];                                // per list position
+    float2 coupling[kTileRows];
+    int32_t row_of[kTileRows];                               // per list position: its row
+    uint16_t column_at[kTileRows / 32][kSliceMaxRow + 1];    // per slice and column: its first entry within the tile
+    uint16_t position[kTileRows];                            // per row of the tile: its position within the tile
+    uint8_t kept[kTileRows];                                 // per list position: its kept entries
+    int32_t slice_total[kTileRows / 32];
+};
+
+__device__ int residual_slices(const InstDev& I, const Tile& T, int tile, int n_free, ResidualShared& S, Acc& a) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int rb = T.row_begin, rows = T.row_end - rb, slices = (rows + 31) >> 5;
+    const int32_t* __restrict__ list = I.free_rows + rb;
+    const int32_t* __restrict__ col = I.col;
+    const float* __restrict__ vhi = I.vhi;
+    const float* __restrict__ vlo = I.vlo;
+    const int4* xq = I.xq;
+    const int tb = __ldg(I.slice_base + (rb >> 5));
+    for (int t = threadIdx.x; t < rows; t += kBlock)
+        S.position[(t & ~(kSliceWindow - 1)) + __ldg(I.slice_row + rb + t)] = static_cast<uint16_t>(t);
+    __syncthreads();
+    // the tile's entries end where the next tile's begin; the last tile's with the matrix
+    const int te = T.row_end < I.n ? __ldg(I.slice_base + (T.row_end >> 5)) : static_cast<int>(I.nnz);
+    const bool staged = te - tb <= kResidualStage;
+    for (int i = 0; i * (kBlock / 32) < slices; ++i) {
+        // a window's slices come in descending length: every other turn in reverse
+        const int s = i * (kBlock / 32) + ((i & 1) ? kBlock / 32 - 1 - warp : warp);
+        if (s >= slices) continue;
+        const int t = s * 32 + lane, p = rb + t;
+        const bool valid = t < rows;
+        const int len = valid ? __ldg(I.slice_len + p) : 0;
+        const int pos = valid ? I.pos_of[p] : -1;
+        const bool is_free = pos >= 0;
+        const int row = valid ? (t & ~(kSliceWindow - 1)) + __ldg(I.slice_row + p) : 0;
+        const int next = valid && row + 1 < rows ? rb + S.position[row + 1] : -1;  // the position of the row after
+        const int longest = __shfl_sync(0xffffffffu, len, 0);
+        int k = __ldg(I.slice_base + (p >> 5)) + lane;
+        float2 acc = make_float2(0.f, 0.f), e_next = make_float2(0.f, 0.f);
+        int kept = 0;
+        for (int j = 0; j < longest; j += kResidualAhead) {  // warp-uniform
+            int c[kResidualAhead], at[kResidualAhead];
+            float h[kResidualAhead], l[kResidualAhead];
+            int4 q4[kResidualAhead];
+#pragma unroll
+            for (int q = 0; q < kResidualAhead; ++q) {
+                const bool in = j + q < len;
+                at[q] = k - tb;
+                if (lane == 0 && j + q < longest) S.column_at[s][j + q] = static_cast<uint16_t>(at[q]);
+                c[q] = in && is_free ? __ldg(col + k) : -1;
+                h[q] = in && is_free ? __ldg(vhi + k) : 0.f;
+                l[q] = in && is_free ? __ldg(vlo + k) : 0.f;
+                k += __popc(__ballot_sync(0xffffffffu, in));
+            }
+#pragma unroll
+            for (int q = 0; q < kResidualAhead; ++q) q4[q] = c[q] >= 0 ? xq[c[q]] : make_int4(0, 0, -1, 0);
+#pragma unroll
+            for (int q = 0; q < kResidualAhead; ++q) {
+                if (c[q] < 0) continue;
+                acc = df_add(acc, df_prod2(h[q], l[q], make_float2(__int_as_float(q4[q].x), __int_as_float(q4[q].y))));
+                if (c[q] == next) e_next = make_float2(e_next.x + h[q], e_next.y + l[q]);
+                kept += q4[q].z >= 0 ? 1 : 0;
+                if (staged) S.place[at[q]] = q4[q].z;
+            }
+        }
+        if (is_free) {
+            const int f = pos - rb;
+            S.row_of[f] = row;
+            S.kept[f] = static_cast<uint8_t>(kept);
+            S.rowsum[f] = acc;
+            S.coupling[f] = e_next;
+        }
+    }
+    __syncthreads();
+    const int ff = (n_free + 31) >> 5;
+    for (int f = warp; f < ff; f += kBlock / 32) {
+        const int j = f * 32 + lane;
+        const int total = static_cast<int>(__reduce_add_sync(0xffffffffu, j < n_free ? static_cast<unsigned>(S.kept[j]) : 0u));
+        if (lane == 0) S.slice_total[f] = total;
+    }
+    __syncthreads();
+    int kept_tile = 0;
+    for (int f = 0; f < ff; ++f) kept_tile += S.slice_total[f];
+    for (int f = warp; f < ff; f += kBlock / 32) {
+        int base = tb;
+        for (int g = 0; g < f; ++g) base += S.slice_total[g];
+        const int j = f * 32 + lane;
+        const int kept = j < n_free ? S.kept[j] : 0;
+        const int t = j < n_free ? list[j] - rb : 0;
+        if (j < n_free) I.cnt_ff[rb + j] = kept;
+        if (lane == 0) I.start_ff[rb + j] = base;
+        const int most = static_cast<int>(__reduce_max_sync(0xffffffffu, static_cast<unsigned>(kept)));
+        int q = 0;
+        for (int i = 0; i < most; ++i) {  // warp-uniform
+            const bool in = i < kept;
+            const unsigned m = __ballot_sync(0xffffffffu, in);
+            if (in) {
+                int at, place;
+                do {  // the row's next kept entry
+                    at = S.column_at[t >> 5][q++] + (t & 31);
+                    place = staged ? S.place[at] : xq[__ldg(col + tb + at)].z;
+                } while (place < 0);
+                const int to = base + __popc(m & ((1u << lane) - 1u));
+                I.col_ff[to] = place;
+                I.hi_ff[to] = __ldg(vhi + tb + at);
+                I.lo_ff[to] = __ldg(vlo + tb + at);
+            }
+            base += __popc(m);
+        }
+    }
+    __syncthreads();  // the places have been read
+    residual_epilogue(I, list, S.row_of, n_free, tile, S.rowsum, S.coupling, S.scratch, a);
+    return kept_tile;
+}
+
+// The residual pass over sliced rows.  It reads the matrix and writes the free part of it; the places
+// of kept entries stay in shared memory between the count and the copy, and both run over a tile's
+// positions in slice order.  Random graph 1M 215 us (the CSR kernel 200), grid 121 us: what it
+// costs here the product gains back.  Four blocks per SM: 1.75 ms of device time per solve, three 1.82.
+__global__ void __launch_bounds__(kBlock, kResidualBlocks) polish_residual_slice_kernel(View v) {
+    extern __shared__ __align__(16) unsigned char dyn_smem[];
+    ResidualShared& S = *reinterpret_cast<ResidualShared*>(dyn_smem);
+    const int nu = v.ctrl->n_units;
+    for (int un = blockIdx.x; un < nu; un += gridDim.x) {
+        const int4 U = v.units[un];  // first tile, tiles, index and units of its instance
+        const Tile T0 = v.tiles[U.x];
+        if (!is_sliced(T0.variant)) continue;
+        InstDev& I = v.inst[T0.inst];
+        if (!polish_phase(I, PH_POLISH_INIT)) continue;
+        const int2 R = v.ranges[T0.inst];
+        Acc a = acc_identity();
+        int kept = 0, n_free_unit = 0;
+        for (int q = 0; q < U.y; ++q) {
+            const int t = U.x + q;
+            if (q > 0) __syncthreads();  // the previous tile's shared arrays have been read
+            const int n_free = I.free_cnt[t - R.x];
+            kept += residual_slices(I, v.tiles[t], t - R.x, n_free, S, a);
+            n_free_unit += n_free;
+        }
+        finish_residual(v, I, T0.inst, R, U, kept, n_free_unit, a);
+    }
+}
+
+constexpr int kProductAhead = 5, kProductBlocks = 4;
+// CG product over the sliced Q_FF: a slice of 32 list positions per warp, a position per lane, its sum and
+// its share of the reduction without leaving the lane; one block reduction and publication per unit.
+// Bound by the pair gathers of p on a random graph (45.5 -> 43 us, cold caches) and by the
+// launch's load-gather-reduce chain on a small one (10k rows 19 -> 16 us; grid 1M 32 us on either).  5
+// columns at 4 blocks per SM; 3 and 5 blocks measured slower.
+__global__ void __launch_bounds__(kBlock, kProductBlocks) cg_matvec_slice_kernel(View v) {
+    constexpr int kAheadPairs = kProductAhead;
+    __shared__ int first_slice[kCgUnitMax + 1];  // prefix of the tiles' slices
+    __shared__ int first_pos[kCgUnitMax];
+    __shared__ int free_of[kCgUnitMax];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    let_next_launch_begin();
+    bool waited = false;
+    const int nu = v.ctrl->n_units;
+    for (int un = blockIdx.x; un < nu; un += gridDim.x) {
+        const int4 U = v.units[un];  // first tile, tiles, index and units of its instance
+        const Tile T = v.tiles[U.x];
+        if (!is_sliced(T.variant)) continue;
+        InstDev& I = v.inst[T.inst];
+        if (I.precision != PREC_MIXED) continue;
+        const int2 R = v.ranges[T.inst];
+        if (warp == 0) {
+            const bool mine = lane < U.y;
+            const int n_free = mine ? I.free_cnt[U.x - R.x + lane] : 0, count = (n_free + 31) >> 5;
+            int incl = count;
+#pragma unroll
+            for (int o = 1; o <= kCgUnitMax; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += y;
+            }
+            if (lane <= U.y) first_slice[lane] = incl - count;  // lane U.y: the total
+            if (mine) {
+                first_pos[lane] = v.tiles[U.x + lane].row_begin;
+                free_of[lane] = n_free;
+            }
+        }
+        if (!waited) wait_for_previous_launch();  // the tables above are those of the whole loop
+        waited = true;
+        if (!polish_phase(I, PH_POLISH_CG)) {
+            __syncthreads();  // the tables are rewritten for the next unit
+            continue;
+        }
+        __syncthreads();
+        const int total = first_slice[U.y];
+        Acc a = acc_identity();
+        for (int f = warp, q = 0; f < total; f += kBlock / 32) {
+            while (f >= first_slice[q + 1]) ++q;
+            const int local = (f - first_slice[q]) * 32;
+            const int pos0 = first_pos[q] + local, pos = pos0 + lane;
+            const bool valid = local + lane < free_of[q];
+            const int cnt = valid ? I.cnt_ff[pos] : 0;
+            int base = I.start_ff[pos0];
+            const double ui = valid ? I.z[pos] : 0.0, ri = valid ? I.r[pos] : 0.0, xi = valid ? I.xf[pos] : 0.0;
+            const int most = static_cast<int>(__reduce_max_sync(0xffffffffu, static_cast<unsigned>(cnt)));
+            float2 acc = make_float2(0.f, 0.f);
+            for (int j = 0; j < most; j += kAheadPairs) {  // warp-uniform
+                SlicePairs<kAheadPairs> e;
+#pragma unroll
+                for (int m = 0; m < kAheadPairs; ++m) {
+                    const bool in = j + m < cnt;
+                    const unsigned who = __ballot_sync(0xffffffffu, in);
+                    const int k = base + __popc(who & ((1u << lane) - 1u));
+                    e.c[m] = in ? __ldg(I.col_ff + k) : -1;
+                    e.h[m] = in ? __ldg(I.hi_ff + k) : 0.f;
+                    e.l[m] = in ? __ldg(I.lo_ff + k) : 0.f;
+                    base += __popc(who);
+                }
+                acc = e.add(I.p2, acc);
+            }
+            if (valid) {
+                const double w = df_value(acc);
+                I.q[pos] = w;
+                a.a = fma(ri, ui, a.a);
+                a.obj = fma(w, ui, a.obj);
+                a.b = umax64(a.b, cg_ratio_bits(ri, xi));
+            }
+        }
+        finish_product(v, I, T.inst, R, U, a);
+    }
+    if (!waited) wait_for_previous_launch();
 }
 
 // CG vector step on the free-list positions: p = u + beta p, s = w + beta s, x += alpha p,
 // r -= alpha s, u = M^-1 r (and its FP32 pairs for the next product), every vector streamed by
 // position.  No reduction: the product kernel's finalizer already chose alpha and beta.  Instances
 // that finished CG write x back to their free rows, snapped into the box, here.
-// In a graph, block 0 also decides whether the CG loop runs another iteration: while an instance
+// In a graph (cap > 0) a body of the CG loop runs kCgTurns iterations, `turn` this one's place among them, and
+// block 0 of the last decides whether another body runs: while an instance
 // still iterates and fewer than `cap` iterations ran (the product kernel, which completed before
 // this launch, counted finishing instances down).
-__global__ void __launch_bounds__(kBlock) cg_vector_kernel(View v, cudaGraphConditionalHandle h_cg, int cap) {
+__global__ void __launch_bounds__(kBlock) cg_vector_kernel(View v, cudaGraphConditionalHandle h_cg, int cap, int turn, int launches) {
+    let_next_launch_begin();
+    wait_for_previous_launch();
+    Ctrl* ctrl = v.ctrl;
+    if (turn > 0 && ctrl->n_cg_before == 0) {  // every instance had finished an iteration ago
+        if (turn == kCgTurns - 1 && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(h_cg, 0u);
+        return;
+    }
     if (cap > 0 && blockIdx.x == 0 && threadIdx.x == 0) {
-        Ctrl* ctrl = v.ctrl;
         const int it = ++ctrl->cg_iters;
-        ctrl->kernels += 2;
-        cudaGraphSetConditional(h_cg, (ctrl->n_cg > 0 && it < cap) ? 1u : 0u);
+        ctrl->kernels += launches;
+        if (turn == kCgTurns - 1) cudaGraphSetConditional(h_cg, (ctrl->n_cg > 0 && it < cap) ? 1u : 0u);
+        static_assert(kCgTurns == 2, "the turn that writes n_cg_before is not one that reads it");
+        if (turn == 0) ctrl->n_cg_before = ctrl->n_cg;
     }
 
     const int nt = v.ctrl->n_tiles;
@@ -2208,10 +2711,11 @@ __global__ void gate_kernel(View v, cudaGraphConditionalHandle h_fp64, cudaGraph
         }
         v.ctrl->n_polish = c.polish;
         v.ctrl->n_cg = c.polish;
+        v.ctrl->n_cg_before = c.polish;
         v.ctrl->cg_iters = 0;
         long long launched = steps.checks + 1;  // check kernels and gate
         for (int k = 0; k < 3; ++k) launched += c.fista[k] > 0 ? steps.n[k] : 0;
-        launched += c.polish > 0 ? 2 : 0;
+        launched += c.polish > 0 ? steps.polish : 0;
         v.ctrl->kernels += launched;
         if (steps.present & 1u) cudaGraphSetConditional(h_fp64, c.fista[0] > 0 ? 1u : 0u);
         if (steps.present & 2u) cudaGraphSetConditional(h_mixed, c.fista[1] > 0 ? 1u : 0u);
@@ -2243,6 +2747,7 @@ __global__ void gate_plain_kernel(View v, int steps) {
         }
         v.ctrl->n_polish = c.polish;
         v.ctrl->n_cg = c.polish;
+        v.ctrl->n_cg_before = c.polish;
         v.ctrl->cg_iters = 0;
     }
 }
@@ -2409,7 +2914,8 @@ __global__ void __launch_bounds__(kGateWarps * 32) convexity_gate_kernel(const i
                                                                           const double* __restrict__ val, int n,
                                                                           GateResult* out, double* __restrict__ diag,
                                                                           float* __restrict__ vhi,
-                                                                          float* __restrict__ vlo) {
+                                                                          float* __restrict__ vlo,
+                                                                          const uint8_t* __restrict__ position_of) {
     __shared__ uint64_t sval[kGateWarps][kGateBuf];  // the values' bit patterns
     __shared__ int32_t scol[kGateWarps][kGateBuf];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -2427,6 +2933,8 @@ __global__ void __launch_bounds__(kGateWarps * 32) convexity_gate_kernel(const i
         const int last = min(n - g * 32, 32) - 1;
         const int kb = __shfl_sync(0xffffffffu, a, 0);
         const int ke = __shfl_sync(0xffffffffu, b, last);
+        // the row's own column and its place in diag: positions where the columns are positions
+        const int own = valid && position_of ? (r & ~(kSliceWindow - 1)) | __ldg(position_of + r) : r;
         float sum_lo = 0.0f, sum_hi = 0.0f, rad_lo = 0.0f, rad_hi = 0.0f;
         int nd = 0, kd = 0;  // diagonal entries of the row and the first one's position
         bool offd = false;   // a nonzero off-diagonal value (check_qp_solution's positive_diagonal)
@@ -2467,7 +2975,7 @@ __global__ void __launch_bounds__(kGateWarps * 32) convexity_gate_kernel(const i
                 abs_bounds_bits(mag, lo, hi);
                 sum_lo = __fadd_rd(sum_lo, __uint_as_float(lo));
                 sum_hi = __fadd_ru(sum_hi, __uint_as_float(hi));
-                if (bc[k] == r) {
+                if (bc[k] == own) {
                     if (nd++ == 0) kd = k + w;
                 } else {
                     rad_lo = __fadd_rd(rad_lo, __uint_as_float(lo));
@@ -2493,7 +3001,7 @@ __global__ void __launch_bounds__(kGateWarps * 32) convexity_gate_kernel(const i
                 d = __ldg(val + kd);
             } else if (nd > 1) {
                 for (int k = kd; k < b; ++k)
-                    if (__ldg(col + k) == r) d += __ldg(val + k);
+                    if (__ldg(col + k) == own) d += __ldg(val + k);
             }
             if (widen_bits(__float_as_uint(sum_hi)) >= floor_seen) {
                 double total = 0.0;
@@ -2514,13 +3022,13 @@ __global__ void __launch_bounds__(kGateWarps * 32) convexity_gate_kernel(const i
             } else {
                 double radius = 0.0;
                 for (int k = a; k < b; ++k)
-                    if (__ldg(col + k) != r) radius += fabs(__ldg(val + k));
+                    if (__ldg(col + k) != own) radius += fabs(__ldg(val + k));
                 below = d < radius;
             }
             if (below) nondominant = 1;
             if (offd) flags |= kGateOffDiagonal;
             if (negative || dm == 0 || dm > 0x7ff0000000000000ull) flags |= kGateNonPositive;  // !(Q_ii > 0)
-            if (diag) diag[r] = d;
+            if (diag) diag[own] = d;
         }
     }
 #pragma unroll
@@ -2612,18 +3120,57 @@ __global__ void __launch_bounds__(kSliceWindow) slice_order_kernel(InstDev I, in
     if (lane == 0 && valid) const_cast<int32_t*>(I.slice_base)[(w0 >> 5) + warp] = base;
 }
 
-// Second kernel: the window's entries, staged in shared memory by coalesced loads where they fit
+// Second kernel: the columns of the uploaded CSR as positions, in place (a gather of one byte per entry;
+// it needs no values, so it runs while they are still being copied: 55 us for 15M entries, which the
+// third kernel would otherwise spend after the copy, 157 us against 101).  A column out of range stays as
+// it is: the gate refuses that solve.
+__global__ void __launch_bounds__(kBlock) slice_columns_kernel(int64_t nnz, int columns, int32_t* __restrict__ col,
+                                                               const uint8_t* __restrict__ position_of) {
+    constexpr int kFlight = 8;
+    const int64_t stride = static_cast<int64_t>(gridDim.x) * kBlock;
+    for (int64_t k0 = static_cast<int64_t>(blockIdx.x) * kBlock + threadIdx.x; k0 < nnz; k0 += kFlight * stride) {
+        int32_t c[kFlight];
+        uint8_t at[kFlight];
+#pragma unroll
+        for (int q = 0; q < kFlight; ++q) c[q] = k0 + q * stride < nnz ? col[k0 + q * stride] : -1;
+#pragma unroll
+        for (int q = 0; q < kFlight; ++q)
+            at[q] = static_cast<uint32_t>(c[q]) < static_cast<uint32_t>(columns) ? __ldg(position_of + c[q]) : 0;
+#pragma unroll
+        for (int q = 0; q < kFlight; ++q)
+            if (static_cast<uint32_t>(c[q]) < static_cast<uint32_t>(columns))
+                col[k0 + q * stride] = (c[q] & ~(kSliceWindow - 1)) | at[q];
+    }
+}
+
+// Third kernel: the window's entries, staged in shared memory by asynchronous copies where they fit
 // (`cap` entries; a fuller window reads its rows from global memory), leave slice by slice, column by
-// column, their columns as positions.  Each entry is read and written once (24 bytes) and its column's
-// position gathered (one byte): 154 us for 15M entries, once per solve.  A column out of range passes through unchanged: the gate refuses
-// that solve.
-__global__ void __launch_bounds__(kSliceWindow) slice_entries_kernel(InstDev I, int n, int columns,
-                                                                    const int32_t* __restrict__ rowptr,
+// column: 24 bytes read and written per entry, once per solve (15M entries: 101 us, cold caches).  SPLIT
+// (mixed engine): the values leave as FP32 pairs.
+__device__ __forceinline__ void split_value(uint64_t vb, float& hi, float& lo) {
+    uint32_t h, l;
+    if (!split_hilo_bits(vb, h, l)) {
+        const double v = bdouble(vb);
+        const float hf = __double2float_rn(v);
+        h = __float_as_uint(hf);
+        l = __float_as_uint(__double2float_rn(v - static_cast<double>(hf)));
+    }
+    hi = __uint_as_float(h);
+    lo = __uint_as_float(l);
+}
+
+struct SliceEntriesOut {
+    int32_t* col;
+    double* val;
+    float* hi;
+    float* lo;
+};
+
+template <bool SPLIT>
+__global__ void __launch_bounds__(kSliceWindow) slice_entries_kernel(InstDev I, int n, const int32_t* __restrict__ rowptr,
                                                                     const int32_t* __restrict__ col,
                                                                     const double* __restrict__ val, int cap,
-                                                                    const uint8_t* __restrict__ position_of,
-                                                                    int32_t* __restrict__ col_out,
-                                                                    double* __restrict__ val_out) {
+                                                                    SliceEntriesOut out) {
     extern __shared__ __align__(16) unsigned char dyn_smem[];
     double* sval = reinterpret_cast<double*>(dyn_smem);
     int32_t* scol = reinterpret_cast<int32_t*>(sval + cap);
@@ -2631,27 +3178,29 @@ __global__ void __launch_bounds__(kSliceWindow) slice_entries_kernel(InstDev I, 
     const int w0 = blockIdx.x * kSliceWindow, rows = min(kSliceWindow, n - w0);
     const int kb = __ldg(rowptr + w0), ke = __ldg(rowptr + w0 + rows);
     const bool staged = ke - kb <= cap;
-    auto place = [&](int32_t c) {
-        return static_cast<uint32_t>(c) < static_cast<uint32_t>(columns) ? (c & ~(kSliceWindow - 1)) | __ldg(position_of + c) : c;
-    };
     if (staged) {
-#pragma unroll 4
         for (int k = t; k < ke - kb; k += kSliceWindow) {
-            sval[k] = __ldg(val + kb + k);
-            scol[k] = place(__ldg(col + kb + k));
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(sval + k))),
+                         "l"(val + kb + k));
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(scol + k))),
+                         "l"(col + kb + k));
         }
     }
     const bool valid = t < rows;
     const int len = valid ? __ldg(I.slice_len + w0 + t) : 0;
     const int src = valid ? __ldg(rowptr + w0 + __ldg(I.slice_row + w0 + t)) - kb : 0;
     int k = valid ? __ldg(I.slice_base + ((w0 + t) >> 5)) + lane : 0;
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     const int longest = __shfl_sync(0xffffffffu, len, 0);
+#pragma unroll 4
     for (int j = 0; j < longest; ++j) {  // warp-uniform
         const bool in = j < len;
         if (in) {
-            val_out[k] = staged ? sval[src + j] : __ldg(val + kb + src + j);
-            col_out[k] = staged ? scol[src + j] : place(__ldg(col + kb + src + j));
+            const double a = staged ? sval[src + j] : __ldg(val + kb + src + j);
+            if constexpr (SPLIT) split_value(dbits(a), out.hi[k], out.lo[k]);
+            else out.val[k] = a;
+            out.col[k] = staged ? scol[src + j] : __ldg(col + kb + src + j);
         }
         k += __popc(__ballot_sync(0xffffffffu, in));
     }
@@ -2739,6 +3288,49 @@ __global__ void __launch_bounds__(kBlock) precond_bound_kernel(InstDev I, int n)
 #pragma unroll
         for (int o = LANES / 2; o > 0; o >>= 1) sum = __fadd_ru(sum, __shfl_xor_sync(0xffffffffu, sum, o));
         if (r < n && sl == 0) best = max(best, __float_as_uint(__fmul_ru(sum, vf[r])));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
+    if (best && best < 0x00800000u) best = 0x00800000u;  // a subnormal bound: 2^-126 above it
+    if ((threadIdx.x & 31) == 0 && best)
+        atomicMax(reinterpret_cast<unsigned long long*>(I.lprec), static_cast<unsigned long long>(widen_bits(best)));
+}
+
+// The same bound over sliced rows, a position per lane; a row's sum keeps the order of LANES lanes (LANES
+// interleaved sums, then their tree), so the bound is the same to the bit (15M entries: 69 us).
+template <int LANES>
+__global__ void __launch_bounds__(kBlock) precond_bound_slice_kernel(InstDev I, int n) {
+    const int slices = (n + 31) / 32, warps = gridDim.x * (kBlock / 32);
+    const float* __restrict__ vf = I.sstep;
+    uint32_t best = 0;
+    for (int s = blockIdx.x * (kBlock / 32) + static_cast<int>(threadIdx.x >> 5); s < slices; s += warps) {
+        const int p = s * 32 + static_cast<int>(threadIdx.x & 31);
+        const int len = p < n ? __ldg(I.slice_len + p) : 0;
+        int k = __ldg(I.slice_base + s) + static_cast<int>(threadIdx.x & 31);
+        const int longest = __shfl_sync(0xffffffffu, len, 0);
+        float sum[LANES];
+#pragma unroll
+        for (int q = 0; q < LANES; ++q) sum[q] = 0.0f;
+        constexpr int kRound = LANES < 4 ? 4 : LANES;
+        for (int j = 0; j < longest; j += kRound) {  // warp-uniform
+#pragma unroll
+            for (int q = 0; q < kRound; ++q) {
+                const bool in = j + q < len;
+                if (in) {
+                    const uint32_t hb = __float_as_uint(__ldg(I.vhi + k)) & 0x7fffffffu;
+                    const float a = __uint_as_float(hb >= 0x7f800000u ? 0x7f800000u : hb + 1u);
+                    const int32_t c = __ldg(I.col + k);  // in range once the gate passes; clamped until then
+                    sum[q % LANES] = __fmaf_ru(a, __ldg(vf + (static_cast<uint32_t>(c) < static_cast<uint32_t>(n) ? c : 0)),
+                                               sum[q % LANES]);
+                }
+                k += __popc(__ballot_sync(0xffffffffu, in));
+            }
+        }
+#pragma unroll
+        for (int o = LANES / 2; o > 0; o >>= 1)
+#pragma unroll
+            for (int q = 0; q < o; ++q) sum[q] = __fadd_ru(sum[q], sum[q + o]);
+        if (p < n) best = max(best, __float_as_uint(__fmul_ru(sum[0], vf[p])));
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
@@ -3049,8 +3641,8 @@ namespace {
 // One full wave (SMs x resident blocks per SM) per tile kernel, computed once per process.
 struct Waves {
     int group[kStepGroups] = {};
-    int slices[4] = {};  // FP64, FP64 small, exact, exact small
-    int check_slices = 0;
+    int slices[6] = {};  // FP64, FP64 small, exact, exact small, mixed, mixed small
+    int check_slices = 0, check_mixed_slices = 0, check_verify_slices = 0, residual_slices = 0, matvec_slices = 0;
     int exact = 0;
     int check = 0, check_mixed = 0, check_verify = 0, polish = 0, matvec = 0, residual = 0;
 };
@@ -3096,10 +3688,27 @@ void group_waves(int sms) {
 // hide latency with whole rows in flight (12 columns, 128 registers: 10k rows 2.95 -> 2.47 ms per solve
 // against 8 columns at 6 blocks).  The two cross at about kSliceSmall rows: 40k rows 6.7 against 7.2 us a
 // step, 100k rows 10.4 against 10.2.
+// A launch that may begin while the one before it in the stream still runs (its kernel waits).
+template <class... P, class... A>
+void launch_dependent(void (*kernel)(P...), int grid, cudaStream_t s, A... args) {
+    cudaLaunchAttribute overlap;
+    overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    overlap.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(static_cast<unsigned>(grid));
+    config.blockDim = dim3(kBlock);
+    config.stream = s;
+    config.attrs = &overlap;
+    config.numAttrs = 1;
+    cudaLaunchKernelEx(&config, kernel, static_cast<P>(args)...);
+}
+
 using SliceKernel = void (*)(View, int, int);
 constexpr int kWideAhead = 5, kWideBlocks = 8, kSmallAhead = 12, kSmallBlocks = 4;
-SliceKernel slice_kernel(bool exact, bool small) {
-    if (exact) return small ? step_slice_kernel<PREC_FP64_EXACT, kSmallAhead, kSmallBlocks> : step_slice_kernel<PREC_FP64_EXACT, kWideAhead, kWideBlocks>;
+constexpr int kMixedAhead = 6, kMixedBlocks = 8;
+SliceKernel slice_kernel(int precision, bool small) {  // 0 FP64, 1 FP64_EXACT, 2 mixed
+    if (precision == 2) return small ? step_slice_f32_kernel<kSmallAhead, kSmallBlocks> : step_slice_f32_kernel<kMixedAhead, kMixedBlocks>;
+    if (precision == 1) return small ? step_slice_kernel<PREC_FP64_EXACT, kSmallAhead, kSmallBlocks> : step_slice_kernel<PREC_FP64_EXACT, kWideAhead, kWideBlocks>;
     return small ? step_slice_kernel<PREC_FP64, kSmallAhead, kSmallBlocks> : step_slice_kernel<PREC_FP64, kWideAhead, kWideBlocks>;
 }
 
@@ -3130,13 +3739,16 @@ int tile_grid(int sms) {
     group_waves<PREC_FP64>(sms);
     group_waves<PREC_MIXED>(sms);
     g_waves.exact = wave_of(step_exact_kernel, sms, 0);
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < 6; ++k) {
         int blocks = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, slice_kernel(k >= 2, k & 1), kSliceThreads, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, slice_kernel(k / 2, (k & 1) != 0), kSliceThreads, 0);
         g_waves.slices[k] = sms * (blocks < 1 ? 1 : blocks);
     }
     g_waves.check_slices = wave_of(check_slice_kernel, sms, 0);
-    cudaFuncSetAttribute(slice_entries_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 12 * kSliceStageMax);
+    g_waves.check_mixed_slices = wave_of(check_slice_mixed_kernel<FAMILY_MIXED>, sms, 0);
+    g_waves.check_verify_slices = wave_of(check_slice_mixed_kernel<FAMILY_VERIFY>, sms, 0);
+    g_waves.residual_slices = wave_of(polish_residual_slice_kernel, sms, sizeof(ResidualShared));
+    g_waves.matvec_slices = wave_of(cg_matvec_slice_kernel, sms, 0);
     g_waves.check = wave_of(check_kernel<FAMILY_FP64>, sms, kSmem8);
     g_waves.check_mixed = wave_of(check_kernel<FAMILY_MIXED>, sms, kSmem8);
     g_waves.check_verify = wave_of(check_kernel<FAMILY_VERIFY>, sms, kSmem8);
@@ -3146,7 +3758,8 @@ int tile_grid(int sms) {
     g_waves.polish = wave_of(cg_vector_kernel, sms, 0);
     int m = g_waves.exact;
     for (int w : g_waves.group) m = w > m ? w : m;
-    for (int w : {g_waves.check, g_waves.matvec, g_waves.polish, g_waves.slices[0], g_waves.slices[1], g_waves.slices[2], g_waves.slices[3]})
+    for (int w : {g_waves.check, g_waves.matvec, g_waves.polish, g_waves.slices[0], g_waves.slices[1], g_waves.slices[2], g_waves.slices[3],
+                  g_waves.slices[4], g_waves.slices[5], g_waves.matvec_slices, g_waves.residual_slices})
         m = w > m ? w : m;
     return m;
 }
@@ -3159,23 +3772,28 @@ void launch_check(const View& v, int families, int grid, cudaStream_t s) {
         check_kernel<FAMILY_VERIFY><<<pick(grid, g_waves.check_verify), kBlock, kSmem8, s>>>(v);
     }
     if (families & kCheckFp64) check_kernel<FAMILY_FP64><<<pick(grid, g_waves.check), kBlock, kSmem8, s>>>(v);
+    if (families & kCheckMixedSlices) {
+        check_slice_mixed_kernel<FAMILY_MIXED><<<pick(grid, g_waves.check_mixed_slices), kBlock, 0, s>>>(v);
+        check_slice_mixed_kernel<FAMILY_VERIFY><<<pick(grid, g_waves.check_verify_slices), kBlock, 0, s>>>(v);
+    }
     if (families & kCheckSlices) check_slice_kernel<<<pick(grid, g_waves.check_slices), kBlock, 0, s>>>(v);
 }
 
 void launch_step_group(const View& v, int group, int j, int grid, cudaStream_t s) {
-    const int wide = step_group(PREC_FP64, VAR_SLICE), small = step_group(PREC_FP64, VAR_SLICE_SMALL);
-    if (group >= kExactSlices || group == wide || group == small) {
-        const bool exact = group >= kExactSlices, is_small = group == small || group == kExactSlices + 1;
+    const int variant = group % kVariants;
+    if (group >= kExactSlices || variant == variant_index(VAR_SLICE) || variant == variant_index(VAR_SLICE_SMALL)) {
+        const int kind = group >= kExactSlices ? 1 : group >= kVariants ? 2 : 0;
+        const bool is_small = group >= kExactSlices ? group == kExactSlices + 1 : variant == variant_index(VAR_SLICE_SMALL);
         cudaLaunchAttribute overlap;
         overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
         overlap.val.programmaticStreamSerializationAllowed = 1;
         cudaLaunchConfig_t config = {};
-        config.gridDim = dim3(static_cast<unsigned>(pick(8 * grid, g_waves.slices[2 * exact + is_small])));
+        config.gridDim = dim3(static_cast<unsigned>(pick(8 * grid, g_waves.slices[2 * kind + is_small])));
         config.blockDim = dim3(kSliceThreads);
         config.stream = s;
         config.attrs = &overlap;
         config.numAttrs = j > 0 ? 1 : 0;  // the first step of a body reads what the kernels before it wrote
-        cudaLaunchKernelEx(&config, slice_kernel(exact, is_small), v, group, j);
+        cudaLaunchKernelEx(&config, slice_kernel(kind, is_small), v, group, j);
     } else if (group >= kVariants) {
         launch_group_of<PREC_MIXED>(v, group, j, grid, s);
     } else {
@@ -3190,14 +3808,19 @@ void launch_step_exact(const View& v, int j, int grid, cudaStream_t s) {
 void launch_polish_init(const View& v, int grid, cudaStream_t s) {
     polish_init_kernel<<<pick(grid, g_waves.polish), kBlock, 0, s>>>(v);
 }
-void launch_polish_residual(const View& v, int grid, cudaStream_t s) {
-    polish_residual_kernel<<<pick(grid, g_waves.residual), kBlock, 0, s>>>(v);
+void launch_polish_residual(const View& v, int families, int grid, cudaStream_t s) {
+    if (families & kCheckMixed) polish_residual_kernel<<<pick(grid, g_waves.residual), kBlock, 0, s>>>(v);
+    if (families & kCheckMixedSlices)
+        polish_residual_slice_kernel<<<pick(grid, g_waves.residual_slices), kBlock, sizeof(ResidualShared), s>>>(v);
 }
-void launch_cg_matvec(const View& v, int grid, cudaStream_t s) {
-    cg_matvec_kernel<<<pick(grid, g_waves.matvec), kBlock, 0, s>>>(v);
+void launch_cg_matvec(const View& v, int families, int grid, cudaStream_t s) {
+    // the first overlaps the vector step before it (in the same body of the loop); both wait before
+    // they read what it wrote
+    if (families & kCheckMixed) launch_dependent(cg_matvec_kernel, pick(grid, g_waves.matvec), s, v);
+    if (families & kCheckMixedSlices) launch_dependent(cg_matvec_slice_kernel, pick(grid, g_waves.matvec_slices), s, v);
 }
-void launch_cg_vector(const View& v, int grid, cudaStream_t s, cudaGraphConditionalHandle cg_loop, int cap) {
-    cg_vector_kernel<<<pick(grid, g_waves.polish), kBlock, 0, s>>>(v, cg_loop, cap);
+void launch_cg_vector(const View& v, int products, int grid, cudaStream_t s, cudaGraphConditionalHandle cg_loop, int cap, int turn) {
+    launch_dependent(cg_vector_kernel, pick(grid, g_waves.polish), s, v, cg_loop, cap, turn, products + 1);
 }
 
 void launch_gate(const View& v, const cudaGraphConditionalHandle* fista, cudaGraphConditionalHandle polish,
@@ -3243,7 +3866,10 @@ void launch_precondition(const InstDev& rec, int64_t n, const double* val, bool 
         if (g > 152 * 16) g = 152 * 16;
         if (g < 1) g = 1;
         const int gi = static_cast<int>(g), ni = static_cast<int>(n);
-        if (lanes == 8) precond_bound_kernel<8><<<gi, kBlock, 0, s>>>(rec, ni);
+        if (rec.slice_len && lanes == 8) precond_bound_slice_kernel<8><<<static_cast<int>(grid), kBlock, 0, s>>>(rec, ni);
+        else if (rec.slice_len && lanes == 4) precond_bound_slice_kernel<4><<<static_cast<int>(grid), kBlock, 0, s>>>(rec, ni);
+        else if (rec.slice_len) precond_bound_slice_kernel<2><<<static_cast<int>(grid), kBlock, 0, s>>>(rec, ni);
+        else if (lanes == 8) precond_bound_kernel<8><<<gi, kBlock, 0, s>>>(rec, ni);
         else if (lanes == 4) precond_bound_kernel<4><<<gi, kBlock, 0, s>>>(rec, ni);
         else precond_bound_kernel<2><<<gi, kBlock, 0, s>>>(rec, ni);
     }
@@ -3286,14 +3912,14 @@ void launch_power_lipschitz(const InstDev& rec, int64_t n, const double* val, bo
 }
 
 void launch_gate_raw(int64_t n, const int32_t* rowptr, const int32_t* col, const double* val, GateResult* out,
-                     double* diag, float* vhi, float* vlo, cudaStream_t s) {
+                     double* diag, float* vhi, float* vlo, const uint8_t* position_of, cudaStream_t s) {
     cudaMemsetAsync(out, 0, sizeof(GateResult), s);
     const int64_t groups = (n + 31) / 32;
     int64_t grid = (groups + kGateWarps - 1) / kGateWarps;
     if (grid > 152 * 8) grid = 152 * 8;
     if (grid < 1) grid = 1;
     convexity_gate_kernel<<<static_cast<int>(grid), kGateWarps * 32, 0, s>>>(rowptr, col, val, static_cast<int>(n), out,
-                                                                             diag, vhi, vlo);
+                                                                             diag, vhi, vlo, position_of);
 }
 
 void launch_slice_order(const InstDev& rec, int64_t n, const int32_t* rowptr, uint8_t* position_of, cudaStream_t s) {
@@ -3301,22 +3927,34 @@ void launch_slice_order(const InstDev& rec, int64_t n, const int32_t* rowptr, ui
     slice_order_kernel<<<windows, kSliceWindow, 0, s>>>(rec, static_cast<int>(n), rowptr, position_of);
 }
 
-void launch_slice_entries(const InstDev& rec, int64_t n, int64_t columns, int64_t nnz, const int32_t* rowptr,
-                          const int32_t* col, const double* val, const uint8_t* position_of, int32_t* col_out,
-                          double* val_out, cudaStream_t s) {
+void launch_slice_columns(int64_t nnz, int64_t columns, int32_t* col, const uint8_t* position_of, cudaStream_t s) {
+    if (nnz <= 0) return;
+    int64_t grid = (nnz + 8 * kBlock - 1) / (8 * kBlock);
+    if (grid > 152 * 8) grid = 152 * 8;
+    slice_columns_kernel<<<static_cast<int>(grid), kBlock, 0, s>>>(nnz, static_cast<int>(columns), col, position_of);
+}
+
+namespace {
+template <bool SPLIT>
+void slice_entries(const InstDev& rec, int64_t n, int64_t nnz, const int32_t* rowptr, const int32_t* col, const double* val,
+                   const SliceEntriesOut& out, cudaStream_t s) {
     // shared memory for a window of average rows and a fifth more
     const int64_t want = kSliceWindow * nnz / n * 6 / 5 + kSliceWindow;
     const int cap = static_cast<int>(want < 1024 ? 1024 : want > kSliceStageMax ? kSliceStageMax : (want + 1) & ~int64_t(1));
     const int windows = static_cast<int>((n + kSliceWindow - 1) / kSliceWindow);
-    cudaFuncSetAttribute(slice_entries_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 12 * kSliceStageMax);
-    slice_entries_kernel<<<windows, kSliceWindow, 12 * cap, s>>>(rec, static_cast<int>(n), static_cast<int>(columns), rowptr, col,
-                                                               val, cap, position_of, col_out, val_out);
+    cudaFuncSetAttribute(slice_entries_kernel<SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 12 * kSliceStageMax);
+    slice_entries_kernel<SPLIT><<<windows, kSliceWindow, 12 * cap, s>>>(rec, static_cast<int>(n), rowptr, col, val, cap, out);
+}
+}  // namespace
+
+void launch_slice_entries(const InstDev& rec, int64_t n, int64_t nnz, const int32_t* rowptr, const int32_t* col,
+                          const double* val, int32_t* col_out, double* val_out, cudaStream_t s) {
+    slice_entries<false>(rec, n, nnz, rowptr, col, val, SliceEntriesOut{col_out, val_out, nullptr, nullptr}, s);
 }
 
-void launch_slice_rows(const InstDev& rec, int64_t n, int64_t nnz, const int32_t* rowptr, const int32_t* col,
-                       const double* val, uint8_t* position_of, int32_t* col_out, double* val_out, cudaStream_t s) {
-    launch_slice_order(rec, n, rowptr, position_of, s);
-    launch_slice_entries(rec, n, n, nnz, rowptr, col, val, position_of, col_out, val_out, s);
+void launch_slice_entries_split(const InstDev& rec, int64_t n, int64_t nnz, const int32_t* rowptr, const int32_t* col,
+                                const double* val, int32_t* col_out, float* hi_out, float* lo_out, cudaStream_t s) {
+    slice_entries<true>(rec, n, nnz, rowptr, col, val, SliceEntriesOut{col_out, nullptr, hi_out, lo_out}, s);
 }
 
 void launch_unslice(int64_t n, const uint8_t* slice_row, const double* x, double* out, cudaStream_t s) {
@@ -3333,10 +3971,9 @@ void launch_slice_vector(int64_t n, const uint8_t* slice_row, const double* x, d
     slice_vector_kernel<<<static_cast<int>(grid), kBlock, 0, s>>>(static_cast<int>(n), slice_row, x, out);
 }
 
-void launch_gate(const InstDev& rec, int64_t n, const double* val, cudaStream_t s) {
-    const bool split = rec.precision == PREC_MIXED;
+void launch_gate(const InstDev& rec, int64_t n, const double* val, bool split, const uint8_t* position_of, cudaStream_t s) {
     launch_gate_raw(n, rec.rowptr, rec.col, val, rec.gate, const_cast<double*>(rec.diag),
-                    split ? const_cast<float*>(rec.vhi) : nullptr, split ? const_cast<float*>(rec.vlo) : nullptr, s);
+                    split ? const_cast<float*>(rec.vhi) : nullptr, split ? const_cast<float*>(rec.vlo) : nullptr, position_of, s);
 }
 
 void launch_prepare_instance(const InstDev& rec, int64_t n, cudaStream_t s) {

@@ -19,16 +19,22 @@ void launch_step_exact(const View& v, int j, int grid, cudaStream_t s);
 // Check kernels of a body: one per family that has instances (bits of kCheck*).
 constexpr int kCheckFp64 = 1;    // FP64 engines over the CSR
 constexpr int kCheckSlices = 2;  // FP64 engines over sliced rows
-constexpr int kCheckMixed = 4;   // mixed engine: the FP32 iterate and the polished point (two kernels)
+constexpr int kCheckMixed = 4;   // mixed engine over the CSR: the FP32 iterate and the polished point (two kernels)
+constexpr int kCheckMixedSlices = 8;  // the same over sliced rows
 constexpr int check_launches(int families) {
-    return ((families & kCheckFp64) ? 1 : 0) + ((families & kCheckSlices) ? 1 : 0) + ((families & kCheckMixed) ? 2 : 0);
+    return ((families & kCheckFp64) ? 1 : 0) + ((families & kCheckSlices) ? 1 : 0) + ((families & kCheckMixed) ? 2 : 0) +
+           ((families & kCheckMixedSlices) ? 2 : 0);
 }
+// Residual and CG product kernels of a body (kCheckMixed, kCheckMixedSlices of `families`).
+constexpr int polish_launches(int families) { return ((families & kCheckMixed) ? 1 : 0) + ((families & kCheckMixedSlices) ? 1 : 0); }
 void launch_polish_init(const View& v, int grid, cudaStream_t s);
-void launch_polish_residual(const View& v, int grid, cudaStream_t s);
-void launch_cg_matvec(const View& v, int grid, cudaStream_t s);
-// cap > 0 (inside a graph): also sets cg_loop, the WHILE handle of the CG loop, allowing at
-// most `cap` iterations per body.  cap = 0: no handle is touched (host-driven launches).
-void launch_cg_vector(const View& v, int grid, cudaStream_t s, cudaGraphConditionalHandle cg_loop = 0, int cap = 0);
+void launch_polish_residual(const View& v, int families, int grid, cudaStream_t s);
+void launch_cg_matvec(const View& v, int families, int grid, cudaStream_t s);
+// cap > 0 (inside a graph): the last of a body's kCgTurns also sets cg_loop, the WHILE handle of the CG
+// loop, allowing at most `cap` iterations per polish branch.  cap = 0: no handle is touched (host-driven launches).
+// products: product kernels launched before it (for the count of kernels)
+void launch_cg_vector(const View& v, int products, int grid, cudaStream_t s, cudaGraphConditionalHandle cg_loop = 0, int cap = 0,
+                      int turn = 0);
 // Single-block control kernels that steer the conditional graph nodes.
 // fista[k]: handle of the IF node of the precision-k step launches; polish: the IF node of the
 // polish branch; cg_loop: the WHILE node of its CG loop.  `steps.n[k]`: kernels inside the
@@ -36,6 +42,7 @@ void launch_cg_vector(const View& v, int grid, cudaStream_t s, cudaGraphConditio
 struct StepLaunches {
     int n[3];
     int checks;        // check kernels of a body
+    int polish;        // kernels at the head of the polish branch
     unsigned present;  // bit k: the graph has a branch for precision k (bit 1: and the polish)
 };
 void launch_gate(const View& v, const cudaGraphConditionalHandle* fista, cudaGraphConditionalHandle polish,
@@ -48,26 +55,26 @@ void launch_control_plain(const View& v, int steps, cudaStream_t s);
 // Admission, first kernel: the convexity gate and Gershgorin bound of the uploaded full CSR
 // (FP64 values `val`) into *rec.gate (cleared first), the FP64 diagonal into rec.diag and, for the
 // mixed engine, the hi/lo FP32 values into rec.vhi/rec.vlo.  The later admission kernels read L there.
-void launch_gate(const InstDev& rec, int64_t n, const double* val, cudaStream_t s);
-// Admission of a sliced instance, after the gate: the order of its rows (slice_len, slice_row,
-// slice_base of `rec`), its vectors (c, l, u, diag) brought into that order in place, and its entries
-// (columns as positions) into col_out, val_out.  rowptr, col, val: the uploaded CSR; position_of: n
-// bytes of scratch.
-void launch_slice_rows(const InstDev& rec, int64_t n, int64_t nnz, const int32_t* rowptr, const int32_t* col,
-                       const double* val, uint8_t* position_of, int32_t* col_out, double* val_out, cudaStream_t s);
-// The two steps by themselves: the order of `n` rows (rec's vectors may be null), and their entries, whose
-// columns (below `columns`) are mapped by position_of.
+// position_of: the columns are positions already (launch_slice_columns); the diagonal goes there too.
+void launch_gate(const InstDev& rec, int64_t n, const double* val, bool split, const uint8_t* position_of, cudaStream_t s);
+// Admission of a sliced instance, three kernels: the order of its rows (slice_len, slice_row, slice_base of
+// `rec`; its vectors c, l, u, diag, where given, move into that order in place) from the uploaded row
+// pointers, with each row's position in its window in position_of (n bytes); the uploaded columns as
+// positions, in place (below `columns`); and the entries in slice order into col_out and val_out, or,
+// for the mixed engine, as FP32 pairs.
 void launch_slice_order(const InstDev& rec, int64_t n, const int32_t* rowptr, uint8_t* position_of, cudaStream_t s);
-void launch_slice_entries(const InstDev& rec, int64_t n, int64_t columns, int64_t nnz, const int32_t* rowptr,
-                          const int32_t* col, const double* val, const uint8_t* position_of, int32_t* col_out,
-                          double* val_out, cudaStream_t s);
+void launch_slice_columns(int64_t nnz, int64_t columns, int32_t* col, const uint8_t* position_of, cudaStream_t s);
+void launch_slice_entries(const InstDev& rec, int64_t n, int64_t nnz, const int32_t* rowptr, const int32_t* col,
+                          const double* val, int32_t* col_out, double* val_out, cudaStream_t s);
+void launch_slice_entries_split(const InstDev& rec, int64_t n, int64_t nnz, const int32_t* rowptr, const int32_t* col,
+                                const double* val, int32_t* col_out, float* hi_out, float* lo_out, cudaStream_t s);
 // A vector brought into slice order: out[position] = x[row].
 void launch_slice_vector(int64_t n, const uint8_t* slice_row, const double* x, double* out, cudaStream_t s);
 // x of a sliced instance in row order: out[row] = x[position].
 void launch_unslice(int64_t n, const uint8_t* slice_row, const double* x, double* out, cudaStream_t s);
 // The same pass on raw device pointers (diag, vhi, vlo may be null: not stored).
 void launch_gate_raw(int64_t n, const int32_t* rowptr, const int32_t* col, const double* val, GateResult* out,
-                     double* diag, float* vhi, float* vlo, cudaStream_t s);
+                     double* diag, float* vhi, float* vlo, const uint8_t* position_of, cudaStream_t s);
 // Admission, mixed engine, after launch_gate on the same stream: 1/diag, preconditioner scales and
 // the FP32 cost and bounds (nothing for the FP64 engines).
 // The record is passed by value: the instance is installed in its slot later, between graph launches.
@@ -91,8 +98,8 @@ void launch_rearm(const View& v, const InstDev* stage, const int32_t* slots, con
 // primals in row order, written to where `jobs` says (spans: job index, first row; all page-locked).
 void launch_collect(const View& v, const CollectJob* jobs, const int2* spans, int n_spans, int32_t* statuses, Ctrl* ctrl,
                     cudaStream_t s);
-// One launch in place of a copy per array: pieces of host memory that the device can read directly
-// (page-locked, or any on a device with access to pageable memory), 4-byte multiples.
+// One launch in place of a copy per array: pieces of page-locked host memory,
+// 4-byte multiples.
 struct UploadPieces {
     static constexpr int kMost = 8;
     int count = 0;

@@ -17,35 +17,39 @@ __device__ __forceinline__ void let_next_launch_begin() { asm volatile("griddepc
 // before it + lane: the lane's address advances by the count of active lanes.  AHEAD columns
 // are loaded together (entries, then gathers) before the first product.
 // EXACT: products and sums rounded separately from 0.0, the reference loop's arithmetic.
-template <int AHEAD>
+template <int AHEAD, class T = double>
 struct SliceColumns {  // AHEAD columns of a slice: this lane's columns (-1: the row has ended) and values
     int c[AHEAD];
-    double a[AHEAD];
-    __device__ __forceinline__ void load(const int32_t* __restrict__ col, const double* __restrict__ val, int left, int& k) {
+    T a[AHEAD];
+    __device__ __forceinline__ void load(const int32_t* __restrict__ col, const T* __restrict__ val, int left, int& k) {
 #pragma unroll
         for (int q = 0; q < AHEAD; ++q) {
             const bool in = q < left;
             c[q] = in ? __ldg(col + k) : -1;
-            a[q] = in ? __ldg(val + k) : 0.0;
+            a[q] = in ? __ldg(val + k) : T(0);
             k += __popc(__ballot_sync(0xffffffffu, in));
         }
     }
     // adds the first `columns` (warp-uniform) of them; a column past the slice's longest row costs
     // no FP64 issue slot
     template <bool EXACT>
-    __device__ __forceinline__ double add(const double* x, int columns, double acc) const {
-        double xv[AHEAD];
+    __device__ __forceinline__ T add(const T* x, int columns, T acc) const {
+        T xv[AHEAD];
 #pragma unroll
-        for (int q = 0; q < AHEAD; ++q) xv[q] = c[q] >= 0 ? x[c[q]] : 0.0;
+        for (int q = 0; q < AHEAD; ++q) xv[q] = c[q] >= 0 ? x[c[q]] : T(0);
         return sum<EXACT, 0>(xv, columns, acc);
     }
 
 private:
     template <bool EXACT, int Q>
-    __device__ __forceinline__ double sum(const double* xv, int columns, double acc) const {
+    __device__ __forceinline__ T sum(const T* xv, int columns, T acc) const {
         if constexpr (Q < AHEAD) {
             if (Q >= columns) return acc;
-            if (c[Q] >= 0) acc = EXACT ? __dadd_rn(acc, __dmul_rn(a[Q], xv[Q])) : fma(a[Q], xv[Q], acc);
+            if constexpr (EXACT) {
+                if (c[Q] >= 0) acc = __dadd_rn(acc, __dmul_rn(a[Q], xv[Q]));
+            } else {
+                if (c[Q] >= 0) acc = fma(a[Q], xv[Q], acc);
+            }
             return sum<EXACT, Q + 1>(xv, columns, acc);
         } else {
             return acc;

@@ -80,7 +80,9 @@ typedef struct bqp_options {
                                  dual-gap gate (src/qp_admm.cpp:72-78,106-116)                  */
     double  offset;           /* constant term of the objective (LinearProblem::offset)          */
     int32_t kernel_variant;   /* SpMV structure of the FISTA step: -1 auto (tuning default), 0 block-
-                                 staged tile, 64 warp-staged rows, 1/2/4/8/16/32 lanes per row     */
+                                 staged tile, 64 warp-staged rows, 1/2/4/8/16/32 lanes per row.
+                                 Mixed instances of short rows run on sliced rows in the order
+                                 of sums that 0, 64, 1 and 2 name                                  */
     int32_t scaling;          /* mixed engine: 0 auto (= 1), 1 diagonally preconditioned FISTA steps
                                  (per-row step 1 / (L' Q_ii), L' the Gershgorin bound of
                                  D^-1/2 Q D^-1/2: FISTA in Jacobi-scaled variables, with iterates,

@@ -94,3 +94,31 @@ def test_resolve_and_batch_of_sliced_solves_keep_their_bits(engine):
             engine.resolve(ids)
     for i in ids:
         engine.release(i)
+
+
+@pytest.mark.parametrize('n,hub,empty', CASES)
+def test_sliced_mixed_engine_is_verified(engine, n, hub, empty):
+    """The mixed engine (FP32 steps, FP64 checks and polish on the same layout): verified at 1e-6 by the
+    oracle, the objective within 1e-7 of the oracle's (the bar of the engine's parity tests)."""
+    rng = np.random.default_rng(100 * n + hub)
+    args = problem(n, rng, hub, empty)
+    rowptr, col, val, _ = rows_of(n, *args[:3])
+    _, _, st_ref = O.solve_box(*args, tol=1e-9, threads=1)
+    o = boxqp.options_struct(1e-6, 60.0, 200000, 'mixed')
+    x, st = engine.solve(rowptr, col, val, *args[3:], o)
+    assert boxqp.STATUS_NAMES[st.status] == 'optimal'
+    assert O.check(*args, x, tol=1e-6)['verified'] == 1.0
+    assert abs(st.objective - st_ref['objective']) <= 1e-7 * (1 + abs(st_ref['objective']))
+
+
+@pytest.mark.parametrize('n', [2, 256, 513, 1025, 70001])
+def test_sliced_chains_keep_the_row_order(engine, n):
+    """Tridiagonal rows (the end rows are shorter, so the order within the first and last window is not
+    the row order): the polish's chains must follow the rows, or CG needs tens of iterations."""
+    inst = boxqp.planted('tridiagonal', n=n, lower_triplets=True)
+    o = boxqp.options_struct(1e-6, 60.0, 200000, 'mixed')
+    x, st = engine.solve(inst['rowptr'], inst['col'], inst['val'], inst['c'], inst['lower'], inst['upper'], o)
+    assert boxqp.STATUS_NAMES[st.status] == 'optimal'
+    assert st.polish_iterations <= 15
+    args = (inst['hrow'], inst['hcol'], inst['hval'], inst['c'], inst['lower'], inst['upper'])
+    assert O.check(*args, x, tol=1e-6)['verified'] == 1.0
