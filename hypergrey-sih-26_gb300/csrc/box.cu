@@ -114,8 +114,8 @@ __global__ void box_start_kernel(int64_t n, const double* l, const double* u, do
 // The verification reduction needs global scratch for its per-block partials, its completion
 // counter and its 8 result values.  bqp_check_device_noalloc takes that scratch from this
 // file-scope device array instead of cudaMalloc: 96 KiB in every context that loads this
-// module, held until the context ends.  At most 1024 blocks of partials fit, which bounds n to
-// kNoAllocMaxRows.  In host code the name of the array is only a host-side stand-in, so its
+// module, held until the context ends (the check's partials, 608 blocks at most, take 49 KiB of it); it
+// serves up to kNoAllocMaxRows rows.  In host code the name of the array is only a host-side stand-in, so its
 // device address is looked up with cudaGetSymbolAddress, with the device current, once per
 // context: the lookup is cached under the current context's unique id (cuCtxGetId), so a
 // context that is destroyed and recreated (cudaDeviceReset) gets a fresh lookup instead of a

@@ -325,16 +325,20 @@ int choose_variant(int64_t n, int64_t nnz, int64_t longest_row, const bqp_option
 }
 
 // CG and check work units of one instance (its `count` tiles at t), appended to `out` as {first tile, tiles,
-// index, units}, the tiles counted from the instance's first: as many units as the product kernel has resident blocks (`slots`), so that one
-// round runs them on the whole GPU, but units of about kCgUnitMin tiles at least; the tiles are
-// spread evenly (sizes differ by one at most), and no unit goes above kCgRowsum rows (the row
-// sums' shared buffer; units of kCgUnitMin tiles always fit).  At least 4 / 2 / 1 tiles: a 10k-row mixed
-// solve 457 / 430 / 420 us, the FP64 one 2.10 / 1.95 / 1.95 ms, 256 uneven solves 2.00 / 2.03 / 2.12 ms
-// on the device.  Depends on the instance alone, so
-// the product's partial sums, and the CG iterates, are the same in a batch as solo.
-void cg_units(const Tile* t, int count, int slots, std::vector<int4>& out) {
+// index, units}, the tiles counted from the instance's first: as many units as the product kernel has
+// resident blocks (`slots`), so that one round runs them on the whole GPU, but units of about
+// kCgUnitMin tiles at least; the tiles are spread evenly (sizes differ by one at most), and no unit
+// goes above kCgRowsum rows (the row sums' shared buffer; units of kCgUnitMin tiles always fit).
+// FP64 instances take single tiles: their units serve the check alone, which the FP64 pipe of the
+// SM bounds (1024 rows of 11 entries take 10 us on one), 10k rows 2.03 -> 1.95 ms.  So do small mixed
+// instances, whose CG iterations are latency: 1k rows 230 -> 197 us, 256 uneven solves 1.33 ms on
+// the device either way; with up to 32 tiles these take 1.42 ms, with any number 1.45 (a unit costs
+// its block a reduction and a publication).  Depends on the instance alone, so the partial sums, and
+// the CG iterates, are the same in a batch as solo.
+void cg_units(const Tile* t, int count, int slots, bool fp64, std::vector<int4>& out) {
     const int fewest = (count + kCgUnitMax - 1) / kCgUnitMax;
-    const int most = std::max(1, (count + kCgUnitMin - 1) / kCgUnitMin);
+    const int least = fp64 || count <= kCgSmall ? 1 : kCgUnitMin;
+    const int most = std::max(1, (count + least - 1) / least);
     int u = std::max(fewest, std::min(std::max(slots, 1), most));
     for (;; ++u) {
         bool fits = true;
@@ -1726,7 +1730,7 @@ bool Engine::install(std::vector<Job*>& jobs, std::string& why) {
         for (Tile& t : j.tiles) t.inst = slot;
         for (Tile& t : j.items) t.inst = slot;
         j.units.clear();
-        cg_units(j.tiles.data(), static_cast<int>(j.tiles.size()), cg_slots_, j.units);
+        cg_units(j.tiles.data(), static_cast<int>(j.tiles.size()), cg_slots_, j.opt.precision != PREC_MIXED, j.units);
     }
     if (!cuda_ok(cudaStreamWaitEvent(stream_, uev_, 0), why, "upload order")) return false;
     if (!rearm(jobs, why)) return false;

@@ -18,6 +18,7 @@ constexpr int kTileNnz = 4096;       // target nonzeros per tile
 constexpr int kTileRows = 512;       // maximum rows per tile
 constexpr int kCgUnitMin = 2;        // tiles per work unit of the polish CG product and the sliced check: about
 constexpr int kCgUnitMax = 8;        //   this many at least, and up to this many for large instances (cg_units)
+constexpr int kCgSmall = 16;         // tiles up to which a mixed instance's units are single tiles (cg_units)
 constexpr int kCgRowsum = 4 * kTileRows;  // rows per CG work unit at most (its row sums, 16 KB)
 constexpr int kCgTurns = 2;          // CG iterations per body of the graph's CG loop (a body's start costs several us)
 constexpr int kCgGroups = 2;         // row groups per warp whose loads the CG product keeps in flight

@@ -121,34 +121,6 @@ __device__ __forceinline__ Acc combine(const Acc& x, const Acc& y) {
     r.flags = x.flags | y.flags;
     return r;
 }
-__device__ __forceinline__ Acc shfl_acc(const Acc& x, int o) {
-    Acc r;
-    r.obj = shfl_xor(x.obj, o); r.bnd = shfl_xor(x.bnd, o); r.sep = shfl_xor(x.sep, o); r.a = shfl_xor(x.a, o);
-    r.stat = shfl_xor(x.stat, o); r.prim = shfl_xor(x.prim, o); r.b = shfl_xor(x.b, o);
-    r.hash = shfl_xor(x.hash, o);
-    r.nact = shfl_xor(x.nact, o);
-    r.flags = shfl_xor(x.flags, o);
-    return r;
-}
-
-// Fixed-order block reduction; the result is valid in thread 0.
-__device__ Acc block_reduce(Acc v) {
-    __shared__ Acc warp_part[kBlock / 32];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = combine(v, shfl_acc(v, o));
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) warp_part[warp] = v;
-    __syncthreads();
-    if (warp == 0) {
-        Acc w = lane < kBlock / 32 ? warp_part[lane] : acc_identity();
-#pragma unroll
-        for (int o = (kBlock / 64); o > 0; o >>= 1) w = combine(w, shfl_acc(w, o));
-        v = w;
-    }
-    __syncthreads();
-    return v;
-}
-
 // The check's reduction: the two FP64 sums it always needs (objective, tangent bound), the
 // separable bound only for the diagonal dual-gap gate (GATE, a template parameter so that no
 // FP64 addition runs for it otherwise), and the integer fields; the CG fields (a, b) stay out.
@@ -364,13 +336,61 @@ __device__ __forceinline__ unsigned mix_index(unsigned k) {
     return k ^ (k >> 13);
 }
 
+// The largest stationarity ratio |x - P(x - g)| / (1 + |x|) without a division per row: rows are ranked
+// by FP32 bounds of their ratios, the only row that can still be a thread's largest waits
+// undivided, and after the last row the lanes whose row can be the warp's largest divide once.  Two rows
+// whose bounds overlap are both divided.  The maximum is the one the plain FP64 form gives, bit
+// for bit.  A division costs a warp as much of the FP64 pipe as the rest of a tridiagonal row's
+// check, and dividing wherever a thread's own maximum might rise divided almost every row: 59 us per
+// check of 1M tridiagonal rows, now 45.
+struct StatMax {
+    unsigned long long num, x;  // bits of the waiting row's |x - P(x - g)| and of its x; num 0: none
+    float lo, up;               // bounds of the largest ratio so far
+};
+// `floor`: the bits of a ratio that other blocks of the check have already reached
+__device__ __forceinline__ StatMax stat_max(unsigned long long floor) {
+    uint32_t rd, ru;
+    abs_bounds_bits(floor, rd, ru);
+    return StatMax{0, 0, __uint_as_float(rd), __uint_as_float(ru)};
+}
+__device__ __forceinline__ unsigned long long stat_ratio(unsigned long long num, unsigned long long x) {
+    const unsigned long long q = dbits(bdouble(num) / (1.0 + fabs(bdouble(x))));
+    return finite_bits(q) ? q : dbits(kInf);
+}
+__device__ __forceinline__ void stat_row(Acc& a, StatMax& m, unsigned long long num, unsigned long long x) {
+    if (!ratio_may_exceed(num, x, widen_bits(__float_as_uint(m.lo)))) return;
+    uint32_t nd, nu, xd, xu;
+    abs_bounds_bits(num, nd, nu);
+    abs_bounds_bits(x & kAbsMask64, xd, xu);
+    // RU(num) / RD(1 + |x|) within 2 units in the last place, and the margins cover that, the three
+    // roundings (a unit each) and those of the FP64 form; outside 2^-60 .. 2^60 the bounds 0 and
+    // num (1 + |x| is at least 1)
+    float lo = 0.f, up = __uint_as_float(nu);
+    const float den = __fadd_rd(1.f, __uint_as_float(xd));
+    if (up > 0x1p-60f && up < 0x1p60f && den < 0x1p60f) {
+        const float q = __fdividef(up, den);
+        lo = q * (1.f - 0x1p-19f);
+        up = q * (1.f + 0x1p-19f);
+    }
+    if (up < m.lo) return;
+    if (lo > m.up) {
+        m = StatMax{num, x, lo, up};
+    } else if (num != m.num || x != m.x) {
+        a.stat = umax64(a.stat, stat_ratio(num, x));
+        if (m.num) a.stat = umax64(a.stat, stat_ratio(m.num, m.x));
+        m = StatMax{0, 0, fmaxf(lo, m.lo), fmaxf(up, m.up)};
+    }
+}
+// After a thread's last row, by every thread of the block.
+__device__ __forceinline__ void stat_settle(Acc& a, const StatMax& m) {
+    const unsigned best = __reduce_max_sync(0xffffffffu, __float_as_uint(m.lo));
+    if (m.num && __float_as_uint(m.up) >= best) a.stat = umax64(a.stat, stat_ratio(m.num, m.x));
+}
+
 // One row of check_qp_solution.  The comparisons and finiteness tests run on the bit patterns
-// (integer pipes) and the stationarity ratio is divided in FP64 only where it can raise the
-// running maximum: this thread's, or `floor`, a maximum other tiles of the same check already
-// reached.  The maximum is the one the plain FP64 form gives, bit for bit.
-__device__ __forceinline__ void check_row(Acc& a, double xi, double gq, double ci, double li, double ui, double di,
-                                          int gate, int row, bool at_lower, bool at_upper,
-                                          unsigned long long floor = 0) {
+// (integer pipes).
+__device__ __forceinline__ void check_row(Acc& a, StatMax& m, double xi, double gq, double ci, double li, double ui,
+                                          double di, int gate, int row, bool at_lower, bool at_upper) {
     const uint64_t xb = dbits(xi);
     if (!finite_bits(xb)) {
         a.flags |= 1;
@@ -386,14 +406,8 @@ __device__ __forceinline__ void check_row(Acc& a, double xi, double gq, double c
     const uint64_t cb = less_bits(lb, mb) ? mb : lb;
     const double num = fabs(xi - bdouble(cb));
     const uint64_t nb = dbits(num);
-    unsigned long long res = 0;  // 0: the ratio leaves the maximum as it is
-    if (!finite_bits(gb) || !finite_bits(nb)) {
-        res = dbits(kInf);
-    } else if (ratio_may_exceed(nb, xb, umax64(a.stat, floor))) {
-        const double q = num / (1.0 + fabs(xi));
-        res = finite_bits(dbits(q)) ? dbits(q) : dbits(kInf);
-    }
-    a.stat = umax64(a.stat, res);
+    if (!finite_bits(gb) || !finite_bits(nb)) a.stat = dbits(kInf);
+    else stat_row(a, m, nb, xb);
     // scaled bound violation, only where the bound is violated (iterates are clamped):
     // li - xi > 0 exactly when xi < li, xi - ui > 0 exactly when ui < xi
     if (less_bits(xb, lb)) a.prim = umax64(a.prim, dbits((li - xi) / (1.0 + fabs(li) + fabs(xi))));
@@ -405,8 +419,8 @@ __device__ __forceinline__ void check_row(Acc& a, double xi, double gq, double c
         else a.flags |= 2;
     }
     if (gate) {
-        double m = smax(li, smin(ui, -ci / di));
-        a.sep += 0.5 * di * m * m + ci * m;
+        const double y = smax(li, smin(ui, -ci / di));
+        a.sep += 0.5 * di * y * y + ci * y;
     }
     if (at_lower) {
         a.hash ^= mix_index(2u * static_cast<unsigned>(row));
@@ -643,6 +657,7 @@ __device__ __forceinline__ double gate_diag(const CheckSrc& s, int r, double fal
 template <int MODE>
 __device__ void check_rows(const CheckSrc& s, int variant, int rb, int re, Acc& a, unsigned long long floor = 0) {
     const int32_t* __restrict__ col = s.col;
+    StatMax m = stat_max(floor);
     if constexpr (MODE == 0) {
         tile_rows<double>(
             variant, s.rowptr, rb, re, [&](int k) { return __ldg(s.val64 + k) * s.x64[__ldg(col + k)]; },
@@ -655,8 +670,8 @@ __device__ void check_rows(const CheckSrc& s, int variant, int rb, int re, Acc& 
                     di = gate_diag(s, r, __ldg(s.rowptr + r + 1) > ks ? __ldg(s.val64 + ks) : 0.0);
                 }
                 const double li = s.l[r], ui = s.u[r];
-                check_row(a, xi, gq, s.c[r], li, ui, di, s.gate, r, less_equal_bits(dbits(xi), dbits(li)),
-                          less_equal_bits(dbits(ui), dbits(xi)), floor);
+                check_row(a, m, xi, gq, s.c[r], li, ui, di, s.gate, r, less_equal_bits(dbits(xi), dbits(li)),
+                          less_equal_bits(dbits(ui), dbits(xi)));
             });
     } else if constexpr (MODE == 1) {
         tile_rows<float2>(
@@ -668,7 +683,7 @@ __device__ void check_rows(const CheckSrc& s, int variant, int rb, int re, Acc& 
                 if (s.gate) {
                     const int ks = __ldg(s.rowptr + r);
                     const double d0 = __ldg(s.rowptr + r + 1) > ks ? static_cast<double>(__ldg(s.vhi + ks)) + __ldg(s.vlo + ks) : 0.0;
-                    check_row(a, static_cast<double>(xf), df_value(acc), s.c[r], s.l[r], s.u[r], gate_diag(s, r, d0),
+                    check_row(a, m, static_cast<double>(xf), df_value(acc), s.c[r], s.l[r], s.u[r], gate_diag(s, r, d0),
                               1, r, xf <= s.l32[r], xf >= s.u32[r]);
                 } else {
                     check_row_f32(a, xf, df_value(acc), s.c[r], s.l[r], s.u[r], r, xf <= s.l32[r], xf >= s.u32[r]);
@@ -687,10 +702,11 @@ __device__ void check_rows(const CheckSrc& s, int variant, int rb, int re, Acc& 
                     di = gate_diag(s, r, __ldg(s.rowptr + r + 1) > ks ? static_cast<double>(__ldg(s.vhi + ks)) + __ldg(s.vlo + ks) : 0.0);
                 }
                 const double li = s.l[r], ui = s.u[r];
-                check_row(a, xi, df_value(acc), s.c[r], li, ui, di, s.gate, r, less_equal_bits(dbits(xi), dbits(li)),
-                          less_equal_bits(dbits(ui), dbits(xi)), floor);
+                check_row(a, m, xi, df_value(acc), s.c[r], li, ui, di, s.gate, r, less_equal_bits(dbits(xi), dbits(li)),
+                          less_equal_bits(dbits(ui), dbits(xi)));
             });
     }
+    stat_settle(a, m);
 }
 
 __device__ __forceinline__ CheckSrc source_of(const InstDev& I) {
@@ -702,24 +718,23 @@ __device__ __forceinline__ CheckSrc source_of(const InstDev& I) {
 }
 
 // ---- the state machine after a check (thread 0 of the finalizing block) -------------------
-// Momenta of iterations [I.it0, I.it0 + count).  The sequence depends on the iteration alone, so it
-// comes from a table the host filled with the same IEEE operations: one thread's recurrence (a
-// square root and two divisions per iteration, each waiting for the one before) took 20 us per
-// chunk of 25 on this GPU's FP64 pipe.  Past the table the recurrence goes on from I.t.
+// Momenta of iterations [I.it0, I.it0 + count), by the whole block.  The sequence depends on the
+// iteration alone, so it comes from a table the host filled with the same IEEE operations: one
+// thread's recurrence (a square root and two divisions per iteration, each waiting for the one
+// before) took 20 us per chunk of 25 on this GPU's FP64 pipe.  Past the table the recurrence goes
+// on from I.t.
 __device__ void fista_betas(const View& v, InstDev& I, int64_t count) {
     const int64_t first = I.it0;
     if (first + count <= kMomentumTable) {
-        double t = I.t;
-#pragma unroll 8
-        for (int64_t j = 0; j < count; ++j) {
+        for (int64_t j = threadIdx.x; j < count; j += blockDim.x) {
             const double2 m = __ldg(v.momentum + first + j);
             I.beta[j] = m.x;
             I.beta32[j] = static_cast<float>(m.x);
-            t = m.y;
+            if (j + 1 == count) I.t = m.y;
         }
-        I.t = t;
         return;
     }
+    if (threadIdx.x != 0) return;
     // t_{k+1} = (1 + sqrt(1 + 4 t_k^2)) / 2, beta_k = (t_k - 1) / t_{k+1}
     // (src/accelerated_qp.cpp:47), each operation rounded as the reference's CPU loop rounds it.
     double t = I.t;
@@ -739,7 +754,8 @@ __device__ void finish(InstDev& I, int status, int src) {
     I.end_ns = now_ns();
 }
 
-__device__ void after_check(const View& v, InstDev& I, const Acc& tot) {
+// Returns the steps of the chunk that it arms (0: none), whose momenta conclude_check fills in.
+__device__ int64_t after_check(InstDev& I, const Acc& tot) {
     const int64_t it_check = I.it_next;
     const int ph = I.phase;
     I.checks++;
@@ -766,10 +782,10 @@ __device__ void after_check(const View& v, InstDev& I, const Acc& tot) {
     I.verified = verified ? 1 : 0;
     I.iterations = it_check;
     const int src = (ph == PH_POLISH_FINISH) ? 2 : (I.precision == PREC_MIXED ? 1 : 0);
-    if (verified) { finish(I, ST_OPTIMAL, src); return; }
-    if (!isfinite(obj) || !isfinite(stat)) { finish(I, ST_NUMERICAL_ERROR, src); return; }
-    if (now_ns() >= I.deadline_ns) { finish(I, ST_TIME_LIMIT, src); return; }
-    if (it_check >= I.max_iter) { finish(I, ST_ITERATION_LIMIT, src); return; }
+    if (verified) { finish(I, ST_OPTIMAL, src); return 0; }
+    if (!isfinite(obj) || !isfinite(stat)) { finish(I, ST_NUMERICAL_ERROR, src); return 0; }
+    if (now_ns() >= I.deadline_ns) { finish(I, ST_TIME_LIMIT, src); return 0; }
+    if (it_check >= I.max_iter) { finish(I, ST_ITERATION_LIMIT, src); return 0; }
     if (ph == PH_POLISH_FINISH) {
         // The polished point failed verification: the active-set guess was wrong.  FISTA
         // resumes from its own untouched state at it_check.
@@ -790,7 +806,7 @@ __device__ void after_check(const View& v, InstDev& I, const Acc& tot) {
             I.cg_it = 0;
             I.ff_nnz = 0;
             I.ff_rows = 0;
-            return;
+            return 0;
         }
     }
     I.phase = PH_FISTA;
@@ -800,9 +816,22 @@ __device__ void after_check(const View& v, InstDev& I, const Acc& tot) {
     I.moved[1] = 0;
     I.it_next = it_check + I.interval < I.max_iter ? it_check + I.interval : I.max_iter;
     const int64_t count = I.it_next - I.it0;
-    fista_betas(v, I, count);
     I.fista_iters += count;
+    return count;
 }
+
+// The whole block that finished an instance's check: its state machine, then the next chunk's momenta.
+__device__ void conclude_check(const View& v, InstDev& I, const Acc& tot) {
+    __shared__ int64_t armed;
+    if (threadIdx.x == 0) {
+        armed = after_check(I, tot);
+        I.stat_floor = 0;  // the next check starts from nothing
+    }
+    __syncthreads();
+    if (armed > 0) fista_betas(v, I, armed);
+    __syncthreads();
+}
+
 
 // ---- step kernel ------------------------------------------------------------------------------
 // Active-set motion (mixed precision): in the last two steps of a chunk the step kernel records
@@ -1348,11 +1377,7 @@ __global__ void __launch_bounds__(kBlock, 3) check_kernel(View v) {
         const int2 R = v.ranges[T.inst];
         if (publish_and_test_last(v, t, T.inst, R.y - R.x, total)) {
             Acc inst_total = reduce_instance(v, R.x, R.y, s.gate != 0);
-            if (threadIdx.x == 0) {
-                after_check(v, I, inst_total);
-                I.stat_floor = 0;  // the next check starts from nothing
-            }
-            __syncthreads();
+            conclude_check(v, I, inst_total);
         }
     }
 }
@@ -1373,26 +1398,26 @@ __global__ void __launch_bounds__(kBlock, 4) check_slice_kernel(View v) {
         const unsigned long long floor = __ldcg(&I.stat_floor);
         const int gate = I.diag_gate, n = I.n;
         Acc a = acc_identity();
+        StatMax m = stat_max(floor);
         for (int s = (T.row_begin >> 5) + static_cast<int>(threadIdx.x >> 5); s < last; s += kBlock / 32) {
             const int p = s * 32 + static_cast<int>(threadIdx.x & 31);
             const bool valid = p < n;
             const int len = valid ? __ldg(I.slice_len + p) : 0;
+            // the row's own numbers are on their way while its products are formed
+            const double xi = valid ? I.x64[p] : 0.0, li = valid ? I.l[p] : 0.0, ui = valid ? I.u[p] : 0.0;
+            const double ci = valid ? I.c[p] : 0.0;
             const double gq = slice_dot<false, 4>(I.col, I.val64, I.x64, __ldg(I.slice_base + s), len);
             if (!valid) continue;
-            const double xi = I.x64[p], li = I.l[p], ui = I.u[p];
-            check_row(a, xi, gq, I.c[p], li, ui, gate ? I.diag[p] : 1.0, gate, p, less_equal_bits(dbits(xi), dbits(li)),
-                      less_equal_bits(dbits(ui), dbits(xi)), floor);
+            check_row(a, m, xi, gq, ci, li, ui, gate ? I.diag[p] : 1.0, gate, p, less_equal_bits(dbits(xi), dbits(li)),
+                      less_equal_bits(dbits(ui), dbits(xi)));
         }
+        stat_settle(a, m);
         Acc total = block_reduce_check(a, gate != 0, true);
         if (threadIdx.x == 0 && total.stat > floor) atomicMax(&I.stat_floor, total.stat);
         const int2 R = v.ranges[T.inst];
         if (publish_and_test_last(v, R.x + U.z, T.inst, U.w, total)) {
             Acc inst_total = reduce_instance(v, R.x, R.x + U.w, gate != 0);
-            if (threadIdx.x == 0) {
-                after_check(v, I, inst_total);
-                I.stat_floor = 0;
-            }
-            __syncthreads();
+            conclude_check(v, I, inst_total);
         }
     }
 }
@@ -1453,6 +1478,7 @@ __global__ void __launch_bounds__(kBlock, 4) check_slice_mixed_kernel(View v) {
         const unsigned long long floor = __ldcg(&I.stat_floor);
         const int gate = I.diag_gate, n = I.n;
         Acc a = acc_identity();
+        StatMax m = stat_max(floor);
         for (int s = (T.row_begin >> 5) + static_cast<int>(threadIdx.x >> 5); s < last; s += kBlock / 32) {
             const int p = s * 32 + static_cast<int>(threadIdx.x & 31);
             const bool valid = p < n;
@@ -1470,25 +1496,22 @@ __global__ void __launch_bounds__(kBlock, 4) check_slice_mixed_kernel(View v) {
             const double gq = df_value(acc), li = I.l[p], ui = I.u[p], ci = I.c[p];
             if constexpr (FAMILY == FAMILY_VERIFY) {
                 const double xi = I.xp[p];
-                check_row(a, xi, gq, ci, li, ui, gate ? I.diag[p] : 1.0, gate, p, less_equal_bits(dbits(xi), dbits(li)),
-                          less_equal_bits(dbits(ui), dbits(xi)), floor);
+                check_row(a, m, xi, gq, ci, li, ui, gate ? I.diag[p] : 1.0, gate, p, less_equal_bits(dbits(xi), dbits(li)),
+                          less_equal_bits(dbits(ui), dbits(xi)));
             } else {
                 const float xf = I.x32[p];
                 const bool at_lower = xf <= I.l32[p], at_upper = xf >= I.u32[p];
-                if (gate) check_row(a, static_cast<double>(xf), gq, ci, li, ui, I.diag[p], 1, p, at_lower, at_upper);
+                if (gate) check_row(a, m, static_cast<double>(xf), gq, ci, li, ui, I.diag[p], 1, p, at_lower, at_upper);
                 else check_row_f32(a, xf, gq, ci, li, ui, p, at_lower, at_upper);
             }
         }
+        stat_settle(a, m);
         Acc total = block_reduce_check(a, gate != 0, true);
         if (threadIdx.x == 0 && total.stat > floor) atomicMax(&I.stat_floor, total.stat);
         const int2 R = v.ranges[T.inst];
         if (publish_and_test_last(v, R.x + U.z, T.inst, U.w, total)) {
             Acc inst_total = reduce_instance(v, R.x, R.x + U.w, gate != 0);
-            if (threadIdx.x == 0) {
-                after_check(v, I, inst_total);
-                I.stat_floor = 0;
-            }
-            __syncthreads();
+            conclude_check(v, I, inst_total);
         }
     }
 }
@@ -2775,8 +2798,8 @@ __device__ __forceinline__ void init_row(const InstDev& I, int r) {
     }
 }
 
-// Start of a solve: clock, deadline and (mixed) the first chunk.  One thread.
-__device__ void start_instance(const View& v, InstDev& I) {
+// Start of a solve: clock, deadline and (mixed) the first chunk, whose steps it returns.  One thread.
+__device__ int64_t start_instance(InstDev& I) {
         const int64_t start = now_ns();
         I.start_ns = start;
         I.deadline_ns = start + I.deadline_ns;  // host stores the budget in nanoseconds
@@ -2792,9 +2815,10 @@ __device__ void start_instance(const View& v, InstDev& I) {
             I.moved[1] = 0;
             const int64_t first = I.interval <= 16 ? I.interval + I.interval / 2 : I.interval;
             I.it_next = first < I.max_iter ? first : I.max_iter;
-            fista_betas(v, I, I.it_next);
             I.fista_iters += I.it_next;
+            return I.it_next;
         }
+        return 0;
 }
 
 // Re-arms a list of resident solves in one launch.  Block b takes rows [span.y, span.y + kRearmRows)
@@ -2811,6 +2835,7 @@ __global__ void __launch_bounds__(kBlock) rearm_kernel(View v, const InstDev* __
         const uint4* src = reinterpret_cast<const uint4*>(&S);
         uint4* dst = reinterpret_cast<uint4*>(&I);
         for (int w = threadIdx.x; w < static_cast<int>(sizeof(InstDev) / 16); w += kBlock) dst[w] = src[w];
+        __shared__ int64_t armed;
         __syncthreads();
         if (threadIdx.x == 0) {
             // the power estimate replaces the host's Gershgorin L (the mixed engine's steps
@@ -2822,8 +2847,10 @@ __global__ void __launch_bounds__(kBlock) rearm_kernel(View v, const InstDev* __
                 I.div_span = I.L >= 0x1p-100 && I.L <= 0x1p100 ? kDivSpan : 0;
                 I.invLf = static_cast<float>(I.invL);
             }
-            start_instance(v, I);
+            armed = start_instance(I);
         }
+        __syncthreads();
+        if (armed > 0) fista_betas(v, I, armed);
     }
 }
 
@@ -3537,6 +3564,11 @@ __global__ void __launch_bounds__(kBlock) lanczos_update_kernel(InstDev I, int n
 }
 
 // ---- standalone check on caller arrays ---------------------------------------------------------
+// On the caller's CSR, a row per lane, so that a row's products are fused and its sum needs no tree:
+// the FP64 pipe (an issue slot of 16 cycles per warp instruction) and the gathers bound it.  On the
+// random graph 1M the verification call (gate and check) takes 346 us; 357 with two lanes a row, 366 with
+// warp-staged rows (rounded products, then sums), 468 with those on 245 blocks of 4096 rows, which left
+// most of the SMs' warps unused.
 struct StandaloneScratch {
     int done;
     int pad[3];
@@ -3545,12 +3577,13 @@ struct StandaloneScratch {
 __global__ void __launch_bounds__(kBlock) check_standalone_kernel(CheckSrc s, int n, double tol, double offset,
                                                                  Partial* partial, StandaloneScratch* scr,
                                                                  double* result) {
-    const int rows_per_block = (n + gridDim.x - 1) / gridDim.x;
-    const int rb = blockIdx.x * rows_per_block;
-    const int re = min(n, rb + rows_per_block);
+    // whole warps of rows; the last blocks may have none
+    const int64_t rows_per_block = (((n + gridDim.x - 1) / gridDim.x) + 31) & ~31;
+    const int64_t rb = blockIdx.x * rows_per_block;
+    const int re = static_cast<int>(min(static_cast<int64_t>(n), rb + rows_per_block));
     Acc a = acc_identity();
-    if (rb < re) check_rows<0>(s, VAR_WARP, rb, re, a);
-    Acc total = block_reduce(a);
+    if (rb < re) check_rows<0>(s, 1, static_cast<int>(rb), re, a);
+    Acc total = block_reduce_check(a, s.gate != 0);
     __shared__ int is_last;
     if (threadIdx.x == 0) {
         store_partial(&partial[blockIdx.x], total);
@@ -3562,7 +3595,7 @@ __global__ void __launch_bounds__(kBlock) check_standalone_kernel(CheckSrc s, in
     __threadfence();
     Acc acc = acc_identity();
     for (int k = threadIdx.x; k < static_cast<int>(gridDim.x); k += kBlock) acc = combine(acc, load_partial(&partial[k]));
-    Acc tot = block_reduce(acc);
+    Acc tot = block_reduce_check(acc, s.gate != 0);
     if (threadIdx.x == 0) {
         scr->done = 0;
         double obj, stat, prim, bound, gap;
@@ -3984,11 +4017,11 @@ void launch_prepare_instance(const InstDev& rec, int64_t n, cudaStream_t s) {
     prepare_kernel<<<static_cast<int>(grid), kBlock, 0, s>>>(rec, static_cast<int>(n));
 }
 
+// Two rows per thread at least, and no more blocks than the SMs hold at a time (4 on each of 152).
+constexpr int64_t kCheckBlocks = 608;
 int check_grid(int64_t n) {
-    int64_t g = (n + 4095) / 4096;
-    if (g > 2048) g = 2048;
-    if (g < 1) g = 1;
-    return static_cast<int>(g);
+    const int64_t g = (n + 511) / 512;
+    return static_cast<int>(g > kCheckBlocks ? kCheckBlocks : g);
 }
 
 size_t check_scratch_bytes(int64_t n) {
