@@ -21,6 +21,7 @@
 // vector is in slice order and host vectors are permuted as they come and go.  The other systems
 // keep CSR with four lanes per row.
 #include "boxqp.h"
+#include "fpbits.h"
 #include "kernels.cuh"
 #include "slices.cuh"
 
@@ -57,6 +58,8 @@ __device__ __forceinline__ unsigned long long umax64(unsigned long long a, unsig
 __device__ __forceinline__ unsigned long long dbits(double v) {
     return static_cast<unsigned long long>(__double_as_longlong(v));
 }
+// the bits of |v| in integer arithmetic (fpbits.h: bits64)
+__device__ __forceinline__ unsigned long long abs_bits(double v) { return bqp::bits64(v) & 0x7fffffffffffffffull; }
 
 // y = M v for rows [0, rows) of a CSR matrix, kLanes lanes per row in a fixed order; returns the
 // row sum in the group's lane 0 (valid for r < rows).
@@ -73,21 +76,23 @@ __device__ __forceinline__ double csr_row(const int32_t* __restrict__ rp, const 
     return s;
 }
 
-// Fixed-order block sums of two doubles and a maximum; the last block (ticket) adds the block
+// Fixed-order block sums of one or two doubles (TWO) and a maximum; the last block (ticket) adds the block
 // partials, all its threads strided over them and then the same fixed tree, and returns true in
-// its thread 0 with the grid totals.
+// its thread 0 with the grid totals.  A sum that nobody reads is left out: its additions take the
+// FP64 pipe 16 cycles per warp and level.
+template <bool TWO>
 __device__ __forceinline__ void block_tree(double& a, double& b, unsigned long long& mx, double* ra, double* rb,
                                            unsigned long long* rm) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         a += __shfl_xor_sync(0xffffffffu, a, o);
-        b += __shfl_xor_sync(0xffffffffu, b, o);
+        if (TWO) b += __shfl_xor_sync(0xffffffffu, b, o);
         mx = umax64(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (lane == 0) {
         ra[warp] = a;
-        rb[warp] = b;
+        if (TWO) rb[warp] = b;
         rm[warp] = mx;
     }
     __syncthreads();
@@ -97,21 +102,22 @@ __device__ __forceinline__ void block_tree(double& a, double& b, unsigned long l
         mx = 0;
         for (int w = 0; w < kB / 32; ++w) {
             a += ra[w];
-            b += rb[w];
+            if (TWO) b += rb[w];
             mx = umax64(mx, rm[w]);
         }
     }
 }
 
+template <bool TWO>
 __device__ bool reduce_last(double a, double b, unsigned long long mx, double* partial, AdmmState* st, double* ta,
                             double* tb, unsigned long long* tm) {
-    __shared__ double ra[kB / 32], rb[kB / 32];
+    __shared__ double ra[kB / 32], rb[TWO ? kB / 32 : 1];
     __shared__ unsigned long long rm[kB / 32];
     __shared__ int last;
-    block_tree(a, b, mx, ra, rb, rm);
+    block_tree<TWO>(a, b, mx, ra, rb, rm);
     if (threadIdx.x == 0) {
         partial[3 * blockIdx.x] = a;
-        partial[3 * blockIdx.x + 1] = b;
+        if (TWO) partial[3 * blockIdx.x + 1] = b;
         partial[3 * blockIdx.x + 2] = __longlong_as_double(static_cast<long long>(mx));
         __threadfence();
         last = atomicAdd(&st->ticket, 1u) == gridDim.x - 1 ? 1 : 0;
@@ -123,10 +129,10 @@ __device__ bool reduce_last(double a, double b, unsigned long long mx, double* p
     unsigned long long sm = 0;
     for (unsigned k = threadIdx.x; k < gridDim.x; k += kB) {
         sa += __ldcg(partial + 3 * k);
-        sb += __ldcg(partial + 3 * k + 1);
+        if (TWO) sb += __ldcg(partial + 3 * k + 1);
         sm = umax64(sm, dbits(__ldcg(partial + 3 * k + 2)));
     }
-    block_tree(sa, sb, sm, ra, rb, rm);  // thread 0 read the first tree's ra/rb/rm before the barrier above
+    block_tree<TWO>(sa, sb, sm, ra, rb, rm);  // thread 0 read the first tree's ra/rb/rm before the barrier above
     if (threadIdx.x != 0) return false;
     st->ticket = 0;
     *ta = sa;
@@ -193,7 +199,7 @@ __global__ void __launch_bounds__(kB) admm_k_kernel(Sys s, const double* __restr
     if (mode == 0) return;
     double ta, tb;
     unsigned long long tm;
-    if (!reduce_last(acc_a, acc_b, acc_m, partial, st, &ta, &tb, &tm)) return;
+    if (!reduce_last<true>(acc_a, acc_b, acc_m, partial, st, &ta, &tb, &tm)) return;
     if (mode == 1) {
         st->rz = ta;
         st->rmax = tm;
@@ -229,7 +235,7 @@ __global__ void __launch_bounds__(kB) admm_update_kernel(Sys s, double* __restri
     }
     double ta, tb;
     unsigned long long tm;
-    if (!reduce_last(acc_a, 0.0, acc_m, partial, st, &ta, &tb, &tm)) return;
+    if (!reduce_last<false>(acc_a, 0.0, acc_m, partial, st, &ta, &tb, &tm)) return;
     st->beta = ta / st->rz;
     st->rz = ta;
     st->rmax = tm;
@@ -248,7 +254,9 @@ __global__ void __launch_bounds__(kB) admm_direction_kernel(int n, double* __res
 // ---- the same over sliced rows ------------------------------------------------------------------
 // Bounds of an iteration on 1M variables, 15M + 2 x 4M entries: 23M random gathers (92 us at the
 // 250 G/s this GPU gathers), 276 MB of entries (41 us), on the FP64 pipe 23M products and about
-// eight operations a row (50 us).  Four lanes per CSR row spent as much FP64 time again on tree
+// eight operations a row (50 us); the L2 hands out a 32-byte sector per gathered number, which with
+// the entries makes 104 us.  Now 154: A d 22, K d 100, update 20, direction and the loop 11 (two
+// iterations per body of the loop: 157).  Four lanes per CSR row spent as much FP64 time again on tree
 // additions and quarter-warp epilogues, and a general division per row: 217 us an iteration.
 // Columns of a row in flight: 5 on large systems (64 registers; 4: 183, 8: 167 us an iteration), whole
 // rows on small ones, which are bound by the latency of their loads.
@@ -342,7 +350,7 @@ __global__ void __launch_bounds__(kB, AHEAD > 8 ? 2 : 4) admm_k_slice_kernel(Sli
             pre[p] = pp;
             d[p] = pp;
             acc_a = fma(rr, pp, acc_a);
-            acc_m = umax64(acc_m, dbits(fabs(rr)));
+            acc_m = umax64(acc_m, abs_bits(rr));
         } else if (mode == 2) {
             acc_a = fma(vp, o, acc_a);
         }
@@ -351,7 +359,7 @@ __global__ void __launch_bounds__(kB, AHEAD > 8 ? 2 : 4) admm_k_slice_kernel(Sli
     if (mode == 0) return;
     double ta, tb;
     unsigned long long tm;
-    if (!reduce_last(acc_a, 0.0, acc_m, partial, st, &ta, &tb, &tm)) return;
+    if (!reduce_last<false>(acc_a, 0.0, acc_m, partial, st, &ta, &tb, &tm)) return;
     if (mode == 1) {
         st->rz = ta;
         st->rmax = tm;
@@ -383,11 +391,11 @@ __global__ void __launch_bounds__(kB) admm_update_slice_kernel(int n, const doub
         r[j] = rr;
         pre[j] = pp;
         acc_a = fma(rr, pp, acc_a);
-        acc_m = umax64(acc_m, dbits(fabs(rr)));
+        acc_m = umax64(acc_m, abs_bits(rr));
     }
     double ta, tb;
     unsigned long long tm;
-    if (!reduce_last(acc_a, 0.0, acc_m, partial, st, &ta, &tb, &tm)) return;
+    if (!reduce_last<false>(acc_a, 0.0, acc_m, partial, st, &ta, &tb, &tm)) return;
     st->beta = ta / st->rz;
     st->rz = ta;
     st->rmax = tm;
@@ -463,12 +471,12 @@ __global__ void __launch_bounds__(kB) admm_rhs_slice_kernel(SliceSys S, const do
             const double v = __dadd_rn(acc, __dsub_rn(__dmul_rn(S.sigma, xa[p]), c[p]));
             rhs[p] = v;
             x0[p] = xa[p];
-            mx = umax64(mx, dbits(fabs(v)));
+            mx = umax64(mx, abs_bits(v));
         }
     }
     double ta, tb;
     unsigned long long tm;
-    if (!reduce_last(0.0, 0.0, mx, partial, st, &ta, &tb, &tm)) return;
+    if (!reduce_last<false>(0.0, 0.0, mx, partial, st, &ta, &tb, &tm)) return;
     const double rmax = __longlong_as_double(static_cast<long long>(tm));
     st->accuracy = __dmul_rn(iteration_factor, __dadd_rn(1.0, rmax));
     st->max_inner = S.k.n * 2LL + 20 < 4000 ? S.k.n * 2LL + 20 : 4000;
@@ -564,7 +572,7 @@ __global__ void __launch_bounds__(kB) admm_rhs_kernel(Sys s, const double* __res
     }
     double ta, tb;
     unsigned long long tm;
-    if (!reduce_last(0.0, 0.0, mx, partial, st, &ta, &tb, &tm)) return;
+    if (!reduce_last<false>(0.0, 0.0, mx, partial, st, &ta, &tb, &tm)) return;
     const double rmax = __longlong_as_double(static_cast<long long>(tm));
     st->accuracy = __dmul_rn(iteration_factor, __dadd_rn(1.0, rmax));
     st->max_inner = s.n * 2LL + 20 < 4000 ? s.n * 2LL + 20 : 4000;

@@ -1432,9 +1432,9 @@ struct SlicePairs {
 #pragma unroll
         for (int q = 0; q < AHEAD; ++q) {
             const bool in = q < left;
-            c[q] = in ? __ldg(col + k) : -1;
-            h[q] = in ? __ldg(vhi + k) : 0.f;
-            l[q] = in ? __ldg(vlo + k) : 0.f;
+            c[q] = in ? load_once(col + k) : -1;
+            h[q] = in ? load_once(vhi + k) : 0.f;
+            l[q] = in ? load_once(vlo + k) : 0.f;
             k += __popc(__ballot_sync(0xffffffffu, in));
         }
     }
@@ -1629,7 +1629,7 @@ __device__ void count_kept(const InstDev& I, const int32_t* __restrict__ list, i
             const int r = list[j];
             const int ks = __ldg(rowptr + r), ke = __ldg(rowptr + r + 1);
 #pragma unroll 4
-            for (int k = ks + sl; k < ke; k += LANES) cnt += pos_of[__ldg(col + k)] >= 0 ? 1 : 0;
+            for (int k = ks + sl; k < ke; k += LANES) cnt += pos_of[load_once(col + k)] >= 0 ? 1 : 0;
         }
 #pragma unroll
         for (int o = LANES / 2; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
@@ -1712,9 +1712,9 @@ __device__ void residual_rows(const InstDev& I, const int32_t* __restrict__ list
             float h = 0.f, lo = 0.f;
             if (valid) {
                 const int k = ks + i + sl;
-                cc = __ldg(col + k);
-                h = __ldg(vhi + k);
-                lo = __ldg(vlo + k);
+                cc = load_once(col + k);
+                h = load_once(vhi + k);
+                lo = load_once(vlo + k);
                 const int4 q = xq[cc];  // the column's pair and position in one gather
                 acc = df_add(acc, df_prod2(h, lo, make_float2(__int_as_float(q.x), __int_as_float(q.y))));
                 pc = q.z;
