@@ -1348,6 +1348,8 @@ constexpr int FAMILY_VERIFY = 2;   // polished point of the mixed engine (once p
 
 template <int FAMILY>
 __global__ void __launch_bounds__(kBlock, 3) check_kernel(View v) {
+    let_next_launch_begin();
+    wait_for_previous_launch();
     if (v.ctrl->check_due[FAMILY] == 0) return;  // no instance due for this family in this body
     const int nt = v.ctrl->n_tiles;
     for (int t = blockIdx.x; t < nt; t += gridDim.x) {
@@ -1386,6 +1388,8 @@ __global__ void __launch_bounds__(kBlock, 3) check_kernel(View v) {
 // as many as resident blocks): a unit's rows accumulate in registers, one reduction and one
 // publication per unit (its partial in its instance's slot R.x + index).
 __global__ void __launch_bounds__(kBlock, 4) check_slice_kernel(View v) {
+    let_next_launch_begin();
+    wait_for_previous_launch();
     if (v.ctrl->check_due[FAMILY_FP64] == 0) return;
     const int nu = v.ctrl->n_units;
     for (int un = blockIdx.x; un < nu; un += gridDim.x) {
@@ -1465,6 +1469,8 @@ struct SlicePairs {
 template <int FAMILY>
 __global__ void __launch_bounds__(kBlock, 4) check_slice_mixed_kernel(View v) {
     constexpr int kAheadPairs = 4;
+    let_next_launch_begin();
+    wait_for_previous_launch();
     if (v.ctrl->check_due[FAMILY] == 0) return;
     const int nu = v.ctrl->n_units;
     for (int un = blockIdx.x; un < nu; un += gridDim.x) {
@@ -2695,7 +2701,7 @@ __device__ Counts count_phases(const View& v, int steps = 0) {
     return c;
 }
 
-// End of a body: every instance that stepped in it (FISTA phase) advances by the steps it ran.
+// Every instance that stepped in the body (FISTA phase) advances by the steps it ran.
 // A mixed solve whose chunk just completed step-stable (no variable crossed a bound in its last
 // two steps) goes straight to its first polish attempt, without the check of the FP32 iterate:
 // the polished point is verified in FP64 anyway, and a failed attempt resumes FISTA from this
@@ -2721,67 +2727,58 @@ __device__ void advance_chunks(const View& v, int steps) {
     __syncthreads();
 }
 
-// The polish branch runs polish_init and the residual, then a CG loop whose iterations the
-// direction kernel counts into Ctrl::kernels.
-__global__ void gate_kernel(View v, cudaGraphConditionalHandle h_fp64, cudaGraphConditionalHandle h_mixed,
-                            cudaGraphConditionalHandle h_exact, cudaGraphConditionalHandle h_polish,
-                            cudaGraphConditionalHandle h_cg, StepLaunches steps, int body_steps) {
-    const Counts c = count_phases(v, body_steps);
-    if (threadIdx.x == 0) {
-        for (int k = 0; k < 3; ++k) {
-            v.ctrl->n_fista[k] = c.fista[k];
-            v.ctrl->step_due[k] = c.step_due[k];
-        }
-        v.ctrl->n_polish = c.polish;
-        v.ctrl->n_cg = c.polish;
-        v.ctrl->n_cg_before = c.polish;
-        v.ctrl->cg_iters = 0;
-        long long launched = steps.checks + 1;  // check kernels and gate
-        for (int k = 0; k < 3; ++k) launched += c.fista[k] > 0 ? steps.n[k] : 0;
-        launched += c.polish > 0 ? steps.polish : 0;
-        v.ctrl->kernels += launched;
-        if (steps.present & 1u) cudaGraphSetConditional(h_fp64, c.fista[0] > 0 ? 1u : 0u);
-        if (steps.present & 2u) cudaGraphSetConditional(h_mixed, c.fista[1] > 0 ? 1u : 0u);
-        if (steps.present & 4u) cudaGraphSetConditional(h_exact, c.fista[2] > 0 ? 1u : 0u);
-        if (steps.present & 2u) cudaGraphSetConditional(h_polish, c.polish > 0 ? 1u : 0u);
-        if (steps.present & 2u) cudaGraphSetConditional(h_cg, c.polish > 0 ? 1u : 0u);
-    }
-}
-
-__global__ void control_kernel(View v, cudaGraphConditionalHandle loop_h, int steps) {
+// After the steps of a body: advances the chunks, counts what the checks will find due, and arms the
+// polish branch (in a graph: in_graph) for the solves whose chunk just ended step-stable, so that a
+// solve can step, polish and be verified in one body.  An instance that is in the polish may finish it
+// before the checks, so all of those count as due for verification (the check kernel tests).
+// The polish branch's CG iterations are counted into Ctrl::kernels by the vector kernel.
+__global__ void __launch_bounds__(1024) advance_kernel(View v, cudaGraphConditionalHandle h_polish, cudaGraphConditionalHandle h_cg,
+                                                       StepLaunches body, int steps, int in_graph) {
+    let_next_launch_begin();
+    wait_for_previous_launch();
     advance_chunks(v, steps);
     const Counts c = count_phases(v);
     if (threadIdx.x == 0) {
-        for (int k = 0; k < 3; ++k) v.ctrl->check_due[k] = c.check_due[k];
         Ctrl* ctrl = v.ctrl;
-        ctrl->bodies++;
-        ctrl->kernels += 1;
-        ctrl->running = c.running;
-        cudaGraphSetConditional(loop_h, (c.running > 0 && ctrl->bodies < ctrl->body_cap) ? 1u : 0u);
+        for (int k = 0; k < 3; ++k) ctrl->check_due[k] = c.check_due[k];
+        ctrl->check_due[FAMILY_VERIFY] += c.polish;
+        ctrl->n_polish = c.polish;
+        ctrl->n_cg = c.polish;
+        ctrl->n_cg_before = c.polish;
+        ctrl->cg_iters = 0;
+        long long launched = 1;
+        for (int k = 0; k < 3; ++k) launched += ctrl->n_fista[k] > 0 || ((body.always >> k) & 1u) ? body.n[k] : 0;
+        ctrl->kernels += launched + (c.polish > 0 ? body.polish : 0);
+        if (in_graph && (body.present & 2u)) {
+            cudaGraphSetConditional(h_polish, c.polish > 0 ? 1u : 0u);
+            cudaGraphSetConditional(h_cg, c.polish > 0 ? 1u : 0u);
+        }
     }
 }
 
-__global__ void gate_plain_kernel(View v, int steps) {
+// After the checks: what steps the next body has, and whether there is one (`ends_body`: 0 before the
+// first).
+__global__ void __launch_bounds__(1024) gate_kernel(View v, cudaGraphConditionalHandle h_fp64, cudaGraphConditionalHandle h_mixed,
+                                                    cudaGraphConditionalHandle h_exact, cudaGraphConditionalHandle h_loop,
+                                                    StepLaunches body, int steps, int ends_body, int in_graph) {
+    let_next_launch_begin();
+    wait_for_previous_launch();
     const Counts c = count_phases(v, steps);
     if (threadIdx.x == 0) {
+        Ctrl* ctrl = v.ctrl;
         for (int k = 0; k < 3; ++k) {
-            v.ctrl->n_fista[k] = c.fista[k];
-            v.ctrl->step_due[k] = c.step_due[k];
+            ctrl->n_fista[k] = c.fista[k];
+            ctrl->step_due[k] = c.step_due[k];
         }
-        v.ctrl->n_polish = c.polish;
-        v.ctrl->n_cg = c.polish;
-        v.ctrl->n_cg_before = c.polish;
-        v.ctrl->cg_iters = 0;
-    }
-}
-
-__global__ void control_plain_kernel(View v, int steps) {
-    advance_chunks(v, steps);
-    const Counts c = count_phases(v);
-    if (threadIdx.x == 0) {
-        for (int k = 0; k < 3; ++k) v.ctrl->check_due[k] = c.check_due[k];
-        v.ctrl->bodies++;
-        v.ctrl->running = c.running;
+        ctrl->bodies += ends_body;
+        ctrl->kernels += body.checks + 1;
+        ctrl->running = c.running;
+        if (!in_graph) return;
+        const unsigned branches = body.present & ~body.always;
+        if (branches & 1u) cudaGraphSetConditional(h_fp64, c.fista[0] > 0 ? 1u : 0u);
+        if (branches & 2u) cudaGraphSetConditional(h_mixed, c.fista[1] > 0 ? 1u : 0u);
+        if (branches & 4u) cudaGraphSetConditional(h_exact, c.fista[2] > 0 ? 1u : 0u);
+        cudaGraphSetConditional(h_loop, (c.running > 0 && ctrl->bodies < ctrl->body_cap) ? 1u : 0u);
     }
 }
 
@@ -3716,27 +3713,32 @@ void group_waves(int sms) {
     group_wave<PREC, VAR_WARP>(sms);
 }
 
-// Columns in flight and blocks per SM: 4 / 5 / 6 columns at 8 blocks (64 registers) measured 6.56 /
-// 6.13 / 6.83 ms per FP64 grid solve and 37.1 / 36.8 / 37.9 ms on the random graph; small instances
-// hide latency with whole rows in flight (12 columns, 128 registers: 10k rows 2.95 -> 2.47 ms per solve
-// against 8 columns at 6 blocks).  The two cross at about kSliceSmall rows: 40k rows 6.7 against 7.2 us a
-// step, 100k rows 10.4 against 10.2.
-// A launch that may begin while the one before it in the stream still runs (its kernel waits).
+// `dependent`: the launch may begin while the one before it in the stream still runs (its kernel waits).
 template <class... P, class... A>
-void launch_dependent(void (*kernel)(P...), int grid, cudaStream_t s, A... args) {
+void launch_after(bool dependent, void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s, A... args) {
     cudaLaunchAttribute overlap;
     overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     overlap.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(static_cast<unsigned>(grid));
-    config.blockDim = dim3(kBlock);
+    config.blockDim = dim3(static_cast<unsigned>(block));
+    config.dynamicSmemBytes = smem;
     config.stream = s;
     config.attrs = &overlap;
-    config.numAttrs = 1;
+    config.numAttrs = dependent ? 1 : 0;
     cudaLaunchKernelEx(&config, kernel, static_cast<P>(args)...);
+}
+template <class... P, class... A>
+void launch_dependent(void (*kernel)(P...), int grid, cudaStream_t s, A... args) {
+    launch_after(true, kernel, grid, kBlock, 0, s, args...);
 }
 
 using SliceKernel = void (*)(View, int, int);
+// Columns in flight and blocks per SM: 4 / 5 / 6 columns at 8 blocks (64 registers) measured 6.56 /
+// 6.13 / 6.83 ms per FP64 grid solve and 37.1 / 36.8 / 37.9 ms on the random graph; small instances
+// hide latency with whole rows in flight (12 columns, 128 registers: 10k rows 2.95 -> 2.47 ms per solve
+// against 8 columns at 6 blocks).  The two cross at about kSliceSmall rows: 40k rows 6.7 against 7.2 us a
+// step, 100k rows 10.4 against 10.2.
 constexpr int kWideAhead = 5, kWideBlocks = 8, kSmallAhead = 12, kSmallBlocks = 4;
 constexpr int kMixedAhead = 6, kMixedBlocks = 8;
 SliceKernel slice_kernel(int precision, bool small) {  // 0 FP64, 1 FP64_EXACT, 2 mixed
@@ -3799,17 +3801,22 @@ int tile_grid(int sms) {
 
 int cg_matvec_slots() { return g_waves.matvec; }
 
-void launch_check(const View& v, int families, int grid, cudaStream_t s) {
+void launch_check(const View& v, int families, int grid, bool dependent, cudaStream_t s) {
+    // each overlaps the launch before it and waits for it before it reads what that wrote
+    auto launch = [&](void (*kernel)(View), int wave, size_t smem) {
+        launch_after(dependent, kernel, pick(grid, wave), kBlock, smem, s, v);
+        dependent = true;
+    };
     if (families & kCheckMixed) {
-        check_kernel<FAMILY_MIXED><<<pick(grid, g_waves.check_mixed), kBlock, kSmem8, s>>>(v);
-        check_kernel<FAMILY_VERIFY><<<pick(grid, g_waves.check_verify), kBlock, kSmem8, s>>>(v);
+        launch(check_kernel<FAMILY_MIXED>, g_waves.check_mixed, kSmem8);
+        launch(check_kernel<FAMILY_VERIFY>, g_waves.check_verify, kSmem8);
     }
-    if (families & kCheckFp64) check_kernel<FAMILY_FP64><<<pick(grid, g_waves.check), kBlock, kSmem8, s>>>(v);
+    if (families & kCheckFp64) launch(check_kernel<FAMILY_FP64>, g_waves.check, kSmem8);
     if (families & kCheckMixedSlices) {
-        check_slice_mixed_kernel<FAMILY_MIXED><<<pick(grid, g_waves.check_mixed_slices), kBlock, 0, s>>>(v);
-        check_slice_mixed_kernel<FAMILY_VERIFY><<<pick(grid, g_waves.check_verify_slices), kBlock, 0, s>>>(v);
+        launch(check_slice_mixed_kernel<FAMILY_MIXED>, g_waves.check_mixed_slices, 0);
+        launch(check_slice_mixed_kernel<FAMILY_VERIFY>, g_waves.check_verify_slices, 0);
     }
-    if (families & kCheckSlices) check_slice_kernel<<<pick(grid, g_waves.check_slices), kBlock, 0, s>>>(v);
+    if (families & kCheckSlices) launch(check_slice_kernel, g_waves.check_slices, 0);
 }
 
 void launch_step_group(const View& v, int group, int j, int grid, cudaStream_t s) {
@@ -3817,16 +3824,9 @@ void launch_step_group(const View& v, int group, int j, int grid, cudaStream_t s
     if (group >= kExactSlices || variant == variant_index(VAR_SLICE) || variant == variant_index(VAR_SLICE_SMALL)) {
         const int kind = group >= kExactSlices ? 1 : group >= kVariants ? 2 : 0;
         const bool is_small = group >= kExactSlices ? group == kExactSlices + 1 : variant == variant_index(VAR_SLICE_SMALL);
-        cudaLaunchAttribute overlap;
-        overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        overlap.val.programmaticStreamSerializationAllowed = 1;
-        cudaLaunchConfig_t config = {};
-        config.gridDim = dim3(static_cast<unsigned>(pick(8 * grid, g_waves.slices[2 * kind + is_small])));
-        config.blockDim = dim3(kSliceThreads);
-        config.stream = s;
-        config.attrs = &overlap;
-        config.numAttrs = j > 0 ? 1 : 0;  // the first step of a body reads what the kernels before it wrote
-        cudaLaunchKernelEx(&config, slice_kernel(kind, is_small), v, group, j);
+        // the first step of a body reads what the kernels before it wrote
+        launch_after(j > 0, slice_kernel(kind, is_small), pick(8 * grid, g_waves.slices[2 * kind + is_small]), kSliceThreads, 0, s, v,
+                     group, j);
     } else if (group >= kVariants) {
         launch_group_of<PREC_MIXED>(v, group, j, grid, s);
     } else {
@@ -3856,15 +3856,15 @@ void launch_cg_vector(const View& v, int products, int grid, cudaStream_t s, cud
     launch_dependent(cg_vector_kernel, pick(grid, g_waves.polish), s, v, cg_loop, cap, turn, products + 1);
 }
 
-void launch_gate(const View& v, const cudaGraphConditionalHandle* fista, cudaGraphConditionalHandle polish,
-                 cudaGraphConditionalHandle cg_loop, StepLaunches steps, int body_steps, cudaStream_t s) {
-    gate_kernel<<<1, 1024, 0, s>>>(v, fista[0], fista[1], fista[2], polish, cg_loop, steps, body_steps);
+void launch_advance(const View& v, cudaGraphConditionalHandle polish, cudaGraphConditionalHandle cg_loop, StepLaunches body,
+                    int steps, bool in_graph, bool dependent, cudaStream_t s) {
+    launch_after(dependent, advance_kernel, 1, 1024, 0, s, v, polish, cg_loop, body, steps, in_graph ? 1 : 0);
 }
-void launch_control(const View& v, cudaGraphConditionalHandle loop, int steps, cudaStream_t s) {
-    control_kernel<<<1, 1024, 0, s>>>(v, loop, steps);
+void launch_gate(const View& v, const cudaGraphConditionalHandle* fista, cudaGraphConditionalHandle loop, StepLaunches body,
+                 int steps, bool ends_body, bool in_graph, cudaStream_t s) {
+    launch_after(true, gate_kernel, 1, 1024, 0, s, v, fista[0], fista[1], fista[2], loop, body, steps, ends_body ? 1 : 0,
+                 in_graph ? 1 : 0);
 }
-void launch_gate_plain(const View& v, int steps, cudaStream_t s) { gate_plain_kernel<<<1, 1024, 0, s>>>(v, steps); }
-void launch_control_plain(const View& v, int steps, cudaStream_t s) { control_plain_kernel<<<1, 1024, 0, s>>>(v, steps); }
 
 void launch_rearm(const View& v, const InstDev* stage, const int32_t* slots, const int2* spans, int n_spans,
                   cudaStream_t s) {

@@ -11,7 +11,8 @@ int tile_grid(int sms);
 // resident blocks of the CG product kernel (after tile_grid)
 int cg_matvec_slots();
 // Tile kernels: grid-stride over the tile table (the grid size is fixed at capture).
-void launch_check(const View& v, int families, int grid, cudaStream_t s);
+// dependent: the first overlaps the launch before it (false behind a conditional node or nothing)
+void launch_check(const View& v, int families, int grid, bool dependent, cudaStream_t s);
 // Step j of a body: the step kernel of one group (step_group(precision, variant)) over the group's
 // tiles, or the FP64_EXACT step over the whole table.
 void launch_step_group(const View& v, int group, int j, int grid, cudaStream_t s);
@@ -35,23 +36,22 @@ void launch_cg_matvec(const View& v, int families, int grid, cudaStream_t s);
 // products: product kernels launched before it (for the count of kernels)
 void launch_cg_vector(const View& v, int products, int grid, cudaStream_t s, cudaGraphConditionalHandle cg_loop = 0, int cap = 0,
                       int turn = 0);
-// Single-block control kernels that steer the conditional graph nodes.
-// fista[k]: handle of the IF node of the precision-k step launches; polish: the IF node of the
-// polish branch; cg_loop: the WHILE node of its CG loop.  `steps.n[k]`: kernels inside the
-// precision-k FISTA body (steps per body x step groups launched).
+// Single-block kernels that steer the conditional graph nodes (in_graph; else they touch no handle).
+// Kernels of a body, for the count of kernels.
 struct StepLaunches {
-    int n[3];
-    int checks;        // check kernels of a body
+    int n[3];          // precision-k step launches
+    int checks;
     int polish;        // kernels at the head of the polish branch
-    unsigned present;  // bit k: the graph has a branch for precision k (bit 1: and the polish)
+    unsigned present;  // bit k: the graph has steps for precision k (bit 1: and the polish)
+    unsigned always;   // bit k: outside an IF node
 };
-void launch_gate(const View& v, const cudaGraphConditionalHandle* fista, cudaGraphConditionalHandle polish,
-                 cudaGraphConditionalHandle cg_loop, StepLaunches steps, int body_steps, cudaStream_t s);
-// `steps`: step launches per body; FISTA-phase instances advance it_cur by up to that many.
-void launch_control(const View& v, cudaGraphConditionalHandle loop, int steps, cudaStream_t s);
-// Host-driven variants of the control kernels (no conditional handles).
-void launch_gate_plain(const View& v, int steps, cudaStream_t s);
-void launch_control_plain(const View& v, int steps, cudaStream_t s);
+// After the steps of a body (`steps`: per instance at most): chunks advance; polish: the IF node of the polish
+// branch; cg_loop: the WHILE node of its CG loop.
+void launch_advance(const View& v, cudaGraphConditionalHandle polish, cudaGraphConditionalHandle cg_loop, StepLaunches body,
+                    int steps, bool in_graph, bool dependent, cudaStream_t s);
+// After the checks.  fista[k]: the IF node of the precision-k steps; loop: the WHILE node around the body.
+void launch_gate(const View& v, const cudaGraphConditionalHandle* fista, cudaGraphConditionalHandle loop, StepLaunches body,
+                 int steps, bool ends_body, bool in_graph, cudaStream_t s);
 // Admission, first kernel: the convexity gate and Gershgorin bound of the uploaded full CSR
 // (FP64 values `val`) into *rec.gate (cleared first), the FP64 diagonal into rec.diag and, for the
 // mixed engine, the hi/lo FP32 values into rec.vhi/rec.vlo.  The later admission kernels read L there.
