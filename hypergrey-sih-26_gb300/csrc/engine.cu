@@ -217,7 +217,8 @@ struct Job {
     int sum_lanes = 0;        // sliced mixed solves: InstDev::sum_lanes
     std::vector<Tile> tiles;  // local tiles (inst field filled at admission)
     std::vector<Tile> items;  // step work items of a sliced solve: its tiles in pieces of kSlicePiece rows
-    std::vector<int4> units;  // CG and check work units, tiles counted from the solve's first (cg_units)
+    std::vector<int4> units;  // CG work units, tiles counted from the solve's first (work_units); none of an FP64 solve
+    std::vector<int4> passes; // check and residual work units
     int state = JOB_QUEUED;
     bool resolve = false;     // re-run of a resident solve
     bool notify = false;      // report completion through the completion queue (bqp_wait_any)
@@ -328,20 +329,20 @@ int choose_variant(int64_t n, int64_t nnz, int64_t longest_row, const bqp_option
     return rows_fit && avg < kSliceMaxAverageMixed && *sums >= 0 ? sliced : named;
 }
 
-// CG and check work units of one instance (its `count` tiles at t), appended to `out` as {first tile, tiles,
-// index, units}, the tiles counted from the instance's first: as many units as the product kernel has
-// resident blocks (`slots`), so that one round runs them on the whole GPU, but units of about
-// kCgUnitMin tiles at least; the tiles are spread evenly (sizes differ by one at most), and no unit
-// goes above kCgRowsum rows (the row sums' shared buffer; units of kCgUnitMin tiles always fit).
-// FP64 instances take single tiles: their units serve the check alone, which the FP64 pipe of the
-// SM bounds (1024 rows of 11 entries take 10 us on one), 10k rows 2.03 -> 1.95 ms.  So do small mixed
-// instances, whose CG iterations are latency: 1k rows 230 -> 197 us, 256 uneven solves 1.33 ms on
-// the device either way; with up to 32 tiles these take 1.42 ms, with any number 1.45 (a unit costs
-// its block a reduction and a publication).  Depends on the instance alone, so the partial sums, and
-// the CG iterates, are the same in a batch as solo.
-void cg_units(const Tile* t, int count, int slots, bool fp64, std::vector<int4>& out) {
+// Work units of one instance (its `count` tiles at t), appended to `out` as {first tile, tiles, index,
+// units}, the tiles counted from the instance's first: as many units as the product kernel has
+// resident blocks (`slots`), so that one round runs them on the whole GPU, but units of about `least`
+// tiles at least; the tiles are spread evenly (sizes differ by one at most), and no unit goes above
+// kCgRowsum rows (the row sums' shared buffer; units of kCgUnitMin tiles always fit).
+// Checks and the residual pass take single tiles where they can: the FP64 pipe of an SM bounds a check
+// (1024 rows of 11 entries take 10 us on one), barriers and latency the residual pass (10k rows 38 us
+// in units of two tiles; a mixed solve of 10k rows 294 -> 275 us).  A CG product is shorter than a unit's reduction and publication cost its
+// block, so its units are single tiles only where an instance has kCgSmall of them at most: 1k
+// rows 230 -> 197 us, 256 uneven solves 1.33 ms on the device either way; with up to 32 tiles these take
+// 1.42 ms, with any number 1.45.  Depends on the instance alone, so the partial sums, and the CG
+// iterates, are the same in a batch as solo.
+void work_units(const Tile* t, int count, int slots, int least, std::vector<int4>& out) {
     const int fewest = (count + kCgUnitMax - 1) / kCgUnitMax;
-    const int least = fp64 || count <= kCgSmall ? 1 : kCgUnitMin;
     const int most = std::max(1, (count + least - 1) / least);
     int u = std::max(fewest, std::min(std::max(slots, 1), most));
     for (;; ++u) {
@@ -680,7 +681,7 @@ private:
     // the device tables (tiles, step groups, work units) hold the solves that run, and no others: a
     // launch's kernels do not walk over the tiles of resident solves that have finished
     std::vector<std::pair<int, uint64_t>> table_jobs_;  // slot and id of each solve in the tables
-    int n_tiles_ = 0, n_units_ = 0;
+    int n_tiles_ = 0, n_units_ = 0, n_passes_ = 0;
     int32_t group_begin_[kStepGroups + 1] = {};
     static constexpr uint32_t kExactCsrBit = 1u << kStepGroups;  // FP64_EXACT instances over the CSR
     uint32_t groups_present_ = 0;         // step groups with tiles (and kExactCsrBit)
@@ -934,7 +935,7 @@ bool Engine::ensure_tables(int need_inst, int need_tiles, std::string& why) {
         if (!cuda_ok(cudaMalloc(&tiles, sizeof(Tile) * cap), why, "tile table")) return false;
         if (!cuda_ok(cudaMalloc(&partial, sizeof(Partial) * cap), why, "partials")) return false;
         if (!cuda_ok(cudaMalloc(&group_tiles, sizeof(Tile) * cap * (kTileRows / kSlicePiece)), why, "step groups")) return false;
-        if (!cuda_ok(cudaMalloc(&units, sizeof(int4) * cap), why, "CG work units")) return false;
+        if (!cuda_ok(cudaMalloc(&units, sizeof(int4) * 2 * cap), why, "work units")) return false;
         cudaFree(d_tiles_);
         cudaFree(d_partial_);
         cudaFree(d_group_tiles_);
@@ -1740,7 +1741,11 @@ bool Engine::install(std::vector<Job*>& jobs, std::string& why) {
         for (Tile& t : j.tiles) t.inst = slot;
         for (Tile& t : j.items) t.inst = slot;
         j.units.clear();
-        cg_units(j.tiles.data(), static_cast<int>(j.tiles.size()), cg_slots_, j.opt.precision != PREC_MIXED, j.units);
+        j.passes.clear();
+        const int tiles = static_cast<int>(j.tiles.size());
+        work_units(j.tiles.data(), tiles, cg_slots_, 1, j.passes);
+        if (j.opt.precision == PREC_MIXED)
+            work_units(j.tiles.data(), tiles, cg_slots_, tiles <= kCgSmall ? 1 : kCgUnitMin, j.units);
     }
     if (!cuda_ok(cudaStreamWaitEvent(stream_, uev_, 0), why, "upload order")) return false;
     if (!rearm(jobs, why)) return false;
@@ -1917,13 +1922,14 @@ bool Engine::upload_tables(const std::vector<Job*>& jobs, std::string& why) {
     ids.reserve(jobs.size());
     for (const Job* j : jobs) ids.emplace_back(j->slot, j->id);
     if (!tables_dirty_ && ids == table_jobs_) return true;
-    size_t tiles = 0, units = 0, items = 0;
+    size_t tiles = 0, units = 0, passes = 0, items = 0;
     int32_t count[kStepGroups + 1] = {};
     groups_present_ = 0;
     auto items_of = [](const Job& j) -> const std::vector<Tile>& { return is_sliced(j.variant) ? j.items : j.tiles; };
     for (const Job* j : jobs) {
         tiles += j->tiles.size();
         units += j->units.size();
+        passes += j->passes.size();
         const int g = step_group(j->opt.precision, j->variant);
         if (g < 0) {
             groups_present_ |= kExactCsrBit;
@@ -1937,7 +1943,7 @@ bool Engine::upload_tables(const std::vector<Job*>& jobs, std::string& why) {
     std::memcpy(group_begin_, count, sizeof(group_begin_));
     if (!ensure_tables(0, static_cast<int>(tiles), why)) return false;
     tables_dirty_ = true;  // until the copies below are queued
-    const size_t b_tiles = sizeof(Tile) * tiles, b_group = sizeof(Tile) * items, b_units = sizeof(int4) * units;
+    const size_t b_tiles = sizeof(Tile) * tiles, b_group = sizeof(Tile) * items, b_units = sizeof(int4) * (units + passes);
     const size_t b_ranges = sizeof(int2) * static_cast<size_t>(std::max(n_inst_, 1));
     const size_t need = b_tiles + b_group + b_units + b_ranges;
     if (need > table_stage_bytes_) {
@@ -1952,6 +1958,7 @@ bool Engine::upload_tables(const std::vector<Job*>& jobs, std::string& why) {
     Tile* t = reinterpret_cast<Tile*>(h_table_stage_);
     Tile* it = t + tiles;
     int4* un = reinterpret_cast<int4*>(it + items);
+    int4* pa = un + units;
     n_tiles_ = 0;
     for (const Job* j : jobs) {
         std::memcpy(t + n_tiles_, j->tiles.data(), sizeof(Tile) * j->tiles.size());
@@ -1962,11 +1969,13 @@ bool Engine::upload_tables(const std::vector<Job*>& jobs, std::string& why) {
             count[g] += static_cast<int32_t>(list.size());
         }
         for (const int4& u : j->units) *un++ = make_int4(u.x + n_tiles_, u.y, u.z, u.w);
+        for (const int4& u : j->passes) *pa++ = make_int4(u.x + n_tiles_, u.y, u.z, u.w);
         h_ranges_[j->slot] = int2{n_tiles_, n_tiles_ + static_cast<int>(j->tiles.size())};
         n_tiles_ += static_cast<int>(j->tiles.size());
     }
     n_units_ = static_cast<int>(units);
-    std::memcpy(un, h_ranges_.data(), b_ranges);
+    n_passes_ = static_cast<int>(passes);
+    std::memcpy(pa, h_ranges_.data(), b_ranges);
     const unsigned char* at = h_table_stage_;
     auto copy = [&](void* dst, size_t bytes) {
         if (bytes) cudaMemcpyAsync(dst, at, bytes, cudaMemcpyHostToDevice, stream_);
@@ -1998,6 +2007,7 @@ bool Engine::run_once(std::string& why) {
     h_ctrl_->n_inst = n_inst_;
     h_ctrl_->n_tiles = n_tiles_;
     h_ctrl_->n_units = n_units_;
+    h_ctrl_->n_passes = n_passes_;
     std::memcpy(h_ctrl_->group_begin, group_begin_, sizeof(group_begin_));
     for (int k = 0; k < 3; ++k) {
         h_ctrl_->check_due[k] = 1;  // the first body checks whatever is due; later ones as counted
@@ -2219,6 +2229,7 @@ int Engine::profile_step(uint64_t id, int launches, double* ms_out, double* byte
     h_ctrl_->n_inst = n_inst_;
     h_ctrl_->n_tiles = n_tiles_;
     h_ctrl_->n_units = n_units_;
+    h_ctrl_->n_passes = n_passes_;
     std::memcpy(h_ctrl_->group_begin, group_begin_, sizeof(group_begin_));
     for (int k = 0; k < 3; ++k) h_ctrl_->step_due[k] = kMaxInterval;
     cudaMemcpyAsync(d_ctrl_, h_ctrl_, sizeof(Ctrl), cudaMemcpyHostToDevice, stream_);
@@ -2283,6 +2294,7 @@ int Engine::profile_cg(uint64_t id, int iterations, double* ms_matvec, double* m
     h_ctrl_->n_inst = n_inst_;
     h_ctrl_->n_tiles = n_tiles_;
     h_ctrl_->n_units = n_units_;
+    h_ctrl_->n_passes = n_passes_;
     h_ctrl_->n_cg = 1;
     cudaMemcpyAsync(d_ctrl_, h_ctrl_, sizeof(Ctrl), cudaMemcpyHostToDevice, stream_);
     const View v = view();

@@ -16,9 +16,9 @@ constexpr int kBlock = 256;          // threads per CTA of every tile kernel
 constexpr int kMaxInterval = 32;     // maximum check interval (iterations per chunk)
 constexpr int kTileNnz = 4096;       // target nonzeros per tile
 constexpr int kTileRows = 512;       // maximum rows per tile
-constexpr int kCgUnitMin = 2;        // tiles per work unit of the polish CG product and the sliced check: about
-constexpr int kCgUnitMax = 8;        //   this many at least, and up to this many for large instances (cg_units)
-constexpr int kCgSmall = 16;         // tiles up to which a mixed instance's units are single tiles (cg_units)
+constexpr int kCgUnitMin = 2;        // tiles per work unit of the polish CG product: about
+constexpr int kCgUnitMax = 8;        //   this many at least, and up to this many for large instances (work_units)
+constexpr int kCgSmall = 16;         // tiles up to which a mixed instance's units are single tiles (work_units)
 constexpr int kCgRowsum = 4 * kTileRows;  // rows per CG work unit at most (its row sums, 16 KB)
 constexpr int kCgTurns = 2;          // CG iterations per body of the graph's CG loop (a body's start costs several us)
 constexpr int kCgGroups = 2;         // row groups per warp whose loads the CG product keeps in flight
@@ -290,6 +290,7 @@ struct Ctrl {
     int32_t n_inst;        // instance records in use
     int32_t n_tiles;       // tiles in use
     int32_t n_units;       // CG work units in use (View::units)
+    int32_t n_passes;      // check and residual work units in use, behind those
     int32_t bodies;        // loop bodies run in the current launch
     int32_t body_cap;      // stop the device loop after this many bodies
     int32_t running;       // instances still running (written by the control kernel)
@@ -324,7 +325,8 @@ struct View {
     const int2* ranges;      // per-instance tile range [x, y) in the tile table
     const Tile* group_tiles;     // the tiles (sliced instances: pieces of kSlicePiece rows) ordered by step group (Ctrl::group_begin)
     const double2* momentum;     // FISTA: beta_k and t_{k+1} for k < kMomentumTable (they depend on k alone)
-    const int4* units;           // CG work units: x the first tile of a run of y consecutive tiles of one
+    const int4* units;           // work units of the CG product, then those of the sliced checks and the residual
+                                 // pass: x the first tile of a run of y consecutive tiles of one
                                  // instance, z the unit's index within the instance, w its unit count
 };
 

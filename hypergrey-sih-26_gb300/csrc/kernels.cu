@@ -1391,9 +1391,9 @@ __global__ void __launch_bounds__(kBlock, 4) check_slice_kernel(View v) {
     let_next_launch_begin();
     wait_for_previous_launch();
     if (v.ctrl->check_due[FAMILY_FP64] == 0) return;
-    const int nu = v.ctrl->n_units;
-    for (int un = blockIdx.x; un < nu; un += gridDim.x) {
-        const int4 U = v.units[un];  // first tile, tiles, index and units of its instance
+    const int first = v.ctrl->n_units, np = v.ctrl->n_passes;
+    for (int un = blockIdx.x; un < np; un += gridDim.x) {
+        const int4 U = v.units[first + un];  // first tile, tiles, index and units of its instance
         const Tile T = v.tiles[U.x];
         if (!is_sliced(T.variant)) continue;
         InstDev& I = v.inst[T.inst];
@@ -1472,9 +1472,9 @@ __global__ void __launch_bounds__(kBlock, 4) check_slice_mixed_kernel(View v) {
     let_next_launch_begin();
     wait_for_previous_launch();
     if (v.ctrl->check_due[FAMILY] == 0) return;
-    const int nu = v.ctrl->n_units;
-    for (int un = blockIdx.x; un < nu; un += gridDim.x) {
-        const int4 U = v.units[un];  // first tile, tiles, index and units of its instance
+    const int first = v.ctrl->n_units, np = v.ctrl->n_passes;
+    for (int un = blockIdx.x; un < np; un += gridDim.x) {
+        const int4 U = v.units[first + un];  // first tile, tiles, index and units of its instance
         const Tile T = v.tiles[U.x];
         if (!is_sliced(T.variant)) continue;
         InstDev& I = v.inst[T.inst];
@@ -2170,13 +2170,13 @@ __device__ void finish_residual(const View& v, InstDev& I, int inst, int2 R, int
 
 // Four blocks per SM (64 registers, a few spills): 2.307 ms per 1M random-graph solve against
 // 2.329 ms at the compiler's three (80 registers); the check kernels measured slower at four.
-// Over the CG product's work units (runs of consecutive tiles of one instance, as many as the
+// Over work units (runs of consecutive tiles of one instance, no more than the
 // resident blocks): one unit per block in one round, the unit's tiles one after the other, one
 // reduction and one publication per unit (the unit's partial in its instance's slot R.x + index).
 __global__ void __launch_bounds__(kBlock, 4) polish_residual_kernel(View v) {
-    const int nu = v.ctrl->n_units;
-    for (int un = blockIdx.x; un < nu; un += gridDim.x) {
-        const int4 U = v.units[un];  // first tile, tiles, index and units of its instance
+    const int first = v.ctrl->n_units, np = v.ctrl->n_passes;
+    for (int un = blockIdx.x; un < np; un += gridDim.x) {
+        const int4 U = v.units[first + un];  // first tile, tiles, index and units of its instance
         const Tile T0 = v.tiles[U.x];
         if (is_sliced(T0.variant)) continue;  // polish_residual_slice_kernel's
         InstDev& I = v.inst[T0.inst];
@@ -2401,9 +2401,9 @@ __device__ int residual_slices(const InstDev& I, const Tile& T, int tile, int n_
 __global__ void __launch_bounds__(kBlock, kResidualBlocks) polish_residual_slice_kernel(View v) {
     extern __shared__ __align__(16) unsigned char dyn_smem[];
     ResidualShared& S = *reinterpret_cast<ResidualShared*>(dyn_smem);
-    const int nu = v.ctrl->n_units;
-    for (int un = blockIdx.x; un < nu; un += gridDim.x) {
-        const int4 U = v.units[un];  // first tile, tiles, index and units of its instance
+    const int first = v.ctrl->n_units, np = v.ctrl->n_passes;
+    for (int un = blockIdx.x; un < np; un += gridDim.x) {
+        const int4 U = v.units[first + un];  // first tile, tiles, index and units of its instance
         const Tile T0 = v.tiles[U.x];
         if (!is_sliced(T0.variant)) continue;
         InstDev& I = v.inst[T0.inst];
