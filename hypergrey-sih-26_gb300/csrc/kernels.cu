@@ -32,6 +32,14 @@ namespace {
 
 #define kInf (__longlong_as_double(0x7ff0000000000000LL))
 
+// Asynchronous copies of BYTES (4 or 8) from global to shared memory, and the wait for a thread's own.
+template <int BYTES>
+__device__ __forceinline__ void copy_async(void* to, const void* from) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(to))), "l"(from),
+                 "n"(BYTES));
+}
+__device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 __device__ __forceinline__ int64_t now_ns() {
     uint64_t t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -2927,7 +2935,8 @@ __device__ __forceinline__ double gate_lipschitz(const InstDev& I) {
 //     The row with the largest sum is always among them, so L is the same bits whatever the
 //     order in which the warps run.
 // A warp takes 32 consecutive rows and walks their entries in windows of kGateBuf: it stages a
-// window's values and columns in shared memory with coalesced loads (writing the split as it
+// window's values and columns in shared memory with coalesced asynchronous copies, all of a window in
+// flight at once (four loads per lane at a time: 22 us more for 15M entries; writing the split as it
 // goes), and each lane then adds the part of its own row inside the window, so every row's sums
 // run in column order whatever its length; the FP64 sums re-read their rows (from L2).
 constexpr int kGateWarps = 4;      // warps per block of the gate kernel
@@ -2964,13 +2973,13 @@ __global__ void __launch_bounds__(kGateWarps * 32) convexity_gate_kernel(const i
         bool offd = false;   // a nonzero off-diagonal value (check_qp_solution's positive_diagonal)
         for (int w = kb; w < ke; w += kGateBuf) {
             const int we = min(ke, w + kGateBuf);
-            // the window's loads first, several per lane in flight; then the entry work from
+            // the whole window in flight at once (asynchronous copies), then the entry work from
             // shared memory
-#pragma unroll 4
             for (int k = w + lane; k < we; k += 32) {
-                bv[k - w] = __ldg(vbits + k);
-                bc[k - w] = __ldg(col + k);
+                copy_async<8>(&bv[k - w], vbits + k);
+                copy_async<4>(&bc[k - w], col + k);
             }
+            copies_done();
             __syncwarp();
             for (int k = w + lane; k < we; k += 32) {
                 const uint64_t vb = bv[k - w];
@@ -3204,17 +3213,15 @@ __global__ void __launch_bounds__(kSliceWindow) slice_entries_kernel(InstDev I, 
     const bool staged = ke - kb <= cap;
     if (staged) {
         for (int k = t; k < ke - kb; k += kSliceWindow) {
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(sval + k))),
-                         "l"(val + kb + k));
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(scol + k))),
-                         "l"(col + kb + k));
+            copy_async<8>(sval + k, val + kb + k);
+            copy_async<4>(scol + k, col + kb + k);
         }
     }
     const bool valid = t < rows;
     const int len = valid ? __ldg(I.slice_len + w0 + t) : 0;
     const int src = valid ? __ldg(rowptr + w0 + __ldg(I.slice_row + w0 + t)) - kb : 0;
     int k = valid ? __ldg(I.slice_base + ((w0 + t) >> 5)) + lane : 0;
-    asm volatile("cp.async.wait_all;" ::: "memory");
+    copies_done();
     __syncthreads();
     const int longest = __shfl_sync(0xffffffffu, len, 0);
 #pragma unroll 4
@@ -3561,17 +3568,18 @@ __global__ void __launch_bounds__(kBlock) lanczos_update_kernel(InstDev I, int n
 }
 
 // ---- standalone check on caller arrays ---------------------------------------------------------
-// On the caller's CSR, a row per lane, so that a row's products are fused and its sum needs no tree:
-// the FP64 pipe (an issue slot of 16 cycles per warp instruction) and the gathers bound it.  On the
-// random graph 1M the verification call (gate and check) takes 346 us; 357 with two lanes a row, 366 with
-// warp-staged rows (rounded products, then sums), 468 with those on 245 blocks of 4096 rows, which left
-// most of the SMs' warps unused.
+// On the caller's CSR, two lanes a row: the gathers bound it, the L1 has to hold the sectors of 16
+// rows' entries until their lanes have used them up, and an FP64 instruction takes a warp 16 cycles.
+// So it runs four blocks an SM (64 registers) and leaves the shared memory to the L1.  On the random
+// graph 1M the verification call (gate and check) takes 252 us; with one lane a row 268, four 254, one
+// lane at three blocks 320; with 48 KB of shared memory per block (unused by then) 342, and
+// with warp-staged rows on 245 blocks of 4096 rows, which left most of the SMs idle, 468.
 struct StandaloneScratch {
     int done;
     int pad[3];
 };
 
-__global__ void __launch_bounds__(kBlock) check_standalone_kernel(CheckSrc s, int n, double tol, double offset,
+__global__ void __launch_bounds__(kBlock, 4) check_standalone_kernel(CheckSrc s, int n, double tol, double offset,
                                                                  Partial* partial, StandaloneScratch* scr,
                                                                  double* result) {
     // whole warps of rows; the last blocks may have none
@@ -3579,7 +3587,7 @@ __global__ void __launch_bounds__(kBlock) check_standalone_kernel(CheckSrc s, in
     const int64_t rb = blockIdx.x * rows_per_block;
     const int re = static_cast<int>(min(static_cast<int64_t>(n), rb + rows_per_block));
     Acc a = acc_identity();
-    if (rb < re) check_rows<0>(s, 1, static_cast<int>(rb), re, a);
+    if (rb < re) check_rows<0>(s, 2, static_cast<int>(rb), re, a);
     Acc total = block_reduce_check(a, s.gate != 0);
     __shared__ int is_last;
     if (threadIdx.x == 0) {
@@ -3789,7 +3797,6 @@ int tile_grid(int sms) {
     g_waves.check_verify = wave_of(check_kernel<FAMILY_VERIFY>, sms, kSmem8);
     g_waves.matvec = wave_of(cg_matvec_kernel, sms, 0);
     g_waves.residual = wave_of(polish_residual_kernel, sms, 0);
-    wave_of(check_standalone_kernel, sms, kSmem8);
     g_waves.polish = wave_of(cg_vector_kernel, sms, 0);
     int m = g_waves.exact;
     for (int w : g_waves.group) m = w > m ? w : m;
@@ -4037,18 +4044,12 @@ void launch_check_standalone(int64_t n, const int32_t* rowptr, const int32_t* co
     src.diag = nullptr;  // a diagonal Hessian's only entry per row is its diagonal
     src.gate = gate;
     const int grid = check_grid(n);
-    // The kernel's dynamic shared memory plus its static reduction buffer exceed the default
-    // 48 KB: opt in on every call (a cheap host call; a per-device flag would go stale when the
-    // caller resets the device and its context is recreated).
-    cudaFuncSetAttribute(check_standalone_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem8);
     auto* scr = static_cast<StandaloneScratch*>(scratch);
     auto* partial = reinterpret_cast<Partial*>(static_cast<char*>(scratch) + 256);
-    check_standalone_kernel<<<grid, kBlock, kSmem8, s>>>(src, static_cast<int>(n), tol, offset, partial, scr, result);
+    check_standalone_kernel<<<grid, kBlock, 0, s>>>(src, static_cast<int>(n), tol, offset, partial, scr, result);
 }
 
 cudaError_t load_check_standalone() {
-    cudaError_t e = cudaFuncSetAttribute(check_standalone_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem8);
-    if (e != cudaSuccess) return e;
     cudaFuncAttributes attr;
     return cudaFuncGetAttributes(&attr, check_standalone_kernel);
 }
