@@ -20,7 +20,7 @@ constexpr int kCgUnitMin = 2;        // tiles per work unit of the polish CG pro
 constexpr int kCgUnitMax = 8;        //   this many at least, and up to this many for large instances (work_units)
 constexpr int kCgSmall = 16;         // tiles up to which a mixed instance's units are single tiles (work_units)
 constexpr int kCgRowsum = 4 * kTileRows;  // rows per CG work unit at most (its row sums, 16 KB)
-constexpr int kCgTurns = 2;          // CG iterations per body of the graph's CG loop (a body's start costs several us)
+constexpr int kCgTurns = 4;          // CG iterations per body of the graph's CG loop (a body's start costs 4 us, an idle turn 2)
 constexpr int kCgGroups = 2;         // row groups per warp whose loads the CG product keeps in flight
 constexpr int kCgUnroll = 2;         // entries per row group and lane (and epilogue rows per thread) per pass of the CG product
 constexpr int kMomentumTable = 8192; // FISTA momenta kept in a table (View::momentum)
@@ -298,7 +298,7 @@ struct Ctrl {
     int32_t n_polish;
     int32_t error;         // non-zero: a kernel detected an inconsistency
     int32_t n_cg;          // instances that may still run CG iterations in this body
-    int32_t n_cg_before;   // n_cg as the last CG vector step found it
+    int32_t n_cg_left[kCgTurns];  // n_cg as each turn's CG vector step of the loop's body found it
     int32_t cg_iters;      // CG iterations run in this body
     long long kernels;     // engine kernels executed by this launch (counted by gate/control)
     int32_t group_begin[kStepGroups + 1];  // step groups: [begin, end) in View::group_tiles

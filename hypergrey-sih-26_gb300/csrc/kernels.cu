@@ -2517,15 +2517,17 @@ __global__ void __launch_bounds__(kBlock, kProductBlocks) cg_matvec_slice_kernel
 // r -= alpha s, u = M^-1 r (and its FP32 pairs for the next product), every vector streamed by
 // position.  No reduction: the product kernel's finalizer already chose alpha and beta.  Instances
 // that finished CG write x back to their free rows, snapped into the box, here.
-// In a graph (cap > 0) a body of the CG loop runs kCgTurns iterations, `turn` this one's place among them, and
-// block 0 of the last decides whether another body runs: while an instance
-// still iterates and fewer than `cap` iterations ran (the product kernel, which completed before
-// this launch, counted finishing instances down).
+// In a graph (cap > 0) a body of the CG loop runs kCgTurns iterations, `turn` this one's place among them
+// (2 turns: 10k rows 266 us, 4: 258, the 1M random graph 1707 and 1697, 6: no better), and block 0 of the
+// last decides whether another body runs: while an instance still iterates and fewer than `cap`
+// iterations ran (the product kernel, which completed before this launch, counted finishing
+// instances down).
 __global__ void __launch_bounds__(kBlock) cg_vector_kernel(View v, cudaGraphConditionalHandle h_cg, int cap, int turn, int launches) {
     let_next_launch_begin();
     wait_for_previous_launch();
     Ctrl* ctrl = v.ctrl;
-    if (turn > 0 && ctrl->n_cg_before == 0) {  // every instance had finished an iteration ago
+    if (turn > 0 && ctrl->n_cg_left[turn - 1] == 0) {  // every instance had finished an iteration ago
+        if (blockIdx.x == 0 && threadIdx.x == 0) ctrl->n_cg_left[turn] = 0;
         if (turn == kCgTurns - 1 && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(h_cg, 0u);
         return;
     }
@@ -2533,8 +2535,7 @@ __global__ void __launch_bounds__(kBlock) cg_vector_kernel(View v, cudaGraphCond
         const int it = ++ctrl->cg_iters;
         ctrl->kernels += launches;
         if (turn == kCgTurns - 1) cudaGraphSetConditional(h_cg, (ctrl->n_cg > 0 && it < cap) ? 1u : 0u);
-        static_assert(kCgTurns == 2, "the turn that writes n_cg_before is not one that reads it");
-        if (turn == 0) ctrl->n_cg_before = ctrl->n_cg;
+        ctrl->n_cg_left[turn] = ctrl->n_cg;
     }
 
     const int nt = v.ctrl->n_tiles;
@@ -2752,7 +2753,6 @@ __global__ void __launch_bounds__(1024) advance_kernel(View v, cudaGraphConditio
         ctrl->check_due[FAMILY_VERIFY] += c.polish;
         ctrl->n_polish = c.polish;
         ctrl->n_cg = c.polish;
-        ctrl->n_cg_before = c.polish;
         ctrl->cg_iters = 0;
         long long launched = 1;
         for (int k = 0; k < 3; ++k) launched += ctrl->n_fista[k] > 0 || ((body.always >> k) & 1u) ? body.n[k] : 0;
