@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(kB) admm_direction_kernel(int n, double* __res
 // Bounds of an iteration on 1M variables, 15M + 2 x 4M entries: 23M random gathers (92 us at the
 // 250 G/s this GPU gathers), 276 MB of entries (41 us), on the FP64 pipe 23M products and about
 // eight operations a row (50 us); the L2 hands out a 32-byte sector per gathered number, which with
-// the entries makes 104 us.  Now 154: A d 22, K d 100, update 20, direction and the loop 11 (two
+// the entries makes 104 us.  Now 152: A d 22, K d 100, update 20, direction and the loop 11 (two
 // iterations per body of the loop: 157).  Four lanes per CSR row spent as much FP64 time again on tree
 // additions and quarter-warp epilogues, and a general division per row: 217 us an iteration.
 // Columns of a row in flight: 5 on large systems (64 registers; 4: 183, 8: 167 us an iteration), whole

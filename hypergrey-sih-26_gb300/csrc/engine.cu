@@ -336,8 +336,8 @@ int choose_variant(int64_t n, int64_t nnz, int64_t longest_row, const bqp_option
 // kCgRowsum rows (the row sums' shared buffer; units of kCgUnitMin tiles always fit).
 // Checks and the residual pass take single tiles where they can: the FP64 pipe of an SM bounds a check
 // (1024 rows of 11 entries take 10 us on one), barriers and latency the residual pass (10k rows 38 us
-// in units of two tiles; a mixed solve of 10k rows 294 -> 275 us).  A CG product is shorter than a unit's reduction and publication cost its
-// block, so its units are single tiles only where an instance has kCgSmall of them at most: 1k
+// in units of two tiles; a mixed solve of 10k rows 294 -> 275 us).  A unit of a CG product costs its
+// block a reduction and a publication, about as long as the product itself, so its units are single tiles only where an instance has kCgSmall of them at most: 1k
 // rows 230 -> 197 us, 256 uneven solves 1.33 ms on the device either way; with up to 32 tiles these take
 // 1.42 ms, with any number 1.45.  Depends on the instance alone, so the partial sums, and the CG
 // iterates, are the same in a batch as solo.

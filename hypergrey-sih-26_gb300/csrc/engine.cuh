@@ -293,7 +293,7 @@ struct Ctrl {
     int32_t n_passes;      // check and residual work units in use, behind those
     int32_t bodies;        // loop bodies run in the current launch
     int32_t body_cap;      // stop the device loop after this many bodies
-    int32_t running;       // instances still running (written by the control kernel)
+    int32_t running;       // instances still running (written by the gate kernel)
     int32_t n_fista[3];    // instances in the FISTA phase, per precision
     int32_t n_polish;
     int32_t error;         // non-zero: a kernel detected an inconsistency

@@ -1,6 +1,8 @@
 // sm_103a kernels of the box-QP engine.
 //
 // Hot path (one launch per FISTA iteration, graph-replayed):
+//   step_slice_*  the step (below) over sliced rows (engine.cuh: VAR_SLICE), a slice of 32 rows per warp turn;
+//                 most instances run on those, and so do their checks and their polish
 //   step_kernel   fused CSR SpMV g = Q w, gradient step, clamp to [l,u], momentum update
 //                 w+ = x+ + beta (x+ - x): reads w from one ping-pong buffer and writes the
 //                 other, so no separate gradient array or second launch is needed
