@@ -75,3 +75,10 @@ def test_product_and_solve(n, m, per_row, wide):
         assert np.max(np.abs(left)) <= 1e-9 * top + 1e-12 * top * (1.0 + float(np.max(size)))
     finally:
         s.close()
+
+
+@pytest.mark.parametrize('n', [38912, 38913, 77825, 155649])
+def test_product_and_solve_at_the_edges_of_the_grid(n):
+    """1216 slices: a slice for each of eight warps on 152 SMs; one more; two blocks' worth and one more;
+    and one more than the largest grid has warps (the rows and the bounds are those above)."""
+    test_product_and_solve(n, 33, 4, 100)
