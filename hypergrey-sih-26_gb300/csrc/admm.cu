@@ -14,16 +14,12 @@
 // each reduction finalizes it in a fixed order and sets the loop condition, so a solve is one
 // graph launch with no host round trip per iteration.  FP64 throughout (the reference's inner
 // products; its long double dot accumulation is not reproduced, so iterates agree to rounding).
-//
-// Systems whose rows allow it (sliceable: H's and A' rows together, and A's) keep sliced rows
-// (engine.cuh): row j of H and row j of A' are one row over the stacked vector [v; t], so K v is one
-// product with one lane per row, its sums without shuffles and its epilogue on full warps; every
-// vector is in slice order and host vectors are permuted as they come and go.  The other systems
-// keep CSR with four lanes per row.
+// CG loses orthogonality and amplifies a difference of one rounding to the size of its accuracy
+// (1M variables, 95 iterations: x 1.5e-9 apart, the count by up to 5), so the order of every sum
+// here is part of the results: four interleaved fused chains a row and their tree, a dot product by
+// the thread that holds the row, and the tree over threads and blocks.  The CPU oracle runs the same
+// order and the tests ask for the same bits.
 #include "boxqp.h"
-#include "fpbits.h"
-#include "kernels.cuh"
-#include "slices.cuh"
 
 #include <cuda_runtime.h>
 
@@ -41,7 +37,7 @@ namespace {
 constexpr int kB = 256;
 constexpr int kLanes = 4;         // lanes per CSR row
 constexpr int kRows = kB / kLanes;
-constexpr int kSms = 152, kMaxBlocks = kSms * 4;
+constexpr int kMaxBlocks = 152 * 4;
 
 struct AdmmState {
     double rz, alpha, beta;
@@ -58,8 +54,6 @@ __device__ __forceinline__ unsigned long long umax64(unsigned long long a, unsig
 __device__ __forceinline__ unsigned long long dbits(double v) {
     return static_cast<unsigned long long>(__double_as_longlong(v));
 }
-// the bits of |v| in integer arithmetic (fpbits.h: bits64)
-__device__ __forceinline__ unsigned long long abs_bits(double v) { return bqp::bits64(v) & 0x7fffffffffffffffull; }
 
 // y = M v for rows [0, rows) of a CSR matrix, kLanes lanes per row in a fixed order; returns the
 // row sum in the group's lane 0 (valid for r < rows).
@@ -76,67 +70,56 @@ __device__ __forceinline__ double csr_row(const int32_t* __restrict__ rp, const 
     return s;
 }
 
-// Fixed-order block sums of one or two doubles (TWO) and a maximum; the last block (ticket) adds the block
-// partials, all its threads strided over them and then the same fixed tree, and returns true in
-// its thread 0 with the grid totals.  A sum that nobody reads is left out: its additions take the
-// FP64 pipe 16 cycles per warp and level.
-template <bool TWO>
-__device__ __forceinline__ void block_tree(double& a, double& b, unsigned long long& mx, double* ra, double* rb,
-                                           unsigned long long* rm) {
+// Fixed-order block sum and maximum; the last block (ticket) adds the block partials, all its
+// threads strided over them and then the same fixed tree, and returns true in its thread 0 with the
+// grid totals.
+__device__ __forceinline__ void block_tree(double& a, unsigned long long& mx, double* ra, unsigned long long* rm) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         a += __shfl_xor_sync(0xffffffffu, a, o);
-        if (TWO) b += __shfl_xor_sync(0xffffffffu, b, o);
         mx = umax64(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (lane == 0) {
         ra[warp] = a;
-        if (TWO) rb[warp] = b;
         rm[warp] = mx;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
         a = 0;
-        b = 0;
         mx = 0;
         for (int w = 0; w < kB / 32; ++w) {
             a += ra[w];
-            if (TWO) b += rb[w];
             mx = umax64(mx, rm[w]);
         }
     }
 }
 
-template <bool TWO>
-__device__ bool reduce_last(double a, double b, unsigned long long mx, double* partial, AdmmState* st, double* ta,
-                            double* tb, unsigned long long* tm) {
-    __shared__ double ra[kB / 32], rb[TWO ? kB / 32 : 1];
+__device__ bool reduce_last(double a, unsigned long long mx, double* partial, AdmmState* st, double* ta,
+                            unsigned long long* tm) {
+    __shared__ double ra[kB / 32];
     __shared__ unsigned long long rm[kB / 32];
     __shared__ int last;
-    block_tree<TWO>(a, b, mx, ra, rb, rm);
+    block_tree(a, mx, ra, rm);
     if (threadIdx.x == 0) {
-        partial[3 * blockIdx.x] = a;
-        if (TWO) partial[3 * blockIdx.x + 1] = b;
-        partial[3 * blockIdx.x + 2] = __longlong_as_double(static_cast<long long>(mx));
+        partial[2 * blockIdx.x] = a;
+        partial[2 * blockIdx.x + 1] = __longlong_as_double(static_cast<long long>(mx));
         __threadfence();
         last = atomicAdd(&st->ticket, 1u) == gridDim.x - 1 ? 1 : 0;
     }
     __syncthreads();
     if (!last) return false;
     __threadfence();
-    double sa = 0, sb = 0;
+    double sa = 0;
     unsigned long long sm = 0;
     for (unsigned k = threadIdx.x; k < gridDim.x; k += kB) {
-        sa += __ldcg(partial + 3 * k);
-        if (TWO) sb += __ldcg(partial + 3 * k + 1);
-        sm = umax64(sm, dbits(__ldcg(partial + 3 * k + 2)));
+        sa += __ldcg(partial + 2 * k);
+        sm = umax64(sm, dbits(__ldcg(partial + 2 * k + 1)));
     }
-    block_tree<TWO>(sa, sb, sm, ra, rb, rm);  // thread 0 read the first tree's ra/rb/rm before the barrier above
+    block_tree(sa, sm, ra, rm);  // thread 0 read the first tree's ra/rm before the barrier above
     if (threadIdx.x != 0) return false;
     st->ticket = 0;
     *ta = sa;
-    *tb = sb;
     *tm = sm;
     return true;
 }
@@ -173,7 +156,7 @@ __global__ void __launch_bounds__(kB) admm_k_kernel(Sys s, const double* __restr
                                                     AdmmState* st, cudaGraphConditionalHandle loop) {
     if (mode == 2 && st->stop) return;
     const int sl = threadIdx.x % kLanes;
-    double acc_a = 0, acc_b = 0;
+    double acc_a = 0;
     unsigned long long acc_m = 0;
     for (int base = blockIdx.x * kRows; base < s.n; base += gridDim.x * kRows) {
         const int j = base + static_cast<int>(threadIdx.x) / kLanes;
@@ -197,9 +180,9 @@ __global__ void __launch_bounds__(kB) admm_k_kernel(Sys s, const double* __restr
         }
     }
     if (mode == 0) return;
-    double ta, tb;
+    double ta;
     unsigned long long tm;
-    if (!reduce_last<true>(acc_a, acc_b, acc_m, partial, st, &ta, &tb, &tm)) return;
+    if (!reduce_last(acc_a, acc_m, partial, st, &ta, &tm)) return;
     if (mode == 1) {
         st->rz = ta;
         st->rmax = tm;
@@ -233,9 +216,9 @@ __global__ void __launch_bounds__(kB) admm_update_kernel(Sys s, double* __restri
         acc_a = fma(rr, pp, acc_a);
         acc_m = umax64(acc_m, dbits(fabs(rr)));
     }
-    double ta, tb;
+    double ta;
     unsigned long long tm;
-    if (!reduce_last<false>(acc_a, 0.0, acc_m, partial, st, &ta, &tb, &tm)) return;
+    if (!reduce_last(acc_a, acc_m, partial, st, &ta, &tm)) return;
     st->beta = ta / st->rz;
     st->rz = ta;
     st->rmax = tm;
@@ -249,280 +232,6 @@ __global__ void __launch_bounds__(kB) admm_direction_kernel(int n, double* __res
     if (st->stop) return;
     const double beta = st->beta;
     for (int j = blockIdx.x * kB + threadIdx.x; j < n; j += gridDim.x * kB) d[j] = __dadd_rn(pre[j], __dmul_rn(beta, d[j]));
-}
-
-// ---- the same over sliced rows ------------------------------------------------------------------
-// Bounds of an iteration on 1M variables, 15M + 2 x 4M entries: 23M random gathers (92 us at the
-// 250 G/s this GPU gathers), 276 MB of entries (41 us), on the FP64 pipe 23M products and about
-// eight operations a row (50 us); the L2 hands out a 32-byte sector per gathered number, which with
-// the entries makes 104 us.  Now 152: A d 22, K d 100, update 20, direction and the loop 11 (two
-// iterations per body of the loop: 157).  Four lanes per CSR row spent as much FP64 time again on tree
-// additions and quarter-warp epilogues, and a general division per row: 217 us an iteration.
-// Columns of a row in flight: 5 on large systems (64 registers; 4: 183, 8: 167 us an iteration), whole
-// rows on small ones, which are bound by the latency of their loads.
-constexpr int kAhead = 5, kAheadSmall = 16;
-constexpr int64_t kSmallRows = 65536;
-constexpr int kSliceBlocks = kMaxBlocks;  // their partial sums share the buffer of kMaxBlocks
-struct SliceRows {
-    int n;
-    const uint8_t* len;
-    const uint8_t* row;
-    const int32_t* base;
-    const int32_t* col;
-    const double* val;
-};
-struct SliceSys {
-    SliceRows k, a;       // [H, A'] over [v; t], and A over v
-    int t0;               // where t begins in a stacked vector
-    const double* rho;    // in A's slice order
-    double sigma;
-    const double* minv;   // 1 / M
-};
-
-// A warp's first slice, of a stride of gridDim.x * kB / 32: a block's warps take neighbours, or, where
-// there are fewer slices than warps, the blocks share them out.
-__device__ __forceinline__ int first_slice(int slices) {
-    const int warp = threadIdx.x >> 5, blocks = gridDim.x;
-    return slices < blocks * (kB / 32) ? warp * blocks + static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x) * (kB / 32) + warp;
-}
-
-// A lane's row of slice s: its sum (0 past the last row).  The first columns are loaded before
-// `wait`, the wait for the launch that wrote the vector.
-template <int AHEAD, class Wait>
-__device__ __forceinline__ double slice_row_sum(const SliceRows& R, int s, const double* v, Wait wait) {
-    const int p = s * 32 + static_cast<int>(threadIdx.x & 31);
-    const int len = p < R.n ? __ldg(R.len + p) : 0;
-    int k = __ldg(R.base + s) + static_cast<int>(threadIdx.x & 31);
-    const int longest = __shfl_sync(0xffffffffu, len, 0);
-    bqp::SliceColumns<AHEAD> e;
-    e.load(R.col, R.val, len, k);
-    wait();
-    double acc = e.add<false>(v, longest, 0.0);
-    for (int j = AHEAD; j < longest; j += AHEAD) {
-        e.load(R.col, R.val, len - j, k);
-        acc = e.add<false>(v, longest - j, acc);
-    }
-    return acc;
-}
-
-// Waits once for the launch before; then whether an earlier kernel ended the loop.
-struct WaitOnce {
-    bool waited = false;
-    __device__ __forceinline__ void operator()() {
-        if (!waited) bqp::wait_for_previous_launch();
-        waited = true;
-    }
-};
-
-// t = rho .* (A v), t behind v
-template <int AHEAD>
-__global__ void __launch_bounds__(kB, AHEAD > 8 ? 2 : 4) admm_a_slice_kernel(SliceSys S, double* v) {
-    bqp::let_next_launch_begin();
-    WaitOnce wait;
-    const int slices = (S.a.n + 31) / 32;
-    for (int s = first_slice(slices); s < slices; s += gridDim.x * (kB / 32)) {
-        const double y = slice_row_sum<AHEAD>(S.a, s, v, wait);
-        const int p = s * 32 + static_cast<int>(threadIdx.x & 31);
-        if (p < S.a.n) v[S.t0 + p] = __ldg(S.rho + p) * y;
-    }
-    wait();
-}
-
-// out = K v by the modes of admm_k_kernel (0 apply, 1 set-up: v = x, 2 iteration: v = d)
-template <int AHEAD>
-__global__ void __launch_bounds__(kB, AHEAD > 8 ? 2 : 4) admm_k_slice_kernel(SliceSys S, const double* v, double* out, int mode, const double* rhs,
-                                                         double* r, double* pre, double* d, double* partial, AdmmState* st,
-                                                         cudaGraphConditionalHandle loop) {
-    bqp::let_next_launch_begin();
-    WaitOnce wait;
-    double acc_a = 0;
-    unsigned long long acc_m = 0;
-    const int slices = (S.k.n + 31) / 32;
-    for (int s = first_slice(slices); s < slices; s += gridDim.x * (kB / 32)) {
-        const double sum = slice_row_sum<AHEAD>(S.k, s, v, wait);
-        const int p = s * 32 + static_cast<int>(threadIdx.x & 31);
-        if (p >= S.k.n) continue;
-        const double vp = v[p], o = fma(S.sigma, vp, sum);
-        out[p] = o;
-        if (mode == 1) {
-            const double rr = rhs[p] - o, pp = rr * __ldg(S.minv + p);
-            r[p] = rr;
-            pre[p] = pp;
-            d[p] = pp;
-            acc_a = fma(rr, pp, acc_a);
-            acc_m = umax64(acc_m, abs_bits(rr));
-        } else if (mode == 2) {
-            acc_a = fma(vp, o, acc_a);
-        }
-    }
-    wait();
-    if (mode == 0) return;
-    double ta, tb;
-    unsigned long long tm;
-    if (!reduce_last<false>(acc_a, 0.0, acc_m, partial, st, &ta, &tb, &tm)) return;
-    if (mode == 1) {
-        st->rz = ta;
-        st->rmax = tm;
-        st->inner = 0;
-        st->stop = 0;
-        cudaGraphSetConditional(loop, (st->max_inner > 0 && __longlong_as_double(static_cast<long long>(tm)) > st->accuracy) ? 1u : 0u);
-    } else {
-        if (!(ta > 0) || !isfinite(ta)) st->stop = 1;
-        else st->alpha = st->rz / ta;
-    }
-}
-
-// x += alpha d, r -= alpha K d, pre = r / M; then rz, beta and the loop condition
-__global__ void __launch_bounds__(kB) admm_update_slice_kernel(int n, const double* __restrict__ minv, double* x, double* r,
-                                                               double* pre, const double* d, const double* kd, double* partial,
-                                                               AdmmState* st, cudaGraphConditionalHandle loop) {
-    bqp::let_next_launch_begin();
-    bqp::wait_for_previous_launch();
-    if (st->stop) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(loop, 0u);
-        return;
-    }
-    const double alpha = st->alpha;
-    double acc_a = 0;
-    unsigned long long acc_m = 0;
-    for (int j = blockIdx.x * kB + threadIdx.x; j < n; j += gridDim.x * kB) {
-        x[j] = fma(alpha, d[j], x[j]);
-        const double rr = fma(-alpha, kd[j], r[j]), pp = rr * __ldg(minv + j);
-        r[j] = rr;
-        pre[j] = pp;
-        acc_a = fma(rr, pp, acc_a);
-        acc_m = umax64(acc_m, abs_bits(rr));
-    }
-    double ta, tb;
-    unsigned long long tm;
-    if (!reduce_last<false>(acc_a, 0.0, acc_m, partial, st, &ta, &tb, &tm)) return;
-    st->beta = ta / st->rz;
-    st->rz = ta;
-    st->rmax = tm;
-    st->inner += 1;
-    cudaGraphSetConditional(loop, (st->inner < st->max_inner && __longlong_as_double(static_cast<long long>(tm)) > st->accuracy) ? 1u : 0u);
-}
-
-// d = pre + beta d
-__global__ void __launch_bounds__(kB) admm_direction_slice_kernel(int n, double* d, const double* pre, const AdmmState* st) {
-    bqp::let_next_launch_begin();
-    bqp::wait_for_previous_launch();
-    if (st->stop) return;
-    const double beta = st->beta;
-    for (int j = blockIdx.x * kB + threadIdx.x; j < n; j += gridDim.x * kB) d[j] = fma(beta, d[j], pre[j]);
-}
-
-// 1 / M, M as admm_precond_kernel forms it: a row holds its H entries, then its A' entries in increasing i
-__global__ void __launch_bounds__(kB) admm_precond_slice_kernel(SliceSys S, double* __restrict__ minv) {
-    const int slices = (S.k.n + 31) / 32;
-    for (int s = first_slice(slices); s < slices; s += gridDim.x * (kB / 32)) {
-        const int p = s * 32 + static_cast<int>(threadIdx.x & 31);
-        const int len = p < S.k.n ? __ldg(S.k.len + p) : 0;
-        const int longest = __shfl_sync(0xffffffffu, len, 0);
-        int k = __ldg(S.k.base + s) + static_cast<int>(threadIdx.x & 31);
-        double dg = 0, m = 0;
-        bool head = true;
-        for (int j = 0; j < longest; ++j) {
-            const bool in = j < len;
-            if (in) {
-                const int c = __ldg(S.k.col + k);
-                const double a = __ldg(S.k.val + k);
-                if (c == p) dg = a;
-                if (c >= S.t0) {
-                    if (head) m = __dadd_rn(dg, S.sigma);
-                    head = false;
-                    m = __dadd_rn(m, __dmul_rn(__dmul_rn(__ldg(S.rho + c - S.t0), a), a));
-                }
-            }
-            k += __popc(__ballot_sync(0xffffffffu, in));
-        }
-        if (head) m = __dadd_rn(dg, S.sigma);
-        if (p < S.k.n) minv[p] = __ddiv_rn(1.0, m);
-    }
-}
-
-// rhs = A'(rho z - y) + (sigma x - c), in two kernels: yz into t, then the A' part of the stacked rows
-// (a row's H entries are skipped; its A' entries follow them)
-__global__ void __launch_bounds__(kB) admm_yz_kernel(int m, const double* __restrict__ rho, const double* __restrict__ z,
-                                                     const double* __restrict__ y, double* __restrict__ t) {
-    for (int i = blockIdx.x * kB + threadIdx.x; i < m; i += gridDim.x * kB)
-        t[i] = __dsub_rn(__dmul_rn(__ldg(rho + i), z[i]), y[i]);  // the reference's yz[i]
-}
-
-__global__ void __launch_bounds__(kB) admm_rhs_slice_kernel(SliceSys S, const double* __restrict__ stacked,
-                                                            const double* __restrict__ xa, const double* __restrict__ c,
-                                                            double* __restrict__ rhs, double* __restrict__ x0, double* partial,
-                                                            AdmmState* st, double iteration_factor) {
-    unsigned long long mx = 0;
-    const int slices = (S.k.n + 31) / 32;
-    for (int s = first_slice(slices); s < slices; s += gridDim.x * (kB / 32)) {
-        const int p = s * 32 + static_cast<int>(threadIdx.x & 31);
-        const int len = p < S.k.n ? __ldg(S.k.len + p) : 0;
-        const int longest = __shfl_sync(0xffffffffu, len, 0);
-        int k = __ldg(S.k.base + s) + static_cast<int>(threadIdx.x & 31);
-        double acc = 0;
-        for (int j = 0; j < longest; ++j) {
-            const bool in = j < len;
-            const int col = in ? __ldg(S.k.col + k) : 0;
-            if (col >= S.t0) acc = fma(__ldg(S.k.val + k), __ldg(stacked + col), acc);
-            k += __popc(__ballot_sync(0xffffffffu, in));
-        }
-        if (p < S.k.n) {
-            const double v = __dadd_rn(acc, __dsub_rn(__dmul_rn(S.sigma, xa[p]), c[p]));
-            rhs[p] = v;
-            x0[p] = xa[p];
-            mx = umax64(mx, abs_bits(v));
-        }
-    }
-    double ta, tb;
-    unsigned long long tm;
-    if (!reduce_last<false>(0.0, 0.0, mx, partial, st, &ta, &tb, &tm)) return;
-    const double rmax = __longlong_as_double(static_cast<long long>(tm));
-    st->accuracy = __dmul_rn(iteration_factor, __dadd_rn(1.0, rmax));
-    st->max_inner = S.k.n * 2LL + 20 < 4000 ? S.k.n * 2LL + 20 : 4000;
-    st->stop = 0;  // a breakdown of the previous inner solve does not carry over
-}
-
-// admm_zy_kernel over sliced rows of A
-__global__ void __launch_bounds__(kB, 4) admm_zy_slice_kernel(SliceSys S, const double* next, double* __restrict__ z,
-                                                           double* __restrict__ y, const double* __restrict__ lo,
-                                                           const double* __restrict__ up, AdmmState* st) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) st->inner_sum += st->inner;
-    const int slices = (S.a.n + 31) / 32;
-    for (int s = first_slice(slices); s < slices; s += gridDim.x * (kB / 32)) {
-        const double ax = slice_row_sum<kAhead>(S.a, s, next, [] {});
-        const int i = s * 32 + static_cast<int>(threadIdx.x & 31);
-        if (i >= S.a.n) continue;
-        const double zi = z[i], yi = y[i], ri = S.rho[i];
-        const double relaxed = __dsub_rn(__dmul_rn(1.6, ax), __dmul_rn(.6, zi));
-        const double w = __dadd_rn(relaxed, __ddiv_rn(yi, ri));
-        const double t = w < up[i] ? w : up[i];  // std::max(lo, std::min(up, w))
-        const double nz = lo[i] < t ? t : lo[i];
-        y[i] = __dadd_rn(yi, __dmul_rn(ri, __dsub_rn(relaxed, nz)));
-        z[i] = nz;
-    }
-}
-
-// Row j of H, then row j of A' (its columns moved behind the variables, at t0), as one CSR row
-__global__ void __launch_bounds__(kB) admm_stack_kernel(int n, int t0, const int32_t* __restrict__ hrp,
-                                                        const int32_t* __restrict__ hci, const double* __restrict__ hva,
-                                                        const int32_t* __restrict__ trp, const int32_t* __restrict__ tci,
-                                                        const double* __restrict__ tva, int32_t* __restrict__ rp,
-                                                        int32_t* __restrict__ ci, double* __restrict__ va) {
-    const int lane = threadIdx.x % 8;
-    if (blockIdx.x == 0 && threadIdx.x == 0) rp[n] = hrp[n] + trp[n];
-    for (int j = (blockIdx.x * kB + static_cast<int>(threadIdx.x)) / 8; j < n; j += gridDim.x * kB / 8) {
-        const int h0 = hrp[j], h = hrp[j + 1] - h0, t_at = trp[j], t = trp[j + 1] - t_at, o = h0 + t_at;
-        if (lane == 0) rp[j] = o;
-        for (int k = lane; k < h; k += 8) {
-            ci[o + k] = hci[h0 + k];
-            va[o + k] = hva[h0 + k];
-        }
-        for (int k = lane; k < t; k += 8) {
-            ci[o + h + k] = t0 + tci[t_at + k];
-            va[o + h + k] = tva[t_at + k];
-        }
-    }
 }
 
 // M = diag(H) + sigma + sum_i rho_i a_ij^2, row j of A' in increasing i (the reference's order)
@@ -570,9 +279,9 @@ __global__ void __launch_bounds__(kB) admm_rhs_kernel(Sys s, const double* __res
             mx = umax64(mx, dbits(fabs(v)));
         }
     }
-    double ta, tb;
+    double ta;
     unsigned long long tm;
-    if (!reduce_last<false>(0.0, 0.0, mx, partial, st, &ta, &tb, &tm)) return;
+    if (!reduce_last(0.0, mx, partial, st, &ta, &tm)) return;
     const double rmax = __longlong_as_double(static_cast<long long>(tm));
     st->accuracy = __dmul_rn(iteration_factor, __dadd_rn(1.0, rmax));
     st->max_inner = s.n * 2LL + 20 < 4000 ? s.n * 2LL + 20 : 4000;
@@ -630,13 +339,6 @@ struct bqp_admm {
     double *xa = nullptr, *c = nullptr, *z = nullptr, *y = nullptr, *lo = nullptr, *up = nullptr;
     double sigma = 0;
     bool rho_set = false;
-    // sliced rows (engine.cuh); x, d and v are then stacked vectors (t0 + m entries), rhs, r, pre, kd, xa, c
-    // in the variables' slice order and rho, z, y, lo, up in the rows' of A
-    bool sliced = false;
-    int64_t t0 = 0;
-    uint8_t *k_len = nullptr, *k_row = nullptr, *a_len = nullptr, *a_row = nullptr;
-    int32_t *k_base = nullptr, *a_base = nullptr, *k_col = nullptr, *a_col = nullptr;
-    double *k_val = nullptr, *a_val = nullptr, *stage = nullptr;  // stage: a host vector in its own order
     cudaGraph_t graph = nullptr, apply_graph = nullptr;
     cudaGraphExec_t exec = nullptr, apply_exec = nullptr;
     std::string error;
@@ -653,57 +355,6 @@ struct bqp_admm {
         s.precond = precond;
         s.t = t;
         return s;
-    }
-    SliceSys slices() const {
-        SliceSys s;
-        s.k = SliceRows{static_cast<int>(n), k_len, k_row, k_base, k_col, k_val};
-        s.a = SliceRows{static_cast<int>(m), a_len, a_row, a_base, a_col, a_val};
-        s.t0 = static_cast<int>(t0);
-        s.rho = rho;
-        s.sigma = sigma;
-        s.minv = precond;
-        return s;
-    }
-    // host vectors of the variables (of the rows of A) to the device and back, through the slice order
-    void put(double* dst, const double* src, int64_t count, const uint8_t* row) {
-        if (count <= 0) return;
-        cudaMemcpyAsync(sliced ? stage : dst, src, sizeof(double) * static_cast<size_t>(count), cudaMemcpyHostToDevice, stream);
-        if (sliced) bqp::launch_slice_vector(count, row, stage, dst, stream);
-    }
-    void get(double* dst, const double* src, int64_t count, const uint8_t* row) {
-        if (count <= 0) return;
-        if (sliced) bqp::launch_unslice(count, row, src, stage, stream);
-        cudaMemcpyAsync(dst, sliced ? stage : src, sizeof(double) * static_cast<size_t>(count), cudaMemcpyDeviceToHost, stream);
-    }
-    cudaError_t slice(int64_t hz, int64_t az);
-    // K x (mode as admm_k_kernel), preceded by t = rho .* (A x); dependent: overlapping the launch before
-    void launch_product(double* x_in, double* out, int mode, cudaGraphConditionalHandle h, bool dependent, cudaStream_t s) {
-        const SliceSys S = slices();
-        const bool small = n <= kSmallRows;
-        if (m) launch(small ? admm_a_slice_kernel<kAheadSmall> : admm_a_slice_kernel<kAhead>, slice_grid(m, small), dependent, s, S, x_in);
-        launch(small ? admm_k_slice_kernel<kAheadSmall> : admm_k_slice_kernel<kAhead>, slice_grid(n, small), m != 0 || dependent, s, S, static_cast<const double*>(x_in), out, mode,
-               static_cast<const double*>(rhs), r, pre, d, partial, st, h);
-    }
-    template <class... P, class... A>
-    static void launch(void (*kernel)(P...), int grid, bool dependent, cudaStream_t s, A... args) {
-        cudaLaunchAttribute overlap;
-        overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        overlap.val.programmaticStreamSerializationAllowed = 1;
-        cudaLaunchConfig_t config = {};
-        config.gridDim = dim3(static_cast<unsigned>(grid));
-        config.blockDim = dim3(kB);
-        config.stream = s;
-        config.attrs = &overlap;
-        config.numAttrs = dependent ? 1 : 0;
-        cudaLaunchKernelEx(&config, kernel, static_cast<P>(args)...);
-    }
-    // A slice per warp as far as the resident blocks go (two of the small kernels on an SM), the same number of
-    // blocks on each SM, no more than that takes: 38k rows 2.89 ms per 77 iterations with 608 blocks in
-    // two rounds, 2.32 with 304, 2.05 with 152.
-    static int slice_grid(int64_t rows, bool small = false) {
-        const int64_t slices = (rows + 31) / 32, per_sm = (slices + kSms * (kB / 32) - 1) / (kSms * (kB / 32));
-        const int64_t blocks = kSms * std::min<int64_t>(per_sm, small ? 2 : kSliceBlocks / kSms);
-        return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(slices, blocks)));
     }
     bool ok(cudaError_t e, const char* what) {
         if (e == cudaSuccess) return true;
@@ -729,12 +380,8 @@ struct bqp_admm {
         bool good = ok(cudaStreamBeginCaptureToGraph(cap, graph, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal), "capture");
         cudaGraphNode_t tail = nullptr;
         if (good) {
-            if (sliced) {
-                launch_product(x, kd, 1, h, false, cap);
-            } else {
-                admm_a_kernel<<<gm, kB, 0, cap>>>(s, x, st);
-                admm_k_kernel<<<gn, kB, 0, cap>>>(s, x, kd, 1, rhs, r, pre, d, partial, st, h);
-            }
+            admm_a_kernel<<<gm, kB, 0, cap>>>(s, x, st);
+            admm_k_kernel<<<gn, kB, 0, cap>>>(s, x, kd, 1, rhs, r, pre, d, partial, st, h);
             cudaStreamCaptureStatus cs;
             const cudaGraphNode_t* last = nullptr;
             size_t nlast = 0;
@@ -754,18 +401,10 @@ struct bqp_admm {
                 cudaGraph_t body = p.conditional.phGraph_out[0];
                 good = ok(cudaStreamBeginCaptureToGraph(cap, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal), "capture");
                 if (good) {
-                    if (sliced) {
-                        launch_product(d, kd, 2, h, false, cap);
-                        launch(admm_update_slice_kernel, gv, true, cap, s.n, static_cast<const double*>(precond), x, r, pre,
-                               static_cast<const double*>(d), static_cast<const double*>(kd), partial, st, h);
-                        launch(admm_direction_slice_kernel, gv, true, cap, s.n, d, static_cast<const double*>(pre),
-                               static_cast<const AdmmState*>(st));
-                    } else {
-                        admm_a_kernel<<<gm, kB, 0, cap>>>(s, d, st);
-                        admm_k_kernel<<<gn, kB, 0, cap>>>(s, d, kd, 2, rhs, r, pre, d, partial, st, h);
-                        admm_update_kernel<<<gv, kB, 0, cap>>>(s, x, r, pre, d, kd, partial, st, h);
-                        admm_direction_kernel<<<gv, kB, 0, cap>>>(s.n, d, pre, st);
-                    }
+                    admm_a_kernel<<<gm, kB, 0, cap>>>(s, d, st);
+                    admm_k_kernel<<<gn, kB, 0, cap>>>(s, d, kd, 2, rhs, r, pre, d, partial, st, h);
+                    admm_update_kernel<<<gv, kB, 0, cap>>>(s, x, r, pre, d, kd, partial, st, h);
+                    admm_direction_kernel<<<gv, kB, 0, cap>>>(s.n, d, pre, st);
                     cudaGraph_t out = nullptr;
                     good = ok(cudaStreamEndCapture(cap, &out), "end capture");
                 }
@@ -776,12 +415,8 @@ struct bqp_admm {
         if (good) good = ok(cudaGraphCreate(&apply_graph, 0), "graph");
         if (good) good = ok(cudaStreamBeginCaptureToGraph(cap, apply_graph, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal), "capture");
         if (good) {
-            if (sliced) {
-                launch_product(v, kd, 0, 0, false, cap);
-            } else {
-                admm_a_kernel<<<gm, kB, 0, cap>>>(s, v, st);
-                admm_k_kernel<<<gn, kB, 0, cap>>>(s, v, kd, 0, rhs, r, pre, d, partial, st, 0);
-            }
+            admm_a_kernel<<<gm, kB, 0, cap>>>(s, v, st);
+            admm_k_kernel<<<gn, kB, 0, cap>>>(s, v, kd, 0, rhs, r, pre, d, partial, st, 0);
             cudaGraph_t out = nullptr;
             good = ok(cudaStreamEndCapture(cap, &out), "end capture");
         }
@@ -800,83 +435,12 @@ struct bqp_admm {
                         static_cast<void*>(rhs), static_cast<void*>(x), static_cast<void*>(r), static_cast<void*>(pre),
                         static_cast<void*>(d), static_cast<void*>(kd), static_cast<void*>(v), static_cast<void*>(partial),
                         static_cast<void*>(st), static_cast<void*>(xa), static_cast<void*>(c), static_cast<void*>(z),
-                        static_cast<void*>(y), static_cast<void*>(lo), static_cast<void*>(up), static_cast<void*>(k_len),
-                        static_cast<void*>(k_row), static_cast<void*>(a_len), static_cast<void*>(a_row),
-                        static_cast<void*>(k_base), static_cast<void*>(a_base), static_cast<void*>(k_col),
-                        static_cast<void*>(a_col), static_cast<void*>(k_val), static_cast<void*>(a_val),
-                        static_cast<void*>(stage)})
+                        static_cast<void*>(y), static_cast<void*>(lo), static_cast<void*>(up)})
             if (p) cudaFree(p);
         if (h_st) cudaFreeHost(h_st);
         if (stream) cudaStreamDestroy(stream);
     }
 };
-
-// Brings the uploaded system (H, A, A' in CSR) into slice order and gives the CSR back.  Without memory
-// for the second copy the system stays in CSR.
-cudaError_t bqp_admm::slice(int64_t hz, int64_t az) {
-    const size_t N = static_cast<size_t>(n), M = static_cast<size_t>(std::max<int64_t>(m, 1));
-    t0 = (n + bqp::kSliceWindow - 1) / bqp::kSliceWindow * bqp::kSliceWindow;
-    const size_t stacked = static_cast<size_t>(t0 + m), kz = static_cast<size_t>(hz + az), Z = static_cast<size_t>(az);
-    int32_t *rp = nullptr, *ci = nullptr;  // the stacked rows in CSR
-    double *va = nullptr, *x2 = nullptr, *d2 = nullptr, *v2 = nullptr;
-    uint8_t* position_of = nullptr;
-    struct Want {
-        void** p;
-        size_t bytes;
-    };
-    auto at = [](auto** p) { return reinterpret_cast<void**>(p); };
-    const Want kept[] = {{at(&k_len), N}, {at(&k_row), N}, {at(&k_base), (N + 31) / 32 * 4}, {at(&k_col), kz * 4 + 16},
-                         {at(&k_val), kz * 8 + 16}, {at(&a_len), M}, {at(&a_row), M}, {at(&a_base), (M + 31) / 32 * 4},
-                         {at(&a_col), Z * 4 + 16}, {at(&a_val), Z * 8 + 16}, {at(&stage), std::max(N, M) * 8},
-                         {at(&x2), stacked * 8}, {at(&d2), stacked * 8}, {at(&v2), stacked * 8}};
-    const Want scratch[] = {{at(&rp), (N + 1) * 4}, {at(&ci), kz * 4 + 16}, {at(&va), kz * 8 + 16}, {at(&position_of), stacked}};
-    auto release = [](const Want& w) {
-        cudaFree(*w.p);
-        *w.p = nullptr;
-    };
-    cudaError_t e = cudaSuccess;
-    for (const Want& w : kept) if (!e) e = cudaMalloc(w.p, w.bytes);
-    for (const Want& w : scratch) if (!e) e = cudaMalloc(w.p, w.bytes);
-    if (!e) {
-        admm_stack_kernel<<<kMaxBlocks, kB, 0, stream>>>(static_cast<int>(n), static_cast<int>(t0), hrp, hci, hva, trp, tci, tva,
-                                                        rp, ci, va);
-        bqp::InstDev k{}, a{};
-        k.slice_len = k_len; k.slice_row = k_row; k.slice_base = k_base;
-        a.slice_len = a_len; a.slice_row = a_row; a.slice_base = a_base;
-        bqp::launch_slice_order(k, n, rp, position_of, stream);
-        if (m) bqp::launch_slice_order(a, m, arp, position_of + t0, stream);
-        bqp::launch_slice_columns(hz + az, t0 + m, ci, position_of, stream);
-        bqp::launch_slice_entries(k, n, hz + az, rp, ci, va, k_col, k_val, stream);
-        if (m) {
-            // into a copy: without success the CSR stays in use
-            cudaMemcpyAsync(ci, aci, Z * 4, cudaMemcpyDeviceToDevice, stream);
-            bqp::launch_slice_columns(az, n, ci, position_of, stream);
-            bqp::launch_slice_entries(a, m, az, arp, ci, ava, a_col, a_val, stream);
-        }
-        e = cudaGetLastError();
-        const cudaError_t done = cudaStreamSynchronize(stream);
-        if (!e) e = done;
-    }
-    for (const Want& w : scratch) release(w);
-    if (e) {
-        for (const Want& w : kept) release(w);
-        if (e != cudaErrorMemoryAllocation) return e;
-        cudaGetLastError();  // not sticky
-        return cudaSuccess;
-    }
-    for (void* p : {static_cast<void*>(hrp), static_cast<void*>(hci), static_cast<void*>(hva), static_cast<void*>(trp),
-                    static_cast<void*>(tci), static_cast<void*>(tva), static_cast<void*>(arp), static_cast<void*>(aci),
-                    static_cast<void*>(ava), static_cast<void*>(t), static_cast<void*>(x), static_cast<void*>(d),
-                    static_cast<void*>(v)})
-        cudaFree(p);
-    hrp = hci = trp = tci = arp = aci = nullptr;
-    hva = tva = ava = t = nullptr;
-    x = x2;
-    d = d2;
-    v = v2;
-    sliced = true;
-    return cudaSuccess;
-}
 
 namespace {
 std::string g_admm_error;
@@ -944,7 +508,7 @@ bqp_admm* bqp_admm_create(int device, int64_t n, int64_t m, const int32_t* h_row
         (e = alloc(&s->trp, N + 1)) || (e = alloc(&s->tci, static_cast<size_t>(az))) || (e = alloc(&s->tva, static_cast<size_t>(az))) ||
         (e = alloc(&s->rho, M)) || (e = alloc(&s->t, M)) || (e = alloc(&s->precond, N)) || (e = alloc(&s->rhs, N)) ||
         (e = alloc(&s->x, N)) || (e = alloc(&s->r, N)) || (e = alloc(&s->pre, N)) || (e = alloc(&s->d, N)) ||
-        (e = alloc(&s->kd, N)) || (e = alloc(&s->v, N)) || (e = alloc(&s->partial, 3 * static_cast<size_t>(kMaxBlocks))) ||
+        (e = alloc(&s->kd, N)) || (e = alloc(&s->v, N)) || (e = alloc(&s->partial, 2 * static_cast<size_t>(kMaxBlocks))) ||
         (e = alloc(&s->st, 1)))
         return fail("allocate", e);
     if ((e = cudaMallocHost(reinterpret_cast<void**>(&s->h_st), sizeof(AdmmState)))) return fail("allocate", e);
@@ -960,13 +524,6 @@ bqp_admm* bqp_admm_create(int device, int64_t n, int64_t m, const int32_t* h_row
     if (az) cudaMemcpy(s->tva, tva.data(), sizeof(double) * static_cast<size_t>(az), cudaMemcpyHostToDevice);
     cudaMemset(s->st, 0, sizeof(AdmmState));
     if ((e = cudaDeviceSynchronize())) return fail("upload", e);
-    int64_t longest_k = 0, longest_a = 0;
-    for (int64_t j = 0; j < n; ++j)
-        longest_k = std::max<int64_t>(longest_k, static_cast<int64_t>(h_rowptr[j + 1]) - h_rowptr[j] + trp[j + 1] - trp[j]);
-    for (int64_t i = 0; i < m; ++i) longest_a = std::max<int64_t>(longest_a, static_cast<int64_t>(a_rowptr[i + 1]) - a_rowptr[i]);
-    const bool fits = hz + az <= 2000000000LL && n + m <= 2000000000LL;  // 32-bit entries and stacked columns
-    if (fits && bqp::sliceable(n, hz + az, longest_k) && (m == 0 || bqp::sliceable(m, az, longest_a)))
-        if ((e = s->slice(hz, az))) return fail("slice rows", e);
     if (prev >= 0) cudaSetDevice(prev);
     return s.release();
 }
@@ -978,10 +535,9 @@ int bqp_admm_set_rho(bqp_admm* s, const double* rho, double sigma) {
     int prev = -1;
     cudaGetDevice(&prev);
     cudaSetDevice(s->device);
-    s->put(s->rho, rho, s->m, s->a_row);
+    if (s->m) cudaMemcpyAsync(s->rho, rho, sizeof(double) * static_cast<size_t>(s->m), cudaMemcpyHostToDevice, s->stream);
     s->sigma = sigma;
-    if (s->sliced) admm_precond_slice_kernel<<<bqp_admm::slice_grid(s->n), kB, 0, s->stream>>>(s->slices(), s->precond);
-    else admm_precond_kernel<<<grid_for(static_cast<int>(s->n), kB), kB, 0, s->stream>>>(s->sys(), s->precond);
+    admm_precond_kernel<<<grid_for(static_cast<int>(s->n), kB), kB, 0, s->stream>>>(s->sys(), s->precond);
     bool good = s->ok(cudaStreamSynchronize(s->stream), "preconditioner") && s->build();
     s->rho_set = good;
     if (prev >= 0) cudaSetDevice(prev);
@@ -999,10 +555,10 @@ int bqp_admm_apply(bqp_admm* s, const double* v, double* out) {
     cudaGetDevice(&prev);
     cudaSetDevice(s->device);
     const size_t N = static_cast<size_t>(s->n);
-    s->put(s->v, v, s->n, s->k_row);
+    cudaMemcpyAsync(s->v, v, sizeof(double) * N, cudaMemcpyHostToDevice, s->stream);
     cudaMemsetAsync(s->st, 0, sizeof(AdmmState), s->stream);
     cudaGraphLaunch(s->apply_exec, s->stream);
-    s->get(out, s->kd, s->n, s->k_row);
+    cudaMemcpyAsync(out, s->kd, sizeof(double) * N, cudaMemcpyDeviceToHost, s->stream);
     const bool good = s->ok(cudaStreamSynchronize(s->stream), "apply");
     if (prev >= 0) cudaSetDevice(prev);
     if (!good) {
@@ -1023,11 +579,11 @@ int bqp_admm_solve(bqp_admm* s, const double* rhs, double* x, double accuracy, i
     std::memset(s->h_st, 0, sizeof(AdmmState));
     s->h_st->accuracy = accuracy;
     s->h_st->max_inner = max_inner;
-    s->put(s->rhs, rhs, s->n, s->k_row);
-    s->put(s->x, x, s->n, s->k_row);
+    cudaMemcpyAsync(s->rhs, rhs, sizeof(double) * N, cudaMemcpyHostToDevice, s->stream);
+    cudaMemcpyAsync(s->x, x, sizeof(double) * N, cudaMemcpyHostToDevice, s->stream);
     cudaMemcpyAsync(s->st, s->h_st, sizeof(AdmmState), cudaMemcpyHostToDevice, s->stream);
     cudaGraphLaunch(s->exec, s->stream);
-    s->get(x, s->x, s->n, s->k_row);
+    cudaMemcpyAsync(x, s->x, sizeof(double) * N, cudaMemcpyDeviceToHost, s->stream);
     cudaMemcpyAsync(s->h_st, s->st, sizeof(AdmmState), cudaMemcpyDeviceToHost, s->stream);
     const bool good = s->ok(cudaStreamSynchronize(s->stream), "solve");
     if (prev >= 0) cudaSetDevice(prev);
@@ -1060,12 +616,15 @@ int bqp_admm_iterate(bqp_admm* s, const double* c, const double* lo, const doubl
             return BQP_ERR_NO_MEMORY;
         }
     }
-    s->put(s->xa, x, s->n, s->k_row);
-    s->put(s->c, c, s->n, s->k_row);
-    s->put(s->z, z, s->m, s->a_row);
-    s->put(s->y, y, s->m, s->a_row);
-    s->put(s->lo, lo, s->m, s->a_row);
-    s->put(s->up, up, s->m, s->a_row);
+    const size_t mb = sizeof(double) * static_cast<size_t>(s->m);
+    cudaMemcpyAsync(s->xa, x, sizeof(double) * N, cudaMemcpyHostToDevice, s->stream);
+    cudaMemcpyAsync(s->c, c, sizeof(double) * N, cudaMemcpyHostToDevice, s->stream);
+    if (mb) {
+        cudaMemcpyAsync(s->z, z, mb, cudaMemcpyHostToDevice, s->stream);
+        cudaMemcpyAsync(s->y, y, mb, cudaMemcpyHostToDevice, s->stream);
+        cudaMemcpyAsync(s->lo, lo, mb, cudaMemcpyHostToDevice, s->stream);
+        cudaMemcpyAsync(s->up, up, mb, cudaMemcpyHostToDevice, s->stream);
+    }
     cudaMemsetAsync(s->st, 0, sizeof(AdmmState), s->stream);
     const Sys sy = s->sys();
     const int gn = grid_for(static_cast<int>(s->n), kRows), gm = grid_for(static_cast<int>(s->m), kRows);
@@ -1073,23 +632,16 @@ int bqp_admm_iterate(bqp_admm* s, const double* c, const double* lo, const doubl
     for (int64_t k = 0; k < iterations; ++k) {
         const double it = static_cast<double>(first_iteration + k + 1);
         const double factor = std::min(1e-7, .05 / std::pow(it, 1.6));
-        if (s->sliced) {
-            const SliceSys S = s->slices();
-            const int sn = bqp_admm::slice_grid(s->n), sm = bqp_admm::slice_grid(s->m);
-            if (s->m) admm_yz_kernel<<<gv, kB, 0, s->stream>>>(S.a.n, s->rho, s->z, s->y, s->v + s->t0);
-            admm_rhs_slice_kernel<<<sn, kB, 0, s->stream>>>(S, s->v, s->xa, s->c, s->rhs, s->x, s->partial, s->st, factor);
-            cudaGraphLaunch(s->exec, s->stream);
-            admm_zy_slice_kernel<<<sm, kB, 0, s->stream>>>(S, s->x, s->z, s->y, s->lo, s->up, s->st);
-        } else {
-            admm_rhs_kernel<<<gn, kB, 0, s->stream>>>(sy, s->z, s->y, s->xa, s->c, s->rhs, s->x, s->partial, s->st, factor);
-            cudaGraphLaunch(s->exec, s->stream);
-            admm_zy_kernel<<<gm, kB, 0, s->stream>>>(sy, s->x, s->z, s->y, s->lo, s->up, s->st);
-        }
+        admm_rhs_kernel<<<gn, kB, 0, s->stream>>>(sy, s->z, s->y, s->xa, s->c, s->rhs, s->x, s->partial, s->st, factor);
+        cudaGraphLaunch(s->exec, s->stream);
+        admm_zy_kernel<<<gm, kB, 0, s->stream>>>(sy, s->x, s->z, s->y, s->lo, s->up, s->st);
         admm_x_kernel<<<gv, kB, 0, s->stream>>>(static_cast<int>(s->n), s->x, s->xa);
     }
-    s->get(x, s->xa, s->n, s->k_row);
-    s->get(z, s->z, s->m, s->a_row);
-    s->get(y, s->y, s->m, s->a_row);
+    cudaMemcpyAsync(x, s->xa, sizeof(double) * N, cudaMemcpyDeviceToHost, s->stream);
+    if (mb) {
+        cudaMemcpyAsync(z, s->z, mb, cudaMemcpyDeviceToHost, s->stream);
+        cudaMemcpyAsync(y, s->y, mb, cudaMemcpyDeviceToHost, s->stream);
+    }
     cudaMemcpyAsync(s->h_st, s->st, sizeof(AdmmState), cudaMemcpyDeviceToHost, s->stream);
     const bool good = s->ok(cudaStreamSynchronize(s->stream), "iterate") && s->ok(cudaGetLastError(), "ADMM kernels");
     if (prev >= 0) cudaSetDevice(prev);

@@ -3239,12 +3239,6 @@ __global__ void __launch_bounds__(kSliceWindow) slice_entries_kernel(InstDev I, 
     }
 }
 
-__global__ void __launch_bounds__(kBlock) slice_vector_kernel(int n, const uint8_t* __restrict__ slice_row,
-                                                              const double* __restrict__ x, double* __restrict__ out) {
-    for (int p = blockIdx.x * kBlock + threadIdx.x; p < n; p += gridDim.x * kBlock)
-        out[p] = x[(p & ~(kSliceWindow - 1)) + __ldg(slice_row + p)];
-}
-
 __global__ void __launch_bounds__(kBlock) unslice_kernel(int n, const uint8_t* __restrict__ slice_row,
                                                          const double* __restrict__ x, double* __restrict__ out) {
     for (int p = blockIdx.x * kBlock + threadIdx.x; p < n; p += gridDim.x * kBlock)
@@ -4004,13 +3998,6 @@ void launch_unslice(int64_t n, const uint8_t* slice_row, const double* x, double
     int64_t grid = (n + kBlock - 1) / kBlock;
     if (grid > 152 * 8) grid = 152 * 8;
     unslice_kernel<<<static_cast<int>(grid), kBlock, 0, s>>>(static_cast<int>(n), slice_row, x, out);
-}
-
-void launch_slice_vector(int64_t n, const uint8_t* slice_row, const double* x, double* out, cudaStream_t s) {
-    if (n <= 0) return;
-    int64_t grid = (n + kBlock - 1) / kBlock;
-    if (grid > 152 * 8) grid = 152 * 8;
-    slice_vector_kernel<<<static_cast<int>(grid), kBlock, 0, s>>>(static_cast<int>(n), slice_row, x, out);
 }
 
 void launch_gate(const InstDev& rec, int64_t n, const double* val, bool split, const uint8_t* position_of, cudaStream_t s) {

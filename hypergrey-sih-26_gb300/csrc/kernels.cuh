@@ -68,8 +68,6 @@ void launch_slice_entries(const InstDev& rec, int64_t n, int64_t nnz, const int3
                           const double* val, int32_t* col_out, double* val_out, cudaStream_t s);
 void launch_slice_entries_split(const InstDev& rec, int64_t n, int64_t nnz, const int32_t* rowptr, const int32_t* col,
                                 const double* val, int32_t* col_out, float* hi_out, float* lo_out, cudaStream_t s);
-// A vector brought into slice order: out[position] = x[row].
-void launch_slice_vector(int64_t n, const uint8_t* slice_row, const double* x, double* out, cudaStream_t s);
 // x of a sliced instance in row order: out[row] = x[position].
 void launch_unslice(int64_t n, const uint8_t* slice_row, const double* x, double* out, cudaStream_t s);
 // The same pass on raw device pointers (diag, vhi, vlo may be null: not stored).

@@ -13,8 +13,7 @@ __device__ __forceinline__ void let_next_launch_begin() { asm volatile("griddepc
 
 // Loads of a matrix that a launch reads once: no line of L1 for them, which the gathers of the vector
 // then have to themselves (what bounds a random matrix is the L2's traffic, a 32-byte sector per
-// gathered number beside the stream): FP64 step of the random graph 1M 71.5 -> 70.9 us, ADMM iteration
-// 158 -> 155 us with it.
+// gathered number beside the stream): FP64 step of the random graph 1M 71.5 -> 70.9 us with it.
 __device__ __forceinline__ int load_once(const int32_t* p) {
     int v;
     asm("ld.global.nc.L1::no_allocate.s32 %0, [%1];" : "=r"(v) : "l"(p));

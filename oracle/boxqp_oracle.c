@@ -464,6 +464,145 @@ int orc_solve_box_csr(int64_t n, const int32_t* rowptr, const int32_t* col, cons
     return ORC_OK;
 }
 
+/* ---- the ADMM inner solve in the order of the device's sums (csrc/admm.cu) ------------------------
+   The reference's Jacobi PCG (src/qp_admm.cpp:262-273) on K = H + sigma I + A' diag(rho) A, with the
+   order of additions that the GPU kernels state, so that its results can be compared bit for bit: CG
+   amplifies a rounding, and a tolerance wide enough for that would hide a changed order.
+     row sum      four interleaved fused chains, then (0 + 2) + (1 + 3)
+     dot product  blocks of 256 threads, 608 at most; a thread adds its elements by fused operations in
+                  turns of the grid; a warp's 32 sums by halves (16, 8, 4, 2, 1), a block's eight warps
+                  in order; the blocks' sums the same way, 256 threads strided over them
+   K d: four threads a row, the first of which holds the row (64 rows a block); vectors: one element a thread. */
+enum { ADMM_B = 256, ADMM_LANES = 4, ADMM_ROWS = ADMM_B / ADMM_LANES, ADMM_BLOCKS = 608 };
+
+typedef struct {
+    int64_t n, m;
+    const int32_t *hrp, *hci, *arp, *aci, *trp, *tci;
+    const double *hva, *ava, *tva, *rho;
+    double sigma;
+    double* t;
+} admm_sys;
+
+static double admm_row(const int32_t* rp, const int32_t* ci, const double* va, const double* v, int64_t r) {
+    double s[ADMM_LANES] = {0, 0, 0, 0};
+    for (int32_t k = rp[r]; k < rp[r + 1]; ++k) {
+        double* lane = &s[(k - rp[r]) % ADMM_LANES];
+        *lane = fma(va[k], v[ci[k]], *lane);
+    }
+    return (s[0] + s[2]) + (s[1] + s[3]);
+}
+
+static void admm_apply(const admm_sys* s, const double* v, double* out) {
+    for (int64_t i = 0; i < s->m; ++i) s->t[i] = s->rho[i] * admm_row(s->arp, s->aci, s->ava, v, i);
+    for (int64_t j = 0; j < s->n; ++j) {
+        double hv = admm_row(s->hrp, s->hci, s->hva, v, j), at = admm_row(s->trp, s->tci, s->tva, s->t, j);
+        out[j] = hv + (s->sigma * v[j] + at);
+    }
+}
+
+static double admm_block_sum(const double* thread) {
+    double total = 0;
+    for (int w = 0; w < ADMM_B / 32; ++w) {
+        double x[32];
+        memcpy(x, thread + 32 * w, sizeof(x));
+        for (int o = 16; o > 0; o >>= 1)
+            for (int i = 0; i < o; ++i) x[i] = x[i] + x[i + o];
+        total += x[0];
+    }
+    return total;
+}
+
+/* per_block: elements a block takes per turn (ADMM_ROWS or ADMM_B), each held by the first of
+   ADMM_B / per_block threads; acc: ADMM_BLOCKS * ADMM_B doubles */
+static double admm_dot(int64_t n, const double* a, const double* b, int per_block, double* acc) {
+    int64_t grid = (n + per_block - 1) / per_block;
+    int step = ADMM_B / per_block;
+    double sums[ADMM_BLOCKS], thread[ADMM_B] = {0};
+    if (grid > ADMM_BLOCKS) grid = ADMM_BLOCKS;
+    memset(acc, 0, sizeof(double) * (size_t)grid * ADMM_B);
+    for (int64_t j = 0; j < n; ++j) {
+        int64_t block = j / per_block % grid;
+        double* mine = &acc[block * ADMM_B + j % per_block * step];
+        *mine = fma(a[j], b[j], *mine);
+    }
+    for (int64_t g = 0; g < grid; ++g) sums[g] = admm_block_sum(acc + g * ADMM_B);
+    for (int64_t g = 0; g < grid; ++g) thread[g % ADMM_B] += sums[g];
+    return admm_block_sum(thread);
+}
+
+static double admm_top(int64_t n, const double* r) {
+    double top = 0;
+    for (int64_t j = 0; j < n; ++j) top = fabs(r[j]) > top ? fabs(r[j]) : top;
+    return top;
+}
+
+/* x: the start in, the solution out; product (n, or null): K x of the start. */
+int orc_admm_solve(int64_t n, int64_t m, const int32_t* hrp, const int32_t* hci, const double* hva, const int32_t* arp,
+                   const int32_t* aci, const double* ava, const double* rho, double sigma, const double* rhs, double* x,
+                   double accuracy, int64_t max_inner, int64_t* inner_out, double* residual_out, double* product) {
+    const size_t N = (size_t)n, Z = (size_t)arp[m];
+    int32_t* trp = (int32_t*)calloc(N + 1, sizeof(int32_t));
+    int32_t* next = (int32_t*)malloc(sizeof(int32_t) * (N + 1));
+    int32_t* tci = (int32_t*)malloc(sizeof(int32_t) * (Z + 1));
+    double* tva = (double*)malloc(sizeof(double) * (Z + 1));
+    double* buf = (double*)malloc(sizeof(double) * (5 * N + (size_t)m + (size_t)ADMM_BLOCKS * ADMM_B));
+    int rc = ORC_OK;
+    if (!trp || !next || !tci || !tva || !buf) {
+        rc = ORC_NO_MEMORY;
+    } else {
+        double *r = buf, *pre = r + N, *d = pre + N, *kd = d + N, *precond = kd + N, *t = precond + N, *acc = t + m;
+        /* A' by a stable counting sort */
+        for (size_t k = 0; k < Z; ++k) trp[aci[k] + 1]++;
+        for (int64_t j = 0; j < n; ++j) trp[j + 1] += trp[j];
+        memcpy(next, trp, sizeof(int32_t) * (N + 1));
+        for (int64_t i = 0; i < m; ++i)
+            for (int32_t k = arp[i]; k < arp[i + 1]; ++k) {
+                int32_t p = next[aci[k]]++;
+                tci[p] = (int32_t)i;
+                tva[p] = ava[k];
+            }
+        for (int64_t j = 0; j < n; ++j) {
+            double p = 0;
+            for (int32_t k = hrp[j]; k < hrp[j + 1]; ++k)
+                if (hci[k] == j) p = hva[k];
+            p += sigma;
+            for (int32_t k = trp[j]; k < trp[j + 1]; ++k) p += rho[tci[k]] * tva[k] * tva[k];
+            precond[j] = p;
+        }
+        admm_sys s = {n, m, hrp, hci, arp, aci, trp, tci, hva, ava, tva, rho, sigma, t};
+        admm_apply(&s, x, kd);
+        if (product) memcpy(product, kd, sizeof(double) * N);
+        for (int64_t j = 0; j < n; ++j) {
+            r[j] = rhs[j] - kd[j];
+            pre[j] = r[j] / precond[j];
+            d[j] = pre[j];
+        }
+        double rz = admm_dot(n, r, pre, ADMM_ROWS, acc), top = admm_top(n, r);
+        int64_t inner = 0;
+        while (inner < max_inner && top > accuracy) {
+            admm_apply(&s, d, kd);
+            double den = admm_dot(n, d, kd, ADMM_ROWS, acc);
+            if (!(den > 0) || !isfinite(den)) break;
+            double alpha = rz / den;
+            for (int64_t j = 0; j < n; ++j) {
+                x[j] = x[j] + alpha * d[j];
+                r[j] = r[j] - alpha * kd[j];
+                pre[j] = r[j] / precond[j];
+            }
+            double old = rz;
+            rz = admm_dot(n, r, pre, ADMM_B, acc);
+            top = admm_top(n, r);
+            double beta = rz / old;
+            ++inner;
+            for (int64_t j = 0; j < n; ++j) d[j] = pre[j] + beta * d[j];
+        }
+        *inner_out = inner;
+        *residual_out = top;
+    }
+    free(trp); free(next); free(tci); free(tva); free(buf);
+    return rc;
+}
+
 int orc_max_threads(void) {
 #ifdef _OPENMP
     return omp_get_max_threads();

@@ -199,6 +199,9 @@ def orc():
         L.orc_max_abs_row_sum.restype = c_double
         L.orc_max_abs_row_sum.argtypes = [c_int64, _I32P, _F64P]
         L.orc_max_threads.restype = c_int
+        L.orc_admm_solve.restype = c_int
+        L.orc_admm_solve.argtypes = [c_int64, c_int64, _I32P, _I32P, _F64P, _I32P, _I32P, _F64P, _F64P, c_double,
+                                     _F64P, _F64P, c_double, c_int64, _I64P, _F64P, _F64P]
         L.bqp_planted_preset.restype = c_int
         L.bqp_planted_preset.argtypes = [c_int32, c_uint64, c_int64, c_int64, POINTER(PlantedSpec)]
         L.bqp_planted_create.restype = c_void_p
@@ -412,6 +415,23 @@ def max_abs_row_sum(rowptr, val):
     rowptr = np.ascontiguousarray(rowptr, np.int32)
     val = np.ascontiguousarray(val, np.float64)
     return orc().orc_max_abs_row_sum(rowptr.shape[0] - 1, _p(rowptr, c_int32), _p(val, c_double))
+
+
+def admm_solve(h, a, n, rho, sigma, rhs, x0, accuracy, max_inner):
+    """(x, inner iterations, final max|r|, K x0) of the ADMM inner solve in the order of the device's
+    sums: the same bits as bqp_admm_solve and bqp_admm_apply."""
+    h = [np.ascontiguousarray(v, t) for v, t in zip(h[:3], (np.int32, np.int32, np.float64))]
+    a = [np.ascontiguousarray(v, t) for v, t in zip(a[:3], (np.int32, np.int32, np.float64))]
+    rho, rhs = np.ascontiguousarray(rho, np.float64), np.ascontiguousarray(rhs, np.float64)
+    x, product = np.array(x0, np.float64, copy=True), np.empty(n)
+    inner, resid = c_int64(0), c_double(0)
+    rc = orc().orc_admm_solve(n, len(a[0]) - 1, _p(h[0], c_int32), _p(h[1], c_int32), _p(h[2], c_double),
+                              _p(a[0], c_int32), _p(a[1], c_int32), _p(a[2], c_double), _p(rho, c_double), float(sigma),
+                              _p(rhs, c_double), _p(x, c_double), float(accuracy), int(max_inner), ctypes.byref(inner),
+                              ctypes.byref(resid), _p(product, c_double))
+    if rc:
+        raise MemoryError('orc_admm_solve')
+    return x, inner.value, resid.value, product
 
 
 def max_threads():
