@@ -184,6 +184,9 @@ def cuda_device_name(device=0):
 # ------------------------------------------------------------------------------------------
 # engine context
 # ------------------------------------------------------------------------------------------
+FAULT_PLACES = ('admission', 'launch')  # BQP_FAULT_* of boxqp.h, in their order
+
+
 class Engine:
     """One engine context on one GPU: resident solves, continuous batching, admission cap."""
 
@@ -280,6 +283,10 @@ class Engine:
     def inject_admission_oom(self, count=1):
         """Host-side fault injection: the next `count` admissions fail as out of memory."""
         self._check(lib().bqp_inject_admission_oom(self._ctx, int(count)))
+
+    def inject_oom(self, place, count=1):
+        """Host-side fault injection: the next `count` allocations at `place` (FAULT_PLACES) fail."""
+        self._check(lib().bqp_inject_oom(self._ctx, FAULT_PLACES.index(place), int(count)))
 
     def load(self):
         q, r, p, b = (N.c_int64(0) for _ in range(4))

@@ -448,7 +448,7 @@ public:
         std::lock_guard<std::mutex> g(mu_);
         latency_ms_ = ms;
     }
-    void inject_admission_oom(int count) { inject_oom_.store(count); }
+    void inject_oom(int place, int count) { inject_oom_[place].store(count); }
     // page-locked slots for the gate results of solves between upload and installation (engine
     // thread); chunks of kGateChunk slots, kept until the engine closes
     GateResult* acquire_gate_slot() {
@@ -526,11 +526,21 @@ private:
     bool run_stream(int cap, std::string& why);
     void update_grid();
     bool select_graph(std::string& why);
-    bool queue_collection(const std::vector<Job*>& jobs, std::string& why);
+    struct LaunchSize {
+        size_t tiles = 0, items = 0, units = 0, passes = 0, spans = 0, primals = 0;  // primals: bytes to page-locked memory
+    };
+    LaunchSize launch_size(const std::vector<Job*>& jobs) const;
+    bool reserve_launch(const std::vector<Job*>& jobs, std::string& why);
+    bool reserve_with_running(const std::vector<Job*>& batch, std::string& why);
+    static bool collected_on_host(const Job& j, size_t primals) {
+        return j.n <= kHostPrimal && primals + sizeof(double) * static_cast<size_t>(j.n) <= kCollectMax;
+    }
+    static const std::vector<Tile>& items_of(const Job& j) { return is_sliced(j.variant) ? j.items : j.tiles; }
+    int prepare_collection(const std::vector<Job*>& jobs);
     void collect(std::unique_lock<std::mutex>& lk);
     void process_frees();
     std::vector<Job*> running_jobs() const;
-    bool upload_tables(const std::vector<Job*>& jobs, std::string& why);
+    void upload_tables(const std::vector<Job*>& jobs);
     // step groups of precision `prec` that a body launches (bits of graph_groups_)
     std::vector<int> body_groups(int prec) const {
         std::vector<int> g;
@@ -718,10 +728,16 @@ private:
     int64_t n_running_ = 0, peak_resident_ = 0;
     size_t resident_bytes_ = 0;
     double latency_ms_ = 0;
-    std::atomic<int> inject_oom_{0};
+    std::atomic<int> inject_oom_[BQP_FAULT_PLACES] = {};  // allocations left to fail per BQP_FAULT_* (host-side fault injection)
+    // takes one injected failure of `place`
+    bool injected(int place) {
+        for (int left = inject_oom_[place].load(); left > 0;)
+            if (inject_oom_[place].compare_exchange_weak(left, left - 1)) return true;
+        return false;
+    }
     static constexpr int kGateChunk = 1024;
     std::vector<GateResult*> gate_chunks_;
-    std::vector<GateResult*> gate_free_;  // admissions left to fail as out of memory (host-side fault injection)
+    std::vector<GateResult*> gate_free_;
     double body_ms_ = 0.5;
     double timer_ms_ = 0;
     int64_t timer_kernels_ = 0, timer_launches_ = 0;
@@ -1460,14 +1476,11 @@ bool Engine::upload_begin(Job& j, std::string& why) {
     const int prec = j.opt.precision;
     j.layout = layout_of(j);
     void* slab = nullptr;
-    // host-side fault injection (bqp_inject_admission_oom): fail as an exhausted pool would,
-    // without any device call
-    for (int left = inject_oom_.load(); left > 0;) {
-        if (inject_oom_.compare_exchange_weak(left, left - 1)) {
-            j.out_of_memory = true;
-            why = "CUDA: allocate solve: out of memory (injected on the host)";
-            return false;
-        }
+    // host-side fault injection: fail as an exhausted pool would, without any device call
+    if (injected(BQP_FAULT_ADMISSION)) {
+        j.out_of_memory = true;
+        why = "CUDA: allocate solve: out of memory (injected on the host)";
+        return false;
     }
     const cudaError_t alloc = cudaMallocFromPoolAsync(&slab, j.layout.total, pool_, ustream_);
     if (alloc == cudaErrorMemoryAllocation) {
@@ -1747,6 +1760,7 @@ bool Engine::install(std::vector<Job*>& jobs, std::string& why) {
         if (j.opt.precision == PREC_MIXED)
             work_units(j.tiles.data(), tiles, cg_slots_, tiles <= kCgSmall ? 1 : kCgUnitMin, j.units);
     }
+    if (!reserve_with_running(jobs, why)) return false;
     if (!cuda_ok(cudaStreamWaitEvent(stream_, uev_, 0), why, "upload order")) return false;
     if (!rearm(jobs, why)) return false;
     return true;
@@ -1914,22 +1928,66 @@ std::vector<Job*> Engine::running_jobs() const {
     return jobs;
 }
 
+// What a launch of `jobs` needs in the tables and in the collection's page-locked buffer.
+Engine::LaunchSize Engine::launch_size(const std::vector<Job*>& jobs) const {
+    LaunchSize z;
+    for (const Job* j : jobs) {
+        z.tiles += j->tiles.size();
+        z.units += j->units.size();
+        z.passes += j->passes.size();
+        if (step_group(j->opt.precision, j->variant) >= 0) z.items += items_of(*j).size();
+        if (collected_on_host(*j, z.primals)) z.primals += sizeof(double) * static_cast<size_t>(j->n);
+        z.spans += static_cast<size_t>((j->n + kCollectRows - 1) / kCollectRows);  // at least as many as are written
+    }
+    return z;
+}
+
+// Everything a launch of `jobs` allocates.  It is called before the solves' records are armed, so that a
+// failure leaves none behind that runs on the device and that no launch finishes.
+bool Engine::reserve_launch(const std::vector<Job*>& jobs, std::string& why) {
+    const LaunchSize z = launch_size(jobs);
+    if (!ensure_tables(0, static_cast<int>(z.tiles), why)) return false;
+    auto grow = [&](unsigned char*& buffer, size_t& have, size_t need, const char* what) {
+        if (need <= have) return true;
+        const size_t cap = std::max(need, 2 * have);
+        if (buffer) cudaFreeHost(buffer);
+        buffer = nullptr;
+        have = 0;
+        if (!cuda_ok(cudaMallocHost(&buffer, cap), why, what)) return false;
+        have = cap;
+        return true;
+    };
+    return grow(h_table_stage_, table_stage_bytes_,
+                sizeof(Tile) * (z.tiles + z.items) + sizeof(int4) * (z.units + z.passes) +
+                    sizeof(int2) * static_cast<size_t>(std::max(n_inst_, 1)), "table staging") &&
+           grow(h_collect_, collect_bytes_,
+                align_up(sizeof(CollectJob) * jobs.size()) + align_up(sizeof(int2) * z.spans) +
+                    align_up(sizeof(InstDev) * jobs.size()) + z.primals, "collection staging");
+}
+
+// The same for the solves that run and those of `batch`, which are about to (their records are unarmed).
+bool Engine::reserve_with_running(const std::vector<Job*>& batch, std::string& why) {
+    std::vector<Job*> jobs;
+    {
+        std::lock_guard<std::mutex> g(mu_);
+        jobs = running_jobs();
+    }
+    jobs.insert(jobs.end(), batch.begin(), batch.end());
+    return reserve_launch(jobs, why);
+}
+
 // Uploads the tables of the solves `jobs` (tiles, step groups: items by (precision, variant), work
 // units, ranges) unless the device already has them.  Each solve keeps its own lists, so this is
-// one copy of each into the page-locked staging buffer.
-bool Engine::upload_tables(const std::vector<Job*>& jobs, std::string& why) {
+// one copy of each into the page-locked staging buffer (reserve_launch).
+void Engine::upload_tables(const std::vector<Job*>& jobs) {
     std::vector<std::pair<int, uint64_t>> ids;
     ids.reserve(jobs.size());
     for (const Job* j : jobs) ids.emplace_back(j->slot, j->id);
-    if (!tables_dirty_ && ids == table_jobs_) return true;
-    size_t tiles = 0, units = 0, passes = 0, items = 0;
+    if (!tables_dirty_ && ids == table_jobs_) return;
+    const LaunchSize z = launch_size(jobs);
     int32_t count[kStepGroups + 1] = {};
     groups_present_ = 0;
-    auto items_of = [](const Job& j) -> const std::vector<Tile>& { return is_sliced(j.variant) ? j.items : j.tiles; };
     for (const Job* j : jobs) {
-        tiles += j->tiles.size();
-        units += j->units.size();
-        passes += j->passes.size();
         const int g = step_group(j->opt.precision, j->variant);
         if (g < 0) {
             groups_present_ |= kExactCsrBit;
@@ -1937,29 +1995,19 @@ bool Engine::upload_tables(const std::vector<Job*>& jobs, std::string& why) {
         }
         groups_present_ |= 1u << g;
         count[g + 1] += static_cast<int32_t>(items_of(*j).size());
-        items += items_of(*j).size();
     }
     for (int g = 0; g < kStepGroups; ++g) count[g + 1] += count[g];
     std::memcpy(group_begin_, count, sizeof(group_begin_));
-    if (!ensure_tables(0, static_cast<int>(tiles), why)) return false;
     tables_dirty_ = true;  // until the copies below are queued
-    const size_t b_tiles = sizeof(Tile) * tiles, b_group = sizeof(Tile) * items, b_units = sizeof(int4) * (units + passes);
+    const size_t b_tiles = sizeof(Tile) * z.tiles, b_group = sizeof(Tile) * z.items, b_units = sizeof(int4) * (z.units + z.passes);
     const size_t b_ranges = sizeof(int2) * static_cast<size_t>(std::max(n_inst_, 1));
-    const size_t need = b_tiles + b_group + b_units + b_ranges;
-    if (need > table_stage_bytes_) {
-        const size_t cap = std::max(need, 2 * table_stage_bytes_);
-        if (h_table_stage_) cudaFreeHost(h_table_stage_);
-        h_table_stage_ = nullptr;
-        table_stage_bytes_ = 0;
-        if (!cuda_ok(cudaMallocHost(&h_table_stage_, cap), why, "table staging")) return false;
-        table_stage_bytes_ = cap;
-    }
     // the staging buffer is rewritten only here, after the engine stream drained
     Tile* t = reinterpret_cast<Tile*>(h_table_stage_);
-    Tile* it = t + tiles;
-    int4* un = reinterpret_cast<int4*>(it + items);
-    int4* pa = un + units;
+    Tile* it = t + z.tiles;
+    int4* un = reinterpret_cast<int4*>(it + z.items);
+    int4* pa = un + z.units;
     n_tiles_ = 0;
+    std::fill(h_ranges_.begin(), h_ranges_.end(), int2{0, 0});  // those of all other solves stay empty (in_launch)
     for (const Job* j : jobs) {
         std::memcpy(t + n_tiles_, j->tiles.data(), sizeof(Tile) * j->tiles.size());
         const int g = step_group(j->opt.precision, j->variant);
@@ -1973,8 +2021,8 @@ bool Engine::upload_tables(const std::vector<Job*>& jobs, std::string& why) {
         h_ranges_[j->slot] = int2{n_tiles_, n_tiles_ + static_cast<int>(j->tiles.size())};
         n_tiles_ += static_cast<int>(j->tiles.size());
     }
-    n_units_ = static_cast<int>(units);
-    n_passes_ = static_cast<int>(passes);
+    n_units_ = static_cast<int>(z.units);
+    n_passes_ = static_cast<int>(z.passes);
     std::memcpy(pa, h_ranges_.data(), b_ranges);
     const unsigned char* at = h_table_stage_;
     auto copy = [&](void* dst, size_t bytes) {
@@ -1987,7 +2035,6 @@ bool Engine::upload_tables(const std::vector<Job*>& jobs, std::string& why) {
     copy(d_ranges_, b_ranges);
     table_jobs_.swap(ids);
     tables_dirty_ = false;
-    return true;
 }
 
 bool Engine::run_once(std::string& why) {
@@ -2000,7 +2047,13 @@ bool Engine::run_once(std::string& why) {
         latency = latency_ms_;
         jobs = running_jobs();
     }
-    if (!upload_tables(jobs, why)) return false;
+    if (injected(BQP_FAULT_LAUNCH)) {
+        why = "CUDA: launch set-up: out of memory (injected on the host)";
+        return false;
+    }
+    if (!reserve_launch(jobs, why)) return false;
+    upload_tables(jobs);
+    const int spans = prepare_collection(jobs);
     const double t_tables = host_profile() ? host_seconds() : 0.0;
     if (!stream_mode_ && !select_graph(why)) return false;
     if (latency > 0) cap = std::max(1, static_cast<int>(latency / std::max(body_ms_, 1e-3)));
@@ -2041,7 +2094,10 @@ bool Engine::run_once(std::string& why) {
                      since(t_gated_), since(t_installed_));
     }
     cudaEventRecord(ev1_, stream_);
-    if (!queue_collection(jobs, why)) return false;
+    launch_collect(view(), reinterpret_cast<const CollectJob*>(h_collect_),
+                   reinterpret_cast<const int2*>(h_collect_ + align_up(sizeof(CollectJob) * jobs.size())), spans, h_status_,
+                   h_ctrl_, stream_);
+    if (!cuda_ok(cudaGetLastError(), why, "collect kernel")) return false;
     // while the device runs the launch, upload the new solves that arrive (they are installed
     // before the next launch)
     launch_done_.store(false);
@@ -2078,54 +2134,39 @@ bool Engine::run_once(std::string& why) {
     return true;
 }
 
-// Queues the collection behind a launch of `jobs`: one kernel writes each finished solve's status,
-// record and primal (in row order) to page-locked memory, so that collect() needs no copies of its
-// own.  A primal of more than kHostPrimal variables stays on the device until bqp_fetch copies it
-// straight to the caller's array, off the engine thread (a sliced one is brought into row order in
-// a buffer that the next run writes before it reads it: the first momentum buffer, or CG's r).
-bool Engine::queue_collection(const std::vector<Job*>& jobs, std::string& why) {
+// Lays out the collection behind a launch of `jobs` in page-locked memory (reserve_launch) and returns its
+// spans: one kernel writes each finished solve's status, record and primal (in row order) there, so
+// that collect() needs no copies of its own.  A primal of more than kHostPrimal variables stays on
+// the device until bqp_fetch copies it straight to the caller's array, off the engine thread (a
+// sliced one is brought into row order in a buffer that the next run writes before it reads it: the
+// first momentum buffer, or CG's r).
+int Engine::prepare_collection(const std::vector<Job*>& jobs) {
     collect_jobs_.clear();
-    size_t spans = 0, primals = 0;
-    for (const Job* j : jobs) {
+    const size_t count = jobs.size();
+    const LaunchSize z = launch_size(jobs);
+    const size_t o_spans = align_up(sizeof(CollectJob) * count), o_records = o_spans + align_up(sizeof(int2) * z.spans);
+    const size_t o_x = o_records + align_up(sizeof(InstDev) * count);
+    int2* const spans = reinterpret_cast<int2*>(h_collect_ + o_spans);
+    int2* sp = spans;
+    size_t primals = 0;
+    for (size_t k = 0; k < count; ++k) {
+        const Job& j = *jobs[k];
         CollectJob c{};
-        c.slot = j->slot;
-        const size_t bytes = sizeof(double) * static_cast<size_t>(j->n);
-        if (j->n <= kHostPrimal && primals + bytes <= kCollectMax) {
-            c.n = static_cast<int32_t>(j->n);
-            primals += bytes;
-        } else if (is_sliced(j->variant)) {
-            c.n = static_cast<int32_t>(j->n);
-            c.x = j->opt.precision == PREC_MIXED ? j->rec.r : j->rec.w64[0];
+        c.slot = j.slot;
+        c.record = reinterpret_cast<InstDev*>(h_collect_ + o_records) + k;
+        if (collected_on_host(j, primals)) {
+            c.n = static_cast<int32_t>(j.n);
+            c.x = reinterpret_cast<double*>(h_collect_ + o_x + primals);
+            primals += sizeof(double) * static_cast<size_t>(j.n);
+        } else if (is_sliced(j.variant)) {
+            c.n = static_cast<int32_t>(j.n);
+            c.x = j.opt.precision == PREC_MIXED ? j.rec.r : j.rec.w64[0];
         }
-        spans += static_cast<size_t>(std::max(1, (c.n + kCollectRows - 1) / kCollectRows));
+        for (int64_t r = 0; r == 0 || r < c.n; r += kCollectRows) *sp++ = int2{static_cast<int>(k), static_cast<int>(r)};
         collect_jobs_.push_back(c);
     }
-    const size_t count = jobs.size();
-    const size_t o_spans = align_up(sizeof(CollectJob) * count), o_records = o_spans + align_up(sizeof(int2) * spans);
-    const size_t o_x = o_records + align_up(sizeof(InstDev) * count), need = o_x + primals;
-    if (need > collect_bytes_) {
-        const size_t cap = std::max(need, 2 * collect_bytes_);
-        if (h_collect_) cudaFreeHost(h_collect_);
-        h_collect_ = nullptr;
-        collect_bytes_ = 0;
-        if (!cuda_ok(cudaMallocHost(&h_collect_, cap), why, "collection staging")) return false;
-        collect_bytes_ = cap;
-    }
-    int2* sp = reinterpret_cast<int2*>(h_collect_ + o_spans);
-    double* x = reinterpret_cast<double*>(h_collect_ + o_x);
-    for (size_t k = 0; k < count; ++k) {
-        CollectJob& c = collect_jobs_[k];
-        c.record = reinterpret_cast<InstDev*>(h_collect_ + o_records) + k;
-        if (c.n > 0 && !c.x) {
-            c.x = x;
-            x += c.n;
-        }
-        for (int r = 0; r == 0 || r < c.n; r += kCollectRows) *sp++ = int2{static_cast<int>(k), r};
-    }
     if (count) std::memcpy(h_collect_, collect_jobs_.data(), sizeof(CollectJob) * count);
-    launch_collect(view(), reinterpret_cast<const CollectJob*>(h_collect_), reinterpret_cast<const int2*>(h_collect_ + o_spans),
-                   static_cast<int>(spans), h_status_, h_ctrl_, stream_);
-    return cuda_ok(cudaGetLastError(), why, "collect kernel");
+    return static_cast<int>(sp - spans);
 }
 
 // Moves finished solves to the done state, their records and primals as the collection wrote them.
@@ -2208,10 +2249,11 @@ int Engine::profile_step(uint64_t id, int launches, double* ms_out, double* byte
     if (j.state != JOB_DONE || !j.resident || n_running_ != 0 || !queue_.empty() || launches < 1) return BQP_ERR_NOT_READY;
     cudaSetDevice(device_);
     std::string why;
-    if (!upload_tables({&j}, why)) {
+    if (!reserve_launch({&j}, why)) {
         set_error(why);
         return BQP_ERR_CUDA;
     }
+    upload_tables({&j});
     update_grid();
     InstDev saved;
     cudaMemcpy(&saved, &d_inst_[j.slot], sizeof(InstDev), cudaMemcpyDeviceToHost);
@@ -2274,10 +2316,11 @@ int Engine::profile_cg(uint64_t id, int iterations, double* ms_matvec, double* m
         return BQP_ERR_NOT_READY;
     cudaSetDevice(device_);
     std::string why;
-    if (!upload_tables({&j}, why)) {
+    if (!reserve_launch({&j}, why)) {
         set_error(why);
         return BQP_ERR_CUDA;
     }
+    upload_tables({&j});
     update_grid();
     InstDev saved;
     cudaMemcpy(&saved, &d_inst_[j.slot], sizeof(InstDev), cudaMemcpyDeviceToHost);
@@ -2367,7 +2410,7 @@ void Engine::loop() {
                 for (Job* b : batch) b->state = JOB_ADMITTING;
                 lk.unlock();
                 std::string why;
-                const bool ok = rearm(batch, why);
+                const bool ok = reserve_with_running(batch, why) && rearm(batch, why);
                 lk.lock();
                 for (Job* b : batch) {
                     if (ok) {
@@ -2457,9 +2500,12 @@ void Engine::loop() {
         lk.unlock();
         std::string why;
         bool ok = run_once(why);
+        // what the failed launch had queued ends first: its buffers are rewritten by the next
+        if (!ok) cudaStreamSynchronize(stream_);
         lk.lock();
         if (!ok) {
-            // A CUDA error on the engine stream: fail every running solve.
+            // A CUDA error on the engine stream: fail every running solve.  Their records may still say
+            // that they run; the next launch leaves them out (in_launch).
             set_error(why);
             for (Job* j : slot_job_) {
                 if (j && j->state == JOB_RUNNING) {
@@ -2902,7 +2948,13 @@ int bqp_set_latency_target(bqp_ctx* ctx, double ms) {
 
 int bqp_inject_admission_oom(bqp_ctx* ctx, int32_t count) {
     if (!ctx || count < 0) return BQP_ERR_INVALID;
-    ctx->engine->inject_admission_oom(count);
+    ctx->engine->inject_oom(BQP_FAULT_ADMISSION, count);
+    return BQP_OK;
+}
+
+int bqp_inject_oom(bqp_ctx* ctx, int32_t place, int32_t count) {
+    if (!ctx || count < 0 || place < 0 || place >= BQP_FAULT_PLACES) return BQP_ERR_INVALID;
+    ctx->engine->inject_oom(place, count);
     return BQP_OK;
 }
 

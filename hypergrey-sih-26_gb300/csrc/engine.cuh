@@ -322,7 +322,8 @@ struct View {
     Partial* partial;
     int32_t* tile_done;    // per-instance count of finished tiles (check / CG reductions)
     Ctrl* ctrl;
-    const int2* ranges;      // per-instance tile range [x, y) in the tile table
+    const int2* ranges;      // per-instance tile range [x, y) in the tile table; empty for an instance that is
+                             // not in this launch, whatever its record says
     const Tile* group_tiles;     // the tiles (sliced instances: pieces of kSlicePiece rows) ordered by step group (Ctrl::group_begin)
     const double2* momentum;     // FISTA: beta_k and t_{k+1} for k < kMomentumTable (they depend on k alone)
     const int4* units;           // work units of the CG product, then those of the sliced checks and the residual

@@ -2667,6 +2667,14 @@ struct Counts {
     int step_due[3];   // per precision: the longest remaining chunk among FISTA instances (capped by steps)
 };
 
+// Whether solve i is one of this launch's: the ranges of the others are empty.  A record can be left
+// running without being (its launch failed on the host before it began): nothing would ever finish
+// it, and a loop that counted it would not end.
+__device__ __forceinline__ bool in_launch(const View& v, int i) {
+    const int2 R = v.ranges[i];
+    return R.x < R.y;
+}
+
 // steps > 0: also the step launches with work per precision (a chunk needs it_next - it_cur more)
 __device__ Counts count_phases(const View& v, int steps = 0) {
     __shared__ int s[11];
@@ -2677,7 +2685,7 @@ __device__ Counts count_phases(const View& v, int steps = 0) {
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         const InstDev& I = v.inst[i];
         const int st = I.status;
-        if (st != ST_RUNNING) continue;
+        if (!in_launch(v, i) || st != ST_RUNNING) continue;
         nr++;
         const int pk = I.precision == PREC_MIXED ? 1 : I.precision == PREC_FP64_EXACT ? 2 : 0;
         if (I.phase == PH_FISTA) {
@@ -2721,7 +2729,7 @@ __device__ void advance_chunks(const View& v, int steps) {
     const int n = v.ctrl->n_inst;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         InstDev& I = v.inst[i];
-        if (I.status != ST_RUNNING || I.phase != PH_FISTA) continue;
+        if (!in_launch(v, i) || I.status != ST_RUNNING || I.phase != PH_FISTA) continue;
         const int64_t to = I.it_cur + steps;
         I.it_cur = to < I.it_next ? to : I.it_next;
         if (I.it_cur == I.it_next && I.precision == PREC_MIXED && I.polish && I.polish_rounds == 0 &&

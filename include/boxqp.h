@@ -186,6 +186,15 @@ int bqp_load(bqp_ctx* ctx, int64_t* queued, int64_t* running, int64_t* peak_resi
  * admission).                                                                                */
 int bqp_inject_admission_oom(bqp_ctx* ctx, int32_t count);
 
+/* The same for the next `count` allocations at `place`:
+ *   BQP_FAULT_ADMISSION      as above;
+ *   BQP_FAULT_LAUNCH         the tables of a launch: the solves that were to run in it end with
+ *                            BQP_ERR_CUDA, the context keeps serving those after them.          */
+#define BQP_FAULT_ADMISSION 0
+#define BQP_FAULT_LAUNCH    1
+#define BQP_FAULT_PLACES    2
+int bqp_inject_oom(bqp_ctx* ctx, int32_t place, int32_t count);
+
 /* ---- measurement -------------------------------------------------------------------------
  * bqp_timer: device time of the engine stream's graph launches and re-arm kernels since the
  * last reset, measured with CUDA events on that stream; `kernels` counts the engine kernels

@@ -1,0 +1,72 @@
+"""Allocations of the engine that fail (on the host, injected: no device call is made for them): what
+the failure ends, and that the engine goes on with the right answers.
+
+Answers are compared bit for bit with those of an engine in which nothing failed."""
+import numpy as np
+import pytest
+
+import boxqp
+
+pytestmark = pytest.mark.gpu
+
+
+def problem(seed, n):
+    p = boxqp.planted('graph10k', seed=seed, n=n)
+    return tuple(p[k] for k in ('rowptr', 'col', 'val', 'c', 'lower', 'upper'))
+
+
+@pytest.fixture()
+def engine():
+    eng = boxqp.Engine(0)
+    yield eng
+    eng.close()
+
+
+@pytest.fixture(scope='module')
+def reference():
+    """x of a solve in an engine of its own, by seed, size and precision."""
+    eng, known = boxqp.Engine(0), {}
+
+    def solve(seed, n, precision):
+        if (seed, n, precision) not in known:
+            known[seed, n, precision] = eng.solve(*problem(seed, n), options(precision))[0]
+        return known[seed, n, precision]
+    yield solve
+    eng.close()
+
+
+def options(precision):
+    return boxqp.options_struct(1e-7, 20.0, 200000, precision)
+
+
+def done(engine, ident, n):
+    assert engine.wait(ident, 60.0)
+    x, st = engine.fetch(ident, n)
+    assert boxqp.STATUS_NAMES[st.status] == 'optimal'
+    return x
+
+
+@pytest.mark.parametrize('precision', ['fp64', 'fp64_exact', 'mixed'])
+def test_a_launch_that_cannot_be_set_up_leaves_nothing_running(engine, reference, precision):
+    """Its solves' records were armed on the device; the next launch, of another solve, must not wait for
+    them, and a re-run of them must still give their answer."""
+    engine.inject_oom('launch')
+    failed = engine.submit(*problem(70, 3000), options(precision))
+    with pytest.raises(boxqp.EngineError, match='injected'):
+        engine.wait(failed, 60.0)
+    other = engine.submit(*problem(71, 5000), options(precision))
+    assert np.array_equal(done(engine, other, 5000), reference(71, 5000, precision))
+    engine.resolve([failed])
+    assert np.array_equal(done(engine, failed, 3000), reference(70, 3000, precision))
+    # a re-run that fails, then the release of the solve whose record it left armed
+    engine.inject_oom('launch')
+    engine.resolve([failed])
+    with pytest.raises(boxqp.EngineError, match='injected'):
+        engine.wait(failed, 60.0)
+    engine.release(failed)
+    engine.resolve([other])
+    assert np.array_equal(done(engine, other, 5000), reference(71, 5000, precision))
+    engine.release(other)
+    # its slot is taken again
+    again = engine.submit(*problem(70, 3000), options(precision))
+    assert np.array_equal(done(engine, again, 3000), reference(70, 3000, precision))
