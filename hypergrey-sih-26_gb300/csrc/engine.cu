@@ -1482,6 +1482,13 @@ bool Engine::upload_begin(Job& j, std::string& why) {
         why = "CUDA: allocate solve: out of memory (injected on the host)";
         return false;
     }
+    // before anything is queued for the solve
+    j.gate_host = injected(BQP_FAULT_GATE_RECORD) ? nullptr : acquire_gate_slot();
+    if (!j.gate_host) {
+        cudaGetLastError();  // not sticky
+        why = "host memory for the convexity gate result";
+        return false;
+    }
     const cudaError_t alloc = cudaMallocFromPoolAsync(&slab, j.layout.total, pool_, ustream_);
     if (alloc == cudaErrorMemoryAllocation) {
         cudaGetLastError();  // not sticky: clear it so later calls do not report it
@@ -1686,11 +1693,6 @@ bool Engine::upload_finish(Job& j, std::string& why) {
         R.col = j.csr_col;
         R.val64 = j.csr_val;
     }
-    j.gate_host = acquire_gate_slot();
-    if (!j.gate_host) {
-        why = "host memory for the convexity gate result";
-        return false;
-    }
     const Layout& L = j.layout;
     const double* uploaded = sliced ? j.csr_val : prec == PREC_MIXED ? static_cast<const double*>(j.tmp) : R.val64;
     const bool placed = slice_early(j);  // the columns are positions already (slice_columns)
@@ -1891,11 +1893,16 @@ void Engine::finish_refused(Job* j) {
 // CUDA error.  Caller holds mu_.
 void Engine::fail_admission(Job* j, size_t reserved, const std::string& why) {
     release_gate_slot(*j);
+    // what the streams still do with the solve's memory comes before its frees (on ustream_, and the slab's
+    // on stream_)
+    if (j->columns_sliced) cudaStreamWaitEvent(ustream_, pev_slice_, 0);
     if (j->tmp) cudaFreeAsync(j->tmp, ustream_);
     if (j->power) cudaFreeAsync(j->power, ustream_);
     j->tmp = j->power = nullptr;
     resident_bytes_ -= reserved;
     if (j->resident) {
+        cudaEventRecord(uev_, ustream_);
+        cudaStreamWaitEvent(stream_, uev_, 0);
         pending_free_.emplace_back(-1, j->slab);
         j->slab = nullptr;
         j->resident = false;

@@ -189,10 +189,12 @@ int bqp_inject_admission_oom(bqp_ctx* ctx, int32_t count);
 /* The same for the next `count` allocations at `place`:
  *   BQP_FAULT_ADMISSION      as above;
  *   BQP_FAULT_LAUNCH         the tables of a launch: the solves that were to run in it end with
- *                            BQP_ERR_CUDA, the context keeps serving those after them.          */
-#define BQP_FAULT_ADMISSION 0
-#define BQP_FAULT_LAUNCH    1
-#define BQP_FAULT_PLACES    2
+ *                            BQP_ERR_CUDA, the context keeps serving those after them;
+ *   BQP_FAULT_GATE_RECORD    the page-locked record of a solve's convexity gate (BQP_ERR_CUDA).  */
+#define BQP_FAULT_ADMISSION   0
+#define BQP_FAULT_LAUNCH      1
+#define BQP_FAULT_GATE_RECORD 2
+#define BQP_FAULT_PLACES      3
 int bqp_inject_oom(bqp_ctx* ctx, int32_t place, int32_t count);
 
 /* ---- measurement -------------------------------------------------------------------------

@@ -70,3 +70,23 @@ def test_a_launch_that_cannot_be_set_up_leaves_nothing_running(engine, reference
     # its slot is taken again
     again = engine.submit(*problem(70, 3000), options(precision))
     assert np.array_equal(done(engine, again, 3000), reference(70, 3000, precision))
+
+
+@pytest.mark.parametrize('precision', ['fp64', 'mixed'])
+@pytest.mark.parametrize('n', [3000, 150000])
+def test_no_record_for_the_gate(engine, reference, n, precision):
+    """The solve ends before any of its memory is in use on a stream; those around it keep their answers
+    (sizes of the staged upload and of the copied one)."""
+    before = engine.submit(*problem(72, n), options(precision))
+    done(engine, before, n)
+    engine.inject_oom('gate_record')
+    failed = engine.submit(*problem(73, n), options(precision))
+    after = engine.submit(*problem(74, n), options(precision))
+    with pytest.raises(boxqp.EngineError, match='convexity gate'):
+        engine.wait(failed, 60.0)
+    assert np.array_equal(done(engine, after, n), reference(74, n, precision))
+    engine.resolve([before])
+    assert np.array_equal(done(engine, before, n), reference(72, n, precision))
+    held = engine.load()['resident_bytes']
+    engine.release(failed)
+    assert engine.load()['resident_bytes'] == held
