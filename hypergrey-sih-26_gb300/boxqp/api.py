@@ -184,7 +184,7 @@ def cuda_device_name(device=0):
 # ------------------------------------------------------------------------------------------
 # engine context
 # ------------------------------------------------------------------------------------------
-FAULT_PLACES = ('admission', 'launch', 'gate_record')  # BQP_FAULT_* of boxqp.h, in their order
+FAULT_PLACES = ('admission', 'launch', 'gate_record', 'upload_buffer')  # BQP_FAULT_* of boxqp.h, in their order
 
 
 class Engine:

@@ -215,6 +215,7 @@ struct Job {
     int diag_gate = 0;  // -1: decided by the admission gate (a diagonal Hessian with a positive diagonal)
     int variant = 0;
     int sum_lanes = 0;        // sliced mixed solves: InstDev::sum_lanes
+    int64_t longest_row = 0;
     std::vector<Tile> tiles;  // local tiles (inst field filled at admission)
     std::vector<Tile> items;  // step work items of a sliced solve: its tiles in pieces of kSlicePiece rows
     std::vector<int4> units;  // CG work units, tiles counted from the solve's first (work_units); none of an FP64 solve
@@ -315,10 +316,10 @@ void set_unsupported(bqp_stats& st) {
 // (slice_sums; not named: the block-staged tile's).  Over the CSR, FP64 rows that the options leave open
 // take the structures that the autotuner's timings (boxqp/tuning.json) rank first or within a few
 // percent of it per class.
-int choose_variant(int64_t n, int64_t nnz, int64_t longest_row, const bqp_options& o, int* sums) {
+int choose_variant(int64_t n, int64_t nnz, int64_t longest_row, bool may_slice, const bqp_options& o, int* sums) {
     const double avg = n > 0 ? static_cast<double>(nnz) / static_cast<double>(n) : 1.0;
     const int sliced = n <= kSliceSmall ? VAR_SLICE_SMALL : VAR_SLICE;
-    const bool rows_fit = sliceable(n, nnz, longest_row) && o.lipschitz != BQP_LIPSCHITZ_POWER;
+    const bool rows_fit = may_slice && sliceable(n, nnz, longest_row) && o.lipschitz != BQP_LIPSCHITZ_POWER;
     if (o.precision == PREC_FP64_EXACT) return rows_fit ? sliced : 1;
     if (o.precision == PREC_FP64) {
         if (o.kernel_variant >= 0) return o.kernel_variant;
@@ -399,6 +400,14 @@ double algorithmic_bytes(int64_t n, int64_t nnz, int precision, int64_t iters, i
     const double b_iter = Z * (sv + 4) + 4 * (N + 1) + 7 * N * sv;
     const double b_check = Z * 12 + 4 * (N + 1) + 32 * N;
     return static_cast<double>(iters) * b_iter + static_cast<double>(checks) * b_check + polish_bytes;
+}
+
+// A sliced solve whose upload buffer cannot be had takes its CSR structure, which needs none (mixed: a
+// smaller one).
+void keep_csr(Job& j) {
+    j.variant = choose_variant(j.n, j.nnz, j.longest_row, false, j.opt, &j.sum_lanes);
+    j.tiles = make_tiles(j.n, j.rowptr, j.variant);
+    j.items.clear();
 }
 
 int status_code(int32_t st) {
@@ -490,13 +499,14 @@ private:
     };
     void loop();
     bool upload(Job& j, std::string& why);
+    bool alloc_slab(Job& j, std::string& why);
     bool alloc_upload(Job& j, size_t bytes, std::string& why);
     static bool slice_early(const Job& j);
     void slice_columns(Job& j);
     bool upload_begin(Job& j, std::string& why);
     bool upload_copy(Job& j, size_t budget);
     bool upload_finish(Job& j, std::string& why);
-    void fail_admission(Job* j, size_t reserved, const std::string& why);  // caller holds mu_
+    void fail_admission(Job* j, const std::string& why);  // caller holds mu_
     void finish_paused_upload(std::unique_lock<std::mutex>& lk);
     // host callback behind a launch that the engine thread no longer polls (kPollSeconds)
     static void CUDART_CB on_launch_done(void* self) {
@@ -851,7 +861,9 @@ void Engine::shutdown() {
         if (ustream_) cudaStreamSynchronize(ustream_);
         if (pstream_) cudaStreamSynchronize(pstream_);
         cudaStreamSynchronize(stream_);
-        for (auto& kv : jobs_) if (kv.second->slab) cudaFreeAsync(kv.second->slab, stream_);
+        for (auto& kv : jobs_)
+            for (void* p : {kv.second->slab, kv.second->tmp, kv.second->power})  // the last two: an upload that was paused
+                if (p) cudaFreeAsync(p, stream_);
         for (auto& pf : pending_free_) if (pf.second) cudaFreeAsync(pf.second, stream_);
         cudaStreamSynchronize(stream_);
     }
@@ -1459,10 +1471,25 @@ bool Engine::upload(Job& j, std::string& why) {
     return upload_finish(j, why);
 }
 
+bool Engine::alloc_slab(Job& j, std::string& why) {
+    const cudaError_t e = cudaMallocFromPoolAsync(&j.slab, j.layout.total, pool_, ustream_);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();  // not sticky: clear it so later calls do not report it
+        j.out_of_memory = true;
+        j.slab = nullptr;
+        why = std::string("CUDA: allocate solve: ") + cudaGetErrorString(e);
+        return false;
+    }
+    if (!cuda_ok(e, why, "allocate solve")) return false;
+    j.resident = true;
+    return true;
+}
+
 // The solve's upload buffer (j.tmp) on ustream_, freed behind the admission kernels; an exhausted
 // pool is reported like one that cannot hold the slab.
 bool Engine::alloc_upload(Job& j, size_t bytes, std::string& why) {
-    const cudaError_t e = cudaMallocFromPoolAsync(&j.tmp, bytes, pool_, ustream_);
+    const cudaError_t e = injected(BQP_FAULT_UPLOAD_BUFFER) ? cudaErrorMemoryAllocation
+                                                            : cudaMallocFromPoolAsync(&j.tmp, bytes, pool_, ustream_);
     if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
         j.out_of_memory = true;
@@ -1475,7 +1502,6 @@ bool Engine::upload_begin(Job& j, std::string& why) {
     j.t_upload = host_seconds();
     const int prec = j.opt.precision;
     j.layout = layout_of(j);
-    void* slab = nullptr;
     // host-side fault injection: fail as an exhausted pool would, without any device call
     if (injected(BQP_FAULT_ADMISSION)) {
         j.out_of_memory = true;
@@ -1489,27 +1515,34 @@ bool Engine::upload_begin(Job& j, std::string& why) {
         why = "host memory for the convexity gate result";
         return false;
     }
-    const cudaError_t alloc = cudaMallocFromPoolAsync(&slab, j.layout.total, pool_, ustream_);
-    if (alloc == cudaErrorMemoryAllocation) {
-        cudaGetLastError();  // not sticky: clear it so later calls do not report it
-        j.out_of_memory = true;
-        why = std::string("CUDA: allocate solve: ") + cudaGetErrorString(alloc);
-        return false;
-    }
-    if (!cuda_ok(alloc, why, "allocate solve")) return false;
-    j.slab = slab;
-    j.resident = true;
-    const Layout& L = j.layout;
     const size_t N = static_cast<size_t>(j.n), Z = static_cast<size_t>(j.nnz);
+    const size_t b_val = align_up(Z * 8 + 64), b_col = align_up(Z * 4 + 64), b_rowptr = align_up((N + 1) * 4);
+    j.tmp = nullptr;
+    if (!alloc_slab(j, why)) return false;
+    if (is_sliced(j.variant) && !alloc_upload(j, b_val + b_col + b_rowptr + N, why)) {
+        if (!j.out_of_memory) return false;
+        j.out_of_memory = false;
+        cudaFreeAsync(j.slab, ustream_);
+        j.slab = nullptr;
+        j.resident = false;
+        cudaStreamSynchronize(ustream_);
+        cudaMemPoolTrimTo(pool_, 0);  // the other slab is of another size
+        keep_csr(j);
+        const size_t was = j.layout.total;
+        j.layout = layout_of(j);
+        {
+            std::lock_guard<std::mutex> g(mu_);
+            resident_bytes_ += j.layout.total - was;
+        }
+        if (!alloc_slab(j, why)) return false;
+    }
+    void* const slab = j.slab;
+    const Layout& L = j.layout;
     j.pieces.clear();
     j.piece = j.piece_off = 0;
     j.columns_sliced = false;
     const bool sliced = is_sliced(j.variant);
-    j.tmp = nullptr;
     if (sliced) {
-        const size_t b_val = align_up(Z * 8 + 64), b_col = align_up(Z * 4 + 64);
-        const size_t b_rowptr = align_up((N + 1) * 4);
-        if (!alloc_upload(j, b_val + b_col + b_rowptr + N, why)) return false;
         j.csr_val = static_cast<double*>(j.tmp);
         j.csr_col = reinterpret_cast<int32_t*>(static_cast<char*>(j.tmp) + b_val);
         j.csr_rowptr = reinterpret_cast<int32_t*>(static_cast<char*>(j.tmp) + b_val + b_col);
@@ -1789,7 +1822,7 @@ void Engine::upload_waiting() {
             const bool ok = upload_begin(*j, why);
             lk.lock();
             if (!ok) {
-                fail_admission(j, need, why);
+                fail_admission(j, why);
                 continue;
             }
             uploading_ = j;
@@ -1803,7 +1836,7 @@ void Engine::upload_waiting() {
         if (copied) {
             uploading_ = nullptr;
             if (ok) uploaded_.push_back(j);
-            else fail_admission(j, j->layout.total, why);
+            else fail_admission(j, why);
         }
     }
 }
@@ -1819,7 +1852,7 @@ void Engine::finish_paused_upload(std::unique_lock<std::mutex>& lk) {
     lk.lock();
     uploading_ = nullptr;
     if (ok) uploaded_.push_back(j);
-    else fail_admission(j, j->layout.total, why);
+    else fail_admission(j, why);
 }
 
 // Decides the convexity gate of solves uploaded since the last installation, once their upload
@@ -1891,7 +1924,7 @@ void Engine::finish_refused(Job* j) {
 
 // A solve whose admission failed: its reserved bytes and any slab go back, it finishes with the
 // CUDA error.  Caller holds mu_.
-void Engine::fail_admission(Job* j, size_t reserved, const std::string& why) {
+void Engine::fail_admission(Job* j, const std::string& why) {
     release_gate_slot(*j);
     // what the streams still do with the solve's memory comes before its frees (on ustream_, and the slab's
     // on stream_)
@@ -1899,7 +1932,7 @@ void Engine::fail_admission(Job* j, size_t reserved, const std::string& why) {
     if (j->tmp) cudaFreeAsync(j->tmp, ustream_);
     if (j->power) cudaFreeAsync(j->power, ustream_);
     j->tmp = j->power = nullptr;
-    resident_bytes_ -= reserved;
+    resident_bytes_ -= j->layout.total;
     if (j->resident) {
         cudaEventRecord(uev_, ustream_);
         cudaStreamWaitEvent(stream_, uev_, 0);
@@ -2464,7 +2497,7 @@ void Engine::loop() {
             const bool ok = upload(*j, why);
             lk.lock();
             if (ok) uploaded_.push_back(j);
-            else fail_admission(j, need, why);
+            else fail_admission(j, why);
         }
         // install what was uploaded here and during the previous launch
         if (!uploaded_.empty()) {
@@ -2777,7 +2810,8 @@ int make_job(int64_t n, int64_t nnz, const int32_t* rowptr, const int32_t* col, 
         *out = j.release();
         return BQP_OK;
     }
-    j->variant = bqp::choose_variant(n, nnz, scan.longest, o, &j->sum_lanes);
+    j->variant = bqp::choose_variant(n, nnz, scan.longest, true, o, &j->sum_lanes);
+    j->longest_row = scan.longest;
     j->tiles = bqp::make_tiles(n, rowptr, j->variant);
     if (bqp::is_sliced(j->variant))
         for (const bqp::Tile& t : j->tiles)

@@ -119,7 +119,9 @@ void bqp_options_default(bqp_options* options);
 
 /* ---- context ----------------------------------------------------------------------------
  * bqp_create: one context on one device.  mem_cap_bytes bounds the device memory of resident
- * solves (0 = 90% of the free memory at creation).  Returns NULL on failure; the reason is
+ * solves (0 = 90% of the free memory at creation); while a solve is admitted its inputs take up to 12
+ * bytes an entry and 5 a row beside that (8 an entry in the mixed precision's CSR structures, nothing
+ * in the FP64 ones, which it is admitted over where there is no memory for more).  Returns NULL on failure; the reason is
  * then available from bqp_last_error(NULL).                                                  */
 bqp_ctx*    bqp_create(int device, size_t mem_cap_bytes);
 void        bqp_destroy(bqp_ctx* ctx);
@@ -190,11 +192,15 @@ int bqp_inject_admission_oom(bqp_ctx* ctx, int32_t count);
  *   BQP_FAULT_ADMISSION      as above;
  *   BQP_FAULT_LAUNCH         the tables of a launch: the solves that were to run in it end with
  *                            BQP_ERR_CUDA, the context keeps serving those after them;
- *   BQP_FAULT_GATE_RECORD    the page-locked record of a solve's convexity gate (BQP_ERR_CUDA).  */
+ *   BQP_FAULT_GATE_RECORD    the page-locked record of a solve's convexity gate (BQP_ERR_CUDA);
+ *   BQP_FAULT_UPLOAD_BUFFER  the device buffer of a solve's inputs during admission (bqp_create): a
+ *                            solve on sliced rows is admitted over its CSR instead, a mixed one
+ *                            over the CSR ends with BQP_ERR_NO_MEMORY.                            */
 #define BQP_FAULT_ADMISSION   0
 #define BQP_FAULT_LAUNCH      1
 #define BQP_FAULT_GATE_RECORD 2
-#define BQP_FAULT_PLACES      3
+#define BQP_FAULT_UPLOAD_BUFFER 3
+#define BQP_FAULT_PLACES      4
 int bqp_inject_oom(bqp_ctx* ctx, int32_t place, int32_t count);
 
 /* ---- measurement -------------------------------------------------------------------------

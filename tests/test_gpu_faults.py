@@ -90,3 +90,36 @@ def test_no_record_for_the_gate(engine, reference, n, precision):
     held = engine.load()['resident_bytes']
     engine.release(failed)
     assert engine.load()['resident_bytes'] == held
+
+
+def test_no_buffer_for_the_upload(engine, reference):
+    """A solve of sliced rows goes on over its CSR: the exact engine with the same bits, the FP64 engine
+    with those of the CSR structure it names (two lanes a row), the mixed one verified.  A solve that
+    runs over its CSR anyway and needs the buffer ends out of memory, as it always did."""
+    n = 30000
+    assert engine.load()['resident_bytes'] == 0
+    for precision in ('fp64_exact', 'fp64', 'mixed'):
+        engine.inject_oom('upload_buffer')
+        ident = engine.submit(*problem(75, n), options(precision))
+        x = done(engine, ident, n)
+        ref = reference(75, n, precision)
+        if precision == 'fp64_exact':
+            assert np.array_equal(x, ref)
+        elif precision == 'fp64':
+            named = boxqp.options_struct(1e-7, 20.0, 200000, precision, kernel_variant=2)
+            assert np.array_equal(x, engine.solve(*problem(75, n), named)[0])
+        else:
+            st = engine.fetch(ident, n)[1]
+            fstar = boxqp.planted('graph10k', seed=75, n=n)['fstar']
+            assert st.verified and abs(st.objective - fstar) <= 1e-7 * (1 + abs(fstar))
+        engine.resolve([ident])
+        assert np.array_equal(done(engine, ident, n), x)
+        engine.release(ident)
+    csr = boxqp.options_struct(1e-7, 20.0, 200000, 'mixed', kernel_variant=8)
+    engine.inject_oom('upload_buffer')
+    ident = engine.submit(*problem(75, n), csr)
+    with pytest.raises(boxqp.EngineError, match='upload buffer'):
+        engine.wait(ident, 60.0)
+    engine.release(ident)
+    assert np.array_equal(engine.solve(*problem(75, n), options('mixed'))[0], reference(75, n, 'mixed'))
+    assert engine.load()['resident_bytes'] == 0
