@@ -308,14 +308,29 @@ void set_unsupported(bqp_stats& st) {
     st.dual_bound = -HUGE_VAL;
 }
 
+// FP64 rows over the CSR.  Without a long row (the power estimate): one lane a row below nine entries, two
+// from there, warp-staged rows on small instances of 6 to 13 (boxqp/tuning.json's timings: within 2 % of
+// the best).  A long row is one lane's serial chain, or a few lanes': 50 iterations with a row of 500 on
+// 16k rows of 3 entries take 4.7 ms with one lane, 1.9 with two, 1.6 with four and 1.5 block-staged; that
+// stays ahead up to about 2,000 entries (2,000 on 131k rows of 11: 5.5 ms, 6.5 with two, 3.9 with four;
+// 4,100 on 16k rows: 24, 14 and 7.5), unless the other rows weigh more than the long one, where two lanes
+// do less per entry (500 on 1M rows of 11: 8.1 ms block-staged, 6.6 with two lanes; on 131k rows 2.33
+// and 2.30; 800 there 2.95 and 3.14).
+int csr_variant_fp64(int64_t n, int64_t nnz, int64_t longest_row) {
+    const double avg = n > 0 ? static_cast<double>(nnz) / static_cast<double>(n) : 1.0;
+    if (avg >= 48) return 32;
+    if (longest_row <= kSliceMaxRow) return avg < 6 ? 1 : n < 30000 && avg < 13 ? VAR_WARP : avg < 9 ? 1 : 2;
+    if (longest_row > kTileNnz / 2) return 4;
+    return avg >= 4 && nnz >= 5000 * longest_row ? 2 : VAR_TILE;
+}
+
 // Structure of a solve's kernels.  Sliced rows unless a row is too long for a lane (kSliceMaxRow), the rows
 // are long on average, where several lanes per row give a small instance more loads in flight
 // (kSliceMaxAverage; the mixed engine's FP32 rows gain from it only below kSliceMaxAverageMixed), or the
 // power estimate wants the CSR.  For the FP64 engine a structure that the options name is taken as named;
 // for the mixed engine it names the order of a row's FP32 sum, which the sliced step keeps
-// (slice_sums; not named: the block-staged tile's).  Over the CSR, FP64 rows that the options leave open
-// take the structures that the autotuner's timings (boxqp/tuning.json) rank first or within a few
-// percent of it per class.
+// (slice_sums; not named: the block-staged tile's).  FP64 rows that the options leave open take
+// csr_variant_fp64 over the CSR.
 int choose_variant(int64_t n, int64_t nnz, int64_t longest_row, bool may_slice, const bqp_options& o, int* sums) {
     const double avg = n > 0 ? static_cast<double>(nnz) / static_cast<double>(n) : 1.0;
     const int sliced = n <= kSliceSmall ? VAR_SLICE_SMALL : VAR_SLICE;
@@ -323,7 +338,7 @@ int choose_variant(int64_t n, int64_t nnz, int64_t longest_row, bool may_slice, 
     if (o.precision == PREC_FP64_EXACT) return rows_fit ? sliced : 1;
     if (o.precision == PREC_FP64) {
         if (o.kernel_variant >= 0) return o.kernel_variant;
-        return rows_fit ? sliced : avg >= 48 ? 32 : avg < 9 ? 1 : 2;
+        return rows_fit ? sliced : csr_variant_fp64(n, nnz, longest_row);
     }
     const int named = o.kernel_variant >= 0 ? o.kernel_variant : avg >= 48 ? 32 : VAR_TILE;
     *sums = slice_sums(named);
