@@ -75,8 +75,8 @@ struct Layout {
     size_t total = 0;
 };
 
-// Sliced FP64 solves hold their rows' order in place of the row pointers, which they need (with the
-// CSR as uploaded) only during admission, in a buffer of its own.
+// Sliced solves hold their rows' order in place of the row pointers, which they need (with the CSR as
+// uploaded) only during admission, in a buffer of its own.
 Layout make_layout(int64_t n, int64_t nnz, int64_t tiles, int precision, bool sliced) {
     Layout L;
     size_t o = 0;
@@ -516,7 +516,6 @@ private:
     bool upload(Job& j, std::string& why);
     bool alloc_slab(Job& j, std::string& why);
     bool alloc_upload(Job& j, size_t bytes, std::string& why);
-    static bool slice_early(const Job& j);
     void slice_columns(Job& j);
     bool upload_begin(Job& j, std::string& why);
     bool upload_copy(Job& j, size_t budget);
@@ -1674,10 +1673,6 @@ bool Engine::upload_begin(Job& j, std::string& why) {
     return true;
 }
 
-// Whether a solve's columns become positions before its gate runs (the power estimate multiplies by the
-// CSR as uploaded, after the gate).
-bool Engine::slice_early(const Job& j) { return is_sliced(j.variant) && j.rec.lip_device == 0; }
-
 // The row order and the columns as positions, on a stream of their own behind what ustream_ has copied so
 // far: row pointers, vectors and columns; the values are still on their way.
 void Engine::slice_columns(Job& j) {
@@ -1726,7 +1721,7 @@ bool Engine::upload_copy(Job& j, size_t budget) {
         if (j.piece_off == p.bytes) {
             ++j.piece;
             j.piece_off = 0;
-            if (j.piece + 1 == j.pieces.size() && slice_early(j)) slice_columns(j);  // all but the values
+            if (j.piece + 1 == j.pieces.size() && is_sliced(j.variant)) slice_columns(j);  // all but the values
         }
     }
     return j.piece == j.pieces.size();
@@ -1743,20 +1738,17 @@ bool Engine::upload_finish(Job& j, std::string& why) {
     }
     const Layout& L = j.layout;
     const double* uploaded = sliced ? j.csr_val : prec == PREC_MIXED ? static_cast<const double*>(j.tmp) : R.val64;
-    const bool placed = slice_early(j);  // the columns are positions already (slice_columns)
-    if (placed && !j.columns_sliced) slice_columns(j);
-    if (placed) cudaStreamWaitEvent(ustream_, pev_slice_, 0);
+    if (sliced) {
+        if (!j.columns_sliced) slice_columns(j);
+        cudaStreamWaitEvent(ustream_, pev_slice_, 0);
+    }
     // the convexity gate and the Gershgorin bound: the other admission kernels read L from
     // its result, and the engine thread reads the result back before it installs the solve
-    launch_gate(R, j.n, uploaded, prec == PREC_MIXED && !sliced, placed ? j.position_of : nullptr, ustream_);
+    launch_gate(R, j.n, uploaded, prec == PREC_MIXED && !sliced, sliced ? j.position_of : nullptr, ustream_);
     cudaMemcpyAsync(j.gate_host, R.gate, sizeof(GateResult), cudaMemcpyDeviceToHost, ustream_);
     if (R.lip_device && prec != PREC_MIXED) {
         cudaMemcpyAsync(R.lprec, &R.gate->lip_bits, sizeof(double), cudaMemcpyDeviceToDevice, ustream_);
         launch_power_lipschitz(R, j.n, uploaded, false, j.power, ustream_);
-    }
-    if (sliced && !placed) {
-        launch_slice_order(R, j.n, R.rowptr, j.position_of, ustream_);
-        launch_slice_columns(j.nnz, j.n, j.csr_col, j.position_of, ustream_);
     }
     if (sliced && prec == PREC_MIXED)
         launch_slice_entries_split(R, j.n, j.nnz, R.rowptr, R.col, uploaded, at<int32_t>(j.slab, L.col), const_cast<float*>(R.vhi),

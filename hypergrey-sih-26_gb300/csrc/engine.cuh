@@ -82,8 +82,9 @@ __host__ __device__ constexpr int step_group(int precision, int variant) {
 constexpr int kSliceWindow = 256;
 constexpr int kSlicePiece = 128;     // rows of a step work item (a block's four warps take a slice each)
 constexpr int64_t kSliceSmall = 65536;  // rows up to which an instance is VAR_SLICE_SMALL
-constexpr int kSliceMaxRow = 127;    // longest row of a sliced instance (a tile holds 32 such rows, so tiles begin on slices)
-constexpr int kSliceMaxAverage = 48; // longer average rows keep the sub-warp structures (default_variant)
+constexpr int kSliceMaxRow = 127;    // longest row of a sliced instance (a window's entries stay within 16-bit offsets; its tiles
+                                     // are whole windows, one at least, whatever they hold)
+constexpr int kSliceMaxAverage = 48; // longer average rows keep the sub-warp structures (choose_variant)
 
 // Mixed instances longer than this on average keep the sub-warp structures: their FP32 steps are bound by the
 // gathers on either layout, while admission and the residual pass cost more on slices.
@@ -223,7 +224,7 @@ struct __align__(16) InstDev {
     int64_t end_ns;
     double L;
     double invL;
-    double invL_lo;        // exact engine: 1/L - invL, and the dividends' exponent range (KnownDivisor)
+    double invL_lo;        // exact engine, sliced: 1/L - invL, and the dividends' exponent range (KnownDivisor)
     float invLf;
     int32_t div_span;
     int32_t result_src;    // where the answer lives: 0 x64, 1 x32, 2 xp

@@ -2858,8 +2858,6 @@ __global__ void __launch_bounds__(kBlock) rearm_kernel(View v, const InstDev* __
             if (I.lip_device) {
                 I.L = *I.lprec;
                 I.invL = 1.0 / I.L;
-                I.invL_lo = __ddiv_rn(__fma_rn(-I.invL, I.L, 1.0), I.L);
-                I.div_span = I.L >= 0x1p-100 && I.L <= 0x1p100 ? kDivSpan : 0;
                 I.invLf = static_cast<float>(I.invL);
             }
             armed = start_instance(I);
