@@ -163,6 +163,13 @@ def cpu_reference_solve(inst, tol, time_limit=600.0, prefer_reference=True, thre
                 'engine': 'the CPU oracle port of src/accelerated_qp.cpp (oracle/boxqp_oracle.c, OpenMP)'}
 
 
+def on_slices(inst, precision):
+    """Whether the engine runs the instance on sliced rows (csrc/engine.cu, choose_variant)."""
+    import numpy as np
+    lengths = np.diff(inst['rowptr'])
+    return bool(lengths.max() <= 127 and lengths.mean() < (20 if precision == 'mixed' else 48))
+
+
 def oracle_check(inst, x, tol):
     """The oracle's check_qp_solution (restated, pinned to the reference) of a primal on the host,
     plus the active-set comparison with the planted optimum."""
@@ -317,8 +324,11 @@ def run_ours(args, world, rank, local, pg):
     tp = ROOT / 'profiles' / 'roofline_traffic.json'
     if tp.exists():
         traffic = json.loads(tp.read_text()).get(f'{args.workload}_{args.precision}')
+    sliced = on_slices(inst, args.precision)
+    step_kernel = ('step_slice_f32_kernel' if args.precision == 'mixed' else 'step_slice_kernel') if sliced else \
+        f'step_kernel<{args.precision}>'
     roofline = {'bound': 'hbm', 'achieved': achieved, 'peak': peak, 'unit': 'GB/s', 'frac': achieved / peak,
-                'traffic': traffic, 'peak_kind': peak_kind, 'kernel': f'step_kernel<{args.precision}>',
+                'traffic': traffic if sliced else None, 'peak_kind': peak_kind, 'kernel': step_kernel,
                 'ms_per_launch': step_ms, 'algorithmic_bytes_per_launch': step_bytes}
     # second roofline entry: the polish CG of this solve (mixed precision), its product kernel
     # (the one that dominates the polish) and its vector kernel, on the packed Q_FF
@@ -328,7 +338,7 @@ def run_ours(args, world, rank, local, pg):
         eng.wait(ident)
         try:
             ms_mv, ms_vec, b_mv, b_vec = eng.profile_cg(ident, 10)
-            roofline_cg = {'bound': 'hbm', 'kernel': 'cg_matvec_kernel', 'achieved': b_mv / (ms_mv * 1e-3) / 1e9,
+            roofline_cg = {'bound': 'hbm', 'kernel': 'cg_matvec_slice_kernel' if sliced else 'cg_matvec_kernel', 'achieved': b_mv / (ms_mv * 1e-3) / 1e9,
                            'peak': peak, 'unit': 'GB/s', 'frac': b_mv / (ms_mv * 1e-3) / 1e9 / peak,
                            'peak_kind': peak_kind, 'ms_per_launch': ms_mv, 'algorithmic_bytes_per_launch': b_mv,
                            'vector_kernel': {'kernel': 'cg_vector_kernel', 'ms_per_launch': ms_vec,
