@@ -556,17 +556,17 @@ private:
         size_t tiles = 0, items = 0, units = 0, passes = 0, spans = 0, primals = 0;  // primals: bytes to page-locked memory
     };
     LaunchSize launch_size(const std::vector<Job*>& jobs) const;
-    bool reserve_launch(const std::vector<Job*>& jobs, std::string& why);
+    bool reserve_launch(const LaunchSize& z, size_t jobs, std::string& why);
     bool reserve_with_running(const std::vector<Job*>& batch, std::string& why);
     static bool collected_on_host(const Job& j, size_t primals) {
         return j.n <= kHostPrimal && primals + sizeof(double) * static_cast<size_t>(j.n) <= kCollectMax;
     }
     static const std::vector<Tile>& items_of(const Job& j) { return is_sliced(j.variant) ? j.items : j.tiles; }
-    int prepare_collection(const std::vector<Job*>& jobs);
+    int prepare_collection(const std::vector<Job*>& jobs, const LaunchSize& z);
     void collect(std::unique_lock<std::mutex>& lk);
     void process_frees();
     std::vector<Job*> running_jobs() const;
-    void upload_tables(const std::vector<Job*>& jobs);
+    void upload_tables(const std::vector<Job*>& jobs, const LaunchSize& z);
     // step groups of precision `prec` that a body launches (bits of graph_groups_)
     std::vector<int> body_groups(int prec) const {
         std::vector<int> g;
@@ -1994,10 +1994,9 @@ Engine::LaunchSize Engine::launch_size(const std::vector<Job*>& jobs) const {
     return z;
 }
 
-// Everything a launch of `jobs` allocates.  It is called before the solves' records are armed, so that a
+// Everything a launch of `jobs` solves of the size `z` allocates.  It is called before the solves' records are armed, so that a
 // failure leaves none behind that runs on the device and that no launch finishes.
-bool Engine::reserve_launch(const std::vector<Job*>& jobs, std::string& why) {
-    const LaunchSize z = launch_size(jobs);
+bool Engine::reserve_launch(const LaunchSize& z, size_t jobs, std::string& why) {
     if (!ensure_tables(0, static_cast<int>(z.tiles), why)) return false;
     auto grow = [&](unsigned char*& buffer, size_t& have, size_t need, const char* what) {
         if (need <= have) return true;
@@ -2013,8 +2012,7 @@ bool Engine::reserve_launch(const std::vector<Job*>& jobs, std::string& why) {
                 sizeof(Tile) * (z.tiles + z.items) + sizeof(int4) * (z.units + z.passes) +
                     sizeof(int2) * static_cast<size_t>(std::max(n_inst_, 1)), "table staging") &&
            grow(h_collect_, collect_bytes_,
-                align_up(sizeof(CollectJob) * jobs.size()) + align_up(sizeof(int2) * z.spans) +
-                    align_up(sizeof(InstDev) * jobs.size()) + z.primals, "collection staging");
+                align_up(sizeof(CollectJob) * jobs) + align_up(sizeof(int2) * z.spans) + align_up(sizeof(InstDev) * jobs) + z.primals, "collection staging");
 }
 
 // The same for the solves that run and those of `batch`, which are about to (their records are unarmed).
@@ -2025,18 +2023,17 @@ bool Engine::reserve_with_running(const std::vector<Job*>& batch, std::string& w
         jobs = running_jobs();
     }
     jobs.insert(jobs.end(), batch.begin(), batch.end());
-    return reserve_launch(jobs, why);
+    return reserve_launch(launch_size(jobs), jobs.size(), why);
 }
 
 // Uploads the tables of the solves `jobs` (tiles, step groups: items by (precision, variant), work
 // units, ranges) unless the device already has them.  Each solve keeps its own lists, so this is
 // one copy of each into the page-locked staging buffer (reserve_launch).
-void Engine::upload_tables(const std::vector<Job*>& jobs) {
+void Engine::upload_tables(const std::vector<Job*>& jobs, const LaunchSize& z) {
     std::vector<std::pair<int, uint64_t>> ids;
     ids.reserve(jobs.size());
     for (const Job* j : jobs) ids.emplace_back(j->slot, j->id);
     if (!tables_dirty_ && ids == table_jobs_) return;
-    const LaunchSize z = launch_size(jobs);
     int32_t count[kStepGroups + 1] = {};
     groups_present_ = 0;
     for (const Job* j : jobs) {
@@ -2103,9 +2100,10 @@ bool Engine::run_once(std::string& why) {
         why = "CUDA: launch set-up: out of memory (injected on the host)";
         return false;
     }
-    if (!reserve_launch(jobs, why)) return false;
-    upload_tables(jobs);
-    const int spans = prepare_collection(jobs);
+    const LaunchSize z = launch_size(jobs);
+    if (!reserve_launch(z, jobs.size(), why)) return false;
+    upload_tables(jobs, z);
+    const int spans = prepare_collection(jobs, z);
     const double t_tables = host_profile() ? host_seconds() : 0.0;
     if (!stream_mode_ && !select_graph(why)) return false;
     if (latency > 0) cap = std::max(1, static_cast<int>(latency / std::max(body_ms_, 1e-3)));
@@ -2195,10 +2193,9 @@ bool Engine::run_once(std::string& why) {
 // the device until bqp_fetch copies it straight to the caller's array, off the engine thread (a
 // sliced one is brought into row order in a buffer that the next run writes before it reads it: the
 // first momentum buffer, or CG's r).
-int Engine::prepare_collection(const std::vector<Job*>& jobs) {
+int Engine::prepare_collection(const std::vector<Job*>& jobs, const LaunchSize& z) {
     collect_jobs_.clear();
     const size_t count = jobs.size();
-    const LaunchSize z = launch_size(jobs);
     const size_t o_spans = align_up(sizeof(CollectJob) * count), o_records = o_spans + align_up(sizeof(int2) * z.spans);
     const size_t o_x = o_records + align_up(sizeof(InstDev) * count);
     int2* const spans = reinterpret_cast<int2*>(h_collect_ + o_spans);
@@ -2304,11 +2301,12 @@ int Engine::profile_step(uint64_t id, int launches, double* ms_out, double* byte
     if (j.state != JOB_DONE || !j.resident || n_running_ != 0 || !queue_.empty() || launches < 1) return BQP_ERR_NOT_READY;
     cudaSetDevice(device_);
     std::string why;
-    if (!reserve_launch({&j}, why)) {
+    const LaunchSize z = launch_size({&j});
+    if (!reserve_launch(z, 1, why)) {
         set_error(why);
         return BQP_ERR_CUDA;
     }
-    upload_tables({&j});
+    upload_tables({&j}, z);
     update_grid();
     InstDev saved;
     cudaMemcpy(&saved, &d_inst_[j.slot], sizeof(InstDev), cudaMemcpyDeviceToHost);
@@ -2371,11 +2369,12 @@ int Engine::profile_cg(uint64_t id, int iterations, double* ms_matvec, double* m
         return BQP_ERR_NOT_READY;
     cudaSetDevice(device_);
     std::string why;
-    if (!reserve_launch({&j}, why)) {
+    const LaunchSize z = launch_size({&j});
+    if (!reserve_launch(z, 1, why)) {
         set_error(why);
         return BQP_ERR_CUDA;
     }
-    upload_tables({&j});
+    upload_tables({&j}, z);
     update_grid();
     InstDev saved;
     cudaMemcpy(&saved, &d_inst_[j.slot], sizeof(InstDev), cudaMemcpyDeviceToHost);

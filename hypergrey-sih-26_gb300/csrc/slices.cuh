@@ -12,8 +12,8 @@ __device__ __forceinline__ void wait_for_previous_launch() { asm volatile("gridd
 __device__ __forceinline__ void let_next_launch_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Loads of a matrix that a launch reads once: no line of L1 for them, which the gathers of the vector
-// then have to themselves (what bounds a random matrix is the L2's traffic, a 32-byte sector per
-// gathered number beside the stream): FP64 step of the random graph 1M 71.5 -> 70.9 us with it.
+// then have to themselves (what bounds a random matrix is its gathers, a request and a 32-byte sector
+// each: the L1s are 83 % busy with them): FP64 step of the random graph 1M 71.5 -> 70.9 us with it.
 __device__ __forceinline__ int load_once(const int32_t* p) {
     int v;
     asm("ld.global.nc.L1::no_allocate.s32 %0, [%1];" : "=r"(v) : "l"(p));
